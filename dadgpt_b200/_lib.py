@@ -6,6 +6,7 @@ import os
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libdadattn.so")
+NATIVE_PATH = os.path.join(PKG, "_native.so")
 SHIM_PATH = os.path.join(PKG, "libdadattn_gpuops.so")
 
 P, I, F, U64, I64, SZ = C.c_void_p, C.c_int, C.c_float, C.c_uint64, C.c_int64, C.c_size_t
@@ -50,6 +51,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 
 
 class DadAttnError(RuntimeError):
@@ -72,6 +74,22 @@ def load() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+def native():
+    """The CPython module (csrc/py_attention.cpp) that checks torch tensors and makes the C calls.
+    Raises, like :func:`load`, if the libraries have not been built."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m dadgpt_b200.build`")
+        import torch  # noqa: F401  (its shared libraries have to be loaded first)
+
+        from . import _native as module
+        module.set_error_class(DadAttnError)
+        _native = module
+    return _native
 
 
 def check(rc: int) -> None:

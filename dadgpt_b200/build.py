@@ -8,6 +8,7 @@ Outputs (next to this file, git-ignored, they travel with the working tree):
     libdadattn.so          kernels + C ABI (include/dadattn.h)
     libdadattn_gpuops.so   the three C++ symbols DadGPT's model.cpp links against
                            (gpu_flash_attention_*, reference cuda/gpu_ops.cuh:115-122)
+    _native.so             CPython module behind attention.py (checks + C call on torch tensors)
 """
 from __future__ import annotations
 
@@ -22,6 +23,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libdadattn.so")
 SHIM = os.path.join(PKG, "libdadattn_gpuops.so")
+NATIVE = os.path.join(PKG, "_native.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -71,7 +73,25 @@ def build(force: bool = False, ptxas: bool = False) -> str:
         cxx = shutil.which("g++") or "g++"
         subprocess.run([cxx, "-std=c++20", "-O2", "-fPIC", "-shared", "-I", os.path.join(ROOT, "include"),
                         shim_src, "-o", SHIM, "-L", PKG, "-ldadattn", "-Wl,-rpath,$ORIGIN"], check=True)
+    native_src = os.path.join(CSRC, "py_attention.cpp")
+    if force or _newer(NATIVE, [native_src, os.path.join(ROOT, "include", "dadattn.h")]):
+        _build_native(native_src)
     return LIB
+
+
+def _build_native(src: str) -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda_inc = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    inc = [x for p in [*include_paths(), cuda_inc, sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
+    subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared",
+                    f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+                    "-I", os.path.join(ROOT, "include"), *inc, src, "-o", NATIVE,
+                    "-L", PKG, "-ldadattn", "-L", lib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+                    "-Wl,-rpath,$ORIGIN"], check=True)
 
 
 if __name__ == "__main__":
