@@ -1,35 +1,36 @@
 // KV-cache decode attention: one new query token per sequence against that sequence's cache.
 //
 // The reference runs this as 61 tiny launches per layer (per-head M=1 cuBLAS products, 256-byte
-// device-to-device appends, one softmax; src/model.cpp:745-790). Here it is ONE split-K kernel
-// per layer call, for any number of concurrent sequences:
-//   * grid = (sequences x heads, splits); a CTA of 8 warps owns `chunk` consecutive cache rows
-//     of one (sequence, head): the whole sequence when there are enough pairs to fill the GPU,
-//     a slice otherwise. Splits are the slow grid dimension, so CTAs whose chunk lies
-//     beyond the sequence's length (they exit at once) are scheduled last, not in between;
-//   * a cache row (D elements) is read by D*sizeof(T)/16 adjacent lanes with one 128-bit load
-//     each, so a warp instruction covers 512 contiguous bytes of the cache; a lane issues the K
-//     and V loads of 4 row groups (128 bytes) before it consumes any, and 16-24 such warps per
-//     SM keep ~100 KB in flight: memory-level parallelism is what a bandwidth-bound kernel
-//     lives on;
-//   * q.k partial sums are reduced over those lanes with warp shuffles; each lane keeps an
-//     online-softmax state (max, sum, D/lanes accumulators) for the rows it has seen;
-//   * the append is fused: the lanes that own row `len` take k_new/v_new from the token's
-//     vectors, use them, and store them into the cache;
-//   * split-K merge without a second kernel and without waiting: a CTA writes (unnormalised
-//     out[D], max, sum) to the workspace, fences, and takes a ticket; whoever draws the last
-//     ticket of its (sequence, head) merges the records and writes `out`. A second ticket per
-//     sequence, taken by every CTA after it has read the length, lets the very last CTA of a
-//     sequence store length + 1. Tickets are returned to zero by their last holder, so a
-//     workspace zeroed once stays usable forever;
-//   * launched with programmatic stream serialization: the next decode call's CTAs are already
-//     resident (parked in griddepcontrol.wait) when this grid drains.
-// In direct mode (one split; the fp32 single-sequence path) the CTA normalises and writes the
-// output itself and no workspace is used.
+// device-to-device appends, one softmax; src/model.cpp:745-790). Here it is ONE kernel per layer
+// call, for any number of concurrent sequences. It is bound by HBM where the caches are large and by
+// latency where they are not:
+//   * a producer thread per CTA streams the cache rows of a (sequence, head) through a ring of 16 KB
+//     stages (8 KB of K, 8 KB of V) with bulk copies; four consumer warps read them from shared
+//     memory 512 contiguous bytes at a time. What is in flight does not depend on how the arithmetic
+//     is getting on: with loads and arithmetic taking turns in the same warps the kernel reached
+//     5.0 TB/s on 64 sequences x 12 heads of up to 1024 rows and 4.1 on 4 x 24 of up to 8000 at head
+//     size 128, now 5.8 and 5.4 (6.7 on 128 x 24 x 128);
+//   * q.k partial sums are reduced over a row's D*sizeof(T)/16 lanes with warp shuffles; each lane
+//     keeps an online-softmax state (max, sum, D/lanes accumulators) for the rows it has seen. The
+//     row groups of a tile are handled without branches so that their latencies overlap: a CTA's
+//     rate is the length of that chain (branching on each row: 12-24 % slower);
+//   * many (sequence, head) pairs: persistent CTAs, the longest sequences first, items handed out by
+//     a counter, the next item's rows already on their way while one is merged. Few pairs: the CTAs
+//     of a cluster share a pair and merge through distributed shared memory. Neither needs records in
+//     global memory, and a pair's merge costs no trip through L2 (8 sequences x 8 heads of up to 400
+//     rows: 6.9 us a layer with records and tickets, 4.0 now);
+//   * the append is fused: the warp that owns row `len` takes k_new/v_new from the token's vectors,
+//     uses them, and stores them into the cache;
+//   * every CTA draws a ticket once it has copied the lengths; the holder of the last one stores
+//     length + 1, while the rows are still streaming. Counters are returned to zero by their last
+//     user, so a workspace zeroed once stays usable forever;
+//   * launched with programmatic stream serialization: the next decode call's CTAs set themselves up
+//     (and, where the caller allows it, fill their rings) while this grid drains.
 #include <cfloat>
 #include <climits>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -41,66 +42,57 @@ namespace {
 constexpr int kDecodeWarps = 4;                         // consumer warps
 constexpr int kDecodeThreads = (kDecodeWarps + 1) * 32;  // and one producer warp
 constexpr int kTileBytes = 8192;                        // K (and V) bytes of one ring stage
-constexpr int kDecodeStages = 4;
-constexpr int kDecodeCtasPerSm = 3;
+// Ring stages, and CTAs an SM holds with that many: calls of few CTAs get the deeper rings.
+constexpr int kFewStages = 4, kFewPerSm = 3;
+constexpr int kManyStages = 3, kManyPerSm = 4;
+constexpr int kMaxStages = 4;
+constexpr int kItemRing = 2;        // items a CTA's producer may be ahead
 constexpr unsigned kTicketGroups = 32;  // first-level counters of the "all lengths read" tickets
-constexpr int kMinChunk = 128;      // smallest number of cache rows worth a CTA's start and a record
-constexpr int kMinRecordChunk = 256;  // what the workspace is sized for
-constexpr int kTargetCtas = 592;    // 4 per SM: below that the cache is split across CTAs
-constexpr int kMaxChunkSeqs = 592;  // split calls have fewer (sequence, head) pairs than kTargetCtas
+constexpr int kMaxRanked = 256;     // sequences whose lengths a CTA copies and can rank
 constexpr int kMaxCluster = 8;      // CTAs that share a head of one sequence (portable cluster size)
-constexpr int kRowsPerRank = 64;    // and the cache rows that are worth one of them
+constexpr long long kBytesPerRank = 262144;   // and the K + V bytes that are worth one of them
 
-// Rows per CTA. With enough (sequence, head) pairs to fill the GPU a CTA walks a whole
-// sequence (measured fastest: no records, no tickets); with few pairs the rows are split so
-// that about kTargetCtas CTAs exist. Depends only on (B, H, max_len), so the workspace size and
-// the kernel agree.
-inline int chunk_rows(int B, int H, int max_len) {
-  const long long pairs = static_cast<long long>(B) * H;
-  long long want_splits = (kTargetCtas + pairs - 1) / pairs;
-  if (want_splits < 1) want_splits = 1;
-  long long rows = (max_len + want_splits - 1) / want_splits;
-  if (rows < kMinRecordChunk) rows = kMinRecordChunk;
-  rows = (rows + 127) / 128 * 128;
-  return static_cast<int>(rows);
-}
-inline int split_count(int B, int H, int max_len) {
-  const int c = chunk_rows(B, H, max_len);
-  return (max_len + c - 1) / c;
-}
-
+// A 16-byte piece of a row as float pairs, and the softmax's exponential. Scores are kept in units
+// that exp_of() takes: natural units and expf for fp32 caches, log2 units and ex2 for bf16 ones
+// (whose 2^-9 rounding of the inputs is far above the difference).
 template <typename T>
 struct Elem;
 template <>
 struct Elem<float> {
   static constexpr int kPerLane = 4;
-  __device__ static void unpack(float (&f)[4], const uint4& raw) {
-    f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y);
-    f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
+  static constexpr float kUnit = 1.0f;
+  __device__ static void unpack(float2 (&f)[2], const uint4& raw) {
+    f[0] = make_float2(__uint_as_float(raw.x), __uint_as_float(raw.y));
+    f[1] = make_float2(__uint_as_float(raw.z), __uint_as_float(raw.w));
   }
+  __device__ static float exp_of(float x) { return expf(x); }
   __device__ static float from_float(float x) { return x; }
 };
 template <>
 struct Elem<__nv_bfloat16> {
   static constexpr int kPerLane = 8;
-  __device__ static void unpack(float (&f)[8], const uint4& raw) {
+  static constexpr float kUnit = 1.4426950408889634f;
+  __device__ static void unpack(float2 (&f)[4], const uint4& raw) {
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[2 * i] = __uint_as_float(w[i] << 16);
-      f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
+    for (int i = 0; i < 4; ++i) f[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
   }
+  __device__ static float exp_of(float x) { return ptx::ex2(x); }
   __device__ static __nv_bfloat16 from_float(float x) { return __float2bfloat16_rn(x); }
 };
 
-// Workspace: one ticket per (sequence, head), then the 1 + kTicketGroups counters of the "all
-// lengths read" tickets (uint32, zero between calls), padded to 256 bytes, then the records [B*H][splits][D + 2] fp32 (unnormalised output, max, sum).
-__host__ __device__ inline size_t partial_stride(int D) { return static_cast<size_t>(D) + 2; }
+// Workspace: B*H words, of which the first is the item counter, then the 1 + kTicketGroups counters
+// of the "all lengths read" tickets (uint32, all zero between calls), padded to 256 bytes. Behind
+// them callers hold what dadattn_decode_workspace_bytes has always asked for, the records of a
+// split-K merge in global memory; this kernel does not use that part.
 inline size_t record_bytes(int B, int H, int D, int max_len) {
-  const int splits = split_count(B, H, max_len);
-  if (splits == 1) return 0;  // every CTA finishes its (sequence, head) itself: no records
-  return static_cast<size_t>(B) * H * splits * partial_stride(D) * sizeof(float);
+  constexpr long long kTargetCtas = 592, kMinRows = 256;
+  const long long pairs = static_cast<long long>(B) * H;
+  const long long want = std::max(1LL, (kTargetCtas + pairs - 1) / pairs);
+  const long long rows = (std::max((max_len + want - 1) / want, kMinRows) + 127) / 128 * 128;
+  const long long splits = (max_len + rows - 1) / rows;
+  if (splits == 1) return 0;
+  return static_cast<size_t>(pairs) * splits * (D + 2) * sizeof(float);
 }
 inline size_t ticket_bytes(int B, int H) {
   return (sizeof(uint32_t) * (static_cast<size_t>(B) * H + 1 + kTicketGroups) + 255) / 256 * 256;
@@ -110,15 +102,11 @@ inline size_t workspace_bytes(int B, int H, int D, int max_len) {
 }
 
 // ---- the kernel --------------------------------------------------------------------------------
-// How a call's work is dealt out (launch_decode_batched, dadattn_decode_f32 choose):
-//   kWhole    CTA = one (sequence, head), all of its rows; hardware schedules the CTAs, the longest
-//             sequences first (rank by counting) when `reorder` is set
-//   kChunks   few (sequence, head) pairs: the rows of all of them are cut into chunks of one length
-//             that the kernel derives from the sequence lengths, CTA c takes chunks c, c + grid, ...
-//   kCluster  one sequence, no workspace: the CTAs of a thread-block cluster share a head's rows and
-//             merge through distributed shared memory
-enum DecodeMode { kWhole = 0, kChunks = 1, kCluster = 2 };
-
+// ranks == 1: persistent CTAs take whole (sequence, head) items, the items of longer sequences first
+// (`reorder`): CTA c item c, then whatever a global counter hands out. The producer is already loading
+// the next item's rows while the consumers finish the current one.
+// ranks > 1: the `ranks` CTAs of a thread-block cluster share the rows of one item and merge
+// through distributed shared memory: no records in global memory, no tickets, no second kernel.
 template <typename T, int D>
 struct DecodeTile {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
@@ -127,24 +115,20 @@ struct DecodeTile {
 };
 
 struct DecodeShared {
-  uint64_t full[kDecodeStages], empty[kDecodeStages];
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t item_ready[kItemRing], item_free[kItemRing];
+  int item[kItemRing];                   // items claimed for this CTA
   int abort_flag;
-  int b, len, last, advance, chunk;
   float m[kDecodeWarps], l[kDecodeWarps];
-  float acc[kDecodeWarps][128];
+  float acc[kDecodeWarps][128];          // [warp][d]
+  __align__(16) int lens[kMaxRanked];    // the sequence lengths (calls of up to kMaxRanked sequences)
   union {
     struct {
-      __align__(16) int lens[kMaxChunkSeqs];   // sequence lengths, resp. rows
-      int first[kMaxChunkSeqs + 1];            // ranks (kWhole), first chunk of a sequence (kChunks)
-    } seq;
-    float record[kMaxCluster][130];            // kCluster: every CTA's partial result, in CTA 0
-  } u;
-};
-
-// How the rows are cut: kChunks: aim at `target` chunks, never more than `capacity` records, never
-// longer than `longest` rows. kCluster: `target` CTAs per head.
-struct DecodeSplit {
-  int target, capacity, longest;
+      int place[kMaxRanked];             // reorder: rank of each sequence
+      int order[kMaxRanked];             // reorder: sequence of each rank
+    };
+    float record[kMaxCluster][130];      // ranks > 1: every CTA's partial result, in CTA 0
+  };
 };
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -168,13 +152,12 @@ __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(kDecodeWarps * 32) : "memory");
 }
 
-template <typename T, int D, int MODE>
-__global__ void __launch_bounds__(kDecodeThreads, kDecodeCtasPerSm)
-decode_kernel(T* __restrict__ out, float* __restrict__ partial, unsigned* __restrict__ tickets,
-              unsigned* __restrict__ seq_tickets, const T* __restrict__ q, const T* __restrict__ k_new,
-              const T* __restrict__ v_new, T* __restrict__ k_cache, T* __restrict__ v_cache,
-              int32_t* __restrict__ lengths, int fixed_len, int B, int H, int max_len, DecodeSplit split,
-              int reorder, int early, float scale, int* __restrict__ status) {
+template <typename T, int D>
+__global__ void __launch_bounds__(kDecodeThreads, kManyPerSm)
+decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned* __restrict__ seq_tickets, const T* __restrict__ q,
+              const T* __restrict__ k_new, const T* __restrict__ v_new, T* __restrict__ k_cache,
+              T* __restrict__ v_cache, int32_t* __restrict__ lengths, int fixed_len, int B, int H, int max_len,
+              int ranks, int stages, int reorder, int early, float scale, int* __restrict__ status) {
   using namespace ptx;
   using Tile = DecodeTile<T, D>;
   constexpr int EPL = Elem<T>::kPerLane;  // elements per lane (16 bytes)
@@ -185,20 +168,23 @@ decode_kernel(T* __restrict__ out, float* __restrict__ partial, unsigned* __rest
   static_assert(kGroups * kDecodeWarps * KPI == Tile::kRows && D <= kDecodeWarps * 32, "tile split");
 
   extern __shared__ __align__(128) uint8_t smem[];
-  DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem + kDecodeStages * 2 * kTileBytes);
+  DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem + stages * 2 * kTileBytes);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
   const int lane = threadIdx.x % 32;
-  const bool producer = warp == kDecodeWarps;
+  const int rank = static_cast<int>(blockIdx.x) % ranks;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kDecodeStages; ++i) {
+    for (int i = 0; i < stages; ++i) {
       mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], kDecodeWarps);
+    }
+    for (int i = 0; i < kItemRing; ++i) {
+      mbar_init(&sh.item_ready[i], 1);
+      mbar_init(&sh.item_free[i], kDecodeWarps);
     }
     sh.abort_flag = 0;
     fence_mbar_init();
   }
-  if (MODE == kCluster) cluster_arrive();   // (every CTA of the cluster has started: waited for below)
   // Everything this grid reads may have been written by the grid before it — unless the caller
   // has promised (dadattn_set_decode_early_start) that the grid before it does not write this
   // call's caches, lengths and workspace: then the lengths are read, and the ring is filled with
@@ -206,245 +192,260 @@ decode_kernel(T* __restrict__ out, float* __restrict__ partial, unsigned* __rest
   if (!early) pdl_wait();
   pdl_launch_dependents();
 
-  // ---- which rows this CTA works on ----
-  if (MODE == kWhole) {
-    const int slot_seq = static_cast<int>(blockIdx.x) / H;
-    if (reorder) {
-      // CTAs are handed to the SMs in blockIdx order, and a CTA lasts as long as its sequence is
-      // long: with the sequences taken longest first, the short ones fill the gaps at the end
-      // instead of a long one starting last. rank(s) = number of sequences that come before s
-      // (longer, or as long with a smaller index); with the count padded to a power of two n_pad
-      // (32..256; padding is INT_MIN and comes last), threads share out the n_pad^2 comparisons.
-      const int t = threadIdx.x;
-      for (int i = t; i < 256; i += kDecodeThreads) {
-        sh.u.seq.lens[i] = i < B ? lengths[i] : INT_MIN;
-        sh.u.seq.first[i] = 0;
-      }
-      __syncthreads();
-      if (t < 128) {
-        const int lg = 32 - __clz(B - 1);   // n_pad = 1 << lg, 5 <= lg <= 8
-        const int n_pad = 1 << lg;
-        const int groups = lg < 7 ? 128 >> lg : 1;
-        const int per = n_pad / groups, g = (t >> lg) & (groups - 1);
-        for (int si = t & (n_pad - 1); si < n_pad; si += 128) {
-          const int mine = sh.u.seq.lens[si];
-          int count = 0;
+  // Up to kMaxRanked lengths are copied to shared memory first; nobody reads the caller's array
+  // after that, so it can be advanced as soon as every CTA has its copy.
+  const bool snapshot = B <= kMaxRanked;
+  if (snapshot)
+    for (int i = threadIdx.x; i < kMaxRanked; i += kDecodeThreads) {
+      sh.lens[i] = i < B ? (lengths ? lengths[i] : fixed_len) : INT_MIN;
+      if (reorder) sh.place[i] = 0;
+    }
+  __syncthreads();
+  if (reorder) {
+    // rank(s) = number of sequences that come before s (longer, or as long with a smaller index);
+    // with the count padded to a power of two n_pad (32..256; padding is INT_MIN and comes last),
+    // 128 threads share out the n_pad^2 comparisons.
+    const int t = threadIdx.x;
+    if (t < 128) {
+      const int lg = 32 - __clz(B - 1);   // n_pad = 1 << lg, 5 <= lg <= 8
+      const int n_pad = 1 << lg;
+      const int groups = lg < 7 ? 128 >> lg : 1;
+      const int per = n_pad / groups, g = (t >> lg) & (groups - 1);
+      for (int si = t & (n_pad - 1); si < n_pad; si += 128) {
+        const int mine = sh.lens[si];
+        int count = 0;
 #pragma unroll 4
-          for (int j = g * per; j < (g + 1) * per; j += 4) {
-            const int4 o = *reinterpret_cast<const int4*>(sh.u.seq.lens + j);   // broadcast reads
-            count += static_cast<int>(o.x > mine) | (static_cast<int>(o.x == mine) & static_cast<int>(j + 0 < si));
-            count += static_cast<int>(o.y > mine) | (static_cast<int>(o.y == mine) & static_cast<int>(j + 1 < si));
-            count += static_cast<int>(o.z > mine) | (static_cast<int>(o.z == mine) & static_cast<int>(j + 2 < si));
-            count += static_cast<int>(o.w > mine) | (static_cast<int>(o.w == mine) & static_cast<int>(j + 3 < si));
-          }
-          if (count) atomicAdd(&sh.u.seq.first[si], count);
+        for (int j = g * per; j < (g + 1) * per; j += 4) {
+          const int4 o = *reinterpret_cast<const int4*>(sh.lens + j);   // broadcast reads
+          count += static_cast<int>(o.x > mine) | (static_cast<int>(o.x == mine) & static_cast<int>(j + 0 < si));
+          count += static_cast<int>(o.y > mine) | (static_cast<int>(o.y == mine) & static_cast<int>(j + 1 < si));
+          count += static_cast<int>(o.z > mine) | (static_cast<int>(o.z == mine) & static_cast<int>(j + 2 < si));
+          count += static_cast<int>(o.w > mine) | (static_cast<int>(o.w == mine) & static_cast<int>(j + 3 < si));
         }
+        if (count) atomicAdd(&sh.place[si], count);
       }
-      __syncthreads();
-      for (int i = t; i < B; i += kDecodeThreads)
-        if (sh.u.seq.first[i] == slot_seq) {
-          sh.b = i;
-          sh.len = sh.u.seq.lens[i];
-        }
-    } else if (threadIdx.x == 0) {
-      sh.b = slot_seq;
-      sh.len = lengths[slot_seq];
     }
-  } else if (MODE == kChunks) {
-    // rows of every sequence (0 where its length is invalid), the chunk length that spreads their
-    // sum over split.target chunks, and each sequence's first chunk
-    if (threadIdx.x == 0) sh.len = 0;
     __syncthreads();
-    int rows = 0;
-    for (int i = threadIdx.x; i < B; i += kDecodeThreads) {
-      const int l = lengths[i];
-      const bool valid = l >= 0 && l < max_len;
-      sh.u.seq.lens[i] = valid ? l + 1 : 0;
-      rows += valid ? l + 1 : 0;
-      if (!valid && blockIdx.x == 0) atomicExch(status, DADATTN_E_ARG);
-    }
-    if (rows) atomicAdd(&sh.len, rows);
+    for (int i = t; i < B; i += kDecodeThreads) sh.order[sh.place[i]] = i;
     __syncthreads();
-    if (warp == 0) {
-      const long long all = static_cast<long long>(sh.len) * H;
-      const int spare = split.capacity - B * H;   // chunks beyond one per (sequence, head)
-      int chunk = split.longest;
-      if (spare > 0) {
-        const long long even = (all + split.target - 1) / split.target, fit = (all + spare - 1) / spare;
-        const long long want = max(max(even, fit), static_cast<long long>(kMinChunk));
-        chunk = static_cast<int>(min(want, static_cast<long long>(chunk)));
-        chunk = (chunk + Tile::kRows - 1) / Tile::kRows * Tile::kRows;
-      }
-      int at = 0;
-      for (int i = 0; i < B; i += 32) {
-        const int own = i + lane < B ? (sh.u.seq.lens[i + lane] + chunk - 1) / chunk : 0;
-        int sum = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int up = __shfl_up_sync(0xffffffffu, sum, o);
-          if (lane >= o) sum += up;
-        }
-        if (i + lane < B) sh.u.seq.first[i + lane] = at + sum - own;
-        at += __shfl_sync(0xffffffffu, sum, 31);
-      }
-      if (lane == 0) {
-        sh.u.seq.first[B] = at;
-        sh.chunk = chunk;
-      }
-    }
   }
-  __syncthreads();  // the CTA's ticket below is taken strictly after the reads of the lengths
+
+  // Item e of the call. A sequence whose length is outside [0, max_len) is skipped (rows = 0) and
+  // reported.
+  struct Item {
+    int b, h, len, row0, row1;
+  };
+  const int n_items = B * H, n_lanes = static_cast<int>(gridDim.x) / ranks;   // items taken up by CTAs at the start
+  auto item = [&](int e) -> Item {
+    Item s;
+    const int p = e / H;
+    s.h = e - p * H;
+    s.b = reorder ? sh.order[p] : p;
+    s.len = snapshot ? sh.lens[s.b] : lengths[s.b];
+    const int rows = s.len >= 0 && s.len < max_len ? s.len + 1 : 0;
+    const int share = (rows + ranks - 1) / ranks;
+    s.row0 = min(rank * share, rows);
+    s.row1 = min(s.row0 + share, rows);
+    return s;
+  };
+
+  const Item first = item(static_cast<int>(blockIdx.x) / ranks);
+  // "this CTA has started and looked its item up" (record shares memory with the ranking): waited
+  // for before the first remote store
+  if (ranks > 1) cluster_arrive();
+
   // Every CTA of the call draws a ticket once it has read the lengths; whoever holds the last one
   // knows that nobody will read them again and advances them. Two levels keep the atomics off one
-  // address: the CTAs are dealt into kTicketGroups groups, a CTA draws its group's ticket here, at
-  // the start, and looks at it only at the very end (the round trip through L2 costs it nothing);
-  // the last of each group then draws from a second counter, and the last of those advances.
-  unsigned my_ticket = 0;
-  if (MODE != kCluster && threadIdx.x == 0)
-    my_ticket = atomicAdd(&seq_tickets[1 + blockIdx.x % kTicketGroups], 1u);
-
-  // Segment i of this CTA: rows [row0, row1) of (b, h); false when there is none. All roles walk
-  // the same list.
-  struct Segment {
-    int b, h, len, row0, row1, parts, record;   // parts: segments the (b, h) is cut into
-  };
-  auto segment = [&](int i, Segment& s) -> bool {
-    if (MODE == kChunks) {
-      const int per_head = sh.u.seq.first[B];
-      const long long c = static_cast<long long>(blockIdx.x) + static_cast<long long>(i) * gridDim.x;
-      if (c >= static_cast<long long>(per_head) * H) return false;
-      s.record = static_cast<int>(c);
-      s.h = s.record / per_head;
-      const int r = s.record - s.h * per_head;
-      int lo = 0, hi = B;                       // the last sequence whose first chunk is <= r
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) / 2;
-        if (sh.u.seq.first[mid] <= r) lo = mid; else hi = mid;
-      }
-      s.b = lo;
-      const int rows = sh.u.seq.lens[lo], j = r - sh.u.seq.first[lo];
-      s.len = rows - 1;
-      s.parts = sh.u.seq.first[lo + 1] - sh.u.seq.first[lo];
-      s.record -= j;                            // records of the pair start here
-      s.row0 = j * sh.chunk;
-      s.row1 = min(s.row0 + sh.chunk, rows);
-      return true;
-    }
-    if (i > 0) return false;
-    s.record = 0;
-    if (MODE == kCluster) {
-      const int ranks = split.target, rank = static_cast<int>(blockIdx.x) % ranks;
-      const int rows = fixed_len + 1, chunk = (rows + ranks - 1) / ranks;
-      s.b = 0, s.h = static_cast<int>(blockIdx.x) / ranks, s.len = fixed_len, s.parts = ranks;
-      s.row0 = min(rank * chunk, rows), s.row1 = min(s.row0 + chunk, rows);
-      return true;
-    }
-    s.b = sh.b, s.h = static_cast<int>(blockIdx.x) % H, s.len = sh.len, s.parts = 1;
-    s.row0 = 0, s.row1 = sh.len + 1;
-    if (sh.len >= 0 && sh.len < max_len) return true;
-    if (threadIdx.x == 0 && s.h == 0) atomicExch(status, DADATTN_E_ARG);
-    return false;
+  // address: the CTAs are dealt into kTicketGroups groups; the last of each group draws from a
+  // second counter, and the last of those advances.
+  const unsigned group = blockIdx.x % kTicketGroups;
+  auto draw_ticket = [&]() { return atomicAdd(&seq_tickets[1 + group], 1u); };
+  auto is_last = [&](unsigned ticket) -> bool {
+    const unsigned all_ctas = gridDim.x;
+    if (ticket != (all_ctas - group + kTicketGroups - 1) / kTicketGroups - 1) return false;
+    seq_tickets[1 + group] = 0;   // ready for the next call
+    const unsigned groups = all_ctas < kTicketGroups ? all_ctas : kTicketGroups;
+    if (atomicAdd(&seq_tickets[0], 1u) != groups - 1) return false;
+    seq_tickets[0] = 0;
+    return true;
   };
 
   volatile int* abort_flag = &sh.abort_flag;
-  float part_acc = 0.f, part_m = -FLT_MAX, part_l = 0.f;   // kCluster: this CTA's share, one d per thread
-  if (producer) {
+  if (warp == kDecodeWarps) {
+    // ------------------------------ producer ------------------------------
     if (elect_one()) {
-      int it = 0;
-      Segment s;
+      // The ticket is drawn now and looked at once the ring is full: its round trip and the advance
+      // of the lengths stay off the path to the kernel's end.
+      bool ticket_due = lengths != nullptr && snapshot;
+      const unsigned ticket = ticket_due ? draw_ticket() : 0;
+      auto settle_ticket = [&]() {
+        if (ticket_due && is_last(ticket))
+          for (int j = 0; j < B; ++j) {
+            const int len = sh.lens[j];
+            if (len >= 0 && len < max_len) lengths[j] = len + 1;   // a full or invalid sequence is left alone
+          }
+        ticket_due = false;
+      };
+      int st = 0, lap = 0;
+      Item s = first;
       bool ok = true;
-      for (int i = 0; ok && segment(i, s); ++i) {
+      for (int n = 0; ok; ++n) {
         const size_t base = (static_cast<size_t>(s.b) * H + s.h) * max_len * D;
         const int end = min(s.row1, s.len);   // the row being appended comes from k_new / v_new
-        for (int r = s.row0; r < end; r += Tile::kRows, ++it) {
-          const int st = it % kDecodeStages;
-          if (it >= kDecodeStages && !(ok = mbar_wait(&sh.empty[st], (it / kDecodeStages - 1) & 1, abort_flag))) break;
+        for (int r = s.row0; r < end; r += Tile::kRows) {
+          if (lap == 1 && st == 0) settle_ticket();
+          if (lap > 0 && !(ok = mbar_wait(&sh.empty[st], (lap - 1) & 1, abort_flag))) break;
           const uint32_t bytes = static_cast<uint32_t>(min(Tile::kRows, end - r)) * Tile::kRowBytes;
           mbar_arrive_expect_tx(&sh.full[st], 2 * bytes);
           bulk_load(smem + st * 2 * kTileBytes, k_cache + base + static_cast<size_t>(r) * D, bytes, &sh.full[st]);
           bulk_load(smem + (st * 2 + 1) * kTileBytes, v_cache + base + static_cast<size_t>(r) * D, bytes, &sh.full[st]);
+          if (++st == stages) st = 0, ++lap;
         }
+        // The item after this one is claimed only when this one's last rows are on their way: what is
+        // in the ring covers the counter's round trip, and a CTA with a long item takes no second one
+        // that an idle CTA could have had (64 sequences x 12 heads: 210 us, 240 when claimed an item ahead).
+        int next = n_items;
+        if (ok && n_lanes < n_items) {
+          const unsigned claim = atomicAdd(item_counter, 1u);
+          next = min(static_cast<int>(claim) + n_lanes, n_items);
+          if (claim == static_cast<unsigned>(n_items - 1)) *item_counter = 0;   // the last claim: ready for the next call
+        }
+        const int slot = n % kItemRing;
+        ok = ok && (n < kItemRing || mbar_wait(&sh.item_free[slot], (n / kItemRing - 1) & 1, abort_flag));
+        if (!ok) break;
+        *reinterpret_cast<volatile int*>(&sh.item[slot]) = next;
+        mbar_arrive(&sh.item_ready[slot]);
+        if (next >= n_items) break;
+        s = item(next);
       }
+      settle_ticket();
     }
   } else {
+    // ------------------------------ consumers ------------------------------
     if (early) pdl_wait();
     const int slot = lane / LPK, part = lane % LPK;
-    int it = 0;
+    const float scale_unit = scale * Elem<T>::kUnit;
+    int st = 0;
+    uint32_t phase = 0;
     bool ok = true;
-    Segment s;
-    for (int i = 0; segment(i, s); ++i) {
+    Item s = first, nxt = first;
+    bool have = true;
+    // token vectors of an item: fetched an item ahead (k_new / v_new by the warp that appends)
+    uint4 q_raw = make_uint4(0, 0, 0, 0), kn_raw = q_raw, vn_raw = q_raw;
+    auto fetch_token = [&](const Item& t) {
+      const size_t off = (static_cast<size_t>(t.b) * H + t.h) * D + part * EPL;
+      q_raw = *reinterpret_cast<const uint4*>(q + off);
+      if (warp == 0 && slot == 0) {
+        kn_raw = *reinterpret_cast<const uint4*>(k_new + off);
+        vn_raw = *reinterpret_cast<const uint4*>(v_new + off);
+      }
+    };
+    fetch_token(s);
+    for (int n = 0; have; ++n, s = nxt) {
       const size_t bh = static_cast<size_t>(s.b) * H + s.h;
-      const size_t vec_off = bh * D + part * EPL;
-      float m = -FLT_MAX, l = 0.f, acc[EPL], qf[EPL];
-      Elem<T>::unpack(qf, *reinterpret_cast<const uint4*>(q + vec_off));
+      float m = -FLT_MAX, l = 0.f;
+      float2 acc[EPL / 2], qf[EPL / 2];
+      Elem<T>::unpack(qf, q_raw);
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
+      for (int e = 0; e < EPL / 2; ++e) acc[e] = make_float2(0.f, 0.f);
 
-      // NR row groups' worth of K / V registers into the lane's online-softmax state
-      auto absorb = [&](const uint4* kr, const uint4* vr, const bool* valid, auto count) {
+      // NR row groups' worth of K / V registers into the lane's online-softmax state. No branches:
+      // the groups' chains (shuffles, exponentials, sums) have to overlap, a CTA's rate is their
+      // latency. Rows that do not count (`valid`, read only when !ALL) come in as zeros.
+      auto absorb = [&](const uint4* kr, const uint4* vr, const bool* valid, auto count, auto all) {
         constexpr int NR = decltype(count)::value;
-        float sc[NR];
+        constexpr bool ALL = decltype(all)::value;
+        float sc[NR], p[NR];
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+          float2 kf[EPL / 2];
+          Elem<T>::unpack(kf, kr[u]);
+          float2 dot = fmul2(qf[0], kf[0]);
+#pragma unroll
+          for (int e = 1; e < EPL / 2; ++e) dot = ffma2(qf[e], kf[e], dot);
+          sc[u] = dot.x + dot.y;
+        }
+#pragma unroll
+        for (int o = LPK / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int u = 0; u < NR; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
         float m_new = m;
 #pragma unroll
         for (int u = 0; u < NR; ++u) {
-          float kf[EPL];
-          Elem<T>::unpack(kf, kr[u]);
-          float dot = 0.f;
-#pragma unroll
-          for (int e = 0; e < EPL; ++e) dot = fmaf(qf[e], kf[e], dot);
-#pragma unroll
-          for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-          sc[u] = valid[u] ? dot * scale : -FLT_MAX;
+          sc[u] = ALL || valid[u] ? sc[u] * scale_unit : -FLT_MAX;
           m_new = fmaxf(m_new, sc[u]);
         }
-        if (m_new > -FLT_MAX) {  // at least one row seen by this lane group so far
-          const float corr = expf(m - m_new);
-          l *= corr;
+        // (while m_new is still -FLT_MAX the state is all zeros: corr = 1 leaves it so)
+        const float corr = Elem<T>::exp_of(m - m_new);
+        float sum = 0.f;
 #pragma unroll
-          for (int e = 0; e < EPL; ++e) acc[e] *= corr;
-#pragma unroll
-          for (int u = 0; u < NR; ++u) {
-            if (!valid[u]) continue;
-            const float p = expf(sc[u] - m_new);
-            l += p;
-            float vf[EPL];
-            Elem<T>::unpack(vf, vr[u]);
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) acc[e] = fmaf(p, vf[e], acc[e]);
-          }
-          m = m_new;
+        for (int u = 0; u < NR; ++u) {
+          p[u] = Elem<T>::exp_of(sc[u] - m_new);
+          if (!ALL && !valid[u]) p[u] = 0.f;
+          sum += p[u];
         }
+        l = fmaf(l, corr, sum);
+#pragma unroll
+        for (int e = 0; e < EPL / 2; ++e) acc[e] = fmul2(acc[e], make_float2(corr, corr));
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+          float2 vf[EPL / 2];
+          Elem<T>::unpack(vf, vr[u]);
+#pragma unroll
+          for (int e = 0; e < EPL / 2; ++e) acc[e] = ffma2(make_float2(p[u], p[u]), vf[e], acc[e]);
+        }
+        m = m_new;
       };
 
-      if (warp == 0 && s.row0 <= s.len && s.row1 == s.len + 1) {   // the token being appended: use its vectors and store them
-        uint4 kr = make_uint4(0, 0, 0, 0), vr = kr;
+      // the token being appended: its vectors are used and stored by the CTA whose share ends there
+      if (warp == 0 && s.row0 < s.row1 && s.row1 == s.len + 1) {
         const bool mine = slot == 0;
         if (mine) {
-          kr = *reinterpret_cast<const uint4*>(k_new + vec_off);
-          vr = *reinterpret_cast<const uint4*>(v_new + vec_off);
           const size_t at = (bh * max_len + s.len) * D + part * EPL;
-          *reinterpret_cast<uint4*>(k_cache + at) = kr;
-          *reinterpret_cast<uint4*>(v_cache + at) = vr;
+          *reinterpret_cast<uint4*>(k_cache + at) = kn_raw;
+          *reinterpret_cast<uint4*>(v_cache + at) = vn_raw;
         }
-        absorb(&kr, &vr, &mine, std::integral_constant<int, 1>{});
+        absorb(&kn_raw, &vn_raw, &mine, std::integral_constant<int, 1>{}, std::false_type{});
       }
       const int end = min(s.row1, s.len);
-      for (int r = s.row0; r < end; r += Tile::kRows, ++it) {
-        const int st = it % kDecodeStages;
-        if (!ok || !(ok = mbar_wait(&sh.full[st], (it / kDecodeStages) & 1, abort_flag))) break;
+      for (int r = s.row0; r < end; r += Tile::kRows) {
+        if (!ok || !(ok = mbar_wait(&sh.full[st], phase, abort_flag))) break;
         const uint4* kt = reinterpret_cast<const uint4*>(smem + st * 2 * kTileBytes) + warp * kGroups * 32 + lane;
         const uint4* vt = kt + kTileBytes / 16;
         uint4 kr[kGroups], vr[kGroups];
-        bool valid[kGroups];
 #pragma unroll
-        for (int u = 0; u < kGroups; ++u) {
-          kr[u] = kt[u * 32];
-          vr[u] = vt[u * 32];
-          valid[u] = r + (warp * kGroups + u) * KPI + slot < end;
+        for (int u = 0; u < kGroups; ++u) kr[u] = kt[u * 32];
+#pragma unroll
+        for (int u = 0; u < kGroups; ++u) vr[u] = vt[u * 32];
+        if (r + Tile::kRows <= end) {
+          absorb(kr, vr, nullptr, std::integral_constant<int, kGroups>{}, std::true_type{});
+        } else {   // an item's last tile: what lies beyond the rows loaded is left over from earlier tiles
+          bool valid[kGroups];
+#pragma unroll
+          for (int u = 0; u < kGroups; ++u) {
+            valid[u] = r + (warp * kGroups + u) * KPI + slot < end;
+            if (!valid[u]) kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+          }
+          absorb(kr, vr, valid, std::integral_constant<int, kGroups>{}, std::false_type{});
         }
-        absorb(kr, vr, valid, std::integral_constant<int, kGroups>{});
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.empty[st]);
+        if (++st == stages) st = 0, phase ^= 1;
+      }
+
+      // the next item; its token vectors arrive while this one is merged
+      have = false;
+      if (ranks == 1) {
+        const int slot_i = n % kItemRing;
+        if (ok && (ok = mbar_wait(&sh.item_ready[slot_i], (n / kItemRing) & 1, abort_flag))) {
+          const int e = *reinterpret_cast<volatile int*>(&sh.item[slot_i]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.item_free[slot_i]);
+          if ((have = e < n_items)) {
+            nxt = item(e);
+            fetch_token(nxt);
+          }
+        }
       }
 
       // Merge the KPI row slots of the warp (lanes with equal `part`), then the warps.
@@ -453,19 +454,22 @@ decode_kernel(T* __restrict__ out, float* __restrict__ partial, unsigned* __rest
         const float m_o = __shfl_xor_sync(0xffffffffu, m, o);
         const float l_o = __shfl_xor_sync(0xffffffffu, l, o);
         const float m_new = fmaxf(m, m_o);
-        const float ca = m > -FLT_MAX ? expf(m - m_new) : 0.f;
-        const float cb = m_o > -FLT_MAX ? expf(m_o - m_new) : 0.f;
+        const float ca = m > -FLT_MAX ? Elem<T>::exp_of(m - m_new) : 0.f;
+        const float cb = m_o > -FLT_MAX ? Elem<T>::exp_of(m_o - m_new) : 0.f;
         l = l * ca + l_o * cb;
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) {
-          const float a_o = __shfl_xor_sync(0xffffffffu, acc[e], o);
-          acc[e] = acc[e] * ca + a_o * cb;
+        for (int e = 0; e < EPL / 2; ++e) {
+          acc[e].x = acc[e].x * ca + __shfl_xor_sync(0xffffffffu, acc[e].x, o) * cb;
+          acc[e].y = acc[e].y * ca + __shfl_xor_sync(0xffffffffu, acc[e].y, o) * cb;
         }
         m = m_new;
       }
       if (slot == 0) {
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) sh.acc[warp][part * EPL + e] = acc[e];
+        for (int e = 0; e < EPL / 2; ++e) {
+          sh.acc[warp][part * EPL + 2 * e] = acc[e].x;
+          sh.acc[warp][part * EPL + 2 * e + 1] = acc[e].y;
+        }
         if (part == 0) {
           sh.m[warp] = m;
           sh.l[warp] = l;
@@ -480,163 +484,107 @@ decode_kernel(T* __restrict__ out, float* __restrict__ partial, unsigned* __rest
         float ll = 0.f, aa = 0.f;
 #pragma unroll
         for (int w = 0; w < kDecodeWarps; ++w) {
-          const float c = sh.m[w] > -FLT_MAX ? expf(sh.m[w] - mm) : 0.f;
+          const float c = sh.m[w] > -FLT_MAX ? Elem<T>::exp_of(sh.m[w] - mm) : 0.f;
           ll += sh.l[w] * c;
           aa += sh.acc[w][d] * c;
         }
-        if (s.parts == 1) {  // the only part of this (sequence, head): finish here
-          out[bh * D + d] = Elem<T>::from_float(aa / ll);
-        } else if (MODE == kCluster) {
-          part_acc = aa, part_m = mm, part_l = ll;   // handed to CTA 0 below
+        if (ranks == 1) {
+          if (s.row1 > 0) out[bh * D + d] = Elem<T>::from_float(aa / ll);
         } else {
-          float* rec = partial + (static_cast<size_t>(s.record) + s.row0 / sh.chunk) * partial_stride(D);
-          rec[d] = aa;
+          // hand the share to CTA 0, which is known to run once the cluster's first barrier is through
+          cluster_wait();
+          const uint32_t rec = cluster_rank0_address(&sh.record[rank][0]);
+          st_cluster(rec + d * 4, aa);
           if (d == 0) {
-            rec[D] = mm;
-            rec[D + 1] = ll;
+            st_cluster(rec + D * 4, mm);
+            st_cluster(rec + D * 4 + 4, ll);
           }
         }
       }
-      if (MODE == kChunks && s.parts > 1) {
-        // Publish the record, then draw a ticket; the holder of the last one merges.
-        __threadfence();
-        consumers_sync();
-        if (threadIdx.x == 0) sh.last = atomicAdd(&tickets[bh], 1u) == static_cast<unsigned>(s.parts - 1);
-        consumers_sync();
-        if (sh.last) {
-          __threadfence();
-          if (d < D) {
-            const float* rec = partial + static_cast<size_t>(s.record) * partial_stride(D);
-            float mm = -FLT_MAX;
-            for (int j = 0; j < s.parts; ++j) mm = fmaxf(mm, __ldcg(rec + j * partial_stride(D) + D));
-            float ll = 0.f, aa = 0.f;
-            for (int j = 0; j < s.parts; ++j) {
-              const float* rj = rec + j * partial_stride(D);
-              const float c = expf(__ldcg(rj + D) - mm);
-              ll += __ldcg(rj + D + 1) * c;
-              aa += __ldcg(rj + d) * c;
-            }
-            out[bh * D + d] = Elem<T>::from_float(aa / ll);
-          }
-          if (threadIdx.x == 0) tickets[bh] = 0;  // ready for the next call
-        }
+      if (ranks == 1) {
+        if (s.row1 == 0 && s.h == 0 && threadIdx.x == 0) atomicExch(status, DADATTN_E_ARG);
+        consumers_sync();   // sh.acc / sh.m are read: the next item may write them
       }
-      if (MODE == kChunks) consumers_sync();   // sh.acc / sh.m are read: the next segment may write them
     }
   }
 
-  if (MODE == kCluster && split.target > 1) {
-    // The CTAs of the cluster hand their shares to CTA 0 through distributed shared memory. All
-    // threads take part in both barriers; the first (arrived at on entry) says that CTA 0 runs.
-    const int ranks = split.target, rank = static_cast<int>(blockIdx.x) % ranks, d = threadIdx.x;
-    cluster_wait();
-    if (d < D) {
-      const uint32_t rec = cluster_rank0_address(&sh.u.record[rank][0]);
-      st_cluster(rec + d * 4, part_acc);
-      if (d == 0) {
-        st_cluster(rec + D * 4, part_m);
-        st_cluster(rec + D * 4 + 4, part_l);
-      }
-    }
+  if (ranks > 1) {
+    // Threads without a share to hand over join the first barrier here; after the second, CTA 0 merges.
+    const int d = threadIdx.x;
+    if (d >= D) cluster_wait();
     cluster_arrive();
     cluster_wait();
-    if (rank == 0 && d < D) {
-      float mm = -FLT_MAX;
-      for (int j = 0; j < ranks; ++j) mm = fmaxf(mm, sh.u.record[j][D]);
-      float ll = 0.f, aa = 0.f;
-      for (int j = 0; j < ranks; ++j) {
-        const float c = expf(sh.u.record[j][D] - mm);   // a share without rows has m = -FLT_MAX: 0
-        ll += sh.u.record[j][D + 1] * c;
-        aa += sh.u.record[j][d] * c;
+    if (rank == 0) {
+      const Item& s = first;
+      if (s.len >= 0 && s.len < max_len) {
+        if (d < D) {
+          float mm = -FLT_MAX;
+          for (int j = 0; j < ranks; ++j) mm = fmaxf(mm, sh.record[j][D]);
+          float ll = 0.f, aa = 0.f;
+          for (int j = 0; j < ranks; ++j) {
+            const float c = Elem<T>::exp_of(sh.record[j][D] - mm);   // a share without rows has m = -FLT_MAX: 0
+            ll += sh.record[j][D + 1] * c;
+            aa += sh.record[j][d] * c;
+          }
+          out[(static_cast<size_t>(s.b) * H + s.h) * D + d] = Elem<T>::from_float(aa / ll);
+        }
+      } else if (s.h == 0 && d == 0) {
+        atomicExch(status, DADATTN_E_ARG);
       }
-      out[static_cast<size_t>(blockIdx.x / ranks) * D + d] = Elem<T>::from_float(aa / ll);
     }
-  } else if (MODE == kCluster) {
-    cluster_wait();
   }
 
-  if (MODE != kCluster) {
+  if (lengths != nullptr && !snapshot) {   // the lengths were read all along: tickets only now
+    __shared__ int sh_advance;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      const unsigned all_ctas = gridDim.x, group = blockIdx.x % kTicketGroups;
-      const unsigned group_size = (all_ctas - group + kTicketGroups - 1) / kTicketGroups;
-      int last = 0;
-      if (my_ticket == group_size - 1) {
-        seq_tickets[1 + group] = 0;   // ready for the next call
-        const unsigned groups = all_ctas < kTicketGroups ? all_ctas : kTicketGroups;
-        last = atomicAdd(&seq_tickets[0], 1u) == groups - 1;
-        if (last) seq_tickets[0] = 0;
-      }
-      sh.advance = last;
-    }
+    if (threadIdx.x == 0) sh_advance = is_last(draw_ticket());
     __syncthreads();
-    if (sh.advance) {
+    if (sh_advance)
       for (int i = threadIdx.x; i < B; i += kDecodeThreads) {
-        const int l = lengths[i];
-        if (l >= 0 && l < max_len) lengths[i] = l + 1;   // a full or invalid sequence is left alone
+        const int len = lengths[i];
+        if (len >= 0 && len < max_len) lengths[i] = len + 1;
       }
-    }
   }
   if (threadIdx.x == 0 && sh.abort_flag) report_timeout(status, sh.abort_flag);
 }
 
-constexpr size_t kDecodeSmem = kDecodeStages * 2 * kTileBytes + sizeof(DecodeShared);
-static_assert((kDecodeSmem + 1024) * kDecodeCtasPerSm <= 228 * 1024, "shared memory of an SM exceeded");
+constexpr size_t decode_smem(int stages) { return static_cast<size_t>(stages) * 2 * kTileBytes + sizeof(DecodeShared); }
+static_assert((decode_smem(kFewStages) + 1024) * kFewPerSm <= 228 * 1024 && kFewStages <= kMaxStages &&
+              (decode_smem(kManyStages) + 1024) * kManyPerSm <= 228 * 1024 && kManyStages <= kMaxStages,
+              "shared memory of an SM exceeded");
 
-// The kernel's opt-in to its dynamic shared memory (a cheap host call: 0.06 us measured).
-template <typename Kernel>
-int allow_decode_smem(Kernel kern) {
-  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDecodeSmem)));
-  return DADATTN_OK;
-}
-
-template <typename T, typename Raw, int DH>
-int launch_decode_batched(Raw* out, const Raw* q, const Raw* k_new, const Raw* v_new, Raw* k_cache,
-                          Raw* v_cache, int32_t* lengths, int B, int H, int max_len, float scale,
-                          unsigned* tickets, float* partial, int* status, int early, cudaStream_t st) {
-  const int splits = split_count(B, H, max_len);
-  unsigned* seq_tickets = tickets + static_cast<size_t>(B) * H;
+template <typename T, int DH>
+int launch_decode(T* out, const T* q, const T* k_new, const T* v_new, T* k_cache, T* v_cache, int32_t* lengths,
+                  int fixed_len, int B, int H, int max_len, float scale, unsigned* tickets, int* status, int early,
+                  cudaStream_t st) {
+  // the workspace's tickets: one per (sequence, head), the first of which counts the items; then those
+  // of the lengths
+  unsigned* item_counter = tickets;
+  unsigned* seq_tickets = tickets ? tickets + static_cast<size_t>(B) * H : nullptr;
+  auto kern = decode_kernel<T, DH>;
+  // (a cheap host call, 0.06 us)
+  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(decode_smem(kMaxStages))));
   int dev = 0, sms = 0;
   DAD_CUDA(cudaGetDevice(&dev));
   DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int pairs = B * H, resident = kDecodeCtasPerSm * sms;
-  DecodeSplit split = {0, 0, 0};
-  int grid = pairs, reorder = 0;
-  auto kern = decode_kernel<T, DH, kWhole>;
-  if (splits > 1) {
-    kern = decode_kernel<T, DH, kChunks>;
-    split.capacity = pairs * splits;
-    split.longest = chunk_rows(B, H, max_len);
-    // Every (sequence, head) ends in a chunk that is half empty on average. With few pairs the
-    // chunks are to fill the GPU once, remainders included; with many, about half of it.
-    split.target = max(resident - pairs, resident / 2);
-    grid = min(split.capacity, resident);
-  } else {
-    // Longest-first order pays once the CTAs no longer all fit on the GPU at the same time; the
-    // in-kernel ranking handles 32..256 sequences.
-    reorder = B >= 32 && B <= 256 && pairs > resident;
-  }
-  if (int rc = allow_decode_smem(kern)) return rc;
-  DAD_CUDA(launch_pdl(kern, dim3(grid), dim3(kDecodeThreads), kDecodeSmem, st, reinterpret_cast<T*>(out), partial,
-                      tickets, seq_tickets, reinterpret_cast<const T*>(q), reinterpret_cast<const T*>(k_new),
-                      reinterpret_cast<const T*>(v_new), reinterpret_cast<T*>(k_cache),
-                      reinterpret_cast<T*>(v_cache), lengths, 0, B, H, max_len, split, reorder, early, scale,
-                      status));
-  return DADATTN_OK;
-}
-
-// One fp32 sequence without a workspace: a cluster of CTAs per head.
-template <int DH>
-int launch_decode_one(float* out, const float* q, const float* k_new, const float* v_new, float* k_cache,
-                      float* v_cache, int H, int max_len, int pos, float scale, int* status, cudaStream_t st) {
-  auto kern = decode_kernel<float, DH, kCluster>;
-  if (int rc = allow_decode_smem(kern)) return rc;
+  const long long pairs = static_cast<long long>(B) * H;
+  // CTAs per (sequence, head): as many as the longest sequence there can be has 256 KB of K and V
+  // for, while all of the call's CTAs still fit on the GPU at once. Beyond that, waiting clusters
+  // cost more than the finer cut gives (4 sequences x 24 heads of up to 8000 rows: 131 us with 4 CTAs
+  // each, 145 with 8).
+  const long long bytes = static_cast<long long>(lengths ? max_len : fixed_len + 1) * 2 * DH * sizeof(T);
+  const int resident = kManyPerSm * sms;
   int ranks = 1;
-  while (ranks < kMaxCluster && ranks * kRowsPerRank < pos + 1 && H * ranks < kTargetCtas) ranks *= 2;
+  while (ranks < kMaxCluster && ranks * kBytesPerRank < bytes && pairs * ranks * 2 <= resident) ranks *= 2;
+  // (without a workspace there is no counter to deal items from: one CTA each)
+  const long long grid = ranks > 1 || !item_counter ? pairs * ranks : min(pairs, static_cast<long long>(resident));
+  const int stages = grid <= static_cast<long long>(kFewPerSm) * sms ? kFewStages : kManyStages;
+  // Longest first pays once a CTA takes more than one item; the in-kernel ranking handles 32..256 sequences.
+  const int reorder = B >= 32 && B <= kMaxRanked && pairs > grid;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(H) * ranks);
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kDecodeThreads);
-  cfg.dynamicSmemBytes = kDecodeSmem;
+  cfg.dynamicSmemBytes = decode_smem(stages);
   cfg.stream = st;
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -644,22 +592,29 @@ int launch_decode_one(float* out, const float* q, const float* k_new, const floa
   attrs[1].id = cudaLaunchAttributeClusterDimension;
   attrs[1].val.clusterDim = {static_cast<unsigned>(ranks), 1, 1};
   cfg.attrs = attrs;
-  cfg.numAttrs = 2;
-  const DecodeSplit split = {ranks, 0, 0};
-  DAD_CUDA(cudaLaunchKernelEx(&cfg, kern, out, static_cast<float*>(nullptr), static_cast<unsigned*>(nullptr),
-                              static_cast<unsigned*>(nullptr), q, k_new, v_new, k_cache, v_cache,
-                              static_cast<int32_t*>(nullptr), pos, 1, H, max_len, split, 0, 0, scale, status));
+  cfg.numAttrs = ranks > 1 ? 2 : 1;
+  DAD_CUDA(cudaLaunchKernelEx(&cfg, kern, out, item_counter, seq_tickets, q, k_new, v_new, k_cache, v_cache, lengths, fixed_len, B,
+                              H, max_len, ranks, stages, reorder, early, scale, status));
   return DADATTN_OK;
 }
 
-template <int DH>
-int launch_decode_bf16(uint16_t* out, const uint16_t* q, const uint16_t* k_new,
-                       const uint16_t* v_new, uint16_t* k_cache, uint16_t* v_cache,
-                       int32_t* lengths, int B, int H, int max_len, float scale,
-                       unsigned* tickets, float* partial, int* status, int early, cudaStream_t st) {
-  return launch_decode_batched<__nv_bfloat16, uint16_t, DH>(out, q, k_new, v_new, k_cache, v_cache, lengths, B,
-                                                            H, max_len, scale, tickets, partial, status,
-                                                            early, st);
+int launch_decode_bf16(uint16_t* out, const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,
+                       uint16_t* k_cache, uint16_t* v_cache, int32_t* lengths, int B, int H, int D, int max_len,
+                       float scale, unsigned* tickets, int* status, int early, cudaStream_t st) {
+  using BF = __nv_bfloat16;
+  auto* launch = D == 64 ? launch_decode<BF, 64> : launch_decode<BF, 128>;
+  return launch(reinterpret_cast<BF*>(out), reinterpret_cast<const BF*>(q), reinterpret_cast<const BF*>(k_new),
+                reinterpret_cast<const BF*>(v_new), reinterpret_cast<BF*>(k_cache), reinterpret_cast<BF*>(v_cache),
+                lengths, 0, B, H, max_len, scale, tickets, status, early, st);
+}
+
+int launch_decode_f32(float* out, const float* q, const float* k_new, const float* v_new, float* k_cache,
+                      float* v_cache, int32_t* lengths, int fixed_len, int B, int H, int D, int max_len, float scale,
+                      unsigned* tickets, int* status, cudaStream_t st) {
+  auto* launch = D == 16 ? launch_decode<float, 16> : D == 32 ? launch_decode<float, 32>
+                 : D == 64 ? launch_decode<float, 64> : launch_decode<float, 128>;
+  return launch(out, q, k_new, v_new, k_cache, v_cache, lengths, fixed_len, B, H, max_len, scale,
+                tickets, status, 0, st);
 }
 
 // Rows 0..n-1 of sequence b's cache from the K / V heads a prefill leaves behind: k_heads,
@@ -729,11 +684,8 @@ extern "C" int dadattn_decode_bf16(uint16_t* out, const uint16_t* q, const uint1
   if (!status) return DADATTN_E_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   unsigned* tickets = static_cast<unsigned*>(workspace);
-  float* partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + ticket_bytes(B, H));
-  return D == 64 ? launch_decode_bf16<64>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H,
-                                          max_len, scale, tickets, partial, status, g_decode_early, st)
-                 : launch_decode_bf16<128>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H,
-                                           max_len, scale, tickets, partial, status, g_decode_early, st);
+  return launch_decode_bf16(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, D, max_len, scale, tickets, status,
+                            g_decode_early, st);
 }
 
 extern "C" int dadattn_set_decode_early_start(int on) {
@@ -758,12 +710,8 @@ extern "C" int dadattn_decode_f32(float* out, const float* q, const float* k_new
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (D) {
-    case 16: return launch_decode_one<16>(out, q, k_new, v_new, k_cache, v_cache, H, max_len, pos, scale, status, st);
-    case 32: return launch_decode_one<32>(out, q, k_new, v_new, k_cache, v_cache, H, max_len, pos, scale, status, st);
-    case 64: return launch_decode_one<64>(out, q, k_new, v_new, k_cache, v_cache, H, max_len, pos, scale, status, st);
-    default: return launch_decode_one<128>(out, q, k_new, v_new, k_cache, v_cache, H, max_len, pos, scale, status, st);
-  }
+  return launch_decode_f32(out, q, k_new, v_new, k_cache, v_cache, nullptr, pos, 1, H, D, max_len, scale, nullptr,
+                           status, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -780,7 +728,7 @@ extern "C" int dadattn_decode_f32(float* out, const float* q, const float* k_new
 //
 // The array is part of the library image: every GPU that loads libdadattn.so holds these
 // 8 MiB until the process exits, whether or not this entry point is ever called. Its first
-// 64 KiB are the tickets, at a fixed place whatever the shape of a call: they are zero when the
+// 64 KiB are the counters, at a fixed place whatever the shape of a call: they are zero when the
 // module is loaded and every call returns them to zero, which is the only state a call needs
 // from its predecessors. The records behind them are written before they are read.
 // A sequence that is already at max_len is skipped and noted in g_decode_noalloc_status, which
@@ -842,13 +790,9 @@ extern "C" int dadattn_decode_bf16_noalloc(uint16_t* out, const uint16_t* q,
   int* status = nullptr;
   if (int rc = noalloc_setup(&scratch, &status)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  unsigned* tickets = reinterpret_cast<unsigned*>(scratch);
-  float* partial = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + kNoAllocTicketBytes);
   // never with early start: every call shares the one scratch array with the call before it
-  return D == 64 ? launch_decode_bf16<64>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H,
-                                          max_len, scale, tickets, partial, status, 0, st)
-                 : launch_decode_bf16<128>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H,
-                                           max_len, scale, tickets, partial, status, 0, st);
+  return launch_decode_bf16(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, D, max_len, scale,
+                            reinterpret_cast<unsigned*>(scratch), status, 0, st);
 }
 
 extern "C" int dadattn_decode_noalloc_status(dadattn_stream_t stream) {
@@ -893,13 +837,8 @@ extern "C" int dadattn_decode_f32_batched(float* out, const float* q, const floa
   if (!status) return DADATTN_E_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   unsigned* tickets = static_cast<unsigned*>(workspace);
-  float* partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + ticket_bytes(B, H));
-  switch (D) {
-    case 16: return launch_decode_batched<float, float, 16>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, max_len, scale, tickets, partial, status, 0, st);
-    case 32: return launch_decode_batched<float, float, 32>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, max_len, scale, tickets, partial, status, 0, st);
-    case 64: return launch_decode_batched<float, float, 64>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, max_len, scale, tickets, partial, status, 0, st);
-    default: return launch_decode_batched<float, float, 128>(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, max_len, scale, tickets, partial, status, 0, st);
-  }
+  return launch_decode_f32(out, q, k_new, v_new, k_cache, v_cache, lengths, 0, B, H, D, max_len, scale, tickets,
+                           status, st);
 }
 
 extern "C" int dadattn_kv_cache_fill(void* k_cache, void* v_cache, int32_t* lengths, const float* k_heads,

@@ -239,8 +239,8 @@ int dadattn_decode_f32(float* out, const float* q, const float* k_new, const flo
  * Caches: [B,H,max_len,D] bf16. lengths[B] (int32, device) holds each sequence's current length
  * L_b; the call writes k_new,v_new [B,H,D] at row L_b, attends over rows 0..L_b, and stores
  * L_b + 1 back. Sequences with L_b >= max_len are left untouched and reported through
- * DADATTN_E_ARG at the next dadattn_device_status(). workspace: split-K tickets and records, at
- * least dadattn_decode_workspace_bytes() bytes, 16-byte aligned. It must be zero-filled
+ * DADATTN_E_ARG at the next dadattn_device_status(). workspace: counters and room for split-K
+ * records, at least dadattn_decode_workspace_bytes() bytes, 16-byte aligned. It must be zero-filled
  * (cudaMemset) before its first use and again whenever B, H or max_len change; between calls of
  * one shape the library leaves it in a reusable state. Two calls that share a workspace must not
  * overlap on the GPU. */
