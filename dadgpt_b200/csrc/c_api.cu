@@ -45,6 +45,20 @@ int* device_status_word() {
   return g_status[dev];
 }
 
+int check_launch_registers(const void* kernel, int expected, std::atomic<int>& seen) {
+  int regs = seen.load(std::memory_order_relaxed);
+  if (regs == 0) {
+    cudaFuncAttributes attr;
+    DAD_CUDA(cudaFuncGetAttributes(&attr, kernel));
+    regs = attr.numRegs;   // the same value for every device
+    seen.store(regs, std::memory_order_relaxed);
+  }
+  if (regs != expected)
+    return fail(DADATTN_E_UNSUPPORTED, "a kernel was compiled with %d registers per thread, its register budgets "
+                "assume %d", regs, expected);
+  return DADATTN_OK;
+}
+
 }  // namespace dadattn
 
 using namespace dadattn;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -34,6 +35,11 @@ int fail(int code, const char* fmt, ...);
 // Device-side sticky status word (one per device that loads the library). Kernels record a
 // DADATTN_E_* code here instead of trapping; dadattn_device_status() reads and clears it.
 int* device_status_word();  // device pointer for the current device, nullptr on failure
+
+// Kernels whose warpgroups move registers between them (setmaxnreg) budget with the count the CTA is
+// launched with; were the compiler to give the kernel fewer, an increase would wait for registers
+// that nobody can give back. Refuses such a launch. `seen` belongs to the kernel.
+int check_launch_registers(const void* kernel, int expected, std::atomic<int>& seen);
 
 // ---- Philox4x32-10 with cuRAND's curand_init(seed, subsequence, offset) counter set-up -------
 // The reference draws one uniform per attention probability with subsequence = flat element
@@ -123,6 +129,14 @@ int launch_fwd_bf16_d64(uint16_t* out, float* lse, const uint16_t* q, const uint
                         const uint16_t* v, int BH, int S, float scale, float rate, uint64_t seed,
                         uint64_t offset, int64_t unit0, const uint32_t* mask_bits, int heads,
                         cudaStream_t st);
+
+// fp32 tensors on the tensor cores, exact operands (flash_f32_tc_*.cu): head sizes 16, 32, 64.
+int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
+                      float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
+                      cudaStream_t st);
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* dout, const float* out, const float* lse,
+                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+                      uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st);
 
 // Launch with programmatic stream serialization: the grid may become resident while its
 // predecessor in the stream drains, runs its set-up (barriers, TMEM, descriptor prefetch), and

@@ -1,0 +1,144 @@
+// Exact fp32 operands on the bf16 tensor cores, shared by the forward and backward of
+// flash_f32_tc_*.cu.
+//
+// An fp32 number is the sum of three bf16 numbers, x = x0 + x1 + x2 with x0 = bf16(x), x1 =
+// bf16(x - x0), x2 = x - x0 - x1: each takes 8 of the 24 significand bits, both subtractions are
+// exact and so is the last conversion. A product of two fp32 matrices is then the sum of the nine
+// products of their planes. The three smallest (x1 y2, x2 y1, x2 y2) are at most 2^-26 of |x||y|,
+// a quarter of what one rounding of an fp32 multiply-add may lose, and are left out; the other six
+// are accumulated in fp32, smallest first, at most 64 products deep, and the accumulator is then
+// added to a register sum in fp32 with round-to-nearest. Nothing is rounded to bf16: the result is
+// that of an fp32 dot product with another order of summation (measured against float64: no larger
+// error than the FFMA kernels of flash_f32.cu).
+#pragma once
+
+#include "common.cuh"
+#include "sm100_ptx.cuh"
+
+namespace dadattn {
+namespace f32tc {
+
+using namespace ptx;
+
+constexpr int kRows = 128;          // rows of the resident tile: one per TMEM lane
+constexpr int kStep = 64;           // rows of the streamed tile per step
+constexpr int kPlaneA = kRows * 128;   // one bf16 plane, 128-byte rows (64 elements), swizzled
+constexpr int kPlaneB = kStep * 128;
+constexpr int kComputeThreads = 256;   // two per row
+constexpr int kLoaderThreads = 7 * 32;
+constexpr int kThreads = 512;          // 8 compute warps, 7 loader warps, 1 issuer warp
+constexpr int kWarpLoader0 = 8, kWarpIssuer = 15;
+// Registers per thread once the warpgroups have rebalanced; the pool is what the CTA starts with.
+constexpr int kRegsLaunch = 128, kRegsCompute = 160, kRegsHelper = 96;
+static_assert(256 * kRegsCompute + 256 * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
+
+// Plane pairs of the six products, smallest first.
+__device__ __forceinline__ constexpr int product_a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
+__device__ __forceinline__ constexpr int product_b(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i == 3 ? 0 : i == 4 ? 1 : 0; }
+
+// Four fp32 values -> three planes of four packed bf16.
+struct Split4 {
+  uint2 p[3];
+};
+__device__ __forceinline__ Split4 split4(float4 x) {
+  Split4 s;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    s.p[i] = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
+    x.x -= __uint_as_float(s.p[i].x << 16);
+    x.y -= __uint_as_float(s.p[i].x & 0xffff0000u);
+    x.z -= __uint_as_float(s.p[i].y << 16);
+    x.w -= __uint_as_float(s.p[i].y & 0xffff0000u);
+  }
+  return s;
+}
+// Columns 4 c4 .. 4 c4 + 3 of a row into the three planes of a tile (128-byte swizzle).
+__device__ __forceinline__ void store_split(uint8_t* tile, int plane_bytes, int row, int c4, const Split4& s) {
+  uint8_t* at = tile + row * 128 + ((((c4 >> 1) ^ (row & 7)) << 4) | ((c4 & 1) << 3));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * plane_bytes) = s.p[i];
+}
+
+// Columns 4 c4 .. of row r of a [S, D] matrix; zeros beyond the sequence. Any 4-byte alignment.
+template <int D>
+__device__ __forceinline__ float4 load4(const float* __restrict__ m, int r, int c4, int S, bool vec_ok) {
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (r < S) {
+    const float* p = m + static_cast<size_t>(r) * D + c4 * 4;
+    if (vec_ok)
+      x = __ldg(reinterpret_cast<const float4*>(p));
+    else
+      x = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  }
+  return x;
+}
+__device__ __forceinline__ float dot4(const float4& a, const float4& b) {
+  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+      "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+// 32 values of a row -> three planes of packed pairs in tensor memory, 16 columns each.
+__device__ __forceinline__ void tmem_store_split(float (&x)[32], uint32_t t0, uint32_t t1, uint32_t t2) {
+  const uint32_t t[3] = {t0, t1, t2};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    uint32_t pk[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      pk[j] = pack_bf16(x[2 * j], x[2 * j + 1]);
+      if (i < 2) {
+        x[2 * j] -= __uint_as_float(pk[j] << 16);
+        x[2 * j + 1] -= __uint_as_float(pk[j] & 0xffff0000u);
+      }
+    }
+    tmem_st16(t[i], pk);
+  }
+}
+// sum[c] += the accumulator's columns taddr + c, c < N (N = 32, 16 or 8)
+template <int N>
+__device__ __forceinline__ void tmem_add(uint32_t taddr, float (&sum)[N]) {
+  if constexpr (N == 32) {
+    uint32_t a[32];
+    tmem_ld32(taddr, a);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < N; ++c) sum[c] += __uint_as_float(a[c]);
+  } else {
+    uint32_t a[16];
+    tmem_ld16(taddr, a);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < N; ++c) sum[c] += __uint_as_float(a[c]);
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_row(float* dst, const float (&x)[N], bool vec_ok) {
+  if (vec_ok) {
+#pragma unroll
+    for (int c = 0; c < N; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < N; ++c) dst[c] = x[c];
+  }
+}
+
+}  // namespace f32tc
+}  // namespace dadattn

@@ -475,6 +475,8 @@ int launch_fwd(float* out, float* lse, const float* q, const float* k, const flo
                int S, float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0,
                cudaStream_t st) {
   const bool vec_ok = aligned(out, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
+  if constexpr (D <= 64)
+    return launch_fwd_f32_tc(out, lse, q, k, v, BH, S, D, scale, DROP ? rate : 0.f, seed, offset, unit0, vec_ok, st);
   auto kern = flash_fwd_f32_kernel<D, DROP>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(fwd_smem_bytes<D>())));
@@ -493,6 +495,9 @@ int launch_bwd(float* dq, float* dk, float* dv, float* delta, const float* dout,
   const bool vec_ok = aligned(dq, 16) && aligned(dk, 16) && aligned(dv, 16) &&
                       aligned(dout, 16) && aligned(out, 16) && aligned(q, 16) &&
                       aligned(k, 16) && aligned(v, 16);
+  if constexpr (D <= 64)
+    return launch_bwd_f32_tc(dq, dk, dv, dout, out, lse, q, k, v, BH, S, D, scale, DROP ? rate : 0.f, seed, offset,
+                             unit0, vec_ok, st);
   const int64_t rows = static_cast<int64_t>(BH) * S;
   const int64_t delta_threads = rows * (D / 4);
   flash_delta_f32_kernel<D><<<static_cast<unsigned>((delta_threads + 255) / 256), 256, 0, st>>>(

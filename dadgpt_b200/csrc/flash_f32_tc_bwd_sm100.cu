@@ -1,0 +1,390 @@
+// fp32 backward on the tensor cores (head sizes 16, 32, 64): dQ, dK and dV in one launch, exact fp32
+// operands as three bf16 planes (f32_split.cuh), no atomics, bit-reproducible.
+//
+// As in the reference (cuda/attention.cu:88-205) the probabilities are formed twice, once where
+// keys are resident and queries stream past (dK, dV) and once the other way round (dQ). Both are
+// the same machine, so both kinds of work item share one grid:
+//     kind    resident A1, A2   streamed B1, B2   X1 = A1 B1^T   X2 = A2 B2^T   sums
+//     dK/dV   K, V              Q, dO             S^T            dP^T           dV += P^T B2, dK += dS^T B1
+//     dQ      Q, dO             K, V              S              dP             dQ += dS B1
+// A CTA owns 128 resident rows (one per TMEM lane) and takes the other side 64 rows at a time:
+//   warps 0-7   two threads per row, 32 columns each: p = exp(s scale - lse), ds = p (dP - delta)
+//               scale, both split into planes and written back to tensor memory, from where the
+//               sums take them as A operands; the sums of each step are added to fp32 registers
+//   warps 8-14  fetch the next step's fp32 rows, split them in registers, and put them into the
+//               shared-memory stage the moment it is released; delta = rowsum(dO o O) on the way
+//   warp 15     issues the products. Order on the tensor pipe: sums of step i, X2 then X1 of step
+//               i + 2 (B2's stage is released before B1's, so its refill hides behind the sums'
+//               last products), sums of step i + 1, ...
+// A step costs 2304 (X) + 2304 (dK/dV) or 1152 (dQ) clocks of tensor pipe at head size 64 (48 for a
+// 128 x 64 x 16 product) and about 1900 issue slots per scheduler of everything else.
+// Tensor memory: X1 / X2 double buffered (buffer b at 128 b), 64 columns at 256 for the planes that
+// do not fit over the scores they came from, sums at 320 and 384.
+#include "f32_split.cuh"
+
+namespace dadattn {
+namespace {
+
+using namespace f32tc;
+
+struct BwdSmem {
+  static constexpr int kA1 = 0, kA2 = 3 * kPlaneA;
+  static constexpr int kStage = 6 * kPlaneA;                   // [2 stages][B1, B2][3 planes]
+  static constexpr int kStageBytes = 6 * kPlaneB;
+  static constexpr int kVec = kStage + 2 * kStageBytes;        // [2 stages][lse, delta][64], or [lse, delta][128]
+  static constexpr int kBars = kVec + 1024;
+  static constexpr int kBytes = kBars + 256;
+  static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
+};
+struct BwdBars {
+  uint64_t a_full, p_full, acc_done;
+  uint64_t b1_full[2], b2_full[2], b1_empty[2], b2_empty[2], x_full[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+static_assert(sizeof(BwdBars) <= 256, "barrier block");
+
+struct BwdArgs {
+  float *dq, *dk, *dv;
+  const float *dout, *out, *lse, *q, *k, *v;
+  int BH, S;
+  float scale, rate;
+  PhiloxKey rng;
+  int64_t unit0;
+  bool vec_ok;
+  int* status;
+};
+
+template <int D, bool DROP>
+__global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const BwdArgs args) {
+  using L = BwdSmem;
+  constexpr uint32_t kExtra = 256, kSum1 = 320, kSum2 = 384;   // kSum1: dV; kSum2: dK or dQ
+  constexpr int V4 = D / 4;                                    // float4 pieces of a row
+  constexpr int NC = D / 2;                                    // columns of a sum per thread
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  BwdBars* bars = reinterpret_cast<BwdBars*>(smem + L::kBars);
+  volatile int* abort_flag = &bars->abort_flag;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+  const int lane = threadIdx.x % 32;
+  const int S = args.S;
+
+  if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
+    if (threadIdx.x == 0) atomicExch(args.status, DADATTN_E_CUDA);
+    return;
+  }
+  // Items in order of their number of steps, the longest first: level i holds the key tiles i and
+  // the query tiles n - 1 - i of every (batch, head).
+  const int n_tiles = (S + kRows - 1) / kRows;
+  const int level = static_cast<int>(blockIdx.x) / (2 * args.BH);
+  const int in_level = static_cast<int>(blockIdx.x) - level * 2 * args.BH;
+  const bool is_q = in_level >= args.BH;
+  const int bh = is_q ? in_level - args.BH : in_level;
+  const int row0 = (is_q ? n_tiles - 1 - level : level) * kRows;     // first resident row
+  const int first = is_q ? 0 : row0;                                 // first streamed row
+  const int last = is_q ? min(row0 + kRows, S) : S;
+  const int n_it = (last - first + kStep - 1) / kStep;
+  const size_t base = static_cast<size_t>(bh) * S * D;
+  const float* lse = args.lse + static_cast<size_t>(bh) * S;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bars->a_full, kComputeThreads);
+    mbar_init(&bars->p_full, kComputeThreads);
+    mbar_init(&bars->acc_done, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bars->b1_full[s], kLoaderThreads);
+      mbar_init(&bars->b2_full[s], kLoaderThreads);
+      mbar_init(&bars->b1_empty[s], 1);
+      mbar_init(&bars->b2_empty[s], 1);
+      mbar_init(&bars->x_full[s], 1);
+    }
+    bars->abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == kWarpIssuer) {
+    tmem_alloc(&bars->tmem_base, 512);
+    tmem_relinquish();
+  }
+  // Columns D..63 of the streamed tiles are read by the sums' products (64 columns wide): zeros.
+  if (D < 64)
+    for (int i = threadIdx.x; i < 2 * L::kStageBytes / 16; i += kThreads)
+      reinterpret_cast<uint4*>(smem + L::kStage)[i] = make_uint4(0, 0, 0, 0);
+  if (D < 64) fence_proxy_async_smem();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = bars->tmem_base;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  if (warp >= kWarpLoader0) {
+    setmaxnreg_dec<kRegsHelper>();
+    if (warp < kWarpIssuer) {
+      // ------------------------------ loaders ------------------------------
+      const int t = threadIdx.x - kWarpLoader0 * 32;
+      constexpr int kPieces = kStep * V4;                                   // float4 pieces of a streamed tile
+      constexpr int kMine = (kPieces + kLoaderThreads - 1) / kLoaderThreads;
+      const float* b1 = (is_q ? args.k : args.q) + base;
+      const float* b2 = (is_q ? args.v : args.dout) + base;
+      const float* oo = args.out + base;
+      float* vec = reinterpret_cast<float*>(smem + L::kVec);
+      bool ok = true;
+      for (int i = 0; ok && i < n_it; ++i) {
+        const int s = i & 1, r0 = first + i * kStep;
+        float4 x1[kMine], x2[kMine], xo[kMine];
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          const int e = t + j * kLoaderThreads;
+          const bool in = e < kPieces;
+          const int r = r0 + e / V4, c4 = e % V4;
+          x2[j] = in ? load4<D>(b2, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (!is_q) xo[j] = in ? load4<D>(oo, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+          x1[j] = in ? load4<D>(b1, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float row_lse = 0.f;
+        if (!is_q && t < kStep && r0 + t < S) row_lse = __ldg(lse + r0 + t);
+        Split4 s2[kMine];
+        float delta[kMine];
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          if (!is_q) {
+            delta[j] = dot4(x2[j], xo[j]);
+#pragma unroll
+            for (int o = V4 / 2; o > 0; o >>= 1) delta[j] += __shfl_xor_sync(0xffffffffu, delta[j], o);
+          }
+          s2[j] = split4(x2[j]);
+        }
+        if (i >= 2 && !(ok = mbar_wait(&bars->b2_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
+        uint8_t* tile = smem + L::kStage + s * L::kStageBytes;
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          const int e = t + j * kLoaderThreads;
+          if (e < kPieces) {
+            store_split(tile + 3 * kPlaneB, kPlaneB, e / V4, e % V4, s2[j]);
+            if (!is_q && e % V4 == 0) vec[s * 128 + 64 + e / V4] = delta[j];
+          }
+        }
+        if (!is_q && t < kStep) vec[s * 128 + t] = row_lse;
+        fence_proxy_async_smem();
+        mbar_arrive(&bars->b2_full[s]);
+        Split4 s1[kMine];
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) s1[j] = split4(x1[j]);
+        if (i >= 2 && !(ok = mbar_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          const int e = t + j * kLoaderThreads;
+          if (e < kPieces) store_split(tile, kPlaneB, e / V4, e % V4, s1[j]);
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(&bars->b1_full[s]);
+      }
+    } else if (elect_one()) {
+      // ------------------------------ MMA issuer ------------------------------
+      constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // A, B K-major
+      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // A from tensor memory, B MN-major
+      const SmemDescBase a1 = make_desc_base_sw128(smem_u32(smem + L::kA1), 0);
+      const SmemDescBase a2 = make_desc_base_sw128(smem_u32(smem + L::kA2), 0);
+      const SmemDescBase b0 = make_desc_base_sw128(smem_u32(smem + L::kStage), 0);
+      auto issue_x = [&](int i) -> bool {
+        const int s = i & 1;
+        const uint32_t par = (i >> 1) & 1, tx = tmem + s * 128;
+        const SmemDescBase b1{b0.lo + s * (L::kStageBytes >> 4), b0.hi};
+        const SmemDescBase b2{b1.lo + (3 * kPlaneB >> 4), b0.hi};
+        auto product = [&](uint32_t td, const SmemDescBase& a, const SmemDescBase& b) {
+#pragma unroll
+          for (int m = 0; m < 6; ++m)
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+              mma_ss(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
+                     idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
+        };
+        if (!mbar_wait(&bars->b2_full[s], par, abort_flag)) return false;
+        tc_fence_after_sync();
+        product(tx + 64, a2, b2);
+        if (!mbar_wait(&bars->b1_full[s], par, abort_flag)) return false;
+        tc_fence_after_sync();
+        product(tx, a1, b1);
+        mma_commit(&bars->x_full[s]);
+        return true;
+      };
+      auto issue_sums = [&](int i) -> bool {
+        const int s = i & 1;
+        const uint32_t tx = tmem + s * 128;
+        const SmemDescBase b1{b0.lo + s * (L::kStageBytes >> 4), b0.hi};
+        const SmemDescBase b2{b1.lo + (3 * kPlaneB >> 4), b0.hi};
+        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        tc_fence_after_sync();
+        // planes of 16 streamed rows kk: half kk / 2 of a row's columns, 8 columns of pairs each
+        if (!is_q) {
+#pragma unroll
+          for (int m = 0; m < 6; ++m)
+#pragma unroll
+            for (int kk = 0; kk < kStep / 16; ++kk) {
+              const uint32_t at = (product_a(m) == 0 ? 0u : product_a(m) == 1 ? 16u : 64u) + (kk >> 1) * 32 + (kk & 1) * 8;
+              mma_ts(tmem + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                     (m > 0 || kk > 0) ? 1u : 0u);
+            }
+        }
+        mma_commit(&bars->b2_empty[s]);
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int kk = 0; kk < kStep / 16; ++kk) {
+            const uint32_t in = (kk >> 1) * 32 + (kk & 1) * 8;
+            const uint32_t at = product_a(m) == 0 ? tx + 64 + 16 + in : tmem + kExtra + (product_a(m) == 1 ? 0u : 16u) + in;
+            mma_ts(tmem + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                   (m > 0 || kk > 0) ? 1u : 0u);
+          }
+        mma_commit(&bars->b1_empty[s]);
+        mma_commit(&bars->acc_done);
+        return true;
+      };
+      bool ok = mbar_wait(&bars->a_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
+      for (int i = 0; ok && i < n_it; ++i) ok = issue_sums(i) && (i + 2 >= n_it || issue_x(i + 2));
+    }
+  } else {
+    setmaxnreg_inc<kRegsCompute>();
+    // ------------------------------ compute ------------------------------
+    const int half = warp / 4, quad = warp % 4;
+    const int row = quad * 32 + lane;           // resident row = TMEM lane
+    const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    float* vec = reinterpret_cast<float*>(smem + L::kVec);
+    bool ok = true;
+    {
+      // the resident tiles, split into planes
+      const float* a1 = (is_q ? args.q : args.k) + base;
+      const float* a2 = (is_q ? args.dout : args.v) + base;
+      const float* oo = args.out + base;
+      constexpr int kMine = kRows * V4 / kComputeThreads;
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) {
+        const int e = threadIdx.x + j * kComputeThreads, r = e / V4, c4 = e % V4;
+        const float4 x1 = load4<D>(a1, row0 + r, c4, S, args.vec_ok);
+        const float4 x2 = load4<D>(a2, row0 + r, c4, S, args.vec_ok);
+        store_split(smem + L::kA1, kPlaneA, r, c4, split4(x1));
+        store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2));
+        if (is_q) {
+          float delta = dot4(x2, load4<D>(oo, row0 + r, c4, S, args.vec_ok));
+#pragma unroll
+          for (int o = V4 / 2; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
+          if (c4 == 0) vec[128 + r] = delta;
+        }
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&bars->a_full);
+      if (is_q) asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory");   // delta of all rows
+    }
+    const int r_own = row0 + row;
+    const bool in_seq = r_own < S;
+    const float own_lse = is_q && in_seq ? __ldg(lse + r_own) : 0.f;
+    const float own_delta = is_q ? vec[128 + row] : 0.f;
+    const float scale = args.scale;
+    const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
+    const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
+
+    float sum1[NC], sum2[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sum1[c] = sum2[c] = 0.f;
+    auto take_sums = [&](int i) -> bool {
+      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      tc_fence_after_sync();
+      if (!is_q) tmem_add<NC>(tlane + kSum1 + half * NC, sum1);
+      tmem_add<NC>(tlane + kSum2 + half * NC, sum2);
+      return true;
+    };
+
+    for (int i = 0; i < n_it; ++i) {
+      const int s = i & 1;
+      const int col0 = first + i * kStep + half * 32;      // streamed row of this thread's first column
+      if (!(ok = mbar_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
+      // (the row scalars came with B2)
+      if (!is_q && !(ok = mbar_wait(&bars->b2_full[s], (i >> 1) & 1, abort_flag))) break;
+      tc_fence_after_sync();
+      const uint32_t tx = tlane + s * 128 + half * 32;
+      float p[32], g[32];
+      {
+        uint32_t x1[32], x2[32];
+        tmem_ld32(tx, x1);
+        tmem_ld32(tx + 64, x2);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) p[c] = __uint_as_float(x1[c]), g[c] = __uint_as_float(x2[c]);
+      }
+      // every pair of the tile visible? (key <= query < S)
+      const bool whole = is_q ? first + i * kStep + kStep - 1 <= row0
+                              : first + i * kStep >= row0 + kRows - 1 && first + i * kStep + kStep <= S;
+      const float* lse_s = vec + s * 128 + half * 32;
+      const float* delta_s = lse_s + 64;
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const float l = is_q ? own_lse : lse_s[c], dl = is_q ? own_delta : delta_s[c];
+        const int other = col0 + c;
+        const int rq = is_q ? r_own : other, ck = is_q ? other : r_own;
+        float pr = expf(fmaf(p[c], scale, -l));
+        if (!whole && !(ck <= rq && rq < S)) pr = 0.f;
+        float gr = g[c];
+        float pd = pr;
+        if (DROP) {
+          const float mk = philox_keep(args.rng, (unit + rq) * S + ck, args.rate) ? keep_scale : 0.f;
+          pd = pr * mk;
+          gr *= mk;
+        }
+        g[c] = pr * (gr - dl) * scale;
+        p[c] = pd;
+      }
+      if (i > 0 && !(ok = take_sums(i - 1))) break;   // and with it the planes of step i - 1 are free
+      if (!is_q) tmem_store_split(p, tx, tx + 16, tx + 64);
+      tmem_store_split(g, tx + 64 + 16, tlane + kExtra + half * 32, tlane + kExtra + half * 32 + 16);
+      tmem_wait_st();
+      tc_fence_before_sync();
+      mbar_arrive(&bars->p_full);
+    }
+    if (ok && take_sums(n_it - 1) && in_seq) {
+      const size_t at = base + static_cast<size_t>(r_own) * D + half * NC;
+      if (is_q) {
+        store_row<NC>(args.dq + at, sum2, args.vec_ok);
+      } else {
+        store_row<NC>(args.dv + at, sum1, args.vec_ok);
+        store_row<NC>(args.dk + at, sum2, args.vec_ok);
+      }
+    }
+    tc_fence_before_sync();
+  }
+
+  __syncthreads();
+  if (warp == kWarpIssuer) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 512);
+  }
+  if (threadIdx.x == 0 && bars->abort_flag) report_timeout(args.status, bars->abort_flag);
+}
+
+template <int D, bool DROP>
+int launch(const BwdArgs& a, cudaStream_t st) {
+  auto kern = flash_bwd_f32_tc_kernel<D, DROP>;
+  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::kBytes));
+  static std::atomic<int> regs{0};
+  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs)) return rc;
+  const long long items = 2LL * a.BH * ((a.S + kRows - 1) / kRows);
+  DAD_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(items)), dim3(kThreads), BwdSmem::kBytes, st, a));
+  return DADATTN_OK;
+}
+
+}  // namespace
+
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* dout, const float* out, const float* lse,
+                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+                      uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st) {
+  int* status = device_status_word();
+  if (!status) return DADATTN_E_CUDA;
+  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, BH, S, scale, rate, make_philox(seed, offset), unit0, vec_ok,
+                     status};
+  const bool drop = rate > 0.f;
+  if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
+  if (D == 32) return drop ? launch<32, true>(a, st) : launch<32, false>(a, st);
+  return drop ? launch<16, true>(a, st) : launch<16, false>(a, st);
+}
+
+}  // namespace dadattn

@@ -1,0 +1,331 @@
+// fp32 forward on the tensor cores (head sizes 16, 32, 64): exact fp32 operands as three bf16 planes
+// (f32_split.cuh), online softmax and output sums in fp32 registers.
+//
+// The arithmetic is that of the reference's flash_fwd_kernel (cuda/attention.cu:17-73). A CTA owns
+// 128 query rows and takes the keys 64 at a time:
+//   warps 0-7   two threads per row, 32 key columns each: row max (exchanged between the two through
+//               shared memory), exponentials, p split into planes and written back to tensor memory
+//               over the scores, from where the P V product takes them as its A operand; each step's
+//               P V is added to an fp32 register sum, so the output is never rescaled in tensor memory
+//   warps 8-14  fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
+//   warp 15     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
+// A step costs 2304 clocks of tensor pipe at head size 64 (24 + 24 products of 48) and about 1700
+// issue slots per scheduler.
+// Tensor memory: score buffer b at 64 b, the third planes at 128, P V at 192.
+#include <cfloat>
+
+#include "f32_split.cuh"
+
+namespace dadattn {
+namespace {
+
+using namespace f32tc;
+
+constexpr int kStages = 3;
+struct FwdSmem {
+  static constexpr int kQ = 0;
+  static constexpr int kK = kQ + 3 * kPlaneA;                  // [stage][3 planes]
+  static constexpr int kV = kK + kStages * 3 * kPlaneB;
+  static constexpr int kMax = kV + kStages * 3 * kPlaneB;      // [2 steps][2 halves][128]
+  static constexpr int kBars = kMax + 2048;
+  static constexpr int kBytes = kBars + 256;
+  static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
+};
+struct FwdBars {
+  uint64_t q_full, p_full, acc_done, x_full[2];
+  uint64_t k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+static_assert(sizeof(FwdBars) <= 256, "barrier block");
+
+struct FwdArgs {
+  float *out, *lse;
+  const float *q, *k, *v;
+  int BH, S;
+  float scale, rate;
+  PhiloxKey rng;
+  int64_t unit0;
+  bool vec_ok;
+  int* status;
+};
+
+template <int D, bool DROP>
+__global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const FwdArgs args) {
+  using L = FwdSmem;
+  constexpr uint32_t kExtra = 128, kSum = 192;
+  constexpr int V4 = D / 4;     // float4 pieces of a row
+  constexpr int NC = D / 2;     // output columns per thread
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  FwdBars* bars = reinterpret_cast<FwdBars*>(smem + L::kBars);
+  volatile int* abort_flag = &bars->abort_flag;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+  const int lane = threadIdx.x % 32;
+  const int S = args.S;
+
+  if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
+    if (threadIdx.x == 0) atomicExch(args.status, DADATTN_E_CUDA);
+    return;
+  }
+  // query tiles with the most keys first
+  const int n_tiles = (S + kRows - 1) / kRows;
+  const int level = static_cast<int>(blockIdx.x) / args.BH;
+  const int bh = static_cast<int>(blockIdx.x) - level * args.BH;
+  const int row0 = (n_tiles - 1 - level) * kRows;
+  const int n_it = (min(row0 + kRows, S) + kStep - 1) / kStep;
+  const size_t base = static_cast<size_t>(bh) * S * D;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bars->q_full, kComputeThreads);
+    mbar_init(&bars->p_full, kComputeThreads);
+    mbar_init(&bars->acc_done, 1);
+    for (int s = 0; s < 2; ++s) mbar_init(&bars->x_full[s], 1);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&bars->k_full[s], kLoaderThreads);
+      mbar_init(&bars->v_full[s], kLoaderThreads);
+      mbar_init(&bars->k_empty[s], 1);
+      mbar_init(&bars->v_empty[s], 1);
+    }
+    bars->abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == kWarpIssuer) {
+    tmem_alloc(&bars->tmem_base, 256);
+    tmem_relinquish();
+  }
+  // Columns D..63 of the V tiles are read by the P V products (64 columns wide): zeros.
+  if (D < 64) {
+    for (int i = threadIdx.x; i < kStages * 3 * kPlaneB / 16; i += kThreads)
+      reinterpret_cast<uint4*>(smem + L::kV)[i] = make_uint4(0, 0, 0, 0);
+    fence_proxy_async_smem();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = bars->tmem_base;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  if (warp >= kWarpLoader0) {
+    setmaxnreg_dec<kRegsHelper>();
+    if (warp < kWarpIssuer) {
+      // ------------------------------ loaders ------------------------------
+      const int t = threadIdx.x - kWarpLoader0 * 32;
+      constexpr int kPieces = kStep * V4;
+      constexpr int kMine = (kPieces + kLoaderThreads - 1) / kLoaderThreads;
+      const float *kk = args.k + base, *vv = args.v + base;
+      bool ok = true;
+      int s = 0, lap = 0;
+      for (int i = 0; ok && i < n_it; ++i) {
+        const int r0 = i * kStep;
+        float4 xk[kMine], xv[kMine];
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          const int e = t + j * kLoaderThreads;
+          const bool in = e < kPieces;
+          xk[j] = in ? load4<D>(kk, r0 + e / V4, e % V4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+          xv[j] = in ? load4<D>(vv, r0 + e / V4, e % V4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        auto put = [&](const float4 (&x)[kMine], uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
+          Split4 sp[kMine];
+#pragma unroll
+          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          if (lap > 0 && !mbar_wait(empty, (lap - 1) & 1, abort_flag)) return false;
+#pragma unroll
+          for (int j = 0; j < kMine; ++j) {
+            const int e = t + j * kLoaderThreads;
+            if (e < kPieces) store_split(tile, kPlaneB, e / V4, e % V4, sp[j]);
+          }
+          fence_proxy_async_smem();
+          mbar_arrive(full);
+          return true;
+        };
+        ok = put(xk, smem + L::kK + s * 3 * kPlaneB, &bars->k_empty[s], &bars->k_full[s]) &&
+             put(xv, smem + L::kV + s * 3 * kPlaneB, &bars->v_empty[s], &bars->v_full[s]);
+        if (++s == kStages) s = 0, ++lap;
+      }
+    } else if (elect_one()) {
+      // ------------------------------ MMA issuer ------------------------------
+      constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // Q, K: K-major
+      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // P from tensor memory, V MN-major
+      const SmemDescBase qd = make_desc_base_sw128(smem_u32(smem + L::kQ), 0);
+      const SmemDescBase k0 = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
+      const SmemDescBase v0 = make_desc_base_sw128(smem_u32(smem + L::kV), 0);
+      auto issue_x = [&](int i) -> bool {
+        const int s = i % kStages;
+        const uint32_t tx = tmem + (i & 1) * 64;
+        const SmemDescBase kd{k0.lo + s * (3 * kPlaneB >> 4), k0.hi};
+        if (!mbar_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            mma_ss(tx, desc_at(qd, product_a(m) * kPlaneA + kk * 32), desc_at(kd, product_b(m) * kPlaneB + kk * 32),
+                   idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(&bars->x_full[i & 1]);
+        mma_commit(&bars->k_empty[s]);
+        return true;
+      };
+      auto issue_pv = [&](int i) -> bool {
+        const int s = i % kStages;
+        const uint32_t tx = tmem + (i & 1) * 64;
+        const SmemDescBase vd{v0.lo + s * (3 * kPlaneB >> 4), v0.hi};
+        if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        tc_fence_after_sync();
+        // planes of 16 keys kk: half kk / 2 of a row's columns, 8 columns of pairs each
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int kk = 0; kk < kStep / 16; ++kk) {
+            const uint32_t in = (kk & 1) * 8;
+            const uint32_t at = product_a(m) == 2 ? tmem + kExtra + (kk >> 1) * 16 + in
+                                                  : tx + (kk >> 1) * 32 + product_a(m) * 16 + in;
+            mma_ts(tmem + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                   (m > 0 || kk > 0) ? 1u : 0u);
+          }
+        mma_commit(&bars->v_empty[s]);
+        mma_commit(&bars->acc_done);
+        return true;
+      };
+      bool ok = mbar_wait(&bars->q_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
+      for (int i = 0; ok && i < n_it; ++i) ok = issue_pv(i) && (i + 2 >= n_it || issue_x(i + 2));
+    }
+  } else {
+    setmaxnreg_inc<kRegsCompute>();
+    // ------------------------------ softmax ------------------------------
+    const int half = warp / 4, quad = warp % 4;
+    const int row = quad * 32 + lane;           // query row of the tile = TMEM lane
+    const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    float* part = reinterpret_cast<float*>(smem + L::kMax);
+    // the two warps that share these 32 rows
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };
+    bool ok = true;
+    {
+      const float* qq = args.q + base;
+#pragma unroll
+      for (int j = 0; j < kRows * V4 / kComputeThreads; ++j) {
+        const int e = threadIdx.x + j * kComputeThreads;
+        store_split(smem + L::kQ, kPlaneA, e / V4, e % V4, split4(load4<D>(qq, row0 + e / V4, e % V4, S, args.vec_ok)));
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&bars->q_full);
+    }
+    const int r = row0 + row;
+    const float scale = args.scale;
+    const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
+    float m = -FLT_MAX, l = 0.f, o[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) o[c] = 0.f;
+    auto take_sums = [&](int i) -> bool {
+      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      tc_fence_after_sync();
+      tmem_add<NC>(tlane + kSum + half * NC, o);
+      return true;
+    };
+
+    for (int i = 0; i < n_it; ++i) {
+      if (!(ok = mbar_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
+      tc_fence_after_sync();
+      const uint32_t tx = tlane + (i & 1) * 64 + half * 32;
+      const int c0 = i * kStep + half * 32;
+      float p[32];
+      {
+        uint32_t x[32];
+        tmem_ld32(tx, x);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) p[c] = __uint_as_float(x[c]) * scale;
+      }
+      if (i * kStep + kStep - 1 > row0) {   // keys beyond a row's own
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          if (c0 + c > r) p[c] = -FLT_MAX;
+      }
+      float mx0 = p[0], mx1 = p[1];
+#pragma unroll
+      for (int c = 2; c < 32; c += 4) {
+        mx0 = fmax3(mx0, p[c], p[c + 1]);
+        if (c + 2 < 32) mx1 = fmax3(mx1, p[c + 2], p[c + 3]);
+      }
+      float* own = part + (i & 1) * 256;
+      own[half * 128 + row] = fmaxf(mx0, mx1);
+      pair_sync();
+      // every row sees key 0 in step 0: the max of both halves is finite from there on
+      const float m_new = fmaxf(m, fmaxf(own[row], own[128 + row]));
+      const float corr = expf(m - m_new);
+      m = m_new;
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        p[c] = p[c] == -FLT_MAX ? 0.f : expf(p[c] - m_new);
+        sum += p[c];
+        if (DROP) {
+          const uint64_t idx = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0 + c;
+          p[c] = philox_keep(args.rng, idx, args.rate) ? p[c] * keep_scale : 0.f;
+        }
+      }
+      l = l * corr + sum;
+      if (i > 0) {   // and with it the planes of step i - 1 are free
+        if (!(ok = take_sums(i - 1))) break;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[c] *= corr;
+      }
+      tmem_store_split(p, tx, tx + 16, tlane + kExtra + half * 16);
+      tmem_wait_st();
+      tc_fence_before_sync();
+      mbar_arrive(&bars->p_full);
+    }
+    if (ok && take_sums(n_it - 1)) {
+      float* own = part + (n_it & 1) * 256;
+      own[half * 128 + row] = l;
+      pair_sync();
+      if (r < S) {
+        const float l_all = own[row] + own[128 + row];
+        const float inv = 1.0f / l_all;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[c] *= inv;
+        store_row<NC>(args.out + base + static_cast<size_t>(r) * D + half * NC, o, args.vec_ok);
+        if (half == 0) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
+      }
+    }
+    tc_fence_before_sync();
+  }
+
+  __syncthreads();
+  if (warp == kWarpIssuer) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 256);
+  }
+  if (threadIdx.x == 0 && bars->abort_flag) report_timeout(args.status, bars->abort_flag);
+}
+
+template <int D, bool DROP>
+int launch(const FwdArgs& a, cudaStream_t st) {
+  auto kern = flash_fwd_f32_tc_kernel<D, DROP>;
+  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::kBytes));
+  static std::atomic<int> regs{0};
+  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs)) return rc;
+  const long long items = static_cast<long long>(a.BH) * ((a.S + kRows - 1) / kRows);
+  DAD_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(items)), dim3(kThreads), FwdSmem::kBytes, st, a));
+  return DADATTN_OK;
+}
+
+}  // namespace
+
+int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
+                      float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
+                      cudaStream_t st) {
+  int* status = device_status_word();
+  if (!status) return DADATTN_E_CUDA;
+  const FwdArgs a = {out, lse, q, k, v, BH, S, scale, rate, make_philox(seed, offset), unit0, vec_ok, status};
+  const bool drop = rate > 0.f;
+  if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
+  if (D == 32) return drop ? launch<32, true>(a, st) : launch<32, false>(a, st);
+  return drop ? launch<16, true>(a, st) : launch<16, false>(a, st);
+}
+
+}  // namespace dadattn
