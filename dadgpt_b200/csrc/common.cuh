@@ -107,6 +107,61 @@ __device__ __forceinline__ bool philox_keep(const PhiloxKey& p, uint64_t subsequ
   return !(u < rate);
 }
 
+// The keep bits of several draws at once, for kernels whose time is the drawing: the mask, stripped to
+// what it needs.
+//  * The round keys come precomputed from the host (kernel parameters: constant-bank operands), both
+//    halves of each 32 x 32 product from one widening multiply, the last rounds compute only what the
+//    first output word depends on, and "uniform < rate" is decided on the integer draw: the uniform
+//    is a non-decreasing function of it (cvt.rn, one fma), so the dropped draws are those below a
+//    threshold that the host finds with the same float arithmetic.
+//  * Of the counter only the low subsequence word changes from draw to draw. The first round's
+//    product with the offset word is one number for the call, the second round's product with what
+//    comes of it one for the thread, and neither reaches the other lane before the third round: 13
+//    widening products, two high and one low are left of 20.
+struct PhiloxRounds {
+  uint32_t k0[10], k1[9];   // key words of rounds 0..9 (the last round needs only k0)
+  uint32_t c0, c1;          // low counter words: offset / 4
+  uint32_t m_lo, m_hi;      // round 0: 0xD2511F53 * c0
+  uint32_t word;            // offset % 4: which word of the block is the draw
+  uint32_t drop_below;      // draws below this are dropped (uniform < rate)
+};
+PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate);
+
+// Bit i (i < n <= 32): whether the probability of flat index at + i * stride is kept.
+template <int UNROLL>
+__device__ __forceinline__ uint32_t philox_keep_bits(const PhiloxRounds& p, uint64_t at, uint32_t stride, int n) {
+  const uint32_t lo = static_cast<uint32_t>(at), hi = static_cast<uint32_t>(at >> 32);
+  uint32_t bits = 0;
+  if (p.word == 0 && lo <= 0xffffffffu - 31ull * stride) {   // (the high word stays put)
+    const uint64_t t = static_cast<uint64_t>(0xCD9E8D57u) * (p.m_hi ^ hi ^ p.k1[0]);
+    const uint32_t x0 = static_cast<uint32_t>(t >> 32) ^ p.k0[1], x1 = static_cast<uint32_t>(t), x2 = p.m_lo ^ p.k1[1];
+#pragma unroll UNROLL
+    for (int i = 0; i < n; ++i) {
+      const uint64_t a = static_cast<uint64_t>(0xCD9E8D57u) * (lo + static_cast<uint32_t>(i) * stride);
+      const uint64_t b = static_cast<uint64_t>(0xD2511F53u) * (static_cast<uint32_t>(a >> 32) ^ p.c1 ^ p.k0[0]);
+      uint32_t c0 = x0 ^ static_cast<uint32_t>(a), c1 = x1;
+      uint32_t c2 = static_cast<uint32_t>(b >> 32) ^ x2, c3 = static_cast<uint32_t>(b);
+#pragma unroll
+      for (int r = 2; r < 8; ++r) {
+        const uint64_t p0 = static_cast<uint64_t>(0xD2511F53u) * c0, p1 = static_cast<uint64_t>(0xCD9E8D57u) * c2;
+        c0 = static_cast<uint32_t>(p1 >> 32) ^ c1 ^ p.k0[r];
+        c2 = static_cast<uint32_t>(p0 >> 32) ^ c3 ^ p.k1[r];
+        c1 = static_cast<uint32_t>(p1);
+        c3 = static_cast<uint32_t>(p0);
+      }
+      const uint32_t n2 = __umulhi(0xD2511F53u, c0) ^ c3 ^ p.k1[8];
+      const uint32_t draw = __umulhi(0xCD9E8D57u, n2) ^ (0xCD9E8D57u * c2) ^ p.k0[9];
+      bits |= (draw >= p.drop_below ? 1u : 0u) << i;
+    }
+    return bits;
+  }
+  const PhiloxKey key = {p.k0[0], p.k1[0], p.c0, p.c1, p.word};
+#pragma unroll 1
+  for (int i = 0; i < n; ++i)
+    bits |= (philox_draw(key, at + static_cast<uint64_t>(i) * stride) >= p.drop_below ? 1u : 0u) << i;
+  return bits;
+}
+
 // ---- bit-packed dropout mask (dadattn_dropout_mask_bits) ----------------------------------------
 // One 16-byte record per (batch x head, 128-query tile qt, 128-key tile kt <= qt, query row of
 // the tile): bit i of 32-bit word w says whether the probability of key 32 w + i of the key tile

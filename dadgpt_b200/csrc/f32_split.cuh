@@ -24,13 +24,13 @@ constexpr int kRows = 128;          // rows of the resident tile: one per TMEM l
 constexpr int kStep = 64;           // rows of the streamed tile per step
 constexpr int kPlaneA = kRows * 128;   // one bf16 plane, 128-byte rows (64 elements), swizzled
 constexpr int kPlaneB = kStep * 128;
-constexpr int kComputeThreads = 256;   // two per row
+constexpr int kComputeThreads = 512;   // four per row, 16 of a step's 64 columns each
 constexpr int kLoaderThreads = 7 * 32;
-constexpr int kThreads = 512;          // 8 compute warps, 7 loader warps, 1 issuer warp
-constexpr int kWarpLoader0 = 8, kWarpIssuer = 15;
+constexpr int kThreads = 768;          // 16 compute warps, 7 loader warps, 1 issuer warp
+constexpr int kWarpLoader0 = 16, kWarpIssuer = 23;
 // Registers per thread once the warpgroups have rebalanced; the pool is what the CTA starts with.
-constexpr int kRegsLaunch = 128, kRegsCompute = 160, kRegsHelper = 96;
-static_assert(256 * kRegsCompute + 256 * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
+constexpr int kRegsLaunch = 80, kRegsCompute = 88, kRegsHelper = 64;
+static_assert(kComputeThreads * kRegsCompute + 256 * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
 
 // Plane pairs of the six products, smallest first.
 __device__ __forceinline__ constexpr int product_a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
@@ -59,12 +59,10 @@ __device__ __forceinline__ void store_split(uint8_t* tile, int plane_bytes, int 
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * plane_bytes) = s.p[i];
 }
 
-// Columns 4 c4 .. of row r of a [S, D] matrix; zeros beyond the sequence. Any 4-byte alignment.
-template <int D>
-__device__ __forceinline__ float4 load4(const float* __restrict__ m, int r, int c4, int S, bool vec_ok) {
+// Four consecutive fp32 values at any 4-byte alignment; zeros when !in.
+__device__ __forceinline__ float4 load4(const float* __restrict__ p, bool in, bool vec_ok) {
   float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (r < S) {
-    const float* p = m + static_cast<size_t>(r) * D + c4 * 4;
+  if (in) {
     if (vec_ok)
       x = __ldg(reinterpret_cast<const float4*>(p));
     else
@@ -76,58 +74,64 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b) {
   return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+// N consecutive columns of the thread's TMEM lane (N = 16, 8 or 4)
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[N]) {
+  if constexpr (N == 16)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+  else if constexpr (N == 8)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(taddr)
+        : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-      "r"(r[15]), "r"(taddr)
-      : "memory");
-}
-// 32 values of a row -> three planes of packed pairs in tensor memory, 16 columns each.
-__device__ __forceinline__ void tmem_store_split(float (&x)[32], uint32_t t0, uint32_t t1, uint32_t t2) {
+// 16 values of a row -> three planes of packed pairs in tensor memory, 8 columns each.
+__device__ __forceinline__ void tmem_store_split(float2 (&x)[8], uint32_t t0, uint32_t t1, uint32_t t2) {
   const uint32_t t[3] = {t0, t1, t2};
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    uint32_t pk[16];
+    uint32_t pk[8];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      pk[j] = pack_bf16(x[2 * j], x[2 * j + 1]);
-      if (i < 2) {
-        x[2 * j] -= __uint_as_float(pk[j] << 16);
-        x[2 * j + 1] -= __uint_as_float(pk[j] & 0xffff0000u);
-      }
+    for (int j = 0; j < 8; ++j) {
+      pk[j] = pack_bf16(x[j].x, x[j].y);
+      if (i < 2)
+        x[j] = ffma2(make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xffff0000u)),
+                     make_float2(-1.f, -1.f), x[j]);   // exact
     }
-    tmem_st16(t[i], pk);
+    tmem_st8(t[i], pk);
   }
 }
-// sum[c] += the accumulator's columns taddr + c, c < N (N = 32, 16 or 8)
+// sum[c] += the accumulator's columns taddr + c
 template <int N>
 __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&sum)[N]) {
-  if constexpr (N == 32) {
-    uint32_t a[32];
-    tmem_ld32(taddr, a);
-    tmem_wait_ld();
+  uint32_t a[N];
+  tmem_ld<N>(taddr, a);
+  tmem_wait_ld();
 #pragma unroll
-    for (int c = 0; c < N; ++c) sum[c] += __uint_as_float(a[c]);
-  } else {
-    uint32_t a[16];
-    tmem_ld16(taddr, a);
-    tmem_wait_ld();
-#pragma unroll
-    for (int c = 0; c < N; ++c) sum[c] += __uint_as_float(a[c]);
-  }
+  for (int c = 0; c < N; ++c) sum[c] += __uint_as_float(a[c]);
+}
+// e^x for x <= 0 (or a masked score's -FLT_MAX, which gives 0)
+__device__ __forceinline__ float2 exp2_of(float2 x) {
+  const float2 t = fmul2(x, make_float2(1.4426950408889634f, 1.4426950408889634f));
+  return make_float2(ex2(t.x), ex2(t.y));
 }
 template <int N>
 __device__ __forceinline__ void store_row(float* dst, const float (&x)[N], bool vec_ok) {

@@ -8,12 +8,12 @@
 //     dK/dV   K, V              Q, dO             S^T            dP^T           dV += P^T B2, dK += dS^T B1
 //     dQ      Q, dO             K, V              S              dP             dQ += dS B1
 // A CTA owns 128 resident rows (one per TMEM lane) and takes the other side 64 rows at a time:
-//   warps 0-7   two threads per row, 32 columns each: p = exp(s scale - lse), ds = p (dP - delta)
+//   warps 0-15  four threads per row, 16 columns each: p = exp(s scale - lse), ds = p (dP - delta)
 //               scale, both split into planes and written back to tensor memory, from where the
 //               sums take them as A operands; the sums of each step are added to fp32 registers
-//   warps 8-14  fetch the next step's fp32 rows, split them in registers, and put them into the
+//   warps 16-22 fetch the next step's fp32 rows, split them in registers, and put them into the
 //               shared-memory stage the moment it is released; delta = rowsum(dO o O) on the way
-//   warp 15     issues the products. Order on the tensor pipe: sums of step i, X2 then X1 of step
+//   warp 23     issues the products. Order on the tensor pipe: sums of step i, X2 then X1 of step
 //               i + 2 (B2's stage is released before B1's, so its refill hides behind the sums'
 //               last products), sums of step i + 1, ...
 // A step costs 2304 (X) + 2304 (dK/dV) or 1152 (dQ) clocks of tensor pipe at head size 64 (48 for a
@@ -49,18 +49,18 @@ struct BwdArgs {
   const float *dout, *out, *lse, *q, *k, *v;
   int BH, S;
   float scale, rate;
-  PhiloxKey rng;
+  PhiloxRounds rng;
   int64_t unit0;
   bool vec_ok;
   int* status;
 };
 
 template <int D, bool DROP>
-__global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const BwdArgs args) {
+__global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __grid_constant__ BwdArgs args) {
   using L = BwdSmem;
   constexpr uint32_t kExtra = 256, kSum1 = 320, kSum2 = 384;   // kSum1: dV; kSum2: dK or dQ
   constexpr int V4 = D / 4;                                    // float4 pieces of a row
-  constexpr int NC = D / 2;                                    // columns of a sum per thread
+  constexpr int NC = D / 4;                                    // columns of a sum per thread
 
   extern __shared__ __align__(1024) uint8_t smem[];
   BwdBars* bars = reinterpret_cast<BwdBars*>(smem + L::kBars);
@@ -121,61 +121,62 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const Bwd
     setmaxnreg_dec<kRegsHelper>();
     if (warp < kWarpIssuer) {
       // ------------------------------ loaders ------------------------------
+      // Thread t takes the same four columns of every kRowStep-th row of a streamed tile.
       const int t = threadIdx.x - kWarpLoader0 * 32;
-      constexpr int kPieces = kStep * V4;                                   // float4 pieces of a streamed tile
-      constexpr int kMine = (kPieces + kLoaderThreads - 1) / kLoaderThreads;
-      const float* b1 = (is_q ? args.k : args.q) + base;
-      const float* b2 = (is_q ? args.v : args.dout) + base;
-      const float* oo = args.out + base;
+      constexpr int kRowStep = kLoaderThreads / V4;
+      constexpr int kMine = (kStep + kRowStep - 1) / kRowStep;
+      const int rt = t / V4, c4 = t % V4;
+      const float* b1 = (is_q ? args.k : args.q) + base + c4 * 4;
+      const float* b2 = (is_q ? args.v : args.dout) + base + c4 * 4;
+      const float* oo = args.out + base + c4 * 4;
       float* vec = reinterpret_cast<float*>(smem + L::kVec);
       bool ok = true;
       for (int i = 0; ok && i < n_it; ++i) {
-        const int s = i & 1, r0 = first + i * kStep;
-        float4 x1[kMine], x2[kMine], xo[kMine];
+        const int s = i & 1, r = first + i * kStep + rt;
+        auto fetch = [&](float4 (&x)[kMine], const float* m) {
+          m += static_cast<size_t>(r) * D;
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          const int e = t + j * kLoaderThreads;
-          const bool in = e < kPieces;
-          const int r = r0 + e / V4, c4 = e % V4;
-          x2[j] = in ? load4<D>(b2, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!is_q) xo[j] = in ? load4<D>(oo, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-          x1[j] = in ? load4<D>(b1, r, c4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        float row_lse = 0.f;
-        if (!is_q && t < kStep && r0 + t < S) row_lse = __ldg(lse + r0 + t);
-        Split4 s2[kMine];
-        float delta[kMine];
+          for (int j = 0; j < kMine; ++j)
+            x[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
+        };
+        uint8_t* tile = smem + L::kStage + s * L::kStageBytes;
+        auto put = [&](uint8_t* to, const Split4 (&x)[kMine]) {
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          if (!is_q) {
-            delta[j] = dot4(x2[j], xo[j]);
+          for (int j = 0; j < kMine; ++j)
+            if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, x[j]);
+        };
+        float4 x[kMine];
+        float delta[kMine], row_lse = 0.f;
+        Split4 sp[kMine];
+        fetch(x, b2);
+        if (!is_q) {
+          float4 xo[kMine];
+          fetch(xo, oo);
+          if (t < kStep && first + i * kStep + t < S) row_lse = __ldg(lse + first + i * kStep + t);
+#pragma unroll
+          for (int j = 0; j < kMine; ++j) {
+            delta[j] = dot4(x[j], xo[j]);
 #pragma unroll
             for (int o = V4 / 2; o > 0; o >>= 1) delta[j] += __shfl_xor_sync(0xffffffffu, delta[j], o);
           }
-          s2[j] = split4(x2[j]);
         }
-        if (i >= 2 && !(ok = mbar_wait(&bars->b2_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
-        uint8_t* tile = smem + L::kStage + s * L::kStageBytes;
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          const int e = t + j * kLoaderThreads;
-          if (e < kPieces) {
-            store_split(tile + 3 * kPlaneB, kPlaneB, e / V4, e % V4, s2[j]);
-            if (!is_q && e % V4 == 0) vec[s * 128 + 64 + e / V4] = delta[j];
-          }
+        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+        fetch(x, b1);   // on its way while B2 goes to shared memory
+        if (i >= 2 && !(ok = mbar_wait(&bars->b2_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
+        put(tile + 3 * kPlaneB, sp);
+        if (!is_q) {
+          if (t < kStep) vec[s * 128 + t] = row_lse;
+#pragma unroll
+          for (int j = 0; j < kMine; ++j)
+            if (c4 == 0 && rt + j * kRowStep < kStep) vec[s * 128 + 64 + rt + j * kRowStep] = delta[j];
         }
-        if (!is_q && t < kStep) vec[s * 128 + t] = row_lse;
         fence_proxy_async_smem();
         mbar_arrive(&bars->b2_full[s]);
-        Split4 s1[kMine];
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) s1[j] = split4(x1[j]);
+        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
         if (i >= 2 && !(ok = mbar_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
-#pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          const int e = t + j * kLoaderThreads;
-          if (e < kPieces) store_split(tile, kPlaneB, e / V4, e % V4, s1[j]);
-        }
+        put(tile, sp);
         fence_proxy_async_smem();
         mbar_arrive(&bars->b1_full[s]);
       }
@@ -215,13 +216,13 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const Bwd
         const SmemDescBase b2{b1.lo + (3 * kPlaneB >> 4), b0.hi};
         if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
-        // planes of 16 streamed rows kk: half kk / 2 of a row's columns, 8 columns of pairs each
+        // the planes of 16 streamed rows kk lie over the 16 columns their scores came from
         if (!is_q) {
 #pragma unroll
           for (int m = 0; m < 6; ++m)
 #pragma unroll
             for (int kk = 0; kk < kStep / 16; ++kk) {
-              const uint32_t at = (product_a(m) == 0 ? 0u : product_a(m) == 1 ? 16u : 64u) + (kk >> 1) * 32 + (kk & 1) * 8;
+              const uint32_t at = (product_a(m) == 0 ? 0u : product_a(m) == 1 ? 8u : 64u) + kk * 16;
               mma_ts(tmem + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 2048), idesc_s,
                      (m > 0 || kk > 0) ? 1u : 0u);
             }
@@ -231,8 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const Bwd
         for (int m = 0; m < 6; ++m)
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
-            const uint32_t in = (kk >> 1) * 32 + (kk & 1) * 8;
-            const uint32_t at = product_a(m) == 0 ? tx + 64 + 16 + in : tmem + kExtra + (product_a(m) == 1 ? 0u : 16u) + in;
+            const uint32_t at = product_a(m) == 0 ? tx + 64 + 8 + kk * 16 : tmem + kExtra + (product_a(m) - 1) * 8 + kk * 16;
             mma_ts(tmem + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 2048), idesc_s,
                    (m > 0 || kk > 0) ? 1u : 0u);
           }
@@ -246,26 +246,26 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const Bwd
   } else {
     setmaxnreg_inc<kRegsCompute>();
     // ------------------------------ compute ------------------------------
-    const int half = warp / 4, quad = warp % 4;
+    const int cg = warp / 4, quad = warp % 4;   // which 16 columns of a step; TMEM lane quadrant
     const int row = quad * 32 + lane;           // resident row = TMEM lane
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     float* vec = reinterpret_cast<float*>(smem + L::kVec);
     bool ok = true;
     {
       // the resident tiles, split into planes
-      const float* a1 = (is_q ? args.q : args.k) + base;
-      const float* a2 = (is_q ? args.dout : args.v) + base;
-      const float* oo = args.out + base;
-      constexpr int kMine = kRows * V4 / kComputeThreads;
+      constexpr int kRowStep = kComputeThreads / V4;
+      const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
+      const size_t at = base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
+      const float *a1 = (is_q ? args.q : args.k) + at, *a2 = (is_q ? args.dout : args.v) + at, *oo = args.out + at;
 #pragma unroll
-      for (int j = 0; j < kMine; ++j) {
-        const int e = threadIdx.x + j * kComputeThreads, r = e / V4, c4 = e % V4;
-        const float4 x1 = load4<D>(a1, row0 + r, c4, S, args.vec_ok);
-        const float4 x2 = load4<D>(a2, row0 + r, c4, S, args.vec_ok);
-        store_split(smem + L::kA1, kPlaneA, r, c4, split4(x1));
+      for (int j = 0; j < kRows / kRowStep; ++j) {
+        const int r = rt + j * kRowStep;
+        const bool in = row0 + r < S;
+        const float4 x2 = load4(a2 + j * kRowStep * D, in, args.vec_ok);
+        store_split(smem + L::kA1, kPlaneA, r, c4, split4(load4(a1 + j * kRowStep * D, in, args.vec_ok)));
         store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2));
         if (is_q) {
-          float delta = dot4(x2, load4<D>(oo, row0 + r, c4, S, args.vec_ok));
+          float delta = dot4(x2, load4(oo + j * kRowStep * D, in, args.vec_ok));
 #pragma unroll
           for (int o = V4 / 2; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
           if (c4 == 0) vec[128 + r] = delta;
@@ -289,59 +289,76 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const Bwd
     auto take_sums = [&](int i) -> bool {
       if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
-      if (!is_q) tmem_add<NC>(tlane + kSum1 + half * NC, sum1);
-      tmem_add<NC>(tlane + kSum2 + half * NC, sum2);
+      if (!is_q) tmem_add<NC>(tlane + kSum1 + cg * NC, sum1);
+      tmem_add<NC>(tlane + kSum2 + cg * NC, sum2);
       return true;
     };
 
     for (int i = 0; i < n_it; ++i) {
       const int s = i & 1;
-      const int col0 = first + i * kStep + half * 32;      // streamed row of this thread's first column
+      const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
       if (!(ok = mbar_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
       // (the row scalars came with B2)
       if (!is_q && !(ok = mbar_wait(&bars->b2_full[s], (i >> 1) & 1, abort_flag))) break;
       tc_fence_after_sync();
-      const uint32_t tx = tlane + s * 128 + half * 32;
-      float p[32], g[32];
+      const uint32_t tx = tlane + s * 128 + cg * 16;
+      float2 p[8], g[8];
       {
-        uint32_t x1[32], x2[32];
-        tmem_ld32(tx, x1);
-        tmem_ld32(tx + 64, x2);
+        uint32_t x1[16], x2[16];
+        tmem_ld<16>(tx, x1);
+        tmem_ld<16>(tx + 64, x2);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; ++c) p[c] = __uint_as_float(x1[c]), g[c] = __uint_as_float(x2[c]);
+        for (int c = 0; c < 8; ++c) {
+          p[c] = make_float2(__uint_as_float(x1[2 * c]), __uint_as_float(x1[2 * c + 1]));
+          g[c] = make_float2(__uint_as_float(x2[2 * c]), __uint_as_float(x2[2 * c + 1]));
+        }
       }
-      // every pair of the tile visible? (key <= query < S)
+      const float2* lse_s = reinterpret_cast<const float2*>(vec + s * 128 + cg * 16);
+      const float2* delta_s = lse_s + 32;
+      // p = exp(s scale - lse)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 l = is_q ? make_float2(own_lse, own_lse) : lse_s[c];
+        p[c] = exp2_of(ffma2(p[c], make_float2(scale, scale), make_float2(-l.x, -l.y)));
+      }
+      // every pair of the step visible (key <= query < S)?
       const bool whole = is_q ? first + i * kStep + kStep - 1 <= row0
                               : first + i * kStep >= row0 + kRows - 1 && first + i * kStep + kStep <= S;
-      const float* lse_s = vec + s * 128 + half * 32;
-      const float* delta_s = lse_s + 64;
+      if (!whole) {
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const float l = is_q ? own_lse : lse_s[c], dl = is_q ? own_delta : delta_s[c];
-        const int other = col0 + c;
-        const int rq = is_q ? r_own : other, ck = is_q ? other : r_own;
-        float pr = expf(fmaf(p[c], scale, -l));
-        if (!whole && !(ck <= rq && rq < S)) pr = 0.f;
-        float gr = g[c];
-        float pd = pr;
-        if (DROP) {
-          const float mk = philox_keep(args.rng, (unit + rq) * S + ck, args.rate) ? keep_scale : 0.f;
-          pd = pr * mk;
-          gr *= mk;
+        for (int c = 0; c < 16; ++c) {
+          const int rq = is_q ? r_own : col0 + c, ck = is_q ? col0 + c : r_own;
+          float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
+          if (ck > rq || rq >= S) x = 0.f;
         }
-        g[c] = pr * (gr - dl) * scale;
-        p[c] = pd;
+      }
+      // ds = p (dP - delta) scale, with dropout on P and dP alike
+      uint32_t keep = 0xffffu;
+      if (DROP) {
+        const uint64_t at = is_q ? (unit + r_own) * S + col0 : (unit + col0) * S + r_own;
+        keep = philox_keep_bits<4>(args.rng, at, is_q ? 1u : static_cast<uint32_t>(S), 16);
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 dl = is_q ? make_float2(own_delta, own_delta) : delta_s[c];
+        const float2 pr = p[c];
+        if (DROP) {
+          const float2 mk = make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f);
+          p[c] = fmul2(p[c], mk);
+          g[c] = fmul2(g[c], mk);
+        }
+        g[c] = fmul2(fmul2(pr, fadd2(g[c], make_float2(-dl.x, -dl.y))), make_float2(scale, scale));
       }
       if (i > 0 && !(ok = take_sums(i - 1))) break;   // and with it the planes of step i - 1 are free
-      if (!is_q) tmem_store_split(p, tx, tx + 16, tx + 64);
-      tmem_store_split(g, tx + 64 + 16, tlane + kExtra + half * 32, tlane + kExtra + half * 32 + 16);
+      if (!is_q) tmem_store_split(p, tx, tx + 8, tx + 64);
+      tmem_store_split(g, tx + 64 + 8, tlane + kExtra + cg * 16, tlane + kExtra + cg * 16 + 8);
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(&bars->p_full);
     }
     if (ok && take_sums(n_it - 1) && in_seq) {
-      const size_t at = base + static_cast<size_t>(r_own) * D + half * NC;
+      const size_t at = base + static_cast<size_t>(r_own) * D + cg * NC;
       if (is_q) {
         store_row<NC>(args.dq + at, sum2, args.vec_ok);
       } else {
@@ -379,7 +396,7 @@ int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* dout, const 
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st) {
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, BH, S, scale, rate, make_philox(seed, offset), unit0, vec_ok,
+  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
                      status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);

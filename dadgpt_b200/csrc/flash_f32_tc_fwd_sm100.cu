@@ -3,12 +3,12 @@
 //
 // The arithmetic is that of the reference's flash_fwd_kernel (cuda/attention.cu:17-73). A CTA owns
 // 128 query rows and takes the keys 64 at a time:
-//   warps 0-7   two threads per row, 32 key columns each: row max (exchanged between the two through
+//   warps 0-15  four threads per row, 16 key columns each: row max (exchanged between them through
 //               shared memory), exponentials, p split into planes and written back to tensor memory
 //               over the scores, from where the P V product takes them as its A operand; each step's
 //               P V is added to an fp32 register sum, so the output is never rescaled in tensor memory
-//   warps 8-14  fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
-//   warp 15     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
+//   warps 16-22 fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
+//   warp 23     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
 // A step costs 2304 clocks of tensor pipe at head size 64 (24 + 24 products of 48) and about 1700
 // issue slots per scheduler.
 // Tensor memory: score buffer b at 64 b, the third planes at 128, P V at 192.
@@ -26,8 +26,8 @@ struct FwdSmem {
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + 3 * kPlaneA;                  // [stage][3 planes]
   static constexpr int kV = kK + kStages * 3 * kPlaneB;
-  static constexpr int kMax = kV + kStages * 3 * kPlaneB;      // [2 steps][2 halves][128]
-  static constexpr int kBars = kMax + 2048;
+  static constexpr int kMax = kV + kStages * 3 * kPlaneB;      // [2 steps][4 column groups][128]
+  static constexpr int kBars = kMax + 4096;
   static constexpr int kBytes = kBars + 256;
   static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
 };
@@ -44,18 +44,18 @@ struct FwdArgs {
   const float *q, *k, *v;
   int BH, S;
   float scale, rate;
-  PhiloxKey rng;
+  PhiloxRounds rng;
   int64_t unit0;
   bool vec_ok;
   int* status;
 };
 
 template <int D, bool DROP>
-__global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const FwdArgs args) {
+__global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __grid_constant__ FwdArgs args) {
   using L = FwdSmem;
   constexpr uint32_t kExtra = 128, kSum = 192;
   constexpr int V4 = D / 4;     // float4 pieces of a row
-  constexpr int NC = D / 2;     // output columns per thread
+  constexpr int NC = D / 4;     // output columns per thread
 
   extern __shared__ __align__(1024) uint8_t smem[];
   FwdBars* bars = reinterpret_cast<FwdBars*>(smem + L::kBars);
@@ -111,38 +111,41 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const Fwd
     setmaxnreg_dec<kRegsHelper>();
     if (warp < kWarpIssuer) {
       // ------------------------------ loaders ------------------------------
+      // Thread t takes the same four columns of every kRowStep-th row of a tile.
       const int t = threadIdx.x - kWarpLoader0 * 32;
-      constexpr int kPieces = kStep * V4;
-      constexpr int kMine = (kPieces + kLoaderThreads - 1) / kLoaderThreads;
-      const float *kk = args.k + base, *vv = args.v + base;
+      constexpr int kRowStep = kLoaderThreads / V4;
+      constexpr int kMine = (kStep + kRowStep - 1) / kRowStep;
+      const int rt = t / V4, c4 = t % V4;
+      const float *kk = args.k + base + c4 * 4, *vv = args.v + base + c4 * 4;
       bool ok = true;
       int s = 0, lap = 0;
       for (int i = 0; ok && i < n_it; ++i) {
-        const int r0 = i * kStep;
-        float4 xk[kMine], xv[kMine];
+        const int r = i * kStep + rt;
+        auto fetch = [&](float4 (&x)[kMine], const float* m) {
+          m += static_cast<size_t>(r) * D;
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          const int e = t + j * kLoaderThreads;
-          const bool in = e < kPieces;
-          xk[j] = in ? load4<D>(kk, r0 + e / V4, e % V4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-          xv[j] = in ? load4<D>(vv, r0 + e / V4, e % V4, S, args.vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        auto put = [&](const float4 (&x)[kMine], uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
-          Split4 sp[kMine];
-#pragma unroll
-          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          for (int j = 0; j < kMine; ++j)
+            x[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
+        };
+        float4 x[kMine];
+        Split4 sp[kMine];
+        auto put = [&](uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
           if (lap > 0 && !mbar_wait(empty, (lap - 1) & 1, abort_flag)) return false;
 #pragma unroll
-          for (int j = 0; j < kMine; ++j) {
-            const int e = t + j * kLoaderThreads;
-            if (e < kPieces) store_split(tile, kPlaneB, e / V4, e % V4, sp[j]);
-          }
+          for (int j = 0; j < kMine; ++j)
+            if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
           fence_proxy_async_smem();
           mbar_arrive(full);
           return true;
         };
-        ok = put(xk, smem + L::kK + s * 3 * kPlaneB, &bars->k_empty[s], &bars->k_full[s]) &&
-             put(xv, smem + L::kV + s * 3 * kPlaneB, &bars->v_empty[s], &bars->v_full[s]);
+        fetch(x, kk);
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+        fetch(x, vv);   // on its way while K goes to shared memory
+        if (!(ok = put(smem + L::kK + s * 3 * kPlaneB, &bars->k_empty[s], &bars->k_full[s]))) break;
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+        ok = put(smem + L::kV + s * 3 * kPlaneB, &bars->v_empty[s], &bars->v_full[s]);
         if (++s == kStages) s = 0, ++lap;
       }
     } else if (elect_one()) {
@@ -175,14 +178,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const Fwd
         if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
         if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
-        // planes of 16 keys kk: half kk / 2 of a row's columns, 8 columns of pairs each
+        // the planes of 16 keys kk lie over the 16 columns their scores came from
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
-            const uint32_t in = (kk & 1) * 8;
-            const uint32_t at = product_a(m) == 2 ? tmem + kExtra + (kk >> 1) * 16 + in
-                                                  : tx + (kk >> 1) * 32 + product_a(m) * 16 + in;
+            const uint32_t at = product_a(m) == 2 ? tmem + kExtra + kk * 8 : tx + kk * 16 + product_a(m) * 8;
             mma_ts(tmem + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 2048), idesc_s,
                    (m > 0 || kk > 0) ? 1u : 0u);
           }
@@ -196,20 +197,21 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const Fwd
   } else {
     setmaxnreg_inc<kRegsCompute>();
     // ------------------------------ softmax ------------------------------
-    const int half = warp / 4, quad = warp % 4;
+    const int cg = warp / 4, quad = warp % 4;   // which 16 keys of a step; TMEM lane quadrant
     const int row = quad * 32 + lane;           // query row of the tile = TMEM lane
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     float* part = reinterpret_cast<float*>(smem + L::kMax);
-    // the two warps that share these 32 rows
-    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };
+    // the four warps that share these 32 rows
+    auto rows_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory"); };
     bool ok = true;
     {
-      const float* qq = args.q + base;
+      constexpr int kRowStep = kComputeThreads / V4;
+      const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
+      const float* qq = args.q + base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
 #pragma unroll
-      for (int j = 0; j < kRows * V4 / kComputeThreads; ++j) {
-        const int e = threadIdx.x + j * kComputeThreads;
-        store_split(smem + L::kQ, kPlaneA, e / V4, e % V4, split4(load4<D>(qq, row0 + e / V4, e % V4, S, args.vec_ok)));
-      }
+      for (int j = 0; j < kRows / kRowStep; ++j)
+        store_split(smem + L::kQ, kPlaneA, rt + j * kRowStep, c4,
+                    split4(load4(qq + j * kRowStep * D, row0 + rt + j * kRowStep < S, args.vec_ok)));
       fence_proxy_async_smem();
       mbar_arrive(&bars->q_full);
     }
@@ -222,73 +224,79 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const Fwd
     auto take_sums = [&](int i) -> bool {
       if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
-      tmem_add<NC>(tlane + kSum + half * NC, o);
+      tmem_add<NC>(tlane + kSum + cg * NC, o);
       return true;
     };
 
     for (int i = 0; i < n_it; ++i) {
       if (!(ok = mbar_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
       tc_fence_after_sync();
-      const uint32_t tx = tlane + (i & 1) * 64 + half * 32;
-      const int c0 = i * kStep + half * 32;
-      float p[32];
+      const uint32_t tx = tlane + (i & 1) * 64 + cg * 16;
+      const int c0 = i * kStep + cg * 16;
+      float2 p[8];
       {
-        uint32_t x[32];
-        tmem_ld32(tx, x);
+        uint32_t x[16];
+        tmem_ld<16>(tx, x);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; ++c) p[c] = __uint_as_float(x[c]) * scale;
+        for (int c = 0; c < 8; ++c)
+          p[c] = fmul2(make_float2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1])), make_float2(scale, scale));
       }
       if (i * kStep + kStep - 1 > row0) {   // keys beyond a row's own
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c0 + c > r) p[c] = -FLT_MAX;
-      }
-      float mx0 = p[0], mx1 = p[1];
-#pragma unroll
-      for (int c = 2; c < 32; c += 4) {
-        mx0 = fmax3(mx0, p[c], p[c + 1]);
-        if (c + 2 < 32) mx1 = fmax3(mx1, p[c + 2], p[c + 3]);
-      }
-      float* own = part + (i & 1) * 256;
-      own[half * 128 + row] = fmaxf(mx0, mx1);
-      pair_sync();
-      // every row sees key 0 in step 0: the max of both halves is finite from there on
-      const float m_new = fmaxf(m, fmaxf(own[row], own[128 + row]));
-      const float corr = expf(m - m_new);
-      m = m_new;
-      float sum = 0.f;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        p[c] = p[c] == -FLT_MAX ? 0.f : expf(p[c] - m_new);
-        sum += p[c];
-        if (DROP) {
-          const uint64_t idx = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0 + c;
-          p[c] = philox_keep(args.rng, idx, args.rate) ? p[c] * keep_scale : 0.f;
+        for (int c = 0; c < 16; ++c) {
+          float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
+          if (c0 + c > r) x = -FLT_MAX;
         }
       }
-      l = l * corr + sum;
+      float mx0 = fmaxf(p[0].x, p[0].y), mx1 = fmaxf(p[1].x, p[1].y);
+#pragma unroll
+      for (int c = 2; c < 8; c += 2) {
+        mx0 = fmax3(mx0, p[c].x, p[c].y);
+        mx1 = fmax3(mx1, p[c + 1].x, p[c + 1].y);
+      }
+      float* own = part + (i & 1) * 512;
+      own[cg * 128 + row] = fmaxf(mx0, mx1);
+      rows_sync();
+      // every row sees key 0 in step 0: the max over all columns is finite from there on
+      const float m_new = fmax3(fmaxf(m, own[row]), fmaxf(own[128 + row], own[256 + row]), own[384 + row]);
+      const float corr = exp2_of(make_float2(m - m_new, 0.f)).x;
+      m = m_new;
+      float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        p[c] = exp2_of(fadd2(p[c], make_float2(-m_new, -m_new)));
+        sum = fadd2(sum, p[c]);
+      }
+      if (DROP) {
+        const uint64_t at = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0;
+        const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, 16);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          p[c] = fmul2(p[c], make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f));
+      }
+      l = fmaf(l, corr, sum.x + sum.y);
       if (i > 0) {   // and with it the planes of step i - 1 are free
         if (!(ok = take_sums(i - 1))) break;
 #pragma unroll
         for (int c = 0; c < NC; ++c) o[c] *= corr;
       }
-      tmem_store_split(p, tx, tx + 16, tlane + kExtra + half * 16);
+      tmem_store_split(p, tx, tx + 8, tlane + kExtra + cg * 8);
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(&bars->p_full);
     }
     if (ok && take_sums(n_it - 1)) {
-      float* own = part + (n_it & 1) * 256;
-      own[half * 128 + row] = l;
-      pair_sync();
+      float* own = part + (n_it & 1) * 512;
+      own[cg * 128 + row] = l;
+      rows_sync();
       if (r < S) {
-        const float l_all = own[row] + own[128 + row];
+        const float l_all = (own[row] + own[128 + row]) + (own[256 + row] + own[384 + row]);
         const float inv = 1.0f / l_all;
 #pragma unroll
         for (int c = 0; c < NC; ++c) o[c] *= inv;
-        store_row<NC>(args.out + base + static_cast<size_t>(r) * D + half * NC, o, args.vec_ok);
-        if (half == 0) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
+        store_row<NC>(args.out + base + static_cast<size_t>(r) * D + cg * NC, o, args.vec_ok);
+        if (cg == 0) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
       }
     }
     tc_fence_before_sync();
@@ -321,7 +329,7 @@ int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, co
                       cudaStream_t st) {
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  const FwdArgs a = {out, lse, q, k, v, BH, S, scale, rate, make_philox(seed, offset), unit0, vec_ok, status};
+  const FwdArgs a = {out, lse, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok, status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
   if (D == 32) return drop ? launch<32, true>(a, st) : launch<32, false>(a, st);
