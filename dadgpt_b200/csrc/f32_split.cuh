@@ -133,16 +133,31 @@ __device__ __forceinline__ float2 exp2_of(float2 x) {
   const float2 t = fmul2(x, make_float2(1.4426950408889634f, 1.4426950408889634f));
   return make_float2(ex2(t.x), ex2(t.y));
 }
-template <int N>
-__device__ __forceinline__ void store_row(float* dst, const float (&x)[N], bool vec_ok) {
-  if (vec_ok) {
+// The 128 x D results of a CTA, N columns of a row per compute thread, through shared memory (free by
+// then) to global memory: written straight from the registers, every lane on a row of its own, a
+// warp's store touches 32 lines and the stores of a tile take as long as two of its steps.
+template <int D, int N>
+__device__ __forceinline__ void stage_rows(float* stage, int row, int col, const float (&x)[N]) {
 #pragma unroll
-    for (int c = 0; c < N; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
-  } else {
+  for (int c = 0; c < N; c += 4)
+    *reinterpret_cast<float4*>(stage + row * (D + 4) + col + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+}
+template <int D>
+__device__ __forceinline__ void write_rows(float* __restrict__ dst, const float* stage, int rows, bool vec_ok) {
+  constexpr int V4 = D / 4;
 #pragma unroll
-    for (int c = 0; c < N; ++c) dst[c] = x[c];
+  for (int j = 0; j < kRows * V4 / kComputeThreads; ++j) {
+    const int e = threadIdx.x + j * kComputeThreads, r = e / V4, c = (e % V4) * 4;
+    if (r >= rows) continue;
+    const float4 x = *reinterpret_cast<const float4*>(stage + r * (D + 4) + c);
+    float* p = dst + static_cast<size_t>(r) * D + c;
+    if (vec_ok)
+      *reinterpret_cast<float4*>(p) = x;
+    else
+      p[0] = x.x, p[1] = x.y, p[2] = x.z, p[3] = x.w;
   }
 }
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 9, %0;" ::"n"(kComputeThreads) : "memory"); }
 
 }  // namespace f32tc
 }  // namespace dadattn

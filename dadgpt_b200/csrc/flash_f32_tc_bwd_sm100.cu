@@ -29,16 +29,18 @@ using namespace f32tc;
 
 struct BwdSmem {
   static constexpr int kA1 = 0, kA2 = 3 * kPlaneA;
-  static constexpr int kStage = 6 * kPlaneA;                   // [2 stages][B1, B2][3 planes]
-  static constexpr int kStageBytes = 6 * kPlaneB;
-  static constexpr int kVec = kStage + 2 * kStageBytes;        // [2 stages][lse, delta][64], or [lse, delta][128]
-  static constexpr int kBars = kVec + 1024;
+  // Three stages for B2: X2 of step i + 2 is the first product after the sums of step i and must not
+  // have to wait for a stage that those sums have just released (two stages: 560 clocks a step idle).
+  static constexpr int kB1 = 6 * kPlaneA;                      // [2 stages][3 planes]
+  static constexpr int kB2 = kB1 + 2 * 3 * kPlaneB;            // [3 stages][3 planes]
+  static constexpr int kVec = kB2 + 3 * 3 * kPlaneB;           // [3 stages][lse, delta][64]; dQ items: delta [128]
+  static constexpr int kBars = kVec + 3 * 512;
   static constexpr int kBytes = kBars + 256;
   static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
 };
 struct BwdBars {
   uint64_t a_full, p_full, acc_done;
-  uint64_t b1_full[2], b2_full[2], b1_empty[2], b2_empty[2], x_full[2];
+  uint64_t b1_full[2], b1_empty[2], b2_full[3], b2_empty[3], x_full[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -93,10 +95,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     mbar_init(&bars->acc_done, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->b1_full[s], kLoaderThreads);
-      mbar_init(&bars->b2_full[s], kLoaderThreads);
       mbar_init(&bars->b1_empty[s], 1);
-      mbar_init(&bars->b2_empty[s], 1);
       mbar_init(&bars->x_full[s], 1);
+    }
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&bars->b2_full[s], kLoaderThreads);
+      mbar_init(&bars->b2_empty[s], 1);
     }
     bars->abort_flag = 0;
     fence_mbar_init();
@@ -107,8 +111,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
   }
   // Columns D..63 of the streamed tiles are read by the sums' products (64 columns wide): zeros.
   if (D < 64)
-    for (int i = threadIdx.x; i < 2 * L::kStageBytes / 16; i += kThreads)
-      reinterpret_cast<uint4*>(smem + L::kStage)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < 5 * 3 * kPlaneB / 16; i += kThreads)
+      reinterpret_cast<uint4*>(smem + L::kB1)[i] = make_uint4(0, 0, 0, 0);
   if (D < 64) fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
@@ -131,28 +135,30 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const float* oo = args.out + base + c4 * 4;
       float* vec = reinterpret_cast<float*>(smem + L::kVec);
       bool ok = true;
+      float4 x[kMine];
+      float row_lse = 0.f;
+      auto fetch = [&](float4 (&to)[kMine], const float* m, int i) {
+        const int r = first + i * kStep + rt;
+        m += static_cast<size_t>(r) * D;
+#pragma unroll
+        for (int j = 0; j < kMine; ++j)
+          to[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
+      };
+      fetch(x, b2, 0);
+      int s2 = 0, lap2 = 0;
       for (int i = 0; ok && i < n_it; ++i) {
-        const int s = i & 1, r = first + i * kStep + rt;
-        auto fetch = [&](float4 (&x)[kMine], const float* m) {
-          m += static_cast<size_t>(r) * D;
+        const int s = i & 1;
+        auto put = [&](uint8_t* to, const Split4 (&v)[kMine]) {
 #pragma unroll
           for (int j = 0; j < kMine; ++j)
-            x[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
+            if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, v[j]);
         };
-        uint8_t* tile = smem + L::kStage + s * L::kStageBytes;
-        auto put = [&](uint8_t* to, const Split4 (&x)[kMine]) {
-#pragma unroll
-          for (int j = 0; j < kMine; ++j)
-            if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, x[j]);
-        };
-        float4 x[kMine];
-        float delta[kMine], row_lse = 0.f;
+        float delta[kMine];
         Split4 sp[kMine];
-        fetch(x, b2);
         if (!is_q) {
           float4 xo[kMine];
-          fetch(xo, oo);
-          if (t < kStep && first + i * kStep + t < S) row_lse = __ldg(lse + first + i * kStep + t);
+          fetch(xo, oo, i);
+          row_lse = t < kStep && first + i * kStep + t < S ? __ldg(lse + first + i * kStep + t) : 0.f;
 #pragma unroll
           for (int j = 0; j < kMine; ++j) {
             delta[j] = dot4(x[j], xo[j]);
@@ -162,21 +168,23 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         }
 #pragma unroll
         for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
-        fetch(x, b1);   // on its way while B2 goes to shared memory
-        if (i >= 2 && !(ok = mbar_wait(&bars->b2_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
-        put(tile + 3 * kPlaneB, sp);
+        fetch(x, b1, i);   // on its way while B2 goes to shared memory
+        if (lap2 > 0 && !(ok = mbar_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
+        put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
         if (!is_q) {
-          if (t < kStep) vec[s * 128 + t] = row_lse;
+          if (t < kStep) vec[s2 * 128 + t] = row_lse;
 #pragma unroll
           for (int j = 0; j < kMine; ++j)
-            if (c4 == 0 && rt + j * kRowStep < kStep) vec[s * 128 + 64 + rt + j * kRowStep] = delta[j];
+            if (c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
         }
         fence_proxy_async_smem();
-        mbar_arrive(&bars->b2_full[s]);
+        mbar_arrive(&bars->b2_full[s2]);
+        if (++s2 == 3) s2 = 0, ++lap2;
 #pragma unroll
         for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+        if (i + 1 < n_it) fetch(x, b2, i + 1);
         if (i >= 2 && !(ok = mbar_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
-        put(tile, sp);
+        put(smem + L::kB1 + s * 3 * kPlaneB, sp);
         fence_proxy_async_smem();
         mbar_arrive(&bars->b1_full[s]);
       }
@@ -186,12 +194,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // A from tensor memory, B MN-major
       const SmemDescBase a1 = make_desc_base_sw128(smem_u32(smem + L::kA1), 0);
       const SmemDescBase a2 = make_desc_base_sw128(smem_u32(smem + L::kA2), 0);
-      const SmemDescBase b0 = make_desc_base_sw128(smem_u32(smem + L::kStage), 0);
+      const SmemDescBase b1_0 = make_desc_base_sw128(smem_u32(smem + L::kB1), 0);
+      const SmemDescBase b2_0 = make_desc_base_sw128(smem_u32(smem + L::kB2), 0);
       auto issue_x = [&](int i) -> bool {
         const int s = i & 1;
         const uint32_t par = (i >> 1) & 1, tx = tmem + s * 128;
-        const SmemDescBase b1{b0.lo + s * (L::kStageBytes >> 4), b0.hi};
-        const SmemDescBase b2{b1.lo + (3 * kPlaneB >> 4), b0.hi};
+        const int s2 = i % 3;
+        const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
+        const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
         auto product = [&](uint32_t td, const SmemDescBase& a, const SmemDescBase& b) {
 #pragma unroll
           for (int m = 0; m < 6; ++m)
@@ -200,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
               mma_ss(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
                      idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
         };
-        if (!mbar_wait(&bars->b2_full[s], par, abort_flag)) return false;
+        if (!mbar_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx + 64, a2, b2);
         if (!mbar_wait(&bars->b1_full[s], par, abort_flag)) return false;
@@ -212,8 +222,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       auto issue_sums = [&](int i) -> bool {
         const int s = i & 1;
         const uint32_t tx = tmem + s * 128;
-        const SmemDescBase b1{b0.lo + s * (L::kStageBytes >> 4), b0.hi};
-        const SmemDescBase b2{b1.lo + (3 * kPlaneB >> 4), b0.hi};
+        const int s2 = i % 3;
+        const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
+        const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
         if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 streamed rows kk lie over the 16 columns their scores came from
@@ -227,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
                      (m > 0 || kk > 0) ? 1u : 0u);
             }
         }
-        mma_commit(&bars->b2_empty[s]);
+        mma_commit(&bars->b2_empty[s2]);
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
@@ -257,28 +268,34 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
       const size_t at = base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
       const float *a1 = (is_q ? args.q : args.k) + at, *a2 = (is_q ? args.dout : args.v) + at, *oo = args.out + at;
+      constexpr int kMine = kRows / kRowStep;
+      float4 x1[kMine], x2[kMine], xo[kMine];   // all in flight at once
 #pragma unroll
-      for (int j = 0; j < kRows / kRowStep; ++j) {
+      for (int j = 0; j < kMine; ++j) {
+        const bool in = row0 + rt + j * kRowStep < S;
+        x1[j] = load4(a1 + j * kRowStep * D, in, args.vec_ok);
+        x2[j] = load4(a2 + j * kRowStep * D, in, args.vec_ok);
+        if (is_q) xo[j] = load4(oo + j * kRowStep * D, in, args.vec_ok);
+      }
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) {
         const int r = rt + j * kRowStep;
-        const bool in = row0 + r < S;
-        const float4 x2 = load4(a2 + j * kRowStep * D, in, args.vec_ok);
-        store_split(smem + L::kA1, kPlaneA, r, c4, split4(load4(a1 + j * kRowStep * D, in, args.vec_ok)));
-        store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2));
+        store_split(smem + L::kA1, kPlaneA, r, c4, split4(x1[j]));
+        store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2[j]));
         if (is_q) {
-          float delta = dot4(x2, load4(oo + j * kRowStep * D, in, args.vec_ok));
+          float delta = dot4(x2[j], xo[j]);
 #pragma unroll
           for (int o = V4 / 2; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
-          if (c4 == 0) vec[128 + r] = delta;
+          if (c4 == 0) vec[r] = delta;
         }
       }
       fence_proxy_async_smem();
       mbar_arrive(&bars->a_full);
-      if (is_q) asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory");   // delta of all rows
+      if (is_q) compute_sync();   // delta of all rows
     }
     const int r_own = row0 + row;
-    const bool in_seq = r_own < S;
-    const float own_lse = is_q && in_seq ? __ldg(lse + r_own) : 0.f;
-    const float own_delta = is_q ? vec[128 + row] : 0.f;
+    const float own_lse = is_q && r_own < S ? __ldg(lse + r_own) : 0.f;
+    const float own_delta = is_q ? vec[row] : 0.f;
     const float scale = args.scale;
     const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
     const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
@@ -299,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
       if (!(ok = mbar_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
       // (the row scalars came with B2)
-      if (!is_q && !(ok = mbar_wait(&bars->b2_full[s], (i >> 1) & 1, abort_flag))) break;
+      if (!is_q && !(ok = mbar_wait(&bars->b2_full[i % 3], (i / 3) & 1, abort_flag))) break;
       tc_fence_after_sync();
       const uint32_t tx = tlane + s * 128 + cg * 16;
       float2 p[8], g[8];
@@ -314,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           g[c] = make_float2(__uint_as_float(x2[2 * c]), __uint_as_float(x2[2 * c + 1]));
         }
       }
-      const float2* lse_s = reinterpret_cast<const float2*>(vec + s * 128 + cg * 16);
+      const float2* lse_s = reinterpret_cast<const float2*>(vec + (i % 3) * 128 + cg * 16);
       const float2* delta_s = lse_s + 32;
       // p = exp(s scale - lse)
 #pragma unroll
@@ -357,14 +374,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       tc_fence_before_sync();
       mbar_arrive(&bars->p_full);
     }
-    if (ok && take_sums(n_it - 1) && in_seq) {
-      const size_t at = base + static_cast<size_t>(r_own) * D + cg * NC;
-      if (is_q) {
-        store_row<NC>(args.dq + at, sum2, args.vec_ok);
-      } else {
-        store_row<NC>(args.dv + at, sum1, args.vec_ok);
-        store_row<NC>(args.dk + at, sum2, args.vec_ok);
-      }
+    if (ok && take_sums(n_it - 1)) {
+      // (every product has completed: the stages are free)
+      float* stage = reinterpret_cast<float*>(smem + L::kB1);
+      const size_t at = base + static_cast<size_t>(row0) * D;
+      const int rows = min(kRows, S - row0);
+      stage_rows<D, NC>(stage, row, cg * NC, sum2);
+      if (!is_q) stage_rows<D, NC>(stage + kRows * (D + 4), row, cg * NC, sum1);
+      compute_sync();
+      write_rows<D>((is_q ? args.dq : args.dk) + at, stage, rows, args.vec_ok);
+      if (!is_q) write_rows<D>(args.dv + at, stage + kRows * (D + 4), rows, args.vec_ok);
     }
     tc_fence_before_sync();
   }

@@ -208,10 +208,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       constexpr int kRowStep = kComputeThreads / V4;
       const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
       const float* qq = args.q + base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
+      constexpr int kMine = kRows / kRowStep;
+      float4 x[kMine];   // all in flight at once
 #pragma unroll
-      for (int j = 0; j < kRows / kRowStep; ++j)
-        store_split(smem + L::kQ, kPlaneA, rt + j * kRowStep, c4,
-                    split4(load4(qq + j * kRowStep * D, row0 + rt + j * kRowStep < S, args.vec_ok)));
+      for (int j = 0; j < kMine; ++j) x[j] = load4(qq + j * kRowStep * D, row0 + rt + j * kRowStep < S, args.vec_ok);
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) store_split(smem + L::kQ, kPlaneA, rt + j * kRowStep, c4, split4(x[j]));
       fence_proxy_async_smem();
       mbar_arrive(&bars->q_full);
     }
@@ -290,14 +292,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       float* own = part + (n_it & 1) * 512;
       own[cg * 128 + row] = l;
       rows_sync();
-      if (r < S) {
-        const float l_all = (own[row] + own[128 + row]) + (own[256 + row] + own[384 + row]);
-        const float inv = 1.0f / l_all;
+      const float l_all = (own[row] + own[128 + row]) + (own[256 + row] + own[384 + row]);
+      const float inv = 1.0f / l_all;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) o[c] *= inv;
-        store_row<NC>(args.out + base + static_cast<size_t>(r) * D + cg * NC, o, args.vec_ok);
-        if (cg == 0) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
-      }
+      for (int c = 0; c < NC; ++c) o[c] *= inv;
+      // (every product has completed: the rings are free)
+      float* stage = reinterpret_cast<float*>(smem + L::kK);
+      stage_rows<D, NC>(stage, row, cg * NC, o);
+      if (cg == 0 && r < S) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
+      compute_sync();
+      write_rows<D>(args.out + base + static_cast<size_t>(row0) * D, stage, min(kRows, S - row0), args.vec_ok);
     }
     tc_fence_before_sync();
   }
