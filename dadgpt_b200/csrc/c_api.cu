@@ -45,6 +45,23 @@ int* device_status_word() {
   return g_status[dev];
 }
 
+int optional_status_word(int** word, cudaStream_t st) {
+  int dev = 0;
+  DAD_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < kMaxDevices) {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    if ((*word = g_status[dev])) return DADATTN_OK;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  DAD_CUDA(cudaStreamIsCapturing(st, &capture));
+  if (capture != cudaStreamCaptureStatusNone) {
+    *word = nullptr;
+    return DADATTN_OK;
+  }
+  *word = device_status_word();
+  return *word ? DADATTN_OK : DADATTN_E_CUDA;
+}
+
 int check_launch_registers(const void* kernel, int expected, std::atomic<int>& seen) {
   int regs = seen.load(std::memory_order_relaxed);
   if (regs == 0) {

@@ -35,6 +35,9 @@ int fail(int code, const char* fmt, ...);
 // Device-side sticky status word (one per device that loads the library). Kernels record a
 // DADATTN_E_* code here instead of trapping; dadattn_device_status() reads and clears it.
 int* device_status_word();  // device pointer for the current device, nullptr on failure
+// The same for calls that may be the first on their device inside a stream capture, where the word
+// cannot be allocated: nullptr (such kernels then report nothing) while `st` is capturing.
+int optional_status_word(int** word, cudaStream_t st);
 
 // Kernels whose warpgroups move registers between them (setmaxnreg) budget with the count the CTA is
 // launched with; were the compiler to give the kernel fewer, an increase would wait for registers
@@ -189,8 +192,9 @@ int launch_fwd_bf16_d64(uint16_t* out, float* lse, const uint16_t* q, const uint
 int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
                       float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
                       cudaStream_t st);
-int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* dout, const float* out, const float* lse,
-                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+// delta = rowsum(dO o O), or nullptr: the kernel then forms it from the rows it loads anyway.
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* delta, const float* dout, const float* out,
+                      const float* lse, const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st);
 
 // Launch with programmatic stream serialization: the grid may become resident while its

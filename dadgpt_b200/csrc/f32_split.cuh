@@ -25,12 +25,17 @@ constexpr int kStep = 64;           // rows of the streamed tile per step
 constexpr int kPlaneA = kRows * 128;   // one bf16 plane, 128-byte rows (64 elements), swizzled
 constexpr int kPlaneB = kStep * 128;
 constexpr int kComputeThreads = 512;   // four per row, 16 of a step's 64 columns each
-constexpr int kLoaderThreads = 7 * 32;
-constexpr int kThreads = 768;          // 16 compute warps, 7 loader warps, 1 issuer warp
-constexpr int kWarpLoader0 = 16, kWarpIssuer = 23;
+constexpr int kLoaderThreads = 11 * 32;
+constexpr int kThreads = 896;          // 16 compute warps, 11 loader warps, 1 issuer warp
+constexpr int kWarpLoader0 = 16, kWarpIssuer = 27;
 // Registers per thread once the warpgroups have rebalanced; the pool is what the CTA starts with.
-constexpr int kRegsLaunch = 80, kRegsCompute = 88, kRegsHelper = 64;
-static_assert(kComputeThreads * kRegsCompute + 256 * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
+constexpr int kRegsLaunch = 72, kRegsCompute = 88, kRegsHelper = 48;
+static_assert(kComputeThreads * kRegsCompute + (kThreads - kComputeThreads) * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
+
+// Waits in these kernels: few plain polls before the suspending form. Sixteen compute warps that poll
+// take issue slots from the loaders, which then set the pace.
+constexpr uint32_t kPolls = 16;
+#define tile_wait(bar, parity, abort_flag) mbar_wait_at<kPolls>(bar, parity, abort_flag, __LINE__)
 
 // Plane pairs of the six products, smallest first.
 __device__ __forceinline__ constexpr int product_a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
@@ -45,10 +50,12 @@ __device__ __forceinline__ Split4 split4(float4 x) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     s.p[i] = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
-    x.x -= __uint_as_float(s.p[i].x << 16);
-    x.y -= __uint_as_float(s.p[i].x & 0xffff0000u);
-    x.z -= __uint_as_float(s.p[i].y << 16);
-    x.w -= __uint_as_float(s.p[i].y & 0xffff0000u);
+    const float2 minus = make_float2(-1.f, -1.f);
+    const float2 a = ffma2(make_float2(__uint_as_float(s.p[i].x << 16), __uint_as_float(s.p[i].x & 0xffff0000u)), minus,
+                           make_float2(x.x, x.y));   // exact
+    const float2 b = ffma2(make_float2(__uint_as_float(s.p[i].y << 16), __uint_as_float(s.p[i].y & 0xffff0000u)), minus,
+                           make_float2(x.z, x.w));
+    x = make_float4(a.x, a.y, b.x, b.y);
   }
   return s;
 }

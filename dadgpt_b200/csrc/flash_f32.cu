@@ -1,9 +1,10 @@
 // fp32 fused causal attention, forward and backward: the drop-in for DadGPT's
 // gpu_flash_attention_forward / gpu_flash_attention_backward (reference cuda/attention.cu).
 //
-// Exact fp32 FFMA arithmetic (no tensor cores: the 1e-5 parity bar against the fp32 reference
-// rules out tf32/bf16 products). Where the reference gives one thread a whole query row and a
-// 32-thread block, these kernels tile 64 queries x 64 keys per 256-thread block with 4x4
+// Head sizes 16, 32 and 64 run on the tensor cores with exactly split operands (flash_f32_tc_*.cu).
+// The kernels here are FFMA arithmetic, for head size 128, whose three planes of four resident and
+// streamed tiles do not fit into a CTA's shared memory. Where the reference gives one thread a whole
+// query row and a 32-thread block, they tile 64 queries x 64 keys per 256-thread block with 4x4
 // register micro-tiles, so a tile of K/V is read from shared memory once per 64 rows instead of
 // once per row. Semantics kept from the reference: lse = rowmax + ln(rowsum) of the scaled
 // scores (cuda/attention.cu:71), key c visible to query r iff c <= r (:50), rows >= S never
@@ -20,6 +21,7 @@ namespace {
 constexpr int kTile = 64;      // queries per block and keys per shared-memory tile
 constexpr int kThreads = 256;  // 16 x 16 threads
 constexpr int kPStride = kTile + 4;
+constexpr int kDeltaKernelFrom = 512;   // sequence length from which delta gets a kernel of its own
 
 template <int N>
 __device__ __forceinline__ void load_vec(float (&dst)[N], const float* src) {
@@ -251,6 +253,8 @@ template <int D>
 __global__ void flash_delta_f32_kernel(float* __restrict__ delta, const float* __restrict__ dout,
                                        const float* __restrict__ out, int64_t rows, bool vec_ok) {
   constexpr int L = D / 4;  // lanes per row: 4, 8, 16, 32
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = t / L;
   const int c = static_cast<int>(t % L) * 4;
@@ -475,8 +479,6 @@ int launch_fwd(float* out, float* lse, const float* q, const float* k, const flo
                int S, float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0,
                cudaStream_t st) {
   const bool vec_ok = aligned(out, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
-  if constexpr (D <= 64)
-    return launch_fwd_f32_tc(out, lse, q, k, v, BH, S, D, scale, DROP ? rate : 0.f, seed, offset, unit0, vec_ok, st);
   auto kern = flash_fwd_f32_kernel<D, DROP>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(fwd_smem_bytes<D>())));
@@ -484,6 +486,14 @@ int launch_fwd(float* out, float* lse, const float* q, const float* k, const flo
   kern<<<grid, kThreads, fwd_smem_bytes<D>(), st>>>(out, lse, q, k, v, S, scale, rate,
                                                    make_philox(seed, offset), unit0, vec_ok);
   DAD_LAUNCH_CHECK("flash_fwd_f32_kernel");
+  return DADATTN_OK;
+}
+
+template <int D>
+int launch_delta(float* delta, const float* dout, const float* out, int64_t rows, bool vec_ok, cudaStream_t st) {
+  const int64_t threads = rows * (D / 4);
+  DAD_CUDA(launch_pdl(flash_delta_f32_kernel<D>, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, st,
+                      delta, dout, out, rows, vec_ok));
   return DADATTN_OK;
 }
 
@@ -495,15 +505,7 @@ int launch_bwd(float* dq, float* dk, float* dv, float* delta, const float* dout,
   const bool vec_ok = aligned(dq, 16) && aligned(dk, 16) && aligned(dv, 16) &&
                       aligned(dout, 16) && aligned(out, 16) && aligned(q, 16) &&
                       aligned(k, 16) && aligned(v, 16);
-  if constexpr (D <= 64)
-    return launch_bwd_f32_tc(dq, dk, dv, dout, out, lse, q, k, v, BH, S, D, scale, DROP ? rate : 0.f, seed, offset,
-                             unit0, vec_ok, st);
-  const int64_t rows = static_cast<int64_t>(BH) * S;
-  const int64_t delta_threads = rows * (D / 4);
-  flash_delta_f32_kernel<D><<<static_cast<unsigned>((delta_threads + 255) / 256), 256, 0, st>>>(
-      delta, dout, out, rows, vec_ok);
-  DAD_LAUNCH_CHECK("flash_delta_f32_kernel");
-
+  if (int rc = launch_delta<D>(delta, dout, out, static_cast<int64_t>(BH) * S, vec_ok, st)) return rc;
   const PhiloxKey rng = make_philox(seed, offset);
   dim3 grid((S + kTile - 1) / kTile, BH);
   auto kkv = flash_bwd_dkdv_f32_kernel<D, DROP>;
@@ -550,16 +552,12 @@ extern "C" int dadattn_flash_fwd_f32_dropout(float* out, float* lse, const float
   if (int rc = check_common(BH, S, d_head, rate)) return rc;
   if (!out || !lse || !q || !k || !v) return fail(DADATTN_E_ARG, "null tensor pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define DAD_FWD(DH)                                                                             \
-  case DH:                                                                                      \
-    return rate > 0.f ? launch_fwd<DH, true>(out, lse, q, k, v, BH, S, scale, rate, seed,       \
-                                             offset, unit0, st)                                 \
-                      : launch_fwd<DH, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
-  switch (d_head) {
-    DAD_FWD(16) DAD_FWD(32) DAD_FWD(64) DAD_FWD(128)
+  if (d_head <= 64) {
+    const bool vec_ok = aligned(out, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
+    return launch_fwd_f32_tc(out, lse, q, k, v, BH, S, d_head, scale, rate, seed, offset, unit0, vec_ok, st);
   }
-#undef DAD_FWD
-  return fail(DADATTN_E_UNSUPPORTED, "flash attention: unsupported d_head %d", d_head);
+  return rate > 0.f ? launch_fwd<128, true>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st)
+                    : launch_fwd<128, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
 }
 
 extern "C" int dadattn_flash_fwd_f32(float* out, float* lse, const float* q, const float* k,
@@ -580,17 +578,24 @@ extern "C" int dadattn_flash_bwd_f32_dropout(float* dq, float* dk, float* dv, fl
   if (!dq || !dk || !dv || !delta || !dout || !out || !lse || !q || !k || !v)
     return fail(DADATTN_E_ARG, "null tensor pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define DAD_BWD(DH)                                                                             \
-  case DH:                                                                                      \
-    return rate > 0.f ? launch_bwd<DH, true>(dq, dk, dv, delta, dout, out, lse, q, k, v, BH, S, \
-                                             scale, rate, seed, offset, unit0, st)              \
-                      : launch_bwd<DH, false>(dq, dk, dv, delta, dout, out, lse, q, k, v, BH,   \
-                                              S, scale, 0.f, 0, 0, 0, st);
-  switch (d_head) {
-    DAD_BWD(16) DAD_BWD(32) DAD_BWD(64) DAD_BWD(128)
+  if (d_head <= 64) {
+    const bool vec_ok = aligned(dq, 16) && aligned(dk, 16) && aligned(dv, 16) && aligned(dout, 16) &&
+                        aligned(out, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
+    // Short sequences save a launch (the tensor-core kernel forms delta itself); in long ones the
+    // extra rows would make its loaders the bottleneck (8 x 2048 x 64: 88 us, 102 without the delta
+    // kernel; 96 x 200 x 32: 30.4 us without it, 31.9 with it).
+    const bool own_delta = S < kDeltaKernelFrom;
+    if (!own_delta) {
+      auto* delta_of = d_head == 64 ? launch_delta<64> : d_head == 32 ? launch_delta<32> : launch_delta<16>;
+      if (int rc = delta_of(delta, dout, out, static_cast<int64_t>(BH) * S, vec_ok, st)) return rc;
+    }
+    return launch_bwd_f32_tc(dq, dk, dv, own_delta ? nullptr : delta, dout, out, lse, q, k, v, BH, S, d_head, scale,
+                             rate, seed, offset, unit0, vec_ok, st);
   }
-#undef DAD_BWD
-  return fail(DADATTN_E_UNSUPPORTED, "flash attention: unsupported d_head %d", d_head);
+  return rate > 0.f ? launch_bwd<128, true>(dq, dk, dv, delta, dout, out, lse, q, k, v, BH, S, scale, rate, seed,
+                                            offset, unit0, st)
+                    : launch_bwd<128, false>(dq, dk, dv, delta, dout, out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0,
+                                             st);
 }
 
 extern "C" int dadattn_flash_bwd_f32(float* dq, float* dk, float* dv, float* delta,

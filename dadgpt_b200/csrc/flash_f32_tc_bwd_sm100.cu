@@ -11,9 +11,9 @@
 //   warps 0-15  four threads per row, 16 columns each: p = exp(s scale - lse), ds = p (dP - delta)
 //               scale, both split into planes and written back to tensor memory, from where the
 //               sums take them as A operands; the sums of each step are added to fp32 registers
-//   warps 16-22 fetch the next step's fp32 rows, split them in registers, and put them into the
+//   warps 16-26 fetch the next step's fp32 rows, split them in registers, and put them into the
 //               shared-memory stage the moment it is released; delta = rowsum(dO o O) on the way
-//   warp 23     issues the products. Order on the tensor pipe: sums of step i, X2 then X1 of step
+//   warp 27     issues the products. Order on the tensor pipe: sums of step i, X2 then X1 of step
 //               i + 2 (B2's stage is released before B1's, so its refill hides behind the sums'
 //               last products), sums of step i + 1, ...
 // A step costs 2304 (X) + 2304 (dK/dV) or 1152 (dQ) clocks of tensor pipe at head size 64 (48 for a
@@ -48,7 +48,7 @@ static_assert(sizeof(BwdBars) <= 256, "barrier block");
 
 struct BwdArgs {
   float *dq, *dk, *dv;
-  const float *dout, *out, *lse, *q, *k, *v;
+  const float *dout, *out, *lse, *delta, *q, *k, *v;   // delta: null, or computed by an earlier kernel
   int BH, S;
   float scale, rate;
   PhiloxRounds rng;
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
   const int S = args.S;
 
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
-    if (threadIdx.x == 0) atomicExch(args.status, DADATTN_E_CUDA);
+    if (threadIdx.x == 0 && args.status) atomicExch(args.status, DADATTN_E_CUDA);
     return;
   }
   // Items in order of their number of steps, the longest first: level i holds the key tiles i and
@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
   const int n_it = (last - first + kStep - 1) / kStep;
   const size_t base = static_cast<size_t>(bh) * S * D;
   const float* lse = args.lse + static_cast<size_t>(bh) * S;
+  const float* pre_delta = args.delta ? args.delta + static_cast<size_t>(bh) * S : nullptr;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->a_full, kComputeThreads);
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       float* vec = reinterpret_cast<float*>(smem + L::kVec);
       bool ok = true;
       float4 x[kMine];
-      float row_lse = 0.f;
+      float row_lse = 0.f, row_delta = 0.f;
       auto fetch = [&](float4 (&to)[kMine], const float* m, int i) {
         const int r = first + i * kStep + rt;
         m += static_cast<size_t>(r) * D;
@@ -156,9 +157,13 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         float delta[kMine];
         Split4 sp[kMine];
         if (!is_q) {
+          const int rv = first + i * kStep + t;
+          row_lse = t < kStep && rv < S ? __ldg(lse + rv) : 0.f;
+          if (pre_delta) row_delta = t < kStep && rv < S ? pre_delta[rv] : 0.f;
+        }
+        if (!is_q && !pre_delta) {
           float4 xo[kMine];
           fetch(xo, oo, i);
-          row_lse = t < kStep && first + i * kStep + t < S ? __ldg(lse + first + i * kStep + t) : 0.f;
 #pragma unroll
           for (int j = 0; j < kMine; ++j) {
             delta[j] = dot4(x[j], xo[j]);
@@ -169,13 +174,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
         for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
         fetch(x, b1, i);   // on its way while B2 goes to shared memory
-        if (lap2 > 0 && !(ok = mbar_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
+        if (lap2 > 0 && !(ok = tile_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
         put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
         if (!is_q) {
           if (t < kStep) vec[s2 * 128 + t] = row_lse;
+          if (t < kStep && pre_delta) vec[s2 * 128 + 64 + t] = row_delta;
 #pragma unroll
           for (int j = 0; j < kMine; ++j)
-            if (c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
+            if (!pre_delta && c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
         }
         fence_proxy_async_smem();
         mbar_arrive(&bars->b2_full[s2]);
@@ -183,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
         for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
         if (i + 1 < n_it) fetch(x, b2, i + 1);
-        if (i >= 2 && !(ok = mbar_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
+        if (i >= 2 && !(ok = tile_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
         put(smem + L::kB1 + s * 3 * kPlaneB, sp);
         fence_proxy_async_smem();
         mbar_arrive(&bars->b1_full[s]);
@@ -210,10 +216,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
               mma_ss(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
                      idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
         };
-        if (!mbar_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
+        if (!tile_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx + 64, a2, b2);
-        if (!mbar_wait(&bars->b1_full[s], par, abort_flag)) return false;
+        if (!tile_wait(&bars->b1_full[s], par, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx, a1, b1);
         mma_commit(&bars->x_full[s]);
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         const int s2 = i % 3;
         const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
         const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
-        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!tile_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 streamed rows kk lie over the 16 columns their scores came from
         if (!is_q) {
@@ -251,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         mma_commit(&bars->acc_done);
         return true;
       };
-      bool ok = mbar_wait(&bars->a_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
+      bool ok = tile_wait(&bars->a_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
       for (int i = 0; ok && i < n_it; ++i) ok = issue_sums(i) && (i + 2 >= n_it || issue_x(i + 2));
     }
   } else {
@@ -275,14 +281,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         const bool in = row0 + rt + j * kRowStep < S;
         x1[j] = load4(a1 + j * kRowStep * D, in, args.vec_ok);
         x2[j] = load4(a2 + j * kRowStep * D, in, args.vec_ok);
-        if (is_q) xo[j] = load4(oo + j * kRowStep * D, in, args.vec_ok);
+        if (is_q && !pre_delta) xo[j] = load4(oo + j * kRowStep * D, in, args.vec_ok);
       }
 #pragma unroll
       for (int j = 0; j < kMine; ++j) {
         const int r = rt + j * kRowStep;
         store_split(smem + L::kA1, kPlaneA, r, c4, split4(x1[j]));
         store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2[j]));
-        if (is_q) {
+        if (is_q && !pre_delta) {
           float delta = dot4(x2[j], xo[j]);
 #pragma unroll
           for (int o = V4 / 2; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
@@ -295,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     }
     const int r_own = row0 + row;
     const float own_lse = is_q && r_own < S ? __ldg(lse + r_own) : 0.f;
-    const float own_delta = is_q ? vec[row] : 0.f;
+    const float own_delta = !is_q ? 0.f : !pre_delta ? vec[row] : r_own < S ? pre_delta[r_own] : 0.f;
     const float scale = args.scale;
     const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
     const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
@@ -304,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
     for (int c = 0; c < NC; ++c) sum1[c] = sum2[c] = 0.f;
     auto take_sums = [&](int i) -> bool {
-      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       if (!is_q) tmem_add<NC>(tlane + kSum1 + cg * NC, sum1);
       tmem_add<NC>(tlane + kSum2 + cg * NC, sum2);
@@ -314,9 +320,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     for (int i = 0; i < n_it; ++i) {
       const int s = i & 1;
       const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
-      if (!(ok = mbar_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
+      if (!(ok = tile_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
       // (the row scalars came with B2)
-      if (!is_q && !(ok = mbar_wait(&bars->b2_full[i % 3], (i / 3) & 1, abort_flag))) break;
+      if (!is_q && !(ok = tile_wait(&bars->b2_full[i % 3], (i / 3) & 1, abort_flag))) break;
       tc_fence_after_sync();
       const uint32_t tx = tlane + s * 128 + cg * 16;
       float2 p[8], g[8];
@@ -353,8 +359,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       // ds = p (dP - delta) scale, with dropout on P and dP alike
       uint32_t keep = 0xffffu;
       if (DROP) {
-        const uint64_t at = is_q ? (unit + r_own) * S + col0 : (unit + col0) * S + r_own;
-        keep = philox_keep_bits<4>(args.rng, at, is_q ? 1u : static_cast<uint32_t>(S), 16);
+        // (draws only for pairs that count: key <= query < S)
+        if (is_q) {
+          keep = philox_keep_bits<2>(args.rng, (unit + r_own) * S + col0, 1u, r_own < S ? min(r_own - col0 + 1, 16) : 0);
+        } else {
+          const int lo = max(r_own - col0, 0), hi = min(S - col0, 16);
+          keep = lo < hi ? philox_keep_bits<2>(args.rng, (unit + col0 + lo) * S + r_own, static_cast<uint32_t>(S), hi - lo) << lo
+                         : 0u;
+        }
       }
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -394,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     tc_fence_after_sync();
     tmem_dealloc(tmem, 512);
   }
-  if (threadIdx.x == 0 && bars->abort_flag) report_timeout(args.status, bars->abort_flag);
+  if (threadIdx.x == 0 && bars->abort_flag && args.status) report_timeout(args.status, bars->abort_flag);
 }
 
 template <int D, bool DROP>
@@ -410,12 +422,12 @@ int launch(const BwdArgs& a, cudaStream_t st) {
 
 }  // namespace
 
-int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* dout, const float* out, const float* lse,
-                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* delta, const float* dout, const float* out,
+                      const float* lse, const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st) {
-  int* status = device_status_word();
-  if (!status) return DADATTN_E_CUDA;
-  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
+  int* status = nullptr;
+  if (int rc = optional_status_word(&status, st)) return rc;
+  const BwdArgs a = {dq, dk, dv, dout, out, lse, delta, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
                      status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);

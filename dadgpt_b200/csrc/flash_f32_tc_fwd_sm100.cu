@@ -7,8 +7,8 @@
 //               shared memory), exponentials, p split into planes and written back to tensor memory
 //               over the scores, from where the P V product takes them as its A operand; each step's
 //               P V is added to an fp32 register sum, so the output is never rescaled in tensor memory
-//   warps 16-22 fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
-//   warp 23     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
+//   warps 16-26 fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
+//   warp 27     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
 // A step costs 2304 clocks of tensor pipe at head size 64 (24 + 24 products of 48) and about 1700
 // issue slots per scheduler.
 // Tensor memory: score buffer b at 64 b, the third planes at 128, P V at 192.
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
   const int S = args.S;
 
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
-    if (threadIdx.x == 0) atomicExch(args.status, DADATTN_E_CUDA);
+    if (threadIdx.x == 0 && args.status) atomicExch(args.status, DADATTN_E_CUDA);
     return;
   }
   // query tiles with the most keys first
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         float4 x[kMine];
         Split4 sp[kMine];
         auto put = [&](uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
-          if (lap > 0 && !mbar_wait(empty, (lap - 1) & 1, abort_flag)) return false;
+          if (lap > 0 && !tile_wait(empty, (lap - 1) & 1, abort_flag)) return false;
 #pragma unroll
           for (int j = 0; j < kMine; ++j)
             if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         const int s = i % kStages;
         const uint32_t tx = tmem + (i & 1) * 64;
         const SmemDescBase kd{k0.lo + s * (3 * kPlaneB >> 4), k0.hi};
-        if (!mbar_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!tile_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int m = 0; m < 6; ++m)
@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         const int s = i % kStages;
         const uint32_t tx = tmem + (i & 1) * 64;
         const SmemDescBase vd{v0.lo + s * (3 * kPlaneB >> 4), v0.hi};
-        if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
-        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!tile_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!tile_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 keys kk lie over the 16 columns their scores came from
 #pragma unroll
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         mma_commit(&bars->acc_done);
         return true;
       };
-      bool ok = mbar_wait(&bars->q_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
+      bool ok = tile_wait(&bars->q_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
       for (int i = 0; ok && i < n_it; ++i) ok = issue_pv(i) && (i + 2 >= n_it || issue_x(i + 2));
     }
   } else {
@@ -224,14 +224,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
 #pragma unroll
     for (int c = 0; c < NC; ++c) o[c] = 0.f;
     auto take_sums = [&](int i) -> bool {
-      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       tmem_add<NC>(tlane + kSum + cg * NC, o);
       return true;
     };
 
     for (int i = 0; i < n_it; ++i) {
-      if (!(ok = mbar_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
+      if (!(ok = tile_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
       tc_fence_after_sync();
       const uint32_t tx = tlane + (i & 1) * 64 + cg * 16;
       const int c0 = i * kStep + cg * 16;
@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       }
       if (DROP) {
         const uint64_t at = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0;
-        const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, 16);
+        // (no draws for keys beyond the row's own nor for rows beyond the sequence)
+        const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, r < S ? min(r - c0 + 1, 16) : 0);
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           p[c] = fmul2(p[c], make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f));
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     tc_fence_after_sync();
     tmem_dealloc(tmem, 256);
   }
-  if (threadIdx.x == 0 && bars->abort_flag) report_timeout(args.status, bars->abort_flag);
+  if (threadIdx.x == 0 && bars->abort_flag && args.status) report_timeout(args.status, bars->abort_flag);
 }
 
 template <int D, bool DROP>
@@ -331,8 +332,8 @@ int launch(const FwdArgs& a, cudaStream_t st) {
 int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
                       float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
                       cudaStream_t st) {
-  int* status = device_status_word();
-  if (!status) return DADATTN_E_CUDA;
+  int* status = nullptr;
+  if (int rc = optional_status_word(&status, st)) return rc;
   const FwdArgs a = {out, lse, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok, status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
