@@ -188,6 +188,16 @@ int launch_fwd_bf16_d64(uint16_t* out, float* lse, const uint16_t* q, const uint
                         uint64_t offset, int64_t unit0, const uint32_t* mask_bits, int heads,
                         cudaStream_t st);
 
+// Whether the calling thread's backward is the single-pass one (dadattn_set_bwd_deterministic).
+bool bwd_single_pass();
+
+// bf16 operands, fp32 results (flash_f32_via_bf16.cu), head size 64.
+int launch_fwd_bf16_d64_f32(float* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v, int BH,
+                            int S, float scale, cudaStream_t st);
+int launch_bwd_fused_d64_f32(float* dq32, float* dk32, float* dv32, const float* delta, int* item_counter,
+                             const uint16_t* dout, const float* lse, const uint16_t* q, const uint16_t* k,
+                             const uint16_t* v, int BH, int S, float scale, cudaStream_t st);
+
 // fp32 tensors on the tensor cores, exact operands (flash_f32_tc_*.cu): head sizes 16, 32, 64.
 int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
                       float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,

@@ -465,6 +465,7 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
 namespace {
 thread_local int g_deterministic = 0;
 }
+bool bwd_single_pass() { return !g_deterministic; }
 }  // namespace dadattn
 
 using namespace dadattn;

@@ -107,6 +107,12 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// TMA store of one [128 rows][32 fp32] panel
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 // TMA store of one [128 rows][64 bf16] swizzled panel from shared memory to (x, row, head, batch)
 // of a tensor in either memory layout (UnitLayout); rows beyond the sequence are dropped.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int x, int y,
@@ -174,8 +180,9 @@ struct ItemFeed {
 };
 
 // DROP: 0 = no dropout, 1 = Philox drawn in the kernel, 2 = keep bits read from `mask_bits`
-// (dadattn_dropout_mask_bits; layout in common.cuh).
-template <int DROP>
+// (dadattn_dropout_mask_bits; layout in common.cuh). F32: dK and dV leave as fp32, through maps like
+// map_dqw, whose tensor is then the caller's own zero-filled fp32 dQ (nothing rounds it afterwards).
+template <int DROP, bool F32>
 __global__ void __launch_bounds__(kFThreads, 1)
 flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -406,11 +413,20 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       ItemFeed feed{bars, abort_flag, 0};
       int cur = feed.fetch(n_items);
       int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
-      int g = 0;
+      int g = 0;   // uses of the dQ staging buffer: one per tile, and with F32 one per item for its dV
       bool ok = true;
       for (int j = 0; ok && cur < n_items; ++j) {
         const Item t = decode_item(cur, BH, n_tiles, group_bh);
         for (int i = 0; ok && i < t.n_it; ++i, ++g) {
+          if (F32 && i + 1 == t.n_it) {
+            if (!(ok = mbar_wait(&bars->dq_staged, g & 1, abort_flag))) break;
+            tma_store_3d(&map_dv, smem + L::kDQ, 0, t.kt * kFT, t.bh);
+            tma_store_3d(&map_dv, smem + L::kDQ + kFPanel, 32, t.kt * kFT, t.bh);
+            bulk_commit();
+            bulk_wait_read0();
+            mbar_arrive(&bars->dq_sent);
+            ++g;
+          }
           if (!(ok = mbar_wait(&bars->dq_staged, g & 1, abort_flag))) break;
           const int q0 = (t.kt + i) * kFT;
           tma_reduce_add_3d(&map_dqw, smem + L::kDQ, 0, q0, t.bh, keep);
@@ -430,9 +446,14 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // The next phase of dkv_staged[j & 1] belongs to item j + 2 and cannot complete
             // before this warp has handed back the staging buffer of item j's last tile.
             if (!(ok = mbar_wait(&bars->dkv_staged[j & 1], (j >> 1) & 1, abort_flag))) break;
-            const int ub = t.bh / heads, uh = t.bh - ub * heads;
-            tma_store_4d(&map_dk, smem + L::kK + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
-            tma_store_4d(&map_dv, smem + L::kV + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
+            if (F32) {   // dK: columns 0-31 in the K buffer, 32-63 in the V buffer
+              tma_store_3d(&map_dk, smem + L::kK + (j & 1) * kFPanel, 0, t.kt * kFT, t.bh);
+              tma_store_3d(&map_dk, smem + L::kV + (j & 1) * kFPanel, 32, t.kt * kFT, t.bh);
+            } else {
+              const int ub = t.bh / heads, uh = t.bh - ub * heads;
+              tma_store_4d(&map_dk, smem + L::kK + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
+              tma_store_4d(&map_dv, smem + L::kV + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
+            }
             bulk_commit();
             bulk_wait_read1();
             mbar_arrive(&bars->dq_sent);
@@ -456,15 +477,43 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     int cur = feed.fetch(n_items);
     int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
     bool ok = true;
-    int g = 0;
+    int g = 0, used = 0;   // tiles; uses of the dQ staging buffer
+    // 64 fp32 accumulator columns -> two swizzled panels [128 rows][32 fp32]
+    auto stage_f32 = [&](uint32_t col, uint8_t* panel0, uint8_t* panel1) {
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[16];
+        tmem_ld16(tlane + col + c * 16, o);
+        tmem_wait_ld();
+        uint8_t* dst = (c < 2 ? panel0 : panel1) + row * 128;
+#pragma unroll
+        for (int c4 = 0; c4 < 4; ++c4)
+          *reinterpret_cast<uint4*>(dst + ((((c & 1) * 4 + c4) ^ (row & 7)) << 4)) =
+              make_uint4(o[4 * c4], o[4 * c4 + 1], o[4 * c4 + 2], o[4 * c4 + 3]);
+      }
+    };
     for (int j = 0; ok && cur < n_items; ++j) {
       const int n_it = decode_item(cur, BH, n_tiles, group_bh).n_it;
-      for (int i = 0; i < n_it; ++i, ++g) {
-        // the staging buffer back from the previous tile's reduce, then this tile's GEMMs
-        if (g > 0 && !(ok = mbar_wait(&bars->dq_sent, (g - 1) & 1, abort_flag))) break;
+      for (int i = 0; i < n_it; ++i, ++g, ++used) {
+        // the staging buffer back from its previous use, then this tile's GEMMs
+        if (used > 0 && !(ok = mbar_wait(&bars->dq_sent, (used - 1) & 1, abort_flag))) break;
         if (!(ok = mbar_wait(&bars->acc_done, g & 1, abort_flag))) break;
         tc_fence_after_sync();
-        if (i + 1 == n_it) {
+        if (F32 && i + 1 == n_it) {
+          // The item is complete: dV through the dQ staging buffer (before this tile's dQ), dK through
+          // the item's own K and V buffers, both as fp32 panels.
+          const int kb = j & 1;
+          stage_f32(kColDV, smem + L::kDQ, smem + L::kDQ + kFPanel);
+          fence_proxy_async_smem();
+          mbar_arrive(&bars->dq_staged);
+          ++used;
+          stage_f32(kColDK, smem + L::kK + kb * kFPanel, smem + L::kV + kb * kFPanel);
+          tc_fence_before_sync();
+          mbar_arrive(&bars->dkv_drained);          // the next item's products may overwrite dV / dK
+          fence_proxy_async_smem();
+          mbar_arrive(&bars->dkv_staged[kb]);
+          if (!(ok = mbar_wait(&bars->dq_sent, (used - 1) & 1, abort_flag))) break;
+        } else if (i + 1 == n_it) {
           // The item is complete: dK / dV, tensor memory -> bf16 rows in the item's own K / V
           // buffers (every GEMM that read them has completed), from where the reducer warp
           // stores them. Sixteen columns at a time; dV is columns [0, 64), dK [64, 128).
@@ -800,6 +849,68 @@ size_t fused_bwd_workspace_bytes(int BH, int S) {
   return delta_bytes + dq_bytes + 256;
 }
 
+// The gradient kernel on bf16 tensors, with delta and the item counter (and a zero-filled dq_ws) ready.
+// f32_dk / f32_dv: fp32 results [BH,S,64] instead of bf16 dk / dv.
+static int launch_fused_kernel(float* dq_ws, uint16_t* dk, uint16_t* dv, float* f32_dk, float* f32_dv, const float* delta,
+                               int* item_counter, const uint16_t* dout, const float* lse, const uint16_t* q,
+                               const uint16_t* k, const uint16_t* v, int BH, int S, const UnitLayout& lay, float scale,
+                               float rate, const PhiloxKey& rng, int64_t unit0, const uint32_t* mask_bits,
+                               cudaStream_t st) {
+  CUtensorMap mq, mk, mv, mdo, mws, mdk, mdv, mlse, mdelta;
+  int lse_shift = 0, delta_shift = 0;   // the workspace is 256-byte aligned: delta needs none
+  if (int rc = make_tensor_map_bf16_units(&mq, q, BH, S, kFD, kFT, lay)) return rc;
+  if (int rc = make_tensor_map_bf16_units(&mk, k, BH, S, kFD, kFT, lay)) return rc;
+  if (int rc = make_tensor_map_bf16_units(&mv, v, BH, S, kFD, kFT, lay)) return rc;
+  if (int rc = make_tensor_map_bf16_units(&mdo, dout, BH, S, kFD, kFT, lay)) return rc;
+  if (f32_dk) {
+    if (int rc = make_dq_workspace_map(&mdk, f32_dk, BH, S)) return rc;
+    if (int rc = make_dq_workspace_map(&mdv, f32_dv, BH, S)) return rc;
+  } else {
+    if (int rc = make_tensor_map_bf16_units(&mdk, dk, BH, S, kFD, kFT, lay)) return rc;
+    if (int rc = make_tensor_map_bf16_units(&mdv, dv, BH, S, kFD, kFT, lay)) return rc;
+  }
+  if (int rc = make_dq_workspace_map(&mws, dq_ws, BH, S)) return rc;
+  // (the kernel indexes the [BH, S] vectors with 32-bit TMA coordinates)
+  if (static_cast<int64_t>(BH) * S > INT32_MAX - 1024)
+    return fail(DADATTN_E_UNSUPPORTED, "BH * S = %lld rows exceed what the fused backward addresses",
+                static_cast<long long>(BH) * S);
+  if (int rc = make_row_scalar_map(&mlse, lse, static_cast<int64_t>(BH) * S, &lse_shift)) return rc;
+  if (int rc = make_row_scalar_map(&mdelta, delta, static_cast<int64_t>(BH) * S, &delta_shift)) return rc;
+  if (delta_shift != 0) return fail(DADATTN_E_ARG, "the backward workspace is not 16-byte aligned");
+  int* status = device_status_word();
+  if (!status) return DADATTN_E_CUDA;
+  // One persistent CTA per SM; the CTAs draw (key tile, batch x head) items from a counter.
+  // Batch x head units are worked on in groups whose Q, dO and dQ rows (1 KiB per query) stay
+  // well inside L2.
+  const int64_t n_items = static_cast<int64_t>((S + kFT - 1) / kFT) * BH;
+  if (n_items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (key tile, batch x head) items");
+  int dev = 0, sms = 0;
+  DAD_CUDA(cudaGetDevice(&dev));
+  DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
+  int group_bh = 65536 / S;
+  group_bh = group_bh < 1 ? 1 : (group_bh > 64 ? 64 : group_bh);
+  const int variant = f32_dk ? 3 : rate > 0.f ? (mask_bits ? 2 : 1) : 0;
+  auto kern = variant == 3 ? flash_bwd_fused_kernel<0, true> : variant == 2 ? flash_bwd_fused_kernel<2, false>
+              : variant == 1 ? flash_bwd_fused_kernel<1, false> : flash_bwd_fused_kernel<0, false>;
+  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem::kBytes));
+  static std::atomic<int> regs_seen[4];
+  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs_seen[variant])) return rc;
+  DAD_CUDA(launch_pdl(kern, grid, dim3(kFThreads), FusedSmem::kBytes, st, mq, mk, mv, mdo, mws, mdk, mdv,
+                      mlse, mdelta, lse_shift, item_counter, BH, S, lay.heads, group_bh, scale, rate,
+                      rng, unit0, mask_bits, status));
+  return DADATTN_OK;
+}
+
+// fp32 results on bf16 operands: dq32 (zero-filled by the caller of this function) collects dQ, delta
+// and the zeroed item counter are ready in the caller's workspace.
+int launch_bwd_fused_d64_f32(float* dq32, float* dk32, float* dv32, const float* delta, int* item_counter,
+                             const uint16_t* dout, const float* lse, const uint16_t* q, const uint16_t* k,
+                             const uint16_t* v, int BH, int S, float scale, cudaStream_t st) {
+  return launch_fused_kernel(dq32, nullptr, nullptr, dk32, dv32, delta, item_counter, dout, lse, q, k, v, BH, S,
+                             unit_layout(BH, 1, S, kFD, false), scale, 0.f, PhiloxKey{}, 0, nullptr, st);
+}
+
 int launch_bwd_fused_d64(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* workspace, const uint16_t* dout,
                          const uint16_t* out, const float* lse, const uint16_t* q, const uint16_t* k,
                          const uint16_t* v, int BH, int S, float scale, float rate, uint64_t seed,
@@ -813,25 +924,6 @@ int launch_bwd_fused_d64(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* workspa
   float* delta = static_cast<float*>(workspace);
   float* dq_ws = reinterpret_cast<float*>(static_cast<char*>(workspace) + delta_bytes);
   int* item_counter = reinterpret_cast<int*>(static_cast<char*>(workspace) + delta_bytes + dq_bytes);
-  CUtensorMap mq, mk, mv, mdo, mws, mdk, mdv, mlse, mdelta;
-  int lse_shift = 0, delta_shift = 0;   // the workspace is 256-byte aligned: delta needs none
-  if (int rc = make_tensor_map_bf16_units(&mq, q, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_tensor_map_bf16_units(&mk, k, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_tensor_map_bf16_units(&mv, v, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_tensor_map_bf16_units(&mdo, dout, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_tensor_map_bf16_units(&mdk, dk, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_tensor_map_bf16_units(&mdv, dv, BH, S, kFD, kFT, lay)) return rc;
-  if (int rc = make_dq_workspace_map(&mws, dq_ws, BH, S)) return rc;
-  // (the kernel indexes the [BH, S] vectors with 32-bit TMA coordinates)
-  if (static_cast<int64_t>(BH) * S > INT32_MAX - 1024)
-    return fail(DADATTN_E_UNSUPPORTED, "BH * S = %lld rows exceed what the fused backward addresses",
-                static_cast<long long>(BH) * S);
-  if (int rc = make_row_scalar_map(&mlse, lse, static_cast<int64_t>(BH) * S, &lse_shift)) return rc;
-  if (int rc = make_row_scalar_map(&mdelta, delta, static_cast<int64_t>(BH) * S, &delta_shift)) return rc;
-  if (delta_shift != 0) return fail(DADATTN_E_ARG, "the backward workspace is not 16-byte aligned");
-  int* status = device_status_word();
-  if (!status) return DADATTN_E_CUDA;
-
   const int64_t rows = static_cast<int64_t>(BH) * S;
   const int64_t prep_threads = rows * (kFD / 8);
   stage_event(0, st);
@@ -840,37 +932,9 @@ int launch_bwd_fused_d64(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* workspa
                       dim3(256), 0, st, delta, dq_ws, item_counter, reinterpret_cast<const BF*>(dout),
                       reinterpret_cast<const BF*>(out), rows, S, lay));
   stage_event(1, st);
-  const PhiloxKey rng = make_philox(seed, offset);
-  // One persistent CTA per SM; the CTAs draw (key tile, batch x head) items from a counter.
-  // Batch x head units are worked on in groups whose Q, dO and dQ rows (1 KiB per query) stay
-  // well inside L2.
-  const int64_t n_items = static_cast<int64_t>((S + kFT - 1) / kFT) * BH;
-  if (n_items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (key tile, batch x head) items");
-  int dev = 0, sms = 0;
-  DAD_CUDA(cudaGetDevice(&dev));
-  DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
-  int group_bh = 65536 / S;
-  group_bh = group_bh < 1 ? 1 : (group_bh > 64 ? 64 : group_bh);
-  auto kern = rate > 0.f ? (mask_bits ? flash_bwd_fused_kernel<2> : flash_bwd_fused_kernel<1>)
-                         : flash_bwd_fused_kernel<0>;
-  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem::kBytes));
-  // The warpgroups' register budgets add up to what a CTA is launched with only if the compiler
-  // gave the kernel kRegsLaunch registers per thread; with fewer, the compute warps' increase
-  // would wait for registers that nobody can give back. Refuse rather than hang.
-  static int regs_seen[3] = {0, 0, 0};   // per kernel variant; the same value for every device
-  int& regs = regs_seen[rate > 0.f ? (mask_bits ? 2 : 1) : 0];
-  if (regs == 0) {
-    cudaFuncAttributes fattr;
-    DAD_CUDA(cudaFuncGetAttributes(&fattr, kern));
-    regs = fattr.numRegs;
-  }
-  if (regs != kRegsLaunch)
-    return fail(DADATTN_E_UNSUPPORTED, "the single-pass backward was compiled with %d registers per thread, "
-                "its register budgets assume %d", regs, kRegsLaunch);
-  DAD_CUDA(launch_pdl(kern, grid, dim3(kFThreads), FusedSmem::kBytes, st, mq, mk, mv, mdo, mws, mdk, mdv,
-                      mlse, mdelta, lse_shift, item_counter, BH, S, lay.heads, group_bh, scale, rate,
-                      rng, unit0, mask_bits, status));
+  if (int rc = launch_fused_kernel(dq_ws, dk, dv, nullptr, nullptr, delta, item_counter, dout, lse, q, k, v, BH, S, lay,
+                                   scale, rate, make_philox(seed, offset), unit0, mask_bits, st))
+    return rc;
   stage_event(2, st);
   const int64_t n8 = rows * kFD / 8;
   DAD_CUDA(launch_pdl(heads > 0 ? fused_convert_kernel<true> : fused_convert_kernel<false>,

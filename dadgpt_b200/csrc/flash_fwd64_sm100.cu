@@ -147,10 +147,11 @@ __device__ __forceinline__ F64Item f64_item(const F64Deal& deal, int k, int BH, 
 }
 
 // DROP: 0 = no dropout, 1 = Philox drawn in the kernel, 2 = keep bits read from `mask_bits`.
-template <int DROP>
+// F32: the output is written as fp32 tensor of bf16 values (heads-split layout only).
+template <int DROP, bool F32>
 __global__ void __launch_bounds__(kFwd64Threads, 1)
 flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                   const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
+                   const __grid_constant__ CUtensorMap map_v, void* __restrict__ out,
                    float* __restrict__ lse, int BH, int S, UnitLayout lay, float scale, float rate,
                    PhiloxKey rng, int64_t unit0, const uint4* __restrict__ mask_bits,
                    int* __restrict__ status, const __grid_constant__ F64Deal deal) {
@@ -500,7 +501,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const float l_tot = s0.y * w0 + s1.y * w1;
       const float f0 = w0 / l_tot, f1 = w1 / l_tot;
       const int ub = it.bh / lay.heads, uh = it.bh - ub * lay.heads;
-      __nv_bfloat16* dst = out + ub * lay.batch + uh * lay.head + r * lay.row + half * 32;
+      const int64_t at = ub * lay.batch + uh * lay.head + r * lay.row + half * 32;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {   // 16 output columns at a time
         uint32_t oa[16], ob[16];
@@ -518,8 +519,18 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               y[e] = __uint_as_float(oa[8 * i + e]) * f0 + __uint_as_float(ob[8 * i + e]) * f1;
-            *reinterpret_cast<uint4*>(dst + c * 16 + i * 8) = make_uint4(
-                pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+            if (F32) {
+              float4* dst = reinterpret_cast<float4*>(static_cast<float*>(out) + at + c * 16 + i * 8);
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {   // rounded to bf16 like every operand, widened again
+                const uint32_t lo = pack_bf16(y[4 * e], y[4 * e + 1]), hi = pack_bf16(y[4 * e + 2], y[4 * e + 3]);
+                dst[e] = make_float4(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u),
+                                     __uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
+              }
+            } else {
+              *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(out) + at + c * 16 + i * 8) = make_uint4(
+                  pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+            }
           }
         }
       }
@@ -578,8 +589,8 @@ const F64Deal& fwd64_deal(int BH, int n_tiles, int G) {
   return d;
 }
 
-template <int DROP>
-int launch_fwd64(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v,
+template <int DROP, bool F32 = false>
+int launch_fwd64(void* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v,
                  int BH, int S, const UnitLayout& lay, float scale, float rate, uint64_t seed,
                  uint64_t offset, int64_t unit0, const uint32_t* mask_bits, cudaStream_t st) {
   CUtensorMap mq, mk, mv;
@@ -594,17 +605,22 @@ int launch_fwd64(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k
   const int n_tiles = (S + kT - 1) / kT;
   const long long n_items = static_cast<long long>(BH) * ((n_tiles + 1) / 2);
   if (n_items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (query tile pair, batch x head) items");
-  auto kern = flash_fwd64_kernel<DROP>;
+  auto kern = flash_fwd64_kernel<DROP, F32>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Smem::kBytes));
   dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
   DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv,
-                      reinterpret_cast<__nv_bfloat16*>(out), lse, BH, S, lay, scale, rate,
-                      make_philox(seed, offset), unit0, reinterpret_cast<const uint4*>(mask_bits), status,
+                      out, lse, BH, S, lay, scale, rate, make_philox(seed, offset), unit0, reinterpret_cast<const uint4*>(mask_bits), status,
                       fwd64_deal(BH, n_tiles, static_cast<int>(grid.x))));
   return DADATTN_OK;
 }
 
 }  // namespace
+
+int launch_fwd_bf16_d64_f32(float* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v, int BH,
+                            int S, float scale, cudaStream_t st) {
+  return launch_fwd64<0, true>(out, lse, q, k, v, BH, S, unit_layout(BH, 1, S, kHD, false), scale, 0.f, 0, 0, 0,
+                               nullptr, st);
+}
 
 // Forward at head size 64. mask_bits != nullptr: keep bits from dadattn_dropout_mask_bits;
 // otherwise rate > 0 draws the Philox mask inside the kernel. heads > 0: q, k, v, out are the
