@@ -122,9 +122,17 @@ struct F64Deal {
   uint16_t item[kDealEntries];
 };
 struct F64Item {
-  int bh, qa, n_a, n_b, n_kv;   // n_b = 0 when the pair's second tile lies beyond the sequence
+  int bh, qa, n_a, n_b, n_kv;   // n_b = 0 when there is nothing for group B
+  // Sequences of one tile (S <= 128): the pair is that tile of units bh and bh + 1. The units share no
+  // K/V: ring tile 0 is group A's, ring tile 1 group B's (off_b). With one unit per item group B would
+  // idle and there would be twice as many items (192 x 128: 10.8 us, now 7.6).
+  int bh_b, off_b;
   bool valid;
 };
+__host__ __device__ inline int f64_items(int BH, int n_tiles) {
+  return n_tiles == 1 ? (BH + 1) / 2 : BH * ((n_tiles + 1) / 2);
+}
+template <bool ONE>   // ONE: sequences of one tile
 __device__ __forceinline__ F64Item f64_item(const F64Deal& deal, int k, int BH, int n_tiles, int n_items) {
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
   int e;
@@ -136,6 +144,15 @@ __device__ __forceinline__ F64Item f64_item(const F64Deal& deal, int k, int BH, 
   }
   F64Item it;
   it.valid = e < n_items;
+  if constexpr (ONE) {
+    it.bh = 2 * e;
+    it.bh_b = it.bh + 1;
+    it.qa = 0;
+    it.n_a = 1;
+    it.n_b = it.off_b = it.bh_b < BH ? 1 : 0;
+    it.n_kv = 1 + it.n_b;
+    return it;
+  }
   const int row = e / BH;
   const int n_pairs = (n_tiles + 1) / 2;
   it.bh = e - row * BH;
@@ -148,7 +165,7 @@ __device__ __forceinline__ F64Item f64_item(const F64Deal& deal, int k, int BH, 
 
 // DROP: 0 = no dropout, 1 = Philox drawn in the kernel, 2 = keep bits read from `mask_bits`.
 // F32: the output is written as fp32 tensor of bf16 values (heads-split layout only).
-template <int DROP, bool F32>
+template <int DROP, bool F32, bool ONE>
 __global__ void __launch_bounds__(kFwd64Threads, 1)
 flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, void* __restrict__ out,
@@ -167,7 +184,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
   const int lane = threadIdx.x % 32;
   const int n_tiles = (S + kT - 1) / kT;
-  const int n_items = BH * ((n_tiles + 1) / 2);
+  const int n_items = f64_items(BH, n_tiles);
 
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
     if (threadIdx.x == 0) atomicExch(status, DADATTN_E_CUDA);
@@ -216,24 +233,26 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       int g = 0;  // K/V tiles loaded so far, over all items
       bool ok = true;
       for (int k = 0; ok; ++k) {
-        const F64Item it = f64_item(deal, k, BH, n_tiles, n_items);
+        const F64Item it = f64_item<ONE>(deal, k, BH, n_tiles, n_items);
         if (!it.valid) break;
         const int qb = k & 1;
         // the Q buffer frees when the last score product of the item before last has completed
         if (k >= 2 && !mbar_wait(&bars->q_empty[qb], ((k >> 1) - 1) & 1, abort_flag)) break;
-        const int ub = it.bh / lay.heads, uh = it.bh - ub * lay.heads;   // (batch, head) of the unit
+        int ub = it.bh / lay.heads, uh = it.bh - ub * lay.heads;   // (batch, head) of the unit
+        const int ub_b = ONE ? it.bh_b / lay.heads : ub, uh_b = ONE ? it.bh_b - ub_b * lay.heads : uh;
         mbar_arrive_expect_tx(&bars->q_full[qb], it.n_b ? 2 * kPanel : kPanel);
         tma_load_4d(smem + L::kQ + (qb * 2 + 0) * kPanel, &map_q, &bars->q_full[qb], 0, it.qa * kT, uh, ub);
         if (it.n_b)
-          tma_load_4d(smem + L::kQ + (qb * 2 + 1) * kPanel, &map_q, &bars->q_full[qb], 0,
-                      (it.qa + 1) * kT, uh, ub);
+          tma_load_4d(smem + L::kQ + (qb * 2 + 1) * kPanel, &map_q, &bars->q_full[qb], 0, (ONE ? 0 : it.qa + 1) * kT, uh_b, ub_b);
         for (int j = 0; j < it.n_kv; ++j, ++g) {
           const int s = g % kKvStages, use = g / kKvStages;
           if (use > 0 && !(ok = mbar_wait(&bars->kv_empty[s], (use - 1) & 1, abort_flag))) break;
+          const int row0 = ONE ? 0 : j * kT;
+          if (ONE && j == 1) ub = ub_b, uh = uh_b;
           mbar_arrive_expect_tx(&bars->k_full[s], kPanel);
-          tma_load_4d(smem + L::kK + s * kPanel, &map_k, &bars->k_full[s], 0, j * kT, uh, ub);
+          tma_load_4d(smem + L::kK + s * kPanel, &map_k, &bars->k_full[s], 0, row0, uh, ub);
           mbar_arrive_expect_tx(&bars->v_full[s], kPanel);
-          tma_load_4d(smem + L::kV + s * kPanel, &map_v, &bars->v_full[s], 0, j * kT, uh, ub);
+          tma_load_4d(smem + L::kV + s * kPanel, &map_v, &bars->v_full[s], 0, row0, uh, ub);
         }
       }
     }
@@ -287,27 +306,29 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         ++n_pv;
         return true;
       };
+      // the group takes part in the item's ring tiles begin_of .. end_of - 1
+      auto begin_of = [&](const F64Item& it) { return ONE && X ? it.off_b : 0; };
+      auto end_of = [&](const F64Item& it) { return X ? (ONE ? it.off_b : 0) + it.n_b : it.n_a; };
       auto n_of = [&](const F64Item& it) { return X ? it.n_b : it.n_a; };
 
-      F64Item cur = f64_item(deal, 0, BH, n_tiles, n_items);
-      F64Item nxt = f64_item(deal, 1, BH, n_tiles, n_items);
+      F64Item cur = f64_item<ONE>(deal, 0, BH, n_tiles, n_items);
+      F64Item nxt = f64_item<ONE>(deal, 1, BH, n_tiles, n_items);
       int g = 0;
       if (cur.valid) {
         ok = mbar_wait(&bars->q_full[0], 0, abort_flag) && mbar_wait(&bars->k_full[0], 0, abort_flag);
         if (ok) {
           tc_fence_after_sync();
-          if (n_of(cur) > 0) {
+          if (n_of(cur) > 0 && begin_of(cur) == 0) {
             issue_s(0, 0, 0);
             issue_s(0, 0, 1);
+            if (end_of(cur) == 1) mma_commit(&bars->q_empty[0]);   // the item's only score products of this group
           }
-          if (n_of(cur) <= 1) {   // the item's only (or no) score products of this group
-            if (n_of(cur) == 1) mma_commit(&bars->q_empty[0]); else mbar_arrive(&bars->q_empty[0]);
-          }
+          if (n_of(cur) == 0) mbar_arrive(&bars->q_empty[0]);
         }
       }
       for (int k = 0; ok && cur.valid; ++k) {
         const int qb = k & 1;
-        const int n_x = n_of(cur);
+        const int n_x = n_of(cur), j0 = begin_of(cur), j1 = end_of(cur);
         for (int j = 0; ok && j < cur.n_kv; ++j, ++g) {
           const int s = g % kKvStages;
           // The tile after this one in the ring: the item's next tile, or the next item's first.
@@ -320,18 +341,18 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           // ahead and arrive twice within one phase of a release barrier.
           bool issued = false;
           ok = mbar_wait(&bars->v_full[s], (g / kKvStages) & 1, abort_flag);
-          const int n_next = have_next ? n_of(ni) : 0;
-          const bool s_next = have_next && nj < n_next;   // the group has scores to form in the next tile
+          // the group has scores to form in the next tile
+          const bool s_next = have_next && n_of(ni) > 0 && nj >= begin_of(ni) && nj < end_of(ni);
           bool next_ready = false;
 #pragma unroll
           for (int c = 0; c < 2 && ok; ++c) {
-            if (j < n_x) {
-              ok = issue_pv(g, c, j == 0 && c == 0);
+            if (j >= j0 && j < j1) {
+              ok = issue_pv(g, c, j == j0 && c == 0);
               issued = ok;
             }
             if (ok && s_next) {
               if (!next_ready) {
-                if (last) ok = mbar_wait(&bars->q_full[nqb], ((k + 1) >> 1) & 1, abort_flag);
+                if (nj == begin_of(ni)) ok = mbar_wait(&bars->q_full[nqb], ((last ? k + 1 : k) >> 1) & 1, abort_flag);
                 ok = ok && mbar_wait(&bars->k_full[(g + 1) % kKvStages], ((g + 1) / kKvStages) & 1, abort_flag);
                 if (ok) tc_fence_after_sync();
                 next_ready = true;
@@ -340,11 +361,11 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 issue_s(nqb, g + 1, c);
                 issued = true;
                 // the item's last scores of this group
-                if (c == 1 && nj + 1 == n_next) mma_commit(&bars->q_empty[nqb]);
+                if (c == 1 && nj + 1 == end_of(ni)) mma_commit(&bars->q_empty[nqb]);
               }
             }
           }
-          if (ok && have_next && !s_next && nj == 0) {
+          if (ok && have_next && n_of(ni) == 0 && nj == 0) {
             // the next item has no tile for this group: hand its Q buffer back (once it is loaded)
             if (last) ok = mbar_wait(&bars->q_full[nqb], ((k + 1) >> 1) & 1, abort_flag);
             if (ok) mbar_arrive(&bars->q_empty[nqb]);
@@ -356,7 +377,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         if (n_x > 0) ++n_done;
         cur = nxt;
-        nxt = f64_item(deal, k + 2, BH, n_tiles, n_items);
+        nxt = f64_item<ONE>(deal, k + 2, BH, n_tiles, n_items);
       }
     }
   } else {
@@ -374,23 +395,23 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     bool ok = true;
 
     for (int k = 0; ok; ++k) {
-      const F64Item it = f64_item(deal, k, BH, n_tiles, n_items);
+      const F64Item it = f64_item<ONE>(deal, k, BH, n_tiles, n_items);
       if (!it.valid) break;
       const int n_x = X ? it.n_b : it.n_a;
-      if (n_x == 0) continue;               // the pair's second tile lies beyond the sequence
-      const int qt = it.qa + X;
+      if (n_x == 0) continue;               // nothing for this group
+      const int qt = ONE ? 0 : it.qa + X, bh = ONE && X ? it.bh_b : it.bh;
       float m = -INFINITY;                  // running max of the scaled scores, log2 units
       float2 l2 = make_float2(0.f, 0.f);    // running sum, two interleaved partial sums
       const uint32_t* bits1 = reinterpret_cast<const uint32_t*>(mask_bits);
       uint32_t keep = ~0u, keep_next = ~0u;
-      if (DROP == 2) keep_next = __ldg(bits1 + mask_bits_record(it.bh, qt, 0, row, n_tiles) * 4 + half);
+      if (DROP == 2) keep_next = __ldg(bits1 + mask_bits_record(bh, qt, 0, row, n_tiles) * 4 + half);
 
       for (int v = 0; v < 2 * n_x; ++v, ++t) {
         const int j = v >> 1, c = v & 1;    // K/V tile and its sub-step; c is also the score buffer
         if (DROP == 2) {
           keep = keep_next;   // fetched a sub-step ahead: its latency hides behind this one's work
           if (v + 1 < 2 * n_x)
-            keep_next = __ldg(bits1 + mask_bits_record(it.bh, qt, (v + 1) >> 1, row, n_tiles) * 4 +
+            keep_next = __ldg(bits1 + mask_bits_record(bh, qt, (v + 1) >> 1, row, n_tiles) * 4 +
                               ((v + 1) & 1) * 2 + half);
         }
         if (!(ok = mbar_wait(&bars->s_full[X][c], (t >> 1) & 1, abort_flag))) break;
@@ -465,7 +486,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           }
           if (i & 2) lb = fadd2(lb, p); else la = fadd2(la, p);
           if (DROP == 1) {
-            const uint64_t idx = (static_cast<uint64_t>(unit0 + it.bh) * S + qt * kT + row) * S + j * kT +
+            const uint64_t idx = (static_cast<uint64_t>(unit0 + bh) * S + qt * kT + row) * S + j * kT +
                                  c * 64 + half * 32 + i;
             p.x = (p.x != 0.f && philox_keep(rng, idx, rate)) ? p.x * keep_scale : 0.f;
             p.y = (p.y != 0.f && philox_keep(rng, idx + 1, rate)) ? p.y * keep_scale : 0.f;
@@ -500,7 +521,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const float w1 = (s1.x == -INFINITY) ? 0.f : ex2(s1.x - m_tot);
       const float l_tot = s0.y * w0 + s1.y * w1;
       const float f0 = w0 / l_tot, f1 = w1 / l_tot;
-      const int ub = it.bh / lay.heads, uh = it.bh - ub * lay.heads;
+      const int ub = bh / lay.heads, uh = bh - ub * lay.heads;
       const int64_t at = ub * lay.batch + uh * lay.head + r * lay.row + half * 32;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {   // 16 output columns at a time
@@ -536,7 +557,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
       ++n_item;
       if (r < S) {
-        if (half == 0) lse[static_cast<size_t>(it.bh) * S + r] = (m_tot + log2f(l_tot)) * kLn2;
+        if (half == 0) lse[static_cast<size_t>(bh) * S + r] = (m_tot + log2f(l_tot)) * kLn2;
       }
     }
   }
@@ -566,8 +587,8 @@ const F64Deal& fwd64_deal(int BH, int n_tiles, int G) {
   F64Deal& d = cache.deal;
   d.rows = 0;
   const int n_pairs = (n_tiles + 1) / 2;
-  const long long n_items = static_cast<long long>(BH) * n_pairs;
-  if (n_items > kDealEntries || G <= 0) return d;   // (every item takes an entry: no table could hold them)
+  const long long n_items = f64_items(BH, n_tiles);
+  if (n_tiles == 1 || n_items > kDealEntries || G <= 0) return d;   // (every item takes an entry: no table could hold them)
   std::vector<int> load(G, 0), count(G, 0);
   std::vector<std::vector<uint16_t>> list(G);
   // G is at most a few hundred and the table small: a linear scan for the least loaded CTA
@@ -603,9 +624,9 @@ int launch_fwd64(void* out, float* lse, const uint16_t* q, const uint16_t* k, co
   DAD_CUDA(cudaGetDevice(&dev));
   DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int n_tiles = (S + kT - 1) / kT;
-  const long long n_items = static_cast<long long>(BH) * ((n_tiles + 1) / 2);
-  if (n_items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (query tile pair, batch x head) items");
-  auto kern = flash_fwd64_kernel<DROP, F32>;
+  if (static_cast<long long>(BH) * ((n_tiles + 1) / 2) > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (query tile pair, batch x head) items");
+  const int n_items = f64_items(BH, n_tiles);
+  auto kern = n_tiles == 1 ? flash_fwd64_kernel<DROP, F32, true> : flash_fwd64_kernel<DROP, F32, false>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Smem::kBytes));
   dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
   DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv,
