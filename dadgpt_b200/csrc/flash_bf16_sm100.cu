@@ -153,7 +153,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                       float* __restrict__ lse, int S, float scale, float rate, PhiloxKey rng,
-                      int64_t unit0, int* __restrict__ status) {
+                      int64_t unit0, LeveledGrid order, int* __restrict__ status) {
   using L = FwdSmem<D>;
   constexpr int kPanels = L::kPanels;
   // TMEM columns. D = 64: S [0,128), O_0 [128,192), O_1 [192,256): 256 columns, two CTAs per SM.
@@ -168,8 +168,9 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // heaviest tiles first
-  const int bh = blockIdx.y;
+  int level, bh;
+  if (!leveled_block(order, level, bh)) return;
+  const int qt = (S + kBM - 1) / kBM - 1 - level;   // heaviest tiles first
   const int q0 = qt * kBM;
   const int n_kv = qt + 1;  // causal: key tiles 0..qt
 
@@ -507,10 +508,10 @@ int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t
   auto kern = flash_fwd_bf16_kernel<D, DROP>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 FwdSmem<D>::kBytes));
-  dim3 grid((S + kBM - 1) / kBM, BH);
-  DAD_CUDA(launch_pdl(kern, grid, dim3(kFwdThreads), FwdSmem<D>::kBytes, st, mq, mk, mv,
-                      reinterpret_cast<__nv_bfloat16*>(out), lse, S, scale, rate,
-                      make_philox(seed, offset), unit0, status));
+  const LeveledGrid order = leveled_grid(32768, S, BH);   // (16384 and 65536: 0-4 % slower or the same)
+  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kBM - 1) / kBM), dim3(kFwdThreads), FwdSmem<D>::kBytes, st,
+                      mq, mk, mv, reinterpret_cast<__nv_bfloat16*>(out), lse, S, scale, rate,
+                      make_philox(seed, offset), unit0, order, status));
   return DADATTN_OK;
 }
 

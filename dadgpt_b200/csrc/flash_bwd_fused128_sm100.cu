@@ -43,6 +43,12 @@ constexpr int kGSubPanel = 64 * 128;       // [64 rows][64 bf16] swizzled panel
 constexpr int kGStages = 3;                // streamed-tile ring depth
 constexpr int kGThreads = 19 * 32;
 constexpr int kGCompute = 16 * 32;
+// Up to this many CTAs the key tiles go level by level (leveled_grid) and the delta kernel clears the
+// workspace: 24 x 2048 135 -> 112 us, 24 x 300 21.3 -> 19.0, 96 x 2048 445 -> 429, 24 x 8192 1354 -> 1305.
+// With more waves the order gains nothing and the cleared lines, by then out of L2, are better written by
+// a memset ahead of the reads (192 x 8192, 12288 CTAs: 10.35 ms, against 10.45 in the other form).
+constexpr int kGLeveledBlocks = 2048;
+constexpr int kPrepareThreads = 256;         // of the delta kernel, whose blocks zero a part of one tile
 constexpr int kGDqTileBytes = kGD * kGSub * 4;   // one dQ^T tile, fp32
 constexpr float kGLog2e = 1.4426950408889634f;
 
@@ -99,14 +105,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // c ^ (row & 15): a warp writing one chunk of 32 consecutive rows then spreads over all banks.
 __host__ __device__ __forceinline__ int dq_chunk(int c, int row) { return c ^ (row & 15); }
 
-template <bool DROP>
+template <bool DROP, bool LEVELED>
 __global__ void __launch_bounds__(kGThreads, 1)
 flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                           __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
                           float* __restrict__ dq_ws, const float* __restrict__ lse,
                           const float* __restrict__ delta, int S, float scale, float rate,
-                          PhiloxKey rng, int64_t unit0, int* __restrict__ status) {
+                          PhiloxKey rng, int64_t unit0, LeveledGrid order, int* __restrict__ status) {
   using L = G128Smem;
   constexpr int D = kGD;
   constexpr uint32_t kTmemCols = 512;
@@ -122,9 +128,9 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n_sub = (S + kGSub - 1) / kGSub;
-  const int bh = blockIdx.y;
   // key tile `own` streams the query sub-tiles 2*own .. n_sub-1 (low `own` = most work = first)
-  const int own = static_cast<int>(blockIdx.x);
+  int own = static_cast<int>(blockIdx.x), bh = blockIdx.y;
+  if (LEVELED && !leveled_block(order, own, bh)) return;
   const int first = 2 * own;
   const int n_it = n_sub - first;
   const int k0 = own * kGKeys;
@@ -422,15 +428,22 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
 }
 
 // delta[r] = sum_d dO[r,d] O[r,d] (reference flash_delta_kernel, cuda/attention.cu:76-85): 16
-// lanes per row of 128.
-__global__ void fused128_delta_kernel(float* __restrict__ delta, const __nv_bfloat16* __restrict__ dout,
-                                      const __nv_bfloat16* __restrict__ out, int64_t rows) {
+// lanes per row of 128. With ZERO also zeros into the workspace, 32 bytes per thread (a memset of its
+// own between two kernels costs short calls about 3 us).
+template <bool ZERO>
+__global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __restrict__ dq_ws,
+                                        const __nv_bfloat16* __restrict__ dout,
+                                        const __nv_bfloat16* __restrict__ out, int64_t rows) {
   constexpr int D = kGD, Lr = D / 8;
   pdl_wait();
   pdl_launch_dependents();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = t / Lr;
   const int c = static_cast<int>(t % Lr) * 8;
+  if (ZERO) {
+    float4* zero = reinterpret_cast<float4*>(dq_ws) + static_cast<int64_t>(blockIdx.x) * (2 * kPrepareThreads);
+    zero[threadIdx.x] = zero[threadIdx.x + kPrepareThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float sum = 0.f;
   if (r < rows) {
     const uint4 a = *reinterpret_cast<const uint4*>(dout + r * D + c);
@@ -500,21 +513,24 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
   if (!status) return DADATTN_E_CUDA;
 
   stage_event(0, st);
-  DAD_CUDA(cudaMemsetAsync(dq_ws, 0, static_cast<size_t>(BH) * n_sub * kGDqTileBytes, st));
   const int64_t rows = static_cast<int64_t>(BH) * S;
-  const int64_t threads = rows * (kGD / 8);
-  DAD_CUDA(launch_pdl(fused128_delta_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256),
-                      0, st, delta, reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out),
-                      rows));
+  const dim3 by_unit((S + kGKeys - 1) / kGKeys, BH);
+  const bool leveled = static_cast<int64_t>(by_unit.x) * BH <= kGLeveledBlocks;
+  if (!leveled) DAD_CUDA(cudaMemsetAsync(dq_ws, 0, static_cast<size_t>(BH) * n_sub * kGDqTileBytes, st));
+  const int64_t blocks = static_cast<int64_t>(BH) * n_sub * (kGDqTileBytes / (32 * kPrepareThreads));
+  DAD_CUDA(launch_pdl(leveled ? fused128_prepare_kernel<true> : fused128_prepare_kernel<false>,
+                      dim3(static_cast<unsigned>(blocks)), dim3(kPrepareThreads), 0, st, delta, dq_ws,
+                      reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out), rows));
   stage_event(1, st);
   const PhiloxKey rng = make_philox(seed, offset);
-  dim3 grid((S + kGKeys - 1) / kGKeys, BH);
+  const LeveledGrid order = leveled_grid(32768, S, BH);
   const bool drop = rate > 0.f;
-  auto kern = drop ? flash_bwd_fused128_kernel<true> : flash_bwd_fused128_kernel<false>;
+  auto kern = leveled ? (drop ? flash_bwd_fused128_kernel<true, true> : flash_bwd_fused128_kernel<false, true>)
+                      : (drop ? flash_bwd_fused128_kernel<true, false> : flash_bwd_fused128_kernel<false, false>);
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G128Smem::kBytes));
-  DAD_CUDA(launch_pdl(kern, grid, dim3(kGThreads), G128Smem::kBytes, st, mk, mv, mq, mdo,
-                      reinterpret_cast<BF*>(dk), reinterpret_cast<BF*>(dv), dq_ws, lse,
-                      static_cast<const float*>(delta), S, scale, rate, rng, unit0, status));
+  DAD_CUDA(launch_pdl(kern, leveled ? leveled_blocks(order, by_unit.x) : by_unit, dim3(kGThreads),
+                      G128Smem::kBytes, st, mk, mv, mq, mdo, reinterpret_cast<BF*>(dk),
+                      reinterpret_cast<BF*>(dv), dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
   stage_event(2, st);
   DAD_CUDA(launch_pdl(fused128_convert_kernel, dim3(n_sub, BH), dim3(256), 0, st,
                       reinterpret_cast<BF*>(dq), static_cast<const float*>(dq_ws), S, n_sub));
