@@ -47,6 +47,7 @@
 #include <cuda_bf16.h>
 
 #include <cfloat>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -121,6 +122,9 @@ struct F64Deal {
   int rows;                      // 0: closed-form deal
   uint16_t item[kDealEntries];
 };
+struct F64NoDeal {};   // sequences of one tile: 3 KB less to copy per launch
+template <bool ONE>
+using F64DealOf = std::conditional_t<ONE, F64NoDeal, F64Deal>;
 struct F64Item {
   int bh, qa, n_a, n_b, n_kv;   // n_b = 0 when there is nothing for group B
   // Sequences of one tile (S <= 128): the pair is that tile of units bh and bh + 1. The units share no
@@ -133,14 +137,14 @@ __host__ __device__ inline int f64_items(int BH, int n_tiles) {
   return n_tiles == 1 ? (BH + 1) / 2 : BH * ((n_tiles + 1) / 2);
 }
 template <bool ONE>   // ONE: sequences of one tile
-__device__ __forceinline__ F64Item f64_item(const F64Deal& deal, int k, int BH, int n_tiles, int n_items) {
+__device__ __forceinline__ F64Item f64_item(const F64DealOf<ONE>& deal, int k, int BH, int n_tiles, int n_items) {
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
-  int e;
-  if (deal.rows > 0) {
-    const uint16_t t = k < deal.rows ? deal.item[k * G + c] : kDealNone;
-    e = t == kDealNone ? n_items : t;
-  } else {
-    e = k * G + ((k & 1) ? (G - 1 - c) : c);
+  int e = k * G + ((k & 1) ? (G - 1 - c) : c);
+  if constexpr (!ONE) {
+    if (deal.rows > 0) {
+      const uint16_t t = k < deal.rows ? deal.item[k * G + c] : kDealNone;
+      e = t == kDealNone ? n_items : t;
+    }
   }
   F64Item it;
   it.valid = e < n_items;
@@ -171,7 +175,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                    const __grid_constant__ CUtensorMap map_v, void* __restrict__ out,
                    float* __restrict__ lse, int BH, int S, UnitLayout lay, float scale, float rate,
                    PhiloxKey rng, int64_t unit0, const uint4* __restrict__ mask_bits,
-                   int* __restrict__ status, const __grid_constant__ F64Deal deal) {
+                   int* __restrict__ status, const __grid_constant__ F64DealOf<ONE> deal) {
   using L = F64Smem;
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kColS = 0, kColO = 256;   // score buffer (X,b) at 128 X + 64 b, O_(X,h) at kColO + 64 (2 X + h)
@@ -588,7 +592,7 @@ const F64Deal& fwd64_deal(int BH, int n_tiles, int G) {
   d.rows = 0;
   const int n_pairs = (n_tiles + 1) / 2;
   const long long n_items = f64_items(BH, n_tiles);
-  if (n_tiles == 1 || n_items > kDealEntries || G <= 0) return d;   // (every item takes an entry: no table could hold them)
+  if (n_items > kDealEntries || G <= 0) return d;   // (every item takes an entry: no table could hold them)
   std::vector<int> load(G, 0), count(G, 0);
   std::vector<std::vector<uint16_t>> list(G);
   // G is at most a few hundred and the table small: a linear scan for the least loaded CTA
@@ -626,13 +630,15 @@ int launch_fwd64(void* out, float* lse, const uint16_t* q, const uint16_t* k, co
   const int n_tiles = (S + kT - 1) / kT;
   if (static_cast<long long>(BH) * ((n_tiles + 1) / 2) > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (query tile pair, batch x head) items");
   const int n_items = f64_items(BH, n_tiles);
-  auto kern = n_tiles == 1 ? flash_fwd64_kernel<DROP, F32, true> : flash_fwd64_kernel<DROP, F32, false>;
-  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Smem::kBytes));
-  dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
-  DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv,
-                      out, lse, BH, S, lay, scale, rate, make_philox(seed, offset), unit0, reinterpret_cast<const uint4*>(mask_bits), status,
-                      fwd64_deal(BH, n_tiles, static_cast<int>(grid.x))));
-  return DADATTN_OK;
+  const dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
+  auto launch = [&](auto kern, const auto& deal) -> int {
+    DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Smem::kBytes));
+    DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv, out, lse, BH, S, lay, scale,
+                        rate, make_philox(seed, offset), unit0, reinterpret_cast<const uint4*>(mask_bits), status, deal));
+    return DADATTN_OK;
+  };
+  return n_tiles == 1 ? launch(flash_fwd64_kernel<DROP, F32, true>, F64NoDeal{})
+                      : launch(flash_fwd64_kernel<DROP, F32, false>, fwd64_deal(BH, n_tiles, static_cast<int>(grid.x)));
 }
 
 }  // namespace
