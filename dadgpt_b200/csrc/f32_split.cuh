@@ -164,6 +164,36 @@ __device__ __forceinline__ void write_rows(float* __restrict__ dst, const float*
       p[0] = x.x, p[1] = x.y, p[2] = x.z, p[3] = x.w;
   }
 }
+// N consecutive results per thread (lane = row of the tile) to global memory. Groups of N/4 lanes first
+// exchange their 16-byte pieces, so that a group's lanes write N consecutive floats of one row: written
+// as they are, every lane on a row of its own, a store touches 32 lines and a tile's stores take as
+// long as two of its steps.
+template <int D, int N>
+__device__ __forceinline__ void write_sums(float* __restrict__ dst, int row, int col, float (&x)[N], int rows, bool vec_ok) {
+  constexpr int kPieces = N / 4;
+  const int a = row & (kPieces - 1);
+#pragma unroll
+  for (int b = 1; b < kPieces; b <<= 1)
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i)
+      if (!(i & b))
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float &lo = x[i * 4 + e], &hi = x[(i | b) * 4 + e];
+          const float got = __shfl_xor_sync(0xffffffffu, (a & b) ? lo : hi, b);
+          if (a & b) lo = got; else hi = got;
+        }
+#pragma unroll
+  for (int j = 0; j < kPieces; ++j) {   // piece `a` of row j of the group
+    const int r = row - a + j;
+    if (r >= rows) continue;
+    float* p = dst + static_cast<size_t>(r) * D + col + a * 4;
+    if (vec_ok)
+      *reinterpret_cast<float4*>(p) = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+    else
+      p[0] = x[4 * j], p[1] = x[4 * j + 1], p[2] = x[4 * j + 2], p[3] = x[4 * j + 3];
+  }
+}
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 9, %0;" ::"n"(kComputeThreads) : "memory"); }
 
 }  // namespace f32tc

@@ -18,6 +18,10 @@
 //               last products), sums of step i + 1, ...
 // A step costs 2304 (X) + 2304 (dK/dV) or 1152 (dQ) clocks of tensor pipe at head size 64 (48 for a
 // 128 x 64 x 16 product) and about 1900 issue slots per scheduler of everything else.
+// CTAs are persistent where there are more items than SMs: the streamed rings run on across items, and
+// the next item's resident tiles are fetched and split, and its first products formed, while this one's
+// last sums complete, so an item adds little to its steps (one CTA per item: about 5 us each; 48 x 1024 x
+// 64: 154 -> 142 us, 148 x 512: 158 -> 134, 32 x 301 x 32: 20.0 -> 17.4).
 // Tensor memory: X1 / X2 double buffered (buffer b at 128 b), 64 columns at 256 for the planes that
 // do not fit over the scores they came from, sums at 320 and 384.
 #include "f32_split.cuh"
@@ -33,8 +37,9 @@ struct BwdSmem {
   // have to wait for a stage that those sums have just released (two stages: 560 clocks a step idle).
   static constexpr int kB1 = 6 * kPlaneA;                      // [2 stages][3 planes]
   static constexpr int kB2 = kB1 + 2 * 3 * kPlaneB;            // [3 stages][3 planes]
-  static constexpr int kVec = kB2 + 3 * 3 * kPlaneB;           // [3 stages][lse, delta][64]; dQ items: delta [128]
-  static constexpr int kBars = kVec + 3 * 512;
+  static constexpr int kVec = kB2 + 3 * 3 * kPlaneB;           // [3 stages][lse, delta][64]; dK/dV items
+  static constexpr int kOwn = kVec + 3 * 512;                  // delta of a dQ item's rows, [2 items][128]
+  static constexpr int kBars = kOwn + 2 * 512;
   static constexpr int kBytes = kBars + 256;
   static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
 };
@@ -57,7 +62,33 @@ struct BwdArgs {
   int* status;
 };
 
-template <int D, bool DROP>
+// Items in order of their number of steps, the longest first: level i holds the key tiles i and the
+// query tiles n - 1 - i of every (batch, head). CTA c of G takes the items k G + (k even ? c : G-1-c).
+struct BwdItem {
+  bool valid, is_q;
+  int bh, row0, first, n_it;   // first resident row, first streamed row, steps
+};
+template <bool MANY>
+__device__ __forceinline__ BwdItem bwd_item(int k, int BH, int S) {
+  if (!MANY && k > 0) return BwdItem{};
+  const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
+  const int n_tiles = (S + kRows - 1) / kRows;
+  const int e = k * G + ((k & 1) ? G - 1 - c : c);
+  const int level = e / (2 * BH), in_level = e - level * 2 * BH;
+  BwdItem it;
+  it.valid = level < n_tiles;
+  // (a last tile of at most one step: the level's key tiles have a step less than its query tiles)
+  const bool q_first = (S - 1) % kRows < kStep;
+  it.is_q = (in_level >= BH) != q_first;
+  it.bh = in_level >= BH ? in_level - BH : in_level;
+  it.row0 = (it.is_q ? n_tiles - 1 - level : level) * kRows;
+  it.first = it.is_q ? 0 : it.row0;
+  const int last = it.is_q ? min(it.row0 + kRows, S) : S;
+  it.n_it = (last - it.first + kStep - 1) / kStep;
+  return it;
+}
+
+template <int D, bool DROP, bool MANY>   // MANY: more items than CTAs
 __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __grid_constant__ BwdArgs args) {
   using L = BwdSmem;
   constexpr uint32_t kExtra = 256, kSum1 = 320, kSum2 = 384;   // kSum1: dV; kSum2: dK or dQ
@@ -75,21 +106,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     if (threadIdx.x == 0 && args.status) atomicExch(args.status, DADATTN_E_CUDA);
     return;
   }
-  // Items in order of their number of steps, the longest first: level i holds the key tiles i and
-  // the query tiles n - 1 - i of every (batch, head).
-  const int n_tiles = (S + kRows - 1) / kRows;
-  const int level = static_cast<int>(blockIdx.x) / (2 * args.BH);
-  const int in_level = static_cast<int>(blockIdx.x) - level * 2 * args.BH;
-  const bool is_q = in_level >= args.BH;
-  const int bh = is_q ? in_level - args.BH : in_level;
-  const int row0 = (is_q ? n_tiles - 1 - level : level) * kRows;     // first resident row
-  const int first = is_q ? 0 : row0;                                 // first streamed row
-  const int last = is_q ? min(row0 + kRows, S) : S;
-  const int n_it = (last - first + kStep - 1) / kStep;
-  const size_t base = static_cast<size_t>(bh) * S * D;
-  const float* lse = args.lse + static_cast<size_t>(bh) * S;
-  const float* pre_delta = args.delta ? args.delta + static_cast<size_t>(bh) * S : nullptr;
-
+  const BwdItem item0 = bwd_item<MANY>(0, args.BH, S);   // used when there is one: formed ahead of the dependency wait
   if (threadIdx.x == 0) {
     mbar_init(&bars->a_full, kComputeThreads);
     mbar_init(&bars->p_full, kComputeThreads);
@@ -131,68 +148,75 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       constexpr int kRowStep = kLoaderThreads / V4;
       constexpr int kMine = (kStep + kRowStep - 1) / kRowStep;
       const int rt = t / V4, c4 = t % V4;
-      const float* b1 = (is_q ? args.k : args.q) + base + c4 * 4;
-      const float* b2 = (is_q ? args.v : args.dout) + base + c4 * 4;
-      const float* oo = args.out + base + c4 * 4;
       float* vec = reinterpret_cast<float*>(smem + L::kVec);
       bool ok = true;
       float4 x[kMine];
       float row_lse = 0.f, row_delta = 0.f;
-      auto fetch = [&](float4 (&to)[kMine], const float* m, int i) {
-        const int r = first + i * kStep + rt;
-        m += static_cast<size_t>(r) * D;
+      auto fetch = [&](float4 (&to)[kMine], const float* m, const BwdItem& it, int i) {
+        const int r = it.first + i * kStep + rt;
+        m += (static_cast<size_t>(it.bh) * S + r) * D + c4 * 4;
 #pragma unroll
         for (int j = 0; j < kMine; ++j)
           to[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
       };
-      fetch(x, b2, 0);
-      int s2 = 0, lap2 = 0;
-      for (int i = 0; ok && i < n_it; ++i) {
-        const int s = i & 1;
-        auto put = [&](uint8_t* to, const Split4 (&v)[kMine]) {
+      BwdItem it = MANY ? bwd_item<MANY>(0, args.BH, S) : item0;
+      fetch(x, it.is_q ? args.v : args.dout, it, 0);
+      int s2 = 0, lap2 = 0, g = 0;   // g: steps so far, over all items
+#pragma unroll(MANY ? 1 : 2)
+      for (int n = 0; ok && it.valid && (MANY || n < 1); ++n) {
+        const BwdItem nxt = bwd_item<MANY>(n + 1, args.BH, S);
+        const bool is_q = it.is_q;
+        const size_t unit = static_cast<size_t>(it.bh) * S;
+        for (int i = 0; i < it.n_it; ++i, ++g) {
+          const int s = g & 1;
+          auto put = [&](uint8_t* to, const Split4 (&v)[kMine]) {
 #pragma unroll
-          for (int j = 0; j < kMine; ++j)
-            if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, v[j]);
-        };
-        float delta[kMine];
-        Split4 sp[kMine];
-        if (!is_q) {
-          const int rv = first + i * kStep + t;
-          row_lse = t < kStep && rv < S ? __ldg(lse + rv) : 0.f;
-          if (pre_delta) row_delta = t < kStep && rv < S ? pre_delta[rv] : 0.f;
-        }
-        if (!is_q && !pre_delta) {
-          float4 xo[kMine];
-          fetch(xo, oo, i);
-#pragma unroll
-          for (int j = 0; j < kMine; ++j) {
-            delta[j] = dot4(x[j], xo[j]);
-#pragma unroll
-            for (int o = V4 / 2; o > 0; o >>= 1) delta[j] += __shfl_xor_sync(0xffffffffu, delta[j], o);
+            for (int j = 0; j < kMine; ++j)
+              if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, v[j]);
+          };
+          float delta[kMine];
+          Split4 sp[kMine];
+          if (!is_q) {
+            const int rv = it.first + i * kStep + t;
+            row_lse = t < kStep && rv < S ? __ldg(args.lse + unit + rv) : 0.f;
+            if (args.delta) row_delta = t < kStep && rv < S ? args.delta[unit + rv] : 0.f;
           }
+          if (!is_q && !args.delta) {
+            float4 xo[kMine];
+            fetch(xo, args.out, it, i);
+#pragma unroll
+            for (int j = 0; j < kMine; ++j) {
+              delta[j] = dot4(x[j], xo[j]);
+#pragma unroll
+              for (int o = V4 / 2; o > 0; o >>= 1) delta[j] += __shfl_xor_sync(0xffffffffu, delta[j], o);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          fetch(x, is_q ? args.k : args.q, it, i);   // on its way while B2 goes to shared memory
+          if (lap2 > 0 && !(ok = tile_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
+          put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
+          if (!is_q) {
+            if (t < kStep) vec[s2 * 128 + t] = row_lse;
+            if (t < kStep && args.delta) vec[s2 * 128 + 64 + t] = row_delta;
+#pragma unroll
+            for (int j = 0; j < kMine; ++j)
+              if (!args.delta && c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
+          }
+          fence_proxy_async_smem();
+          mbar_arrive(&bars->b2_full[s2]);
+          if (++s2 == 3) s2 = 0, ++lap2;
+#pragma unroll
+          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          const bool more = i + 1 < it.n_it;
+          if (more || nxt.valid)
+            fetch(x, (more ? is_q : nxt.is_q) ? args.v : args.dout, more ? it : nxt, more ? i + 1 : 0);
+          if (g >= 2 && !(ok = tile_wait(&bars->b1_empty[s], ((g >> 1) - 1) & 1, abort_flag))) break;
+          put(smem + L::kB1 + s * 3 * kPlaneB, sp);
+          fence_proxy_async_smem();
+          mbar_arrive(&bars->b1_full[s]);
         }
-#pragma unroll
-        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
-        fetch(x, b1, i);   // on its way while B2 goes to shared memory
-        if (lap2 > 0 && !(ok = tile_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
-        put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
-        if (!is_q) {
-          if (t < kStep) vec[s2 * 128 + t] = row_lse;
-          if (t < kStep && pre_delta) vec[s2 * 128 + 64 + t] = row_delta;
-#pragma unroll
-          for (int j = 0; j < kMine; ++j)
-            if (!pre_delta && c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
-        }
-        fence_proxy_async_smem();
-        mbar_arrive(&bars->b2_full[s2]);
-        if (++s2 == 3) s2 = 0, ++lap2;
-#pragma unroll
-        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
-        if (i + 1 < n_it) fetch(x, b2, i + 1);
-        if (i >= 2 && !(ok = tile_wait(&bars->b1_empty[s], ((i >> 1) - 1) & 1, abort_flag))) break;
-        put(smem + L::kB1 + s * 3 * kPlaneB, sp);
-        fence_proxy_async_smem();
-        mbar_arrive(&bars->b1_full[s]);
+        it = nxt;
       }
     } else if (elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
@@ -225,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         mma_commit(&bars->x_full[s]);
         return true;
       };
-      auto issue_sums = [&](int i) -> bool {
+      auto issue_sums = [&](int i, bool is_q) -> bool {
         const int s = i & 1;
         const uint32_t tx = tmem + s * 128;
         const int s2 = i % 3;
@@ -257,8 +281,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         mma_commit(&bars->acc_done);
         return true;
       };
-      bool ok = tile_wait(&bars->a_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
-      for (int i = 0; ok && i < n_it; ++i) ok = issue_sums(i) && (i + 2 >= n_it || issue_x(i + 2));
+      bool ok = true;
+      int g = 0;   // steps so far, over all items
+#pragma unroll(MANY ? 1 : 2)
+      for (int n = 0; ok && (MANY || n < 1); ++n) {
+        const BwdItem it = MANY ? bwd_item<MANY>(n, args.BH, S) : item0;
+        if (!it.valid) break;
+        ok = tile_wait(&bars->a_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        for (int i = 0; ok && i < it.n_it; ++i) ok = issue_sums(g + i, it.is_q) && (i + 2 >= it.n_it || issue_x(g + i + 2));
+        g += it.n_it;
+      }
     }
   } else {
     setmaxnreg_inc<kRegsCompute>();
@@ -267,135 +299,175 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     const int row = quad * 32 + lane;           // resident row = TMEM lane
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     float* vec = reinterpret_cast<float*>(smem + L::kVec);
+    const float scale = args.scale;
+    const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
     bool ok = true;
-    {
-      // the resident tiles, split into planes
+    // The resident tiles of item n, split into planes. For every item but the first this happens while
+    // the sums of the item before it are still being formed (its last scores have been seen, so
+    // nothing reads the tiles any more), and the rows come from L2.
+    auto load_resident = [&](const BwdItem& it, int n) {
       constexpr int kRowStep = kComputeThreads / V4;
       const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
-      const size_t at = base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
-      const float *a1 = (is_q ? args.q : args.k) + at, *a2 = (is_q ? args.dout : args.v) + at, *oo = args.out + at;
+      const size_t at = (static_cast<size_t>(it.bh) * S + it.row0 + rt) * D + c4 * 4;
+      const float *a1 = (it.is_q ? args.q : args.k) + at, *a2 = (it.is_q ? args.dout : args.v) + at, *oo = args.out + at;
+      float* own = reinterpret_cast<float*>(smem + L::kOwn) + (n & 1) * kRows;
       constexpr int kMine = kRows / kRowStep;
-      float4 x1[kMine], x2[kMine], xo[kMine];   // all in flight at once
+      float4 x1[kMine], x2[kMine];   // all in flight at once
 #pragma unroll
       for (int j = 0; j < kMine; ++j) {
-        const bool in = row0 + rt + j * kRowStep < S;
+        const bool in = it.row0 + rt + j * kRowStep < S;
         x1[j] = load4(a1 + j * kRowStep * D, in, args.vec_ok);
         x2[j] = load4(a2 + j * kRowStep * D, in, args.vec_ok);
-        if (is_q && !pre_delta) xo[j] = load4(oo + j * kRowStep * D, in, args.vec_ok);
       }
+      const bool form_delta = it.is_q && !args.delta;
+      float4 xo[kMine];
+      auto load_out = [&]() {
 #pragma unroll
-      for (int j = 0; j < kMine; ++j) {
-        const int r = rt + j * kRowStep;
-        store_split(smem + L::kA1, kPlaneA, r, c4, split4(x1[j]));
-        store_split(smem + L::kA2, kPlaneA, r, c4, split4(x2[j]));
-        if (is_q && !pre_delta) {
+        for (int j = 0; j < kMine; ++j) xo[j] = load4(oo + j * kRowStep * D, it.row0 + rt + j * kRowStep < S, args.vec_ok);
+      };
+      if (form_delta && D < 64) load_out();
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) store_split(smem + L::kA1, kPlaneA, rt + j * kRowStep, c4, split4(x1[j]));
+      if (form_delta && D == 64) load_out();   // (into x1's registers)
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) store_split(smem + L::kA2, kPlaneA, rt + j * kRowStep, c4, split4(x2[j]));
+      if (form_delta) {
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
           float delta = dot4(x2[j], xo[j]);
 #pragma unroll
           for (int o = V4 / 2; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
-          if (c4 == 0) vec[r] = delta;
+          if (c4 == 0) own[rt + j * kRowStep] = delta;
         }
       }
       fence_proxy_async_smem();
       mbar_arrive(&bars->a_full);
-      if (is_q) compute_sync();   // delta of all rows
-    }
-    const int r_own = row0 + row;
-    const float own_lse = is_q && r_own < S ? __ldg(lse + r_own) : 0.f;
-    const float own_delta = !is_q ? 0.f : !pre_delta ? vec[row] : r_own < S ? pre_delta[r_own] : 0.f;
-    const float scale = args.scale;
-    const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
-    const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
+    };
+    // Rows of 128 bytes of the item's tiles into L2, a step or more ahead of load_resident.
+    auto prefetch_resident = [&](const BwdItem& it) {
+      const float* a = (threadIdx.x < kComputeThreads / 2 ? (it.is_q ? args.q : args.k) : (it.is_q ? args.dout : args.v)) +
+                       (static_cast<size_t>(it.bh) * S + it.row0) * D;
+      const int at = (threadIdx.x % (kComputeThreads / 2)) * 32;   // 256 lines of 32 floats at head size 64
+      if (at < min(kRows, S - it.row0) * D) asm volatile("prefetch.global.L2 [%0];" ::"l"(a + at));
+    };
 
     float sum1[NC], sum2[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) sum1[c] = sum2[c] = 0.f;
-    auto take_sums = [&](int i) -> bool {
+    auto take_sums = [&](int i, bool is_q) -> bool {
       if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       if (!is_q) tmem_add<NC>(tlane + kSum1 + cg * NC, sum1);
       tmem_add<NC>(tlane + kSum2 + cg * NC, sum2);
       return true;
     };
+    BwdItem it{}, nxt = MANY ? bwd_item<MANY>(0, args.BH, S) : item0;
+    int step = 0;   // over all items
+#pragma unroll(MANY ? 1 : 2)
+    for (int n = 0; MANY || n < 2; ++n) {
+      if (nxt.valid) load_resident(nxt, n);
+      if (n > 0) {   // the results of the item before
+        if (!(ok = take_sums(step - 1, it.is_q))) break;
+        const int rows = min(kRows, S - it.row0);
+        const size_t at = (static_cast<size_t>(it.bh) * S + it.row0) * D;
+        if constexpr (MANY) {
+          write_sums<D, NC>((it.is_q ? args.dq : args.dk) + at, row, cg * NC, sum2, rows, args.vec_ok);
+          if (!it.is_q) write_sums<D, NC>(args.dv + at, row, cg * NC, sum1, rows, args.vec_ok);
+        } else {   // (every product has completed: the stages are free)
+          float* stage = reinterpret_cast<float*>(smem + L::kB1);
+          stage_rows<D, NC>(stage, row, cg * NC, sum2);
+          if (!it.is_q) stage_rows<D, NC>(stage + kRows * (D + 4), row, cg * NC, sum1);
+          compute_sync();
+          write_rows<D>((it.is_q ? args.dq : args.dk) + at, stage, rows, args.vec_ok);
+          if (!it.is_q) write_rows<D>(args.dv + at, stage + kRows * (D + 4), rows, args.vec_ok);
+        }
+      }
+      it = nxt;
+      if (!it.valid) break;
+      nxt = bwd_item<MANY>(n + 1, args.BH, S);
+      const bool is_q = it.is_q;
+      const int row0 = it.row0, first = it.first, n_it = it.n_it, bh = it.bh;
+      if (nxt.valid) prefetch_resident(nxt);
+      if (is_q && !args.delta) compute_sync();   // delta of all rows
+      const int r_own = row0 + row;
+      const size_t at_own = static_cast<size_t>(bh) * S + r_own;
+      const float own_lse = is_q && r_own < S ? __ldg(args.lse + at_own) : 0.f;
+      const float own_delta = !is_q ? 0.f
+                              : !args.delta ? reinterpret_cast<const float*>(smem + L::kOwn)[(n & 1) * kRows + row]
+                              : r_own < S ? args.delta[at_own] : 0.f;
+      const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
 
-    for (int i = 0; i < n_it; ++i) {
-      const int s = i & 1;
-      const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
-      if (!(ok = tile_wait(&bars->x_full[s], (i >> 1) & 1, abort_flag))) break;
-      // (the row scalars came with B2)
-      if (!is_q && !(ok = tile_wait(&bars->b2_full[i % 3], (i / 3) & 1, abort_flag))) break;
-      tc_fence_after_sync();
-      const uint32_t tx = tlane + s * 128 + cg * 16;
-      float2 p[8], g[8];
-      {
-        uint32_t x1[16], x2[16];
-        tmem_ld<16>(tx, x1);
-        tmem_ld<16>(tx + 64, x2);
-        tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < NC; ++c) sum1[c] = sum2[c] = 0.f;
+
+      for (int i = 0; i < n_it; ++i, ++step) {
+        const int s = step & 1;
+        const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
+        if (!(ok = tile_wait(&bars->x_full[s], (step >> 1) & 1, abort_flag))) break;
+        // (the row scalars came with B2)
+        if (!is_q && !(ok = tile_wait(&bars->b2_full[step % 3], (step / 3) & 1, abort_flag))) break;
+        tc_fence_after_sync();
+        const uint32_t tx = tlane + s * 128 + cg * 16;
+        float2 p[8], g[8];
+        {
+          uint32_t x1[16], x2[16];
+          tmem_ld<16>(tx, x1);
+          tmem_ld<16>(tx + 64, x2);
+          tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            p[c] = make_float2(__uint_as_float(x1[2 * c]), __uint_as_float(x1[2 * c + 1]));
+            g[c] = make_float2(__uint_as_float(x2[2 * c]), __uint_as_float(x2[2 * c + 1]));
+          }
+        }
+        const float2* lse_s = reinterpret_cast<const float2*>(vec + (step % 3) * 128 + cg * 16);
+        const float2* delta_s = lse_s + 32;
+        // p = exp(s scale - lse)
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          p[c] = make_float2(__uint_as_float(x1[2 * c]), __uint_as_float(x1[2 * c + 1]));
-          g[c] = make_float2(__uint_as_float(x2[2 * c]), __uint_as_float(x2[2 * c + 1]));
+          const float2 l = is_q ? make_float2(own_lse, own_lse) : lse_s[c];
+          p[c] = exp2_of(ffma2(p[c], make_float2(scale, scale), make_float2(-l.x, -l.y)));
         }
-      }
-      const float2* lse_s = reinterpret_cast<const float2*>(vec + (i % 3) * 128 + cg * 16);
-      const float2* delta_s = lse_s + 32;
-      // p = exp(s scale - lse)
+        // every pair of the step visible (key <= query < S)?
+        const bool whole = is_q ? first + i * kStep + kStep - 1 <= row0
+                                : first + i * kStep >= row0 + kRows - 1 && first + i * kStep + kStep <= S;
+        if (!whole) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float2 l = is_q ? make_float2(own_lse, own_lse) : lse_s[c];
-        p[c] = exp2_of(ffma2(p[c], make_float2(scale, scale), make_float2(-l.x, -l.y)));
-      }
-      // every pair of the step visible (key <= query < S)?
-      const bool whole = is_q ? first + i * kStep + kStep - 1 <= row0
-                              : first + i * kStep >= row0 + kRows - 1 && first + i * kStep + kStep <= S;
-      if (!whole) {
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const int rq = is_q ? r_own : col0 + c, ck = is_q ? col0 + c : r_own;
-          float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
-          if (ck > rq || rq >= S) x = 0.f;
+          for (int c = 0; c < 16; ++c) {
+            const int rq = is_q ? r_own : col0 + c, ck = is_q ? col0 + c : r_own;
+            float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
+            if (ck > rq || rq >= S) x = 0.f;
+          }
         }
-      }
-      // ds = p (dP - delta) scale, with dropout on P and dP alike
-      uint32_t keep = 0xffffu;
-      if (DROP) {
-        // (draws only for pairs that count: key <= query < S)
-        if (is_q) {
-          keep = philox_keep_bits<2>(args.rng, (unit + r_own) * S + col0, 1u, r_own < S ? min(r_own - col0 + 1, 16) : 0);
-        } else {
-          const int lo = max(r_own - col0, 0), hi = min(S - col0, 16);
-          keep = lo < hi ? philox_keep_bits<2>(args.rng, (unit + col0 + lo) * S + r_own, static_cast<uint32_t>(S), hi - lo) << lo
-                         : 0u;
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float2 dl = is_q ? make_float2(own_delta, own_delta) : delta_s[c];
-        const float2 pr = p[c];
+        // ds = p (dP - delta) scale, with dropout on P and dP alike
+        uint32_t keep = 0xffffu;
         if (DROP) {
-          const float2 mk = make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f);
-          p[c] = fmul2(p[c], mk);
-          g[c] = fmul2(g[c], mk);
+          // (draws only for pairs that count: key <= query < S)
+          if (is_q) {
+            keep = philox_keep_bits<2>(args.rng, (unit + r_own) * S + col0, 1u, r_own < S ? min(r_own - col0 + 1, 16) : 0);
+          } else {
+            const int lo = max(r_own - col0, 0), hi = min(S - col0, 16);
+            keep = lo < hi ? philox_keep_bits<2>(args.rng, (unit + col0 + lo) * S + r_own, static_cast<uint32_t>(S), hi - lo) << lo
+                           : 0u;
+          }
         }
-        g[c] = fmul2(fmul2(pr, fadd2(g[c], make_float2(-dl.x, -dl.y))), make_float2(scale, scale));
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float2 dl = is_q ? make_float2(own_delta, own_delta) : delta_s[c];
+          const float2 pr = p[c];
+          if (DROP) {
+            const float2 mk = make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f);
+            p[c] = fmul2(p[c], mk);
+            g[c] = fmul2(g[c], mk);
+          }
+          g[c] = fmul2(fmul2(pr, fadd2(g[c], make_float2(-dl.x, -dl.y))), make_float2(scale, scale));
+        }
+        if (i > 0 && !(ok = take_sums(step - 1, is_q))) break;   // and with it the planes of step i - 1 are free
+        if (!is_q) tmem_store_split(p, tx, tx + 8, tx + 64);
+        tmem_store_split(g, tx + 64 + 8, tlane + kExtra + cg * 16, tlane + kExtra + cg * 16 + 8);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(&bars->p_full);
       }
-      if (i > 0 && !(ok = take_sums(i - 1))) break;   // and with it the planes of step i - 1 are free
-      if (!is_q) tmem_store_split(p, tx, tx + 8, tx + 64);
-      tmem_store_split(g, tx + 64 + 8, tlane + kExtra + cg * 16, tlane + kExtra + cg * 16 + 8);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive(&bars->p_full);
-    }
-    if (ok && take_sums(n_it - 1)) {
-      // (every product has completed: the stages are free)
-      float* stage = reinterpret_cast<float*>(smem + L::kB1);
-      const size_t at = base + static_cast<size_t>(row0) * D;
-      const int rows = min(kRows, S - row0);
-      stage_rows<D, NC>(stage, row, cg * NC, sum2);
-      if (!is_q) stage_rows<D, NC>(stage + kRows * (D + 4), row, cg * NC, sum1);
-      compute_sync();
-      write_rows<D>((is_q ? args.dq : args.dk) + at, stage, rows, args.vec_ok);
-      if (!is_q) write_rows<D>(args.dv + at, stage + kRows * (D + 4), rows, args.vec_ok);
+      if (!ok) break;
     }
     tc_fence_before_sync();
   }
@@ -409,15 +481,25 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
   if (threadIdx.x == 0 && bars->abort_flag && args.status) report_timeout(args.status, bars->abort_flag);
 }
 
-template <int D, bool DROP>
-int launch(const BwdArgs& a, cudaStream_t st) {
-  auto kern = flash_bwd_f32_tc_kernel<D, DROP>;
+template <int D, bool DROP, bool MANY>
+int launch(const BwdArgs& a, unsigned grid, cudaStream_t st) {
+  auto kern = flash_bwd_f32_tc_kernel<D, DROP, MANY>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::kBytes));
   static std::atomic<int> regs{0};
   if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs)) return rc;
-  const long long items = 2LL * a.BH * ((a.S + kRows - 1) / kRows);
-  DAD_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(items)), dim3(kThreads), BwdSmem::kBytes, st, a));
+  DAD_CUDA(launch_pdl(kern, dim3(grid), dim3(kThreads), BwdSmem::kBytes, st, a));
   return DADATTN_OK;
+}
+template <int D, bool DROP>
+int launch(const BwdArgs& a, cudaStream_t st) {
+  const long long items = 2LL * a.BH * ((a.S + kRows - 1) / kRows);
+  int dev = 0, sms = 0;
+  DAD_CUDA(cudaGetDevice(&dev));
+  DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (tile, batch x head) items");
+  // (an item loop that runs once costs the smallest calls 1.3 us of 7)
+  return items <= sms ? launch<D, DROP, false>(a, static_cast<unsigned>(items), st)
+                      : launch<D, DROP, true>(a, static_cast<unsigned>(sms), st);
 }
 
 }  // namespace

@@ -63,3 +63,21 @@ def test_unaligned_tensors_and_repeatability(cuda):
     b = _run(*(x.clone() for x in (q, k, v, dout)), 0.125)
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("rate", [0.0, 0.25])
+@pytest.mark.parametrize("BH,S,D", [(150, 100, 16), (149, 129, 64), (75, 193, 32), (50, 300, 64), (110, 513, 64), (37, 700, 32)])
+def test_several_items_per_cta(cuda, BH, S, D, rate):
+    """More tiles than CTAs, ragged, so that a CTA goes from key tiles to query tiles and back."""
+    g = torch.Generator(device=cuda).manual_seed(S + D)
+    q, k, v, dout = (torch.randn(BH, S, D, device=cuda, generator=g) for _ in range(4))
+    keep, drop = None, {}
+    if rate:
+        drop = {"rate": rate, "seed": 5, "offset": 0, "unit0": 2}
+        keep = torch.empty(BH * S * S, dtype=torch.uint8, device=cuda)
+        dad.dropout_mask(keep, rate, 5, 0, first=2 * S * S)
+        keep = keep.view(BH, S, S)
+    got = _run(q, k, v, dout, D ** -0.5, **drop)
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), got, _reference(q, k, v, dout, D ** -0.5, keep, rate)):
+        err = (a.double() - b).flatten(1).norm(dim=1) / b.flatten(1).norm(dim=1)
+        assert err.max().item() < 3e-6, name
