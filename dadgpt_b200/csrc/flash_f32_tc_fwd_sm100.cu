@@ -50,7 +50,27 @@ struct FwdArgs {
   int* status;
 };
 
-template <int D, bool DROP>
+// Query tiles with the most keys first; CTA c of G takes the items k G + (k even ? c : G-1-c).
+struct FwdItem {
+  bool valid;
+  int bh, row0, n_it;   // first query row, steps
+};
+template <bool MANY>
+__device__ __forceinline__ FwdItem fwd_item(int k, int BH, int S) {
+  if (!MANY && k > 0) return FwdItem{};
+  const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
+  const int n_tiles = (S + kRows - 1) / kRows;
+  const int e = k * G + ((k & 1) ? G - 1 - c : c);
+  const int level = e / BH;
+  FwdItem it;
+  it.valid = level < n_tiles;
+  it.bh = e - level * BH;
+  it.row0 = (n_tiles - 1 - level) * kRows;
+  it.n_it = (min(it.row0 + kRows, S) + kStep - 1) / kStep;
+  return it;
+}
+
+template <int D, bool DROP, bool MANY>   // MANY: more items than CTAs
 __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __grid_constant__ FwdArgs args) {
   using L = FwdSmem;
   constexpr uint32_t kExtra = 128, kSum = 192;
@@ -68,13 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     if (threadIdx.x == 0 && args.status) atomicExch(args.status, DADATTN_E_CUDA);
     return;
   }
-  // query tiles with the most keys first
-  const int n_tiles = (S + kRows - 1) / kRows;
-  const int level = static_cast<int>(blockIdx.x) / args.BH;
-  const int bh = static_cast<int>(blockIdx.x) - level * args.BH;
-  const int row0 = (n_tiles - 1 - level) * kRows;
-  const int n_it = (min(row0 + kRows, S) + kStep - 1) / kStep;
-  const size_t base = static_cast<size_t>(bh) * S * D;
+  const FwdItem item0 = fwd_item<MANY>(0, args.BH, S);   // used when there is one: formed ahead of the dependency wait
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, kComputeThreads);
@@ -116,37 +130,42 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       constexpr int kRowStep = kLoaderThreads / V4;
       constexpr int kMine = (kStep + kRowStep - 1) / kRowStep;
       const int rt = t / V4, c4 = t % V4;
-      const float *kk = args.k + base + c4 * 4, *vv = args.v + base + c4 * 4;
       bool ok = true;
       int s = 0, lap = 0;
-      for (int i = 0; ok && i < n_it; ++i) {
-        const int r = i * kStep + rt;
-        auto fetch = [&](float4 (&x)[kMine], const float* m) {
-          m += static_cast<size_t>(r) * D;
+      for (int n = 0; ok && (MANY || n < 1); ++n) {
+        const FwdItem it = MANY ? fwd_item<MANY>(n, args.BH, S) : item0;
+        if (!it.valid) break;
+        const size_t base = static_cast<size_t>(it.bh) * S * D + c4 * 4;
+        const float *kk = args.k + base, *vv = args.v + base;
+        for (int i = 0; ok && i < it.n_it; ++i) {
+          const int r = i * kStep + rt;
+          auto fetch = [&](float4 (&x)[kMine], const float* m) {
+            m += static_cast<size_t>(r) * D;
 #pragma unroll
-          for (int j = 0; j < kMine; ++j)
-            x[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
-        };
-        float4 x[kMine];
-        Split4 sp[kMine];
-        auto put = [&](uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
-          if (lap > 0 && !tile_wait(empty, (lap - 1) & 1, abort_flag)) return false;
+            for (int j = 0; j < kMine; ++j)
+              x[j] = load4(m + j * kRowStep * D, rt + j * kRowStep < kStep && r + j * kRowStep < S, args.vec_ok);
+          };
+          float4 x[kMine];
+          Split4 sp[kMine];
+          auto put = [&](uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
+            if (lap > 0 && !tile_wait(empty, (lap - 1) & 1, abort_flag)) return false;
 #pragma unroll
-          for (int j = 0; j < kMine; ++j)
-            if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
-          fence_proxy_async_smem();
-          mbar_arrive(full);
-          return true;
-        };
-        fetch(x, kk);
+            for (int j = 0; j < kMine; ++j)
+              if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
+            fence_proxy_async_smem();
+            mbar_arrive(full);
+            return true;
+          };
+          fetch(x, kk);
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
-        fetch(x, vv);   // on its way while K goes to shared memory
-        if (!(ok = put(smem + L::kK + s * 3 * kPlaneB, &bars->k_empty[s], &bars->k_full[s]))) break;
+          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          fetch(x, vv);   // on its way while K goes to shared memory
+          if (!(ok = put(smem + L::kK + s * 3 * kPlaneB, &bars->k_empty[s], &bars->k_full[s]))) break;
 #pragma unroll
-        for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
-        ok = put(smem + L::kV + s * 3 * kPlaneB, &bars->v_empty[s], &bars->v_full[s]);
-        if (++s == kStages) s = 0, ++lap;
+          for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
+          ok = put(smem + L::kV + s * 3 * kPlaneB, &bars->v_empty[s], &bars->v_full[s]);
+          if (++s == kStages) s = 0, ++lap;
+        }
       }
     } else if (elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
@@ -191,8 +210,15 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         mma_commit(&bars->acc_done);
         return true;
       };
-      bool ok = tile_wait(&bars->q_full, 0, abort_flag) && issue_x(0) && (n_it < 2 || issue_x(1));
-      for (int i = 0; ok && i < n_it; ++i) ok = issue_pv(i) && (i + 2 >= n_it || issue_x(i + 2));
+      bool ok = true;
+      int g = 0;   // steps so far, over all items
+      for (int n = 0; ok && (MANY || n < 1); ++n) {
+        const FwdItem it = MANY ? fwd_item<MANY>(n, args.BH, S) : item0;
+        if (!it.valid) break;
+        ok = tile_wait(&bars->q_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        for (int i = 0; ok && i < it.n_it; ++i) ok = issue_pv(g + i) && (i + 2 >= it.n_it || issue_x(g + i + 2));
+        g += it.n_it;
+      }
     }
   } else {
     setmaxnreg_inc<kRegsCompute>();
@@ -204,105 +230,131 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     // the four warps that share these 32 rows
     auto rows_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory"); };
     bool ok = true;
-    {
+    // Q of an item, split into planes: for every item but the first while the last sums of the item
+    // before it are still being formed (its last scores have been seen, so nothing reads Q any more).
+    auto load_resident = [&](const FwdItem& it) {
       constexpr int kRowStep = kComputeThreads / V4;
       const int rt = threadIdx.x / V4, c4 = threadIdx.x % V4;
-      const float* qq = args.q + base + static_cast<size_t>(row0 + rt) * D + c4 * 4;
+      const float* qq = args.q + (static_cast<size_t>(it.bh) * S + it.row0 + rt) * D + c4 * 4;
       constexpr int kMine = kRows / kRowStep;
       float4 x[kMine];   // all in flight at once
 #pragma unroll
-      for (int j = 0; j < kMine; ++j) x[j] = load4(qq + j * kRowStep * D, row0 + rt + j * kRowStep < S, args.vec_ok);
+      for (int j = 0; j < kMine; ++j) x[j] = load4(qq + j * kRowStep * D, it.row0 + rt + j * kRowStep < S, args.vec_ok);
 #pragma unroll
       for (int j = 0; j < kMine; ++j) store_split(smem + L::kQ, kPlaneA, rt + j * kRowStep, c4, split4(x[j]));
       fence_proxy_async_smem();
       mbar_arrive(&bars->q_full);
-    }
-    const int r = row0 + row;
+    };
+    // Q of an item into L2, a step or more ahead of load_resident
+    auto prefetch_resident = [&](const FwdItem& it) {
+      const int at = threadIdx.x * 32;   // 128 bytes per thread
+      if (at < min(kRows, S - it.row0) * D)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(args.q + (static_cast<size_t>(it.bh) * S + it.row0) * D + at));
+    };
     const float scale = args.scale;
     const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
     float m = -FLT_MAX, l = 0.f, o[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) o[c] = 0.f;
     auto take_sums = [&](int i) -> bool {
       if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       tmem_add<NC>(tlane + kSum + cg * NC, o);
       return true;
     };
-
-    for (int i = 0; i < n_it; ++i) {
-      if (!(ok = tile_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
-      tc_fence_after_sync();
-      const uint32_t tx = tlane + (i & 1) * 64 + cg * 16;
-      const int c0 = i * kStep + cg * 16;
-      float2 p[8];
-      {
-        uint32_t x[16];
-        tmem_ld<16>(tx, x);
-        tmem_wait_ld();
+    FwdItem it{}, nxt = MANY ? fwd_item<MANY>(0, args.BH, S) : item0;
+    int step = 0;   // over all items
+#pragma unroll(MANY ? 1 : 2)
+    for (int n = 0; MANY || n < 2; ++n) {
+      if (nxt.valid) load_resident(nxt);
+      if (n > 0) {   // the results of the item before
+        if (!(ok = take_sums(step - 1))) break;
+        float* own = part + ((step + n - 1) & 1) * 512;   // (the buffers of `part` alternate over steps and results)
+        own[cg * 128 + row] = l;
+        rows_sync();
+        const float l_all = (own[row] + own[128 + row]) + (own[256 + row] + own[384 + row]);
+        const float inv = 1.0f / l_all;
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          p[c] = fmul2(make_float2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1])), make_float2(scale, scale));
-      }
-      if (i * kStep + kStep - 1 > row0) {   // keys beyond a row's own
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
-          if (c0 + c > r) x = -FLT_MAX;
+        for (int c = 0; c < NC; ++c) o[c] *= inv;
+        const size_t at = static_cast<size_t>(it.bh) * S + it.row0;
+        const int rows = min(kRows, S - it.row0);
+        if (cg == 0 && row < rows) args.lse[at + row] = m + logf(l_all);
+        if constexpr (MANY) {
+          write_sums<D, NC>(args.out + at * D, row, cg * NC, o, rows, args.vec_ok);
+        } else {   // (every product has completed: the rings are free)
+          float* stage = reinterpret_cast<float*>(smem + L::kK);
+          stage_rows<D, NC>(stage, row, cg * NC, o);
+          compute_sync();
+          write_rows<D>(args.out + at * D, stage, rows, args.vec_ok);
         }
       }
-      float mx0 = fmaxf(p[0].x, p[0].y), mx1 = fmaxf(p[1].x, p[1].y);
+      it = nxt;
+      if (!it.valid) break;
+      nxt = fwd_item<MANY>(n + 1, args.BH, S);
+      if (nxt.valid) prefetch_resident(nxt);
+      const int row0 = it.row0, n_it = it.n_it, bh = it.bh, r = row0 + row;
+      m = -FLT_MAX, l = 0.f;
 #pragma unroll
-      for (int c = 2; c < 8; c += 2) {
-        mx0 = fmax3(mx0, p[c].x, p[c].y);
-        mx1 = fmax3(mx1, p[c + 1].x, p[c + 1].y);
+      for (int c = 0; c < NC; ++c) o[c] = 0.f;
+
+      for (int i = 0; i < n_it; ++i, ++step) {
+        if (!(ok = tile_wait(&bars->x_full[step & 1], (step >> 1) & 1, abort_flag))) break;
+        tc_fence_after_sync();
+        const uint32_t tx = tlane + (step & 1) * 64 + cg * 16;
+        const int c0 = i * kStep + cg * 16;
+        float2 p[8];
+        {
+          uint32_t x[16];
+          tmem_ld<16>(tx, x);
+          tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            p[c] = fmul2(make_float2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1])), make_float2(scale, scale));
+        }
+        if (i * kStep + kStep - 1 > row0) {   // keys beyond a row's own
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            float& x = (c & 1) ? p[c / 2].y : p[c / 2].x;
+            if (c0 + c > r) x = -FLT_MAX;
+          }
+        }
+        float mx0 = fmaxf(p[0].x, p[0].y), mx1 = fmaxf(p[1].x, p[1].y);
+#pragma unroll
+        for (int c = 2; c < 8; c += 2) {
+          mx0 = fmax3(mx0, p[c].x, p[c].y);
+          mx1 = fmax3(mx1, p[c + 1].x, p[c + 1].y);
+        }
+        float* own = part + ((step + n) & 1) * 512;
+        own[cg * 128 + row] = fmaxf(mx0, mx1);
+        rows_sync();
+        // every row sees key 0 in step 0: the max over all columns is finite from there on
+        const float m_new = fmax3(fmaxf(m, own[row]), fmaxf(own[128 + row], own[256 + row]), own[384 + row]);
+        const float corr = exp2_of(make_float2(m - m_new, 0.f)).x;
+        m = m_new;
+        float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          p[c] = exp2_of(fadd2(p[c], make_float2(-m_new, -m_new)));
+          sum = fadd2(sum, p[c]);
+        }
+        if (DROP) {
+          const uint64_t at = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0;
+          // (no draws for keys beyond the row's own nor for rows beyond the sequence)
+          const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, r < S ? min(r - c0 + 1, 16) : 0);
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            p[c] = fmul2(p[c], make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f));
+        }
+        l = fmaf(l, corr, sum.x + sum.y);
+        if (i > 0) {   // and with it the planes of step i - 1 are free
+          if (!(ok = take_sums(step - 1))) break;
+#pragma unroll
+          for (int c = 0; c < NC; ++c) o[c] *= corr;
+        }
+        tmem_store_split(p, tx, tx + 8, tlane + kExtra + cg * 8);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(&bars->p_full);
       }
-      float* own = part + (i & 1) * 512;
-      own[cg * 128 + row] = fmaxf(mx0, mx1);
-      rows_sync();
-      // every row sees key 0 in step 0: the max over all columns is finite from there on
-      const float m_new = fmax3(fmaxf(m, own[row]), fmaxf(own[128 + row], own[256 + row]), own[384 + row]);
-      const float corr = exp2_of(make_float2(m - m_new, 0.f)).x;
-      m = m_new;
-      float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        p[c] = exp2_of(fadd2(p[c], make_float2(-m_new, -m_new)));
-        sum = fadd2(sum, p[c]);
-      }
-      if (DROP) {
-        const uint64_t at = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0;
-        // (no draws for keys beyond the row's own nor for rows beyond the sequence)
-        const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, r < S ? min(r - c0 + 1, 16) : 0);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          p[c] = fmul2(p[c], make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f));
-      }
-      l = fmaf(l, corr, sum.x + sum.y);
-      if (i > 0) {   // and with it the planes of step i - 1 are free
-        if (!(ok = take_sums(i - 1))) break;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) o[c] *= corr;
-      }
-      tmem_store_split(p, tx, tx + 8, tlane + kExtra + cg * 8);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive(&bars->p_full);
-    }
-    if (ok && take_sums(n_it - 1)) {
-      float* own = part + (n_it & 1) * 512;
-      own[cg * 128 + row] = l;
-      rows_sync();
-      const float l_all = (own[row] + own[128 + row]) + (own[256 + row] + own[384 + row]);
-      const float inv = 1.0f / l_all;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) o[c] *= inv;
-      // (every product has completed: the rings are free)
-      float* stage = reinterpret_cast<float*>(smem + L::kK);
-      stage_rows<D, NC>(stage, row, cg * NC, o);
-      if (cg == 0 && r < S) args.lse[static_cast<size_t>(bh) * S + r] = m + logf(l_all);
-      compute_sync();
-      write_rows<D>(args.out + base + static_cast<size_t>(row0) * D, stage, min(kRows, S - row0), args.vec_ok);
+      if (!ok) break;
     }
     tc_fence_before_sync();
   }
@@ -316,15 +368,24 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
   if (threadIdx.x == 0 && bars->abort_flag && args.status) report_timeout(args.status, bars->abort_flag);
 }
 
-template <int D, bool DROP>
-int launch(const FwdArgs& a, cudaStream_t st) {
-  auto kern = flash_fwd_f32_tc_kernel<D, DROP>;
+template <int D, bool DROP, bool MANY>
+int launch(const FwdArgs& a, unsigned grid, cudaStream_t st) {
+  auto kern = flash_fwd_f32_tc_kernel<D, DROP, MANY>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::kBytes));
   static std::atomic<int> regs{0};
   if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs)) return rc;
-  const long long items = static_cast<long long>(a.BH) * ((a.S + kRows - 1) / kRows);
-  DAD_CUDA(launch_pdl(kern, dim3(static_cast<unsigned>(items)), dim3(kThreads), FwdSmem::kBytes, st, a));
+  DAD_CUDA(launch_pdl(kern, dim3(grid), dim3(kThreads), FwdSmem::kBytes, st, a));
   return DADATTN_OK;
+}
+template <int D, bool DROP>
+int launch(const FwdArgs& a, cudaStream_t st) {
+  const long long items = static_cast<long long>(a.BH) * ((a.S + kRows - 1) / kRows);
+  int dev = 0, sms = 0;
+  DAD_CUDA(cudaGetDevice(&dev));
+  DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (query tile, batch x head) items");
+  return items <= sms ? launch<D, DROP, false>(a, static_cast<unsigned>(items), st)
+                      : launch<D, DROP, true>(a, static_cast<unsigned>(sms), st);
 }
 
 }  // namespace
