@@ -68,6 +68,8 @@ struct BwdItem {
   bool valid, is_q;
   int bh, row0, first, n_it;   // first resident row, first streamed row, steps
 };
+// (A table dealt out by the host and a work queue both balance 48 x 1050 better, but what they keep in
+// registers slows every step by more.)
 template <bool MANY>
 __device__ __forceinline__ BwdItem bwd_item(int k, int BH, int S) {
   if (!MANY && k > 0) return BwdItem{};
