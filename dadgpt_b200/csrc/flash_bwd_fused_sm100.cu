@@ -709,10 +709,9 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 }
 
 // delta[r] = sum_d dO[r,d] O[r,d] (reference flash_delta_kernel, cuda/attention.cu:76-85) and the
-// zero fill of the fp32 dQ workspace, in one pass over the rows. The zero fill does not depend on
-// the kernel before this one in the stream (normally the forward pass), so it runs ahead of the
-// dependency wait and overlaps that kernel's tail. The only kernel that reads the workspace,
-// fused_convert_kernel, releases its dependents after its reads.
+// zero fill of the fp32 dQ workspace, in one pass over the rows. The fill waits for the kernel ahead
+// like every other access: the workspace may lie where that kernel still reads or writes (an arena
+// hands its bytes on from call to call), and kernels release their dependents before they are done.
 template <bool INTERLEAVED>
 __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restrict__ dq_ws,
                                      int* __restrict__ item_counter,
@@ -723,16 +722,14 @@ __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restric
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = t / Lr;   // row of the [BH, S] index space: delta and the workspace are heads-split
   const int c = static_cast<int>(t % Lr) * 8;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (t == 0) *item_counter = 0;
+  float sum = 0.f;
   if (r < rows) {
     float4* z = reinterpret_cast<float4*>(dq_ws + r * D + c);
     z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
     z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  if (t == 0) *item_counter = 0;
-  pdl_wait();
-  pdl_launch_dependents();
-  float sum = 0.f;
-  if (r < rows) {
     // where row r = (unit, s) lies in dO and O: heads-split rows are simply consecutive
     int64_t at = r * D + c;
     if (INTERLEAVED) {
@@ -754,33 +751,26 @@ __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restric
   if (r < rows && c == 0) delta[r] = sum;
 }
 
-// dQ workspace (fp32) -> dq (bf16). Dependents are released only after the workspace has been
-// read: the next backward call's prepare kernel clears it ahead of its own dependency wait.
+// dQ workspace (fp32) -> dq (bf16).
 template <bool INTERLEAVED>
 __global__ void fused_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict__ dq_ws,
                                      int64_t n8, int S, UnitLayout lay) {
   pdl_wait();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-  if (t < n8) {
-    a = *reinterpret_cast<const float4*>(dq_ws + t * 8);
-    b = *reinterpret_cast<const float4*>(dq_ws + t * 8 + 4);
-  }
-  // the loads have returned once their values are used; keep the trigger behind that use
-  const uint4 w = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
-  if (t < n8) {
-    // workspace row r = (unit, s), 8 elements at column c; heads-split dq has the same order
-    int64_t at = t * 8;
-    if (INTERLEAVED) {
-      const int64_t r = t / (kFD / 8);
-      const int c = static_cast<int>(t - r * (kFD / 8)) * 8;
-      const int unit = static_cast<int>(r / S), srow = static_cast<int>(r - static_cast<int64_t>(unit) * S);
-      const int ub = unit / lay.heads, uh = unit - ub * lay.heads;
-      at = ub * lay.batch + uh * lay.head + srow * lay.row + c;
-    }
-    *reinterpret_cast<uint4*>(dq + at) = w;
-  }
   pdl_launch_dependents();
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= n8) return;
+  const float4 a = *reinterpret_cast<const float4*>(dq_ws + t * 8), b = *reinterpret_cast<const float4*>(dq_ws + t * 8 + 4);
+  // workspace row r = (unit, s), 8 elements at column c; heads-split dq has the same order
+  int64_t at = t * 8;
+  if (INTERLEAVED) {
+    const int64_t r = t / (kFD / 8);
+    const int c = static_cast<int>(t - r * (kFD / 8)) * 8;
+    const int unit = static_cast<int>(r / S), srow = static_cast<int>(r - static_cast<int64_t>(unit) * S);
+    const int ub = unit / lay.heads, uh = unit - ub * lay.heads;
+    at = ub * lay.batch + uh * lay.head + srow * lay.row + c;
+  }
+  *reinterpret_cast<uint4*>(dq + at) =
+      make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,

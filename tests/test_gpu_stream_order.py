@@ -1,0 +1,59 @@
+"""GPU: the library's kernels start while the kernel ahead of them in the stream drains; none of them may
+touch what that kernel still reads or writes."""
+import pytest
+import torch
+
+from dadgpt_b200 import attention as dad
+from tests import kernel_ahead
+
+pytestmark = pytest.mark.gpu
+
+NAN = 0x7fc00000
+
+
+@pytest.mark.parametrize("path,D", [("split", 64), ("interleaved", 64), ("split", 128), ("via_bf16", 64)])
+def test_backward_workspace_may_be_the_bytes_of_a_call_before(cuda, path, D):
+    """The kernel ahead writes all over the bytes that the backward takes as workspace (in an arena: the
+    results of an earlier call), late. What the backward clears, it has to clear after that."""
+    B, H, S = 2, 2, 300
+    BH, scale = B * H, D ** -0.5
+    shape = (B * S, H * D) if path == "interleaved" else (BH, S, D)
+    g = torch.Generator(device=cuda).manual_seed(D)
+    dtype = torch.float32 if path == "via_bf16" else torch.bfloat16
+    q, k, v, do = (torch.randn(shape, device=cuda, generator=g).to(dtype) for _ in range(4))
+    out, lse = torch.empty_like(q), torch.empty(BH, S, device=cuda)
+    nbytes = (dad.flash_f32_via_bf16_workspace_bytes if path == "via_bf16"
+              else dad.flash_backward_bf16_workspace_bytes)(BH, S, D)
+    ws = torch.zeros(nbytes // 4, dtype=torch.float32, device=cuda)
+    grads = [torch.empty_like(q) for _ in range(3)]
+
+    def backward():
+        if path == "via_bf16":
+            dad.gpu_flash_attention_backward_via_bf16(*grads, do, out, lse, q, k, v, BH, S, D, scale, ws)
+        elif path == "interleaved":
+            dad.gpu_flash_attention_backward_bf16_interleaved(*grads, ws, do, out, lse, q, k, v, B, H, S, D, scale)
+        else:
+            dad.gpu_flash_attention_backward_bf16(*grads, ws, do, out, lse, q, k, v, BH, S, D, scale)
+
+    if path == "via_bf16":
+        dad.gpu_flash_attention_forward_via_bf16(out, lse, q, k, v, BH, S, D, scale, ws)
+    elif path == "interleaved":
+        dad.gpu_flash_attention_forward_bf16_interleaved(out, lse, q, k, v, B, H, S, D, scale)
+    else:
+        dad.gpu_flash_attention_forward_bf16(out, lse, q, k, v, BH, S, D, scale)
+    backward()
+    torch.cuda.synchronize()
+    want = [x.clone() for x in grads]
+    for x in grads:
+        x.fill_(float("nan"))
+    kernel_ahead.launch(ws, value=NAN)   # (loads its module: outside the pair that is tested)
+    torch.cuda.synchronize()
+    kernel_ahead.launch(ws, value=NAN)
+    backward()
+    assert dad.device_status() == 0
+    for got, ref, name in zip(grads, want, ("dq", "dk", "dv")):
+        # dK and dV are summed in a fixed order; dQ in the order of arrival, rounded to bf16 (2^-8) at most
+        if name == "dq":
+            assert (got.float() - ref.float()).norm() <= 1e-2 * ref.float().norm(), name
+        else:
+            assert torch.equal(got, ref), name
