@@ -279,11 +279,13 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
       bool ticket_due = lengths != nullptr && snapshot;
       const unsigned ticket = ticket_due ? draw_ticket() : 0;
       auto settle_ticket = [&]() {
-        if (ticket_due && is_last(ticket))
+        if (ticket_due && is_last(ticket)) {
+          if (early) pdl_wait();   // the kernel ahead may still read the lengths
           for (int j = 0; j < B; ++j) {
             const int len = sh.lens[j];
             if (len >= 0 && len < max_len) lengths[j] = len + 1;   // a full or invalid sequence is left alone
           }
+        }
         ticket_due = false;
       };
       int st = 0, lap = 0;

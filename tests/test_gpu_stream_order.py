@@ -57,3 +57,35 @@ def test_backward_workspace_may_be_the_bytes_of_a_call_before(cuda, path, D):
             assert (got.float() - ref.float()).norm() <= 1e-2 * ref.float().norm(), name
         else:
             assert torch.equal(got, ref), name
+
+
+@pytest.fixture
+def early_start():
+    dad.set_decode_early_start(True)
+    yield
+    dad.set_decode_early_start(False)
+
+
+def _cache(B, H, max_len, D, g):
+    cache = dad.KVCacheBF16(B, H, max_len, D)
+    cache.k.normal_(generator=g)
+    cache.v.normal_(generator=g)
+    cache.lengths.copy_(torch.randint(0, max_len - 8, (B,), generator=g, device="cuda", dtype=torch.int32))
+    return cache
+
+
+# clusters, one CTA per pair, persistent CTAs, more sequences than lengths are copied for
+@pytest.mark.parametrize("B,H,max_len", [(2, 3, 4000), (3, 4, 60), (64, 12, 300), (300, 3, 60)])
+def test_decode_with_early_start_leaves_the_lengths_to_the_kernel_ahead(cuda, early_start, B, H, max_len):
+    """The kernel ahead may read the lengths (positions of the tokens): it sees them as they were."""
+    g = torch.Generator(device=cuda).manual_seed(B)
+    cache = _cache(B, H, max_len, 64, g)
+    x = torch.randn(B, H, 64, device=cuda, generator=g).bfloat16()
+    out, seen = torch.empty_like(x), torch.empty_like(cache.lengths)
+    kernel_ahead.launch(seen, src=cache.lengths)
+    before = cache.lengths.clone()
+    torch.cuda.synchronize()
+    kernel_ahead.launch(seen.fill_(-1), src=cache.lengths)
+    dad.decode_attention_bf16(out, x, x, x, cache, 0.125)
+    assert dad.device_status() == 0
+    assert torch.equal(seen, before) and torch.equal(cache.lengths, before + 1)
