@@ -189,8 +189,12 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
   // has promised (dadattn_set_decode_early_start) that the grid before it does not write this
   // call's caches, lengths and workspace: then the lengths are read, and the ring is filled with
   // the first cache rows, while that grid drains, and only the token vectors wait for it.
-  if (!early) pdl_wait();
-  pdl_launch_dependents();
+  // Dependents are released behind that wait in either case: of several early calls in a row each
+  // overlaps the one ahead of it and no other, so that a cache written two calls ago may be read.
+  if (!early) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
 
   // Up to kMaxRanked lengths are copied to shared memory first; nobody reads the caller's array
   // after that, so it can be advanced as soon as every CTA has its copy.
@@ -324,7 +328,10 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
     }
   } else {
     // ------------------------------ consumers ------------------------------
-    if (early) pdl_wait();
+    if (early) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
     const int slot = lane / LPK, part = lane % LPK;
     const float scale_unit = scale * Elem<T>::kUnit;
     int st = 0;

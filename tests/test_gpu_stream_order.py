@@ -89,3 +89,34 @@ def test_decode_with_early_start_leaves_the_lengths_to_the_kernel_ahead(cuda, ea
     dad.decode_attention_bf16(out, x, x, x, cache, 0.125)
     assert dad.device_status() == 0
     assert torch.equal(seen, before) and torch.equal(cache.lengths, before + 1)
+
+
+def test_decode_with_early_start_overlaps_the_call_ahead_and_no_other(cuda, early_start):
+    """Two layers' caches in turn, all calls early: the call on a cache may start beside the other
+    cache's call, but not beside the one before it on its own cache, whose rows and lengths it needs.
+    The kernel ahead of them all holds everything up until the last call is in the stream."""
+    B, H, D, steps = 1, 4, 64, 4
+    g = torch.Generator(device=cuda).manual_seed(3)
+    caches = [_cache(B, H, 60, D, g) for _ in range(2)]
+    again = [_cache(B, H, 60, D, g) for _ in range(2)]
+    for c, a in zip(caches, again):
+        for name in ("k", "v", "lengths"):
+            getattr(a, name).copy_(getattr(c, name))
+    x = torch.randn(3, steps, 2, B, H, D, device=cuda, generator=g).bfloat16()
+    out, want = torch.empty_like(x[0]), torch.empty_like(x[0])
+    dummy = torch.zeros(4, device=cuda)
+    kernel_ahead.launch(dummy)
+    torch.cuda.synchronize()
+    kernel_ahead.launch(dummy, pause=2000)
+    for i in range(steps):
+        for layer, c in enumerate(caches):
+            dad.decode_attention_bf16(out[i, layer], *x[:, i, layer], c, 0.125)
+    assert dad.device_status() == 0
+    dad.set_decode_early_start(False)
+    for i in range(steps):
+        for layer, c in enumerate(again):
+            dad.decode_attention_bf16(want[i, layer], *x[:, i, layer], c, 0.125)
+    assert dad.device_status() == 0
+    assert torch.equal(out, want)
+    for c, a in zip(caches, again):
+        assert torch.equal(c.lengths, a.lengths) and torch.equal(c.k, a.k) and torch.equal(c.v, a.v)
