@@ -23,7 +23,7 @@
 //     uses them, and stores them into the cache;
 //   * every CTA draws a ticket once it has copied the lengths; the holder of the last one stores
 //     length + 1, while the rows are still streaming. Counters are returned to zero by their last
-//     user, so a workspace zeroed once stays usable forever;
+//     user, also where a bounded wait ran out, so a workspace zeroed once stays usable forever;
 //   * launched with programmatic stream serialization: the next decode call's CTAs set themselves up
 //     (and, where the caller allows it, fill their rings) while this grid drains.
 #include <cfloat>
@@ -292,7 +292,16 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
         }
         ticket_due = false;
       };
+      // One claim per item beyond the CTAs' first ones and one per CTA that finds nothing left: n_items
+      // in all, of which the last returns the counter to zero.
+      auto claim = [&]() -> int {
+        if (n_lanes >= n_items) return n_items;
+        const unsigned c = atomicAdd(item_counter, 1u);
+        if (c == static_cast<unsigned>(n_items - 1)) *item_counter = 0;
+        return min(static_cast<int>(c) + n_lanes, n_items);
+      };
       int st = 0, lap = 0;
+      int next = 0;   // the last claim
       Item s = first;
       bool ok = true;
       for (int n = 0; ok; ++n) {
@@ -310,12 +319,7 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
         // The item after this one is claimed only when this one's last rows are on their way: what is
         // in the ring covers the counter's round trip, and a CTA with a long item takes no second one
         // that an idle CTA could have had (64 sequences x 12 heads: 210 us, 240 when claimed an item ahead).
-        int next = n_items;
-        if (ok && n_lanes < n_items) {
-          const unsigned claim = atomicAdd(item_counter, 1u);
-          next = min(static_cast<int>(claim) + n_lanes, n_items);
-          if (claim == static_cast<unsigned>(n_items - 1)) *item_counter = 0;   // the last claim: ready for the next call
-        }
+        if (ok) next = claim();
         const int slot = n % kItemRing;
         ok = ok && (n < kItemRing || mbar_wait(&sh.item_free[slot], (n / kItemRing - 1) & 1, abort_flag));
         if (!ok) break;
@@ -324,6 +328,8 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
         if (next >= n_items) break;
         s = item(next);
       }
+      // After a wait that ran out the claims are made all the same: the workspace stays usable.
+      while (next < n_items) next = claim();
       settle_ticket();
     }
   } else {

@@ -243,8 +243,8 @@ int dadattn_decode_f32(float* out, const float* q, const float* k_new, const flo
  * DADATTN_E_ARG at the next dadattn_device_status(). workspace: counters and room for split-K
  * records, at least dadattn_decode_workspace_bytes() bytes, 16-byte aligned. It must be zero-filled
  * (cudaMemset) before its first use and again whenever B, H or max_len change; between calls of
- * one shape the library leaves it in a reusable state. Two calls that share a workspace must not
- * overlap on the GPU. */
+ * one shape the library leaves it in a reusable state, also where a bounded wait ran out. Two
+ * calls that share a workspace must not overlap on the GPU. */
 size_t dadattn_decode_workspace_bytes(int B, int H, int D, int max_len);
 int dadattn_decode_bf16(uint16_t* out, const uint16_t* q, const uint16_t* k_new,
                         const uint16_t* v_new, uint16_t* k_cache, uint16_t* v_cache,
@@ -304,7 +304,7 @@ int dadattn_set_decode_early_start(int on);
  *    (cudaGetSymbolAddress); make that first call before starting any stream capture.
  *  - All calls share the one array and it keeps the previous call's contents. Only the tickets
  *    have to be zero when a call starts: they are zero when the library is loaded and every call
- *    hands them back zeroed (records are written before they are read within a call). Two calls
+ *    hands them back zeroed, also one in which a bounded wait ran out. Two calls
  *    that overlap on the GPU (different streams, or threads) race on the array: serialise them.
  *  - A sequence already at max_len is skipped as in dadattn_decode_bf16 and noted in a word
  *    beside the array; dadattn_decode_noalloc_status reads it (dadattn_device_status belongs to
@@ -314,8 +314,9 @@ int dadattn_decode_bf16_noalloc(uint16_t* out, const uint16_t* q, const uint16_t
                                 int32_t* lengths, int B, int H, int D, int max_len, float scale,
                                 dadattn_stream_t stream);
 /* Waits for `stream`, then returns and clears the status word of dadattn_decode_bf16_noalloc on
- * the current device: 0, or DADATTN_E_ARG when a call since the last read skipped a sequence
- * whose length was outside [0, max_len). Copies from and to a symbol of the library image, so it
+ * the current device: 0, DADATTN_E_ARG when a call since the last read skipped a sequence whose
+ * length was outside [0, max_len), or DADATTN_E_TIMEOUT when a bounded wait ran out (the array
+ * stays usable). Copies from and to a symbol of the library image, so it
  * allocates nothing either. No counterpart in the reference. */
 int dadattn_decode_noalloc_status(dadattn_stream_t stream);
 
