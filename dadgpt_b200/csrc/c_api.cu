@@ -1,6 +1,5 @@
 // Library-wide pieces of the C ABI: error text, version, the device-side status word.
 #include <cstring>
-#include <mutex>
 
 #include "common.cuh"
 
@@ -9,8 +8,10 @@ namespace dadattn {
 namespace {
 thread_local char g_error[512] = "";
 constexpr int kMaxDevices = 64;
-int* g_status[kMaxDevices] = {};
-std::mutex g_status_mutex;
+// Status, and a detail for it: the source line of a wait that ran out. Part of the library image on
+// every device, zero when it is loaded.
+__device__ int g_status_words[2];
+std::atomic<int*> g_status[kMaxDevices] = {};
 }  // namespace
 
 char* error_buffer() { return g_error; }
@@ -23,43 +24,26 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
-// Two 4-byte words per device (status, and a detail for it: the source line of a wait that ran
-// out), allocated the first time a kernel that can report a condition is launched on that
-// device; they live until exit.
+// In host code the name g_status_words is only a handle; the address a kernel can use is looked up per
+// device, with that device current. No allocation, so a first call may come while a stream is being
+// captured, its own or another.
 int* device_status_word() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
     fail(DADATTN_E_CUDA, "no current CUDA device");
     return nullptr;
   }
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  if (!g_status[dev]) {
-    int* p = nullptr;
-    if (cudaMalloc(&p, 2 * sizeof(int)) != cudaSuccess || cudaMemset(p, 0, 2 * sizeof(int)) != cudaSuccess) {
-      fail(DADATTN_E_CUDA, "cannot allocate the device status word: %s",
-           cudaGetErrorString(cudaGetLastError()));
+  int* word = g_status[dev].load(std::memory_order_relaxed);
+  if (!word) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_status_words) != cudaSuccess) {
+      fail(DADATTN_E_CUDA, "cannot find the device status word: %s", cudaGetErrorString(cudaGetLastError()));
       return nullptr;
     }
-    g_status[dev] = p;
+    word = static_cast<int*>(p);
+    g_status[dev].store(word, std::memory_order_relaxed);   // (the same address whoever looks it up)
   }
-  return g_status[dev];
-}
-
-int optional_status_word(int** word, cudaStream_t st) {
-  int dev = 0;
-  DAD_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < kMaxDevices) {
-    std::lock_guard<std::mutex> lock(g_status_mutex);
-    if ((*word = g_status[dev])) return DADATTN_OK;
-  }
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  DAD_CUDA(cudaStreamIsCapturing(st, &capture));
-  if (capture != cudaStreamCaptureStatusNone) {
-    *word = nullptr;
-    return DADATTN_OK;
-  }
-  *word = device_status_word();
-  return *word ? DADATTN_OK : DADATTN_E_CUDA;
+  return word;
 }
 
 int check_launch_registers(const void* kernel, int expected, std::atomic<int>& seen) {

@@ -35,9 +35,6 @@ int fail(int code, const char* fmt, ...);
 // Device-side sticky status word (one per device that loads the library). Kernels record a
 // DADATTN_E_* code here instead of trapping; dadattn_device_status() reads and clears it.
 int* device_status_word();  // device pointer for the current device, nullptr on failure
-// The same for calls that may be the first on their device inside a stream capture, where the word
-// cannot be allocated: nullptr (such kernels then report nothing) while `st` is capturing.
-int optional_status_word(int** word, cudaStream_t st);
 
 // Kernels whose warpgroups move registers between them (setmaxnreg) budget with the count the CTA is
 // launched with; were the compiler to give the kernel fewer, an increase would wait for registers

@@ -738,8 +738,7 @@ extern "C" int dadattn_decode_f32(float* out, const float* q, const float* k_new
 // synchronisation an allocation implies; and DadGPT itself sizes all of its buffers once, in
 // model_alloc / kv_cache_alloc, and never allocates inside generate_tokens. For such callers the
 // split-K tickets and records live in the fixed array below instead of a caller-provided
-// workspace, and the bad-length report goes to a fixed word instead of the lazily allocated
-// status word.
+// workspace, and the bad-length report goes to a word of its own beside the array.
 //
 // The array is part of the library image: every GPU that loads libdadattn.so holds these
 // 8 MiB until the process exits, whether or not this entry point is ever called. Its first

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
   const int S = args.S;
 
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
-    if (threadIdx.x == 0 && args.status) atomicExch(args.status, DADATTN_E_CUDA);
+    if (threadIdx.x == 0) atomicExch(args.status, DADATTN_E_CUDA);
     return;
   }
   const FwdItem item0 = fwd_item<MANY>(0, args.BH, S);   // used when there is one: formed ahead of the dependency wait
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     tc_fence_after_sync();
     tmem_dealloc(tmem, 256);
   }
-  if (threadIdx.x == 0 && bars->abort_flag && args.status) report_timeout(args.status, bars->abort_flag);
+  if (threadIdx.x == 0 && bars->abort_flag) report_timeout(args.status, bars->abort_flag);
 }
 
 template <int D, bool DROP, bool MANY>
@@ -396,8 +396,8 @@ int launch(const FwdArgs& a, cudaStream_t st) {
 int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
                       float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
                       cudaStream_t st) {
-  int* status = nullptr;
-  if (int rc = optional_status_word(&status, st)) return rc;
+  int* status = device_status_word();
+  if (!status) return DADATTN_E_CUDA;
   const FwdArgs a = {out, lse, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok, status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);

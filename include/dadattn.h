@@ -6,11 +6,7 @@
  * returns without synchronising. Return value: 0 on success, a negative DADATTN_E_* code
  * otherwise; dadattn_last_error() then describes the failure (thread-local string).
  * All tensors and workspaces belong to the caller. What the library itself holds on a device:
- *  - two 4-byte status words (see dadattn_device_status), allocated with cudaMalloc by the first
- *    bf16, decode or fp32-decode call on that device (or fp32 attention call outside a stream
- *    capture) and kept until exit. Because of that allocation the FIRST bf16, decode or
- *    fp32-decode call on a device must come before any stream capture; later calls allocate
- *    nothing;
+ *  - two 4-byte status words in the library image (see dadattn_device_status);
  *  - the grow-only buffer behind dadattn_library_scratch, only if that function is called;
  *  - an 8 MiB array in the library image for dadattn_decode_bf16_noalloc (no allocation call).
  * There is no CPU fallback: without a CUDA device every compute call fails.
