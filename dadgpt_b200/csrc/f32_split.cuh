@@ -10,6 +10,13 @@
 // added to a register sum in fp32 with round-to-nearest. Nothing is rounded to bf16: the result is
 // that of an fp32 dot product with another order of summation (measured against float64: no larger
 // error than the FFMA kernels of flash_f32.cu).
+//
+// Range. Every finite x: the first plane saturates at bf16's largest number, 3.3895e38, what a larger x
+// has beyond it goes to the second. Below 2^-110 the last bits of the third plane fall under bf16's
+// smallest number, an absolute error of at most 2^-134. An infinite or NaN element (its planes hold a
+// NaN) makes NaN of every result that its tile's products add it to: the rows and columns that see it,
+// and for V, K in the dQ product, dO and Q in the dK / dV products also rows or keys of the same tile
+// for which its weight is a masked 0 (0 x NaN).
 #pragma once
 
 #include "common.cuh"
@@ -41,6 +48,14 @@ constexpr uint32_t kPolls = 16;
 __device__ __forceinline__ constexpr int product_a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
 __device__ __forceinline__ constexpr int product_b(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i == 3 ? 0 : i == 4 ? 1 : 0; }
 
+// (lo, hi) -> packed bf16 as plane i of a split
+template <int I>
+__device__ __forceinline__ uint32_t pack_plane(float lo, float hi) {
+  if (I > 0) return pack_bf16(lo, hi);   // (not saturating: an infinity may not end as a finite sum)
+  uint32_t r;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
 // Four fp32 values -> three planes of four packed bf16.
 struct Split4 {
   uint2 p[3];
@@ -49,7 +64,8 @@ __device__ __forceinline__ Split4 split4(float4 x) {
   Split4 s;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    s.p[i] = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
+    s.p[i] = i == 0 ? make_uint2(pack_plane<0>(x.x, x.y), pack_plane<0>(x.z, x.w))
+                    : make_uint2(pack_plane<1>(x.x, x.y), pack_plane<1>(x.z, x.w));
     const float2 minus = make_float2(-1.f, -1.f);
     const float2 a = ffma2(make_float2(__uint_as_float(s.p[i].x << 16), __uint_as_float(s.p[i].x & 0xffff0000u)), minus,
                            make_float2(x.x, x.y));   // exact
@@ -118,7 +134,7 @@ __device__ __forceinline__ void tmem_store_split(float2 (&x)[8], uint32_t t0, ui
     uint32_t pk[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      pk[j] = pack_bf16(x[j].x, x[j].y);
+      pk[j] = i == 0 ? pack_plane<0>(x[j].x, x[j].y) : pack_plane<1>(x[j].x, x[j].y);
       if (i < 2)
         x[j] = ffma2(make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xffff0000u)),
                      make_float2(-1.f, -1.f), x[j]);   // exact

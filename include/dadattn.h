@@ -50,7 +50,12 @@ int dadattn_flash_supported(int d_head);
 
 /* Replaces gpu_flash_attention_forward (reference cuda/gpu_ops.cuh:116-117,
  * cuda/attention.cu:234-239): out = softmax(causal(q k^T * scale)) v, lse = rowmax + ln(rowsum)
- * of the scaled scores. q,k,v,out: [BH,S,d_head] fp32; lse: [BH,S] fp32. */
+ * of the scaled scores. q,k,v,out: [BH,S,d_head] fp32; lse: [BH,S] fp32.
+ * Range at head sizes 16-64, forward and backward (each operand is the sum of three bf16 numbers):
+ * every finite number; the last bits of one below 2^-110 may be lost, an error of at most 2^-134.
+ * Where an fp32 sum would be infinite because an INPUT is, the result is NaN; and an infinite or
+ * NaN row makes NaN of the queries (in the backward: keys) of its 128-row tile that do not see it,
+ * too, as it does in the bf16 kernels. Other tiles and units are not touched. */
 int dadattn_flash_fwd_f32(float* out, float* lse, const float* q, const float* k, const float* v,
                           int BH, int S, int d_head, float scale, dadattn_stream_t stream);
 
