@@ -19,6 +19,18 @@ def test_values_beyond_the_largest_bf16(cuda, D, value):
     assert torch.equal(out, v)
 
 
+@pytest.mark.parametrize("exponent", [-149, -130, -126, -120, -112, -108, -90])
+def test_small_values(cuda, exponent):
+    """One key again. Half the spacing of bf16's smallest numbers, 2^-133, is all that may be lost."""
+    g = torch.Generator(device=cuda).manual_seed(7)
+    q = torch.ones(50, 1, 64, device=cuda)
+    v = ((1 + torch.rand(50, 1, 64, device=cuda, generator=g, dtype=torch.float64)) * 2.0 ** exponent).float()
+    out, lse, dq, dk, dv = _run(q, q, v, torch.zeros_like(q), 0.125)
+    assert (out.double() - v.double()).abs().max().item() <= 2.0 ** -134
+    if exponent >= -109:
+        assert torch.equal(out, v)
+
+
 @pytest.mark.parametrize("D", [16, 64])
 @pytest.mark.parametrize("S", [65, 300])
 def test_products_of_the_largest_numbers(cuda, D, S):
