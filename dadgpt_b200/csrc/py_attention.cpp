@@ -213,13 +213,14 @@ PyObject* fwd_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t unit0 = p.integer64();
     need_shapes({{"out", out}, {"q", q}, {"k", k}, {"v", v}}, {BH, S, D});
     need_shape("lse", lse, {BH, S});
-    const uint32_t* bits = p.none() ? nullptr : static_cast<const uint32_t*>(ptr(p.tensor("mask_bits")));
+    const bool masked = !p.none();   // (an empty tensor's pointer is null: the library refuses it)
+    const uint32_t* bits = masked ? static_cast<const uint32_t*>(ptr(p.tensor("mask_bits"))) : nullptr;
     const dadattn_stream_t st = stream();
     return done(without_gil([&] {
-      return bits ? dadattn_flash_fwd_bf16_masked(b16(out), f32(lse), b16(q), b16(k), b16(v), BH, S, D, scale, rate,
-                                                  bits, st)
-                  : dadattn_flash_fwd_bf16(b16(out), f32(lse), b16(q), b16(k), b16(v), BH, S, D, scale, rate, seed,
-                                           offset, unit0, st);
+      return masked ? dadattn_flash_fwd_bf16_masked(b16(out), f32(lse), b16(q), b16(k), b16(v), BH, S, D, scale, rate,
+                                                    bits, st)
+                    : dadattn_flash_fwd_bf16(b16(out), f32(lse), b16(q), b16(k), b16(v), BH, S, D, scale, rate, seed,
+                                             offset, unit0, st);
     }));
   });
 }
@@ -238,15 +239,16 @@ PyObject* bwd_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     need_shapes({{"dq", dq}, {"dk", dk}, {"dv", dv}, {"dout", dout}, {"out", out}, {"q", q}, {"k", k}, {"v", v}},
                 {BH, S, D});
     need_shape("lse", lse, {BH, S});
-    const uint32_t* bits = p.none() ? nullptr : static_cast<const uint32_t*>(ptr(p.tensor("mask_bits")));
+    const bool masked = !p.none();   // (an empty tensor's pointer is null: the library refuses it)
+    const uint32_t* bits = masked ? static_cast<const uint32_t*>(ptr(p.tensor("mask_bits"))) : nullptr;
     void* const w = ptr(ws);
     const size_t bytes = ws.nbytes();
     const dadattn_stream_t st = stream();
     return done(without_gil([&] {
-      return bits ? dadattn_flash_bwd_bf16_masked(b16(dq), b16(dk), b16(dv), w, bytes, b16(dout), b16(out), f32(lse),
-                                                  b16(q), b16(k), b16(v), BH, S, D, scale, rate, bits, st)
-                  : dadattn_flash_bwd_bf16(b16(dq), b16(dk), b16(dv), w, bytes, b16(dout), b16(out), f32(lse), b16(q),
-                                           b16(k), b16(v), BH, S, D, scale, rate, seed, offset, unit0, st);
+      return masked ? dadattn_flash_bwd_bf16_masked(b16(dq), b16(dk), b16(dv), w, bytes, b16(dout), b16(out), f32(lse),
+                                                    b16(q), b16(k), b16(v), BH, S, D, scale, rate, bits, st)
+                    : dadattn_flash_bwd_bf16(b16(dq), b16(dk), b16(dv), w, bytes, b16(dout), b16(out), f32(lse),
+                                             b16(q), b16(k), b16(v), BH, S, D, scale, rate, seed, offset, unit0, st);
     }));
   });
 }
