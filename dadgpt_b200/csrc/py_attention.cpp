@@ -72,9 +72,12 @@ class Args {
     ++i_;
     return true;
   }
-  int integer() {
-    const long long v = PyLong_AsLongLong(a_[i_++]);
-    if (v == -1 && PyErr_Occurred()) throw Bad{};
+  int integer() {   // a size: larger ones than an int fit no tensor
+    const int64_t v = integer64();
+    if (v != static_cast<int>(v)) {
+      PyErr_Format(PyExc_ValueError, "size %lld out of range", static_cast<long long>(v));
+      throw Bad{};
+    }
     return static_cast<int>(v);
   }
   int64_t integer64() {
@@ -362,7 +365,7 @@ PyObject* decode_f32(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Args p(a, n, 8, "decode_f32");
     const at::Tensor &out = p.need("out", kF), &q = p.need("q", kF), &kn = p.need("k_new", kF),
                      &vn = p.need("v_new", kF), &k = p.need("k_cache", kF), &v = p.need("v_cache", kF);
-    const int pos = p.integer();
+    const int64_t pos = p.integer64();
     const float scale = p.real();
     if (k.dim() != 3) {
       PyErr_SetString(PyExc_ValueError, "k_cache must be [H, max_len, D]");
@@ -370,13 +373,15 @@ PyObject* decode_f32(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     const int H = static_cast<int>(k.size(0)), max_len = static_cast<int>(k.size(1)), D = static_cast<int>(k.size(2));
     if (pos < 0 || pos >= max_len) {
-      PyErr_Format(PyExc_IndexError, "model_forward_cached: pos %d outside context length %d", pos, max_len);
+      PyErr_Format(PyExc_IndexError, "model_forward_cached: pos %lld outside context length %d",
+                   static_cast<long long>(pos), max_len);
       return nullptr;
     }
     need_shape("v_cache", v, {H, max_len, D});
     const dadattn_stream_t st = stream();
     return done(without_gil([&] {
-      return dadattn_decode_f32(f32(out), f32(q), f32(kn), f32(vn), f32(k), f32(v), H, max_len, D, pos, scale, st);
+      return dadattn_decode_f32(f32(out), f32(q), f32(kn), f32(vn), f32(k), f32(v), H, max_len, D,
+                                static_cast<int>(pos), scale, st);
     }));
   });
 }
