@@ -13,6 +13,7 @@ Outputs (next to this file, git-ignored, they travel with the working tree):
 from __future__ import annotations
 
 import glob
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -24,6 +25,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libdadattn.so")
 SHIM = os.path.join(PKG, "libdadattn_gpuops.so")
 NATIVE = os.path.join(PKG, "_native.so")
+NATIVE_ABI = os.path.join(PKG, "build", "_native.abi")   # what NATIVE was built for
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -74,9 +76,22 @@ def build(force: bool = False, ptxas: bool = False) -> str:
         subprocess.run([cxx, "-std=c++20", "-O2", "-fPIC", "-shared", "-I", os.path.join(ROOT, "include"),
                         shim_src, "-o", SHIM, "-L", PKG, "-ldadattn", "-Wl,-rpath,$ORIGIN"], check=True)
     native_src = os.path.join(CSRC, "py_attention.cpp")
-    if force or _newer(NATIVE, [native_src, os.path.join(ROOT, "include", "dadattn.h")]):
+    if force or _newer(NATIVE, [native_src, os.path.join(ROOT, "include", "dadattn.h")]) or not _native_current():
         _build_native(native_src)
     return LIB
+
+
+def _native_abi() -> str:
+    """What the native module is bound to besides its sources: torch's C++ ABI and CPython's."""
+    return f"torch {importlib.metadata.version('torch')}, {sys.implementation.cache_tag}\n"
+
+
+def _native_current() -> bool:
+    try:
+        with open(NATIVE_ABI) as f:
+            return f.read() == _native_abi()
+    except FileNotFoundError:
+        return False
 
 
 def _build_native(src: str) -> None:
@@ -92,6 +107,9 @@ def _build_native(src: str) -> None:
                     "-I", os.path.join(ROOT, "include"), *inc, src, "-o", NATIVE,
                     "-L", PKG, "-ldadattn", "-L", lib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
                     "-Wl,-rpath,$ORIGIN"], check=True)
+    os.makedirs(os.path.dirname(NATIVE_ABI), exist_ok=True)
+    with open(NATIVE_ABI, "w") as f:
+        f.write(_native_abi())
 
 
 if __name__ == "__main__":
