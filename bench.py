@@ -895,7 +895,7 @@ def bench_strong(cx, dad, W, ws_bytes, large_1gpu, decode_1gpu, verify=True):
                         "gbs_total": float(tot.item()) / (d["ms_total"] * 1e-3),
                         "verify": d.get("verify"),
                         "note": "few (sequence, head) pairs per GPU: the cache rows of a pair are "
-                                "split across CTAs and merged through tickets (split-K branch)"}
+                                "split across the CTAs of a cluster"}
     strong["ok"] = bool((not verify) or (strong["large_shape"]["verify"]["ok"] and d["verify"]["ok"]))
     return strong
 

@@ -137,7 +137,7 @@ def decode_attention_f32(out, q, k_new, v_new, k_cache, v_cache, pos, scale):
 
 class KVCacheBF16:
     """Batched counterpart of the reference's ``struct KVCache`` (src/model.hpp:140-152) for one
-    layer: k, v [B,H,max_len,D] bf16, per-sequence lengths on the device, split-K workspace."""
+    layer: k, v [B,H,max_len,D] bf16, per-sequence lengths on the device, the decode kernel's workspace."""
 
     def __init__(self, B, H, max_len, D, device="cuda"):
         self.B, self.H, self.max_len, self.D = B, H, max_len, D
@@ -145,7 +145,7 @@ class KVCacheBF16:
         self.v = torch.zeros_like(self.k)
         self.lengths = torch.zeros(B, dtype=torch.int32, device=device)
         nbytes = int(_lib.load().dadattn_decode_workspace_bytes(B, H, D, max_len))
-        # zero-filled once: the split-K tickets must start at zero (include/dadattn.h)
+        # zero-filled once: the counters must start at zero (include/dadattn.h)
         self.workspace = torch.zeros(nbytes, dtype=torch.uint8, device=device)
 
 

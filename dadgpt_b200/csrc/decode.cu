@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -82,9 +83,10 @@ struct Elem<__nv_bfloat16> {
 };
 
 // Workspace: B*H words, of which the first is the item counter, then the 1 + kTicketGroups counters
-// of the "all lengths read" tickets (uint32, all zero between calls), padded to 256 bytes. Behind
-// them callers hold what dadattn_decode_workspace_bytes has always asked for, the records of a
-// split-K merge in global memory; this kernel does not use that part.
+// of the "all lengths read" tickets (uint32, all zero between calls), padded to 256 bytes. No more is
+// used. The sizes that callers are asked for, and the shapes that the allocation-free entry point
+// refuses, are part of the interface and count room for the records of a split-K merge, too, which an
+// earlier kernel kept in global memory.
 inline size_t record_bytes(int B, int H, int D, int max_len) {
   constexpr long long kTargetCtas = 592, kMinRows = 256;
   const long long pairs = static_cast<long long>(B) * H;
@@ -737,47 +739,42 @@ extern "C" int dadattn_decode_f32(float* out, const float* q, const float* k_new
 // for a later cudaMalloc; a latency-critical decode loop cannot afford the device-wide
 // synchronisation an allocation implies; and DadGPT itself sizes all of its buffers once, in
 // model_alloc / kv_cache_alloc, and never allocates inside generate_tokens. For such callers the
-// split-K tickets and records live in the fixed array below instead of a caller-provided
-// workspace, and the bad-length report goes to a word of its own beside the array.
+// counters live in the fixed array below instead of a caller-provided workspace, and the bad-length
+// report goes to a word of its own beside the array.
 //
-// The array is part of the library image: every GPU that loads libdadattn.so holds these
-// 8 MiB until the process exits, whether or not this entry point is ever called. Its first
-// 64 KiB are the counters, at a fixed place whatever the shape of a call: they are zero when the
-// module is loaded and every call returns them to zero, which is the only state a call needs
-// from its predecessors. The records behind them are written before they are read.
+// The array is part of the library image: every GPU that loads libdadattn.so holds these 64 KiB until
+// the process exits, whether or not this entry point is ever called. The counters are at a fixed place
+// whatever the shape of a call: they are zero when the module is loaded and every call returns them to
+// zero, which is the only state a call needs from its predecessors.
 // A sequence that is already at max_len is skipped and noted in g_decode_noalloc_status, which
 // dadattn_decode_noalloc_status() reads and clears (a symbol copy: no allocation either).
 // ---------------------------------------------------------------------------------------------
 namespace dadattn {
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = size_t(8) << 20;
 constexpr size_t kNoAllocTicketBytes = size_t(64) << 10;
-static __device__ __align__(256) unsigned char g_decode_scratch[kNoAllocScratchBytes];
+constexpr size_t kNoAllocLimitBytes = size_t(8) << 20;   // largest workspace of a shape that is taken
+static __device__ __align__(256) unsigned g_decode_tickets[kNoAllocTicketBytes / sizeof(unsigned)];
 static __device__ int g_decode_noalloc_status[2];   // status and its detail, as in device_status_word()
 
 constexpr int kNoAllocMaxDevices = 64;
-float* g_scratch_ptr[kNoAllocMaxDevices] = {};
-int* g_noalloc_status_ptr[kNoAllocMaxDevices] = {};
+std::atomic<unsigned*> g_tickets_ptr[kNoAllocMaxDevices] = {};
+std::atomic<int*> g_noalloc_status_ptr[kNoAllocMaxDevices] = {};
 
-// In host code the names g_decode_scratch / g_decode_noalloc_status are only handles; the
+// In host code the names g_decode_tickets / g_decode_noalloc_status are only handles; the
 // device addresses a kernel can use come from cudaGetSymbolAddress, per device, with that
 // device current. Looked up on the first call on each device and cached.
-int noalloc_setup(float** scratch, int** status) {
+int noalloc_setup(unsigned** tickets, int** status) {
   int dev = 0;
   DAD_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kNoAllocMaxDevices)
     return fail(DADATTN_E_UNSUPPORTED, "device ordinal %d not supported", dev);
-  if (!g_scratch_ptr[dev] || !g_noalloc_status_ptr[dev]) {
-    float* s = nullptr;
-    int* w = nullptr;
-    DAD_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&s), g_decode_scratch));
-    DAD_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&w), g_decode_noalloc_status));
-    g_noalloc_status_ptr[dev] = w;
-    g_scratch_ptr[dev] = s;
+  if (!(*tickets = g_tickets_ptr[dev]) || !(*status = g_noalloc_status_ptr[dev])) {
+    DAD_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(tickets), g_decode_tickets));
+    DAD_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(status), g_decode_noalloc_status));
+    g_tickets_ptr[dev] = *tickets;
+    g_noalloc_status_ptr[dev] = *status;
   }
-  *scratch = g_scratch_ptr[dev];
-  *status = g_noalloc_status_ptr[dev];
   return DADATTN_OK;
 }
 
@@ -792,21 +789,20 @@ extern "C" int dadattn_decode_bf16_noalloc(uint16_t* out, const uint16_t* q,
   if (int rc = check_decode_bf16(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, D, max_len))
     return rc;
   const size_t need_tickets = ticket_bytes(B, H), need_records = record_bytes(B, H, D, max_len);
-  if (need_tickets > kNoAllocTicketBytes || need_records > kNoAllocScratchBytes - kNoAllocTicketBytes)
+  if (need_tickets > kNoAllocTicketBytes || need_records > kNoAllocLimitBytes - kNoAllocTicketBytes)
     return fail(DADATTN_E_WORKSPACE,
-                "decode (no-alloc): B=%d H=%d D=%d max_len=%d needs %zu bytes of tickets and %zu "
-                "bytes of split-K records; the built-in array of %zu bytes holds %zu and %zu; use "
+                "decode (no-alloc): B=%d H=%d D=%d max_len=%d counts as %zu bytes of tickets and %zu "
+                "bytes of split-K records; of %zu bytes in all, %zu and %zu are taken; use "
                 "dadattn_decode_bf16 with your own workspace",
-                B, H, D, max_len, need_tickets, need_records,
-                static_cast<size_t>(kNoAllocScratchBytes), static_cast<size_t>(kNoAllocTicketBytes),
-                static_cast<size_t>(kNoAllocScratchBytes - kNoAllocTicketBytes));
-  float* scratch = nullptr;
+                B, H, D, max_len, need_tickets, need_records, kNoAllocLimitBytes, kNoAllocTicketBytes,
+                kNoAllocLimitBytes - kNoAllocTicketBytes);
+  unsigned* tickets = nullptr;
   int* status = nullptr;
-  if (int rc = noalloc_setup(&scratch, &status)) return rc;
+  if (int rc = noalloc_setup(&tickets, &status)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // never with early start: every call shares the one scratch array with the call before it
-  return launch_decode_bf16(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, D, max_len, scale,
-                            reinterpret_cast<unsigned*>(scratch), status, 0, st);
+  // never with early start: every call shares the one array with the call before it
+  return launch_decode_bf16(out, q, k_new, v_new, k_cache, v_cache, lengths, B, H, D, max_len, scale, tickets, status,
+                            0, st);
 }
 
 extern "C" int dadattn_decode_noalloc_status(dadattn_stream_t stream) {

@@ -8,7 +8,7 @@
  * All tensors and workspaces belong to the caller. What the library itself holds on a device:
  *  - two 4-byte status words in the library image (see dadattn_device_status);
  *  - the grow-only buffer behind dadattn_library_scratch, only if that function is called;
- *  - an 8 MiB array in the library image for dadattn_decode_bf16_noalloc (no allocation call).
+ *  - a 64 KiB array in the library image for dadattn_decode_bf16_noalloc (no allocation call).
  * There is no CPU fallback: without a CUDA device every compute call fails.
  *
  * Device-side waits are bounded. If one runs out, the kernel records DADATTN_E_TIMEOUT and
@@ -241,11 +241,11 @@ int dadattn_decode_f32(float* out, const float* q, const float* k_new, const flo
  * Caches: [B,H,max_len,D] bf16. lengths[B] (int32, device) holds each sequence's current length
  * L_b; the call writes k_new,v_new [B,H,D] at row L_b, attends over rows 0..L_b, and stores
  * L_b + 1 back. Sequences with L_b >= max_len are left untouched and reported through
- * DADATTN_E_ARG at the next dadattn_device_status(). workspace: counters and room for split-K
- * records, at least dadattn_decode_workspace_bytes() bytes, 16-byte aligned. It must be zero-filled
- * (cudaMemset) before its first use and again whenever B, H or max_len change; between calls of
- * one shape the library leaves it in a reusable state, also where a bounded wait ran out. Two
- * calls that share a workspace must not overlap on the GPU. */
+ * DADATTN_E_ARG at the next dadattn_device_status(). workspace: counters, at least
+ * dadattn_decode_workspace_bytes() bytes, 16-byte aligned. It must be zero-filled (cudaMemset)
+ * before its first use and again whenever B, H or max_len change; between calls of one shape the
+ * library leaves it in a reusable state, also where a bounded wait ran out. Two calls that share a
+ * workspace must not overlap on the GPU. */
 size_t dadattn_decode_workspace_bytes(int B, int H, int D, int max_len);
 int dadattn_decode_bf16(uint16_t* out, const uint16_t* q, const uint16_t* k_new,
                         const uint16_t* v_new, uint16_t* k_cache, uint16_t* v_cache,
@@ -290,26 +290,23 @@ int dadattn_set_decode_early_start(int on);
  * own KV-cache pool at start-up, a decode loop that must not hit the device-wide stall of an
  * allocation, or DadGPT's own generation loop, which sizes every buffer once in kv_cache_alloc
  * and never allocates afterwards. Same arguments and results as dadattn_decode_bf16 minus the
- * workspace: the split-K partials go to a fixed 8 MiB array inside the library image (held by
+ * workspace: the call's counters live in a fixed 64 KiB array inside the library image (held by
  * every GPU that loads the library, until exit). The call performs no cudaMalloc/cudaFree and
  * uses no allocating routine.
- *  - Limit: the array is 8 MiB (8388608 bytes). Its first 64 KiB hold the tickets, which need
- *    B*H + 33 <= 16384, i.e. B*H <= 16351: that is the binding limit for any shape with
- *    B*H >= 592, where each CTA walks a whole sequence and there are no records at all. With
- *    fewer (sequence, head) pairs the cache rows are split across CTAs and the records
- *    (B*H*splits*(D+2)*4 bytes, at most ~5 splits) must fit in the remaining 8 MiB - 64 KiB,
- *    which they do for every max_len up to about 100 000 rows at D = 64.
- *    dadattn_decode_workspace_bytes(B,H,D,max_len) tells what a shape needs; shapes beyond the
- *    array return DADATTN_E_WORKSPACE.
+ *  - Limit: the counters, 4 bytes each, may take 64 KiB: B*H + 33 <= 16384, i.e. B*H <= 16351.
+ *    That is the binding limit for any shape with B*H >= 592. For fewer (sequence, head) pairs
+ *    dadattn_decode_workspace_bytes also counts split-K records (B*H*splits*(D+2)*4 bytes, at
+ *    most ~5 splits); those may make up the rest of 8 MiB (8388608 bytes), as they do for every
+ *    max_len up to about 100 000 rows at D = 64. Shapes beyond it return DADATTN_E_WORKSPACE.
  *  - The first call on each device looks up the array's device address
  *    (cudaGetSymbolAddress); make that first call before starting any stream capture.
- *  - All calls share the one array and it keeps the previous call's contents. Only the tickets
- *    have to be zero when a call starts: they are zero when the library is loaded and every call
- *    hands them back zeroed, also one in which a bounded wait ran out. Two calls
- *    that overlap on the GPU (different streams, or threads) race on the array: serialise them.
+ *  - All calls share the one array. The counters have to be zero when a call starts: they are
+ *    zero when the library is loaded and every call hands them back zeroed, also one in which a
+ *    bounded wait ran out. Two calls that overlap on the GPU (different streams, or threads) race
+ *    on the array: serialise them.
  *  - A sequence already at max_len is skipped as in dadattn_decode_bf16 and noted in a word
  *    beside the array; dadattn_decode_noalloc_status reads it (dadattn_device_status belongs to
- *    the allocating calls and does not see it). */
+ *    the other calls and does not see it). */
 int dadattn_decode_bf16_noalloc(uint16_t* out, const uint16_t* q, const uint16_t* k_new,
                                 const uint16_t* v_new, uint16_t* k_cache, uint16_t* v_cache,
                                 int32_t* lengths, int B, int H, int D, int max_len, float scale,
@@ -317,8 +314,7 @@ int dadattn_decode_bf16_noalloc(uint16_t* out, const uint16_t* q, const uint16_t
 /* Waits for `stream`, then returns and clears the status word of dadattn_decode_bf16_noalloc on
  * the current device: 0, DADATTN_E_ARG when a call since the last read skipped a sequence whose
  * length was outside [0, max_len), or DADATTN_E_TIMEOUT when a bounded wait ran out (the array
- * stays usable). Copies from and to a symbol of the library image, so it
- * allocates nothing either. No counterpart in the reference. */
+ * stays usable). No counterpart in the reference. */
 int dadattn_decode_noalloc_status(dadattn_stream_t stream);
 
 /* Synchronises the stream and returns the sticky device-side status word of this device
