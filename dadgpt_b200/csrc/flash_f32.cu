@@ -2,8 +2,9 @@
 // gpu_flash_attention_forward / gpu_flash_attention_backward (reference cuda/attention.cu).
 //
 // Head sizes 16, 32 and 64 run on the tensor cores with exactly split operands (flash_f32_tc_*.cu).
-// The kernels here are FFMA arithmetic, for head size 128, whose three planes of four resident and
-// streamed tiles do not fit into a CTA's shared memory. Where the reference gives one thread a whole
+// The kernels here are FFMA arithmetic, for head size 128: in the backward as laid out there the three
+// planes of a 128-wide item's tiles exceed a CTA's shared memory (Q and dO alone 192 KB); the forward's
+// would fit, with smaller steps (Q 96 KB, two stages of 32 rows of K and V 96 KB), and is not built. Where the reference gives one thread a whole
 // query row and a 32-thread block, they tile 64 queries x 64 keys per 256-thread block with 4x4
 // register micro-tiles, so a tile of K/V is read from shared memory once per 64 rows instead of
 // once per row. Semantics kept from the reference: lse = rowmax + ln(rowsum) of the scaled
@@ -23,35 +24,20 @@ constexpr int kThreads = 256;  // 16 x 16 threads
 constexpr int kPStride = kTile + 4;
 constexpr int kDeltaKernelFrom = 512;   // sequence length from which delta gets a kernel of its own
 
-template <int N>
+template <int N>   // a multiple of 4
 __device__ __forceinline__ void load_vec(float (&dst)[N], const float* src) {
-  if constexpr (N % 4 == 0) {
 #pragma unroll
-    for (int i = 0; i < N; i += 4) {
-      float4 t = *reinterpret_cast<const float4*>(src + i);
-      dst[i] = t.x; dst[i + 1] = t.y; dst[i + 2] = t.z; dst[i + 3] = t.w;
-    }
-  } else if constexpr (N == 2) {
-    float2 t = *reinterpret_cast<const float2*>(src);
-    dst[0] = t.x; dst[1] = t.y;
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; ++i) dst[i] = src[i];
+  for (int i = 0; i < N; i += 4) {
+    float4 t = *reinterpret_cast<const float4*>(src + i);
+    dst[i] = t.x; dst[i + 1] = t.y; dst[i + 2] = t.z; dst[i + 3] = t.w;
   }
 }
 
 template <int N>
 __device__ __forceinline__ void store_vec(float* dst, const float (&src)[N]) {
-  if constexpr (N % 4 == 0) {
 #pragma unroll
-    for (int i = 0; i < N; i += 4)
-      *reinterpret_cast<float4*>(dst + i) = make_float4(src[i], src[i + 1], src[i + 2], src[i + 3]);
-  } else if constexpr (N == 2) {
-    *reinterpret_cast<float2*>(dst) = make_float2(src[0], src[1]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; ++i) dst[i] = src[i];
-  }
+  for (int i = 0; i < N; i += 4)
+    *reinterpret_cast<float4*>(dst + i) = make_float4(src[i], src[i + 1], src[i + 2], src[i + 3]);
 }
 
 // Copies rows [row0, row0+64) of a [S, D] matrix into shared memory (row stride D+4), zero
