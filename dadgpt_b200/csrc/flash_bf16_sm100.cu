@@ -12,17 +12,16 @@
 //               warp_id % 4). Each half keeps its OWN running max / sum and its OWN output
 //               accumulator in TMEM, so the two threads of a row never synchronise inside the
 //               loop; the halves are merged once, in the epilogue (split-K inside the CTA).
-//               Eight softmax warps give every scheduler two (four with two CTAs per SM) warps
-//               to hide the FFMA -> MUFU -> FADD latencies behind each other.
-//               A thread reads its 64 scores with tcgen05.ld, writes P as bf16 into shared
-//               memory in the 128-byte-swizzled layout the MMA reads, and rescales its O half
-//               in TMEM only when its max grew by more than 2^8 (lazy rescale; exact result).
+//               Eight softmax warps give every scheduler two warps to hide the FFMA -> MUFU ->
+//               FADD latencies behind each other.
+//               A thread reads its 64 scores with tcgen05.ld, writes P as packed bf16 over them,
+//               and rescales its O half in TMEM only when its max grew by more than 2^8 (lazy
+//               rescale; exact result).
 // S_{j+1} is issued before P_j V_j, so the tensor core works on the next tile while the
-// exponentials of the current one are computed; at D = 64 two CTAs share an SM, at D = 128 the
-// scores are double-buffered in TMEM instead.
+// exponentials of the current one are computed; the scores are double-buffered in TMEM.
 //
-// The kernel template takes head sizes 64 and 128; the library instantiates it for 128 only: head
-// size 64 is served by the persistent two-tile kernel of flash_fwd64_sm100.cu.
+// Head size 128; size 64 has the persistent two-tile kernel of flash_fwd64_sm100.cu. The entry points
+// of both are here.
 //
 // Every mbarrier wait is bounded (sm100_ptx.cuh). If one runs out, the CTA raises its abort
 // flag, everybody falls through to the common exit, TMEM is freed, and DADATTN_E_TIMEOUT is
@@ -109,45 +108,40 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8
 
-template <int D>
+constexpr int kD = 128;           // head size
+constexpr int kPanels = kD / 64;  // 128-byte wide panels of a row
+
+// The probabilities P live in tensor memory between the softmax warps and the P V MMA, written over
+// the scores they were computed from and read by the MMA as its A operand: an MMA with both operands
+// in shared memory reads 8 KB per 64 clocks, all of an SM's shared-memory bandwidth, so every byte of
+// P kept out of shared memory counts.
 struct FwdSmem {
-  static constexpr int kPanels = D / 64;
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kPanels * kPanelBytes;
   static constexpr int kV = kK + kStages * kPanels * kPanelBytes;
-  static constexpr int kP = kV + kStages * kPanels * kPanelBytes;
-  // Where the probabilities P live between the softmax warps and the P V MMA. D = 128: in
-  // tensor memory, written over the scores they were computed from and read by the MMA as its
-  // A operand (an MMA with both operands in shared memory reads 8 KB per 64 clocks, all of an
-  // SM's shared-memory bandwidth, so every byte of P kept out of shared memory counts).
-  // D = 64: one bf16 tile in shared memory.
-  static constexpr bool kPTmem = D == 128;
-  static constexpr int kBars = kP + (kPTmem ? 0 : 2 * kPanelBytes);
+  static constexpr int kBars = kV + kStages * kPanels * kPanelBytes;
   static constexpr int kBytes = kBars + 256;
 };
 
 struct FwdBars {
   uint64_t q_full, k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
-  uint64_t s_full[2], s_free[2], p_full, o_done[2], stat_full;  // P_j V_j commits to o_done[j & 1]
+  uint64_t s_full[2], p_full, o_done[2], stat_full;  // P_j V_j commits to o_done[j & 1]
   uint32_t tmem_base;
   int abort_flag;
 };
 
-template <int D, bool DROP>
-__global__ void __launch_bounds__(kFwdThreads, D == 64 ? 2 : 1)
+template <bool DROP>
+__global__ void __launch_bounds__(kFwdThreads, 1)
 flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                       float* __restrict__ lse, int S, float scale, float rate, PhiloxKey rng,
                       int64_t unit0, LeveledGrid order, int* __restrict__ status) {
-  using L = FwdSmem<D>;
-  constexpr int kPanels = L::kPanels;
-  // TMEM columns. D = 64: S [0,128), O_0 [128,192), O_1 [192,256): 256 columns, two CTAs per SM.
-  // D = 128 (one CTA per SM): two S buffers [0,256) so that Q K^T of the next tile runs while
-  // this tile's softmax still reads its scores, O_0 [256,384), O_1 [384,512).
-  constexpr int kSBufs = D == 128 ? 2 : 1;
-  constexpr uint32_t kTmemCols = D == 128 ? 512 : 256;
-  constexpr uint32_t kColS = 0, kColO = 128 * kSBufs;
+  using L = FwdSmem;
+  // TMEM columns: two S buffers [0,256) so that Q K^T of the next tile runs while this tile's softmax
+  // still reads its scores, O_0 [256,384), O_1 [384,512).
+  constexpr uint32_t kTmemCols = 512;
+  constexpr uint32_t kColS = 0, kColO = 256;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   FwdBars* bars = reinterpret_cast<FwdBars*>(smem + L::kBars);
@@ -173,10 +167,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_init(&bars->k_empty[s], 1);
       mbar_init(&bars->v_empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&bars->s_full[b], 1);
-      mbar_init(&bars->s_free[b], kSoftmaxThreads);
-    }
+    for (int b = 0; b < 2; ++b) mbar_init(&bars->s_full[b], 1);
     mbar_init(&bars->p_full, kSoftmaxThreads);
     mbar_init(&bars->o_done[0], 1);
     mbar_init(&bars->o_done[1], 1);
@@ -225,9 +216,8 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     // ------------------------------ MMA issuer ------------------------------
     if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(kBM, kBN, 0, 0);  // Q, K: K-major
-      constexpr uint32_t idesc_o = make_idesc_bf16(kBM, D, 0, 1);    // P K-major, V MN-major
+      constexpr uint32_t idesc_o = make_idesc_bf16(kBM, kD, 0, 1);   // P K-major, V MN-major
       const SmemDescBase q_desc = make_desc_base_sw128(smem_u32(smem + L::kQ), 0);
-      const SmemDescBase p_desc = make_desc_base_sw128(smem_u32(smem + L::kP), 0);
       const SmemDescBase k_desc0 = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
       const SmemDescBase v_desc0 = make_desc_base_sw128(smem_u32(smem + L::kV), kPanelBytes);
       constexpr uint32_t kStageBytes = kPanels * kPanelBytes;
@@ -240,19 +230,14 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         const SmemDescBase v_desc{v_desc0.lo + s * (kStageBytes >> 4), v_desc0.hi};
-        // One MMA per 16 keys covers all D output columns: the V tile is MN-major, its 64-column
+        // One MMA per 16 keys covers all 128 output columns: the V tile is MN-major, its 64-column
         // panels are kPanelBytes apart, which is what the descriptor's leading byte offset says.
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            if (L::kPTmem)  // P_i sits in the first 32 columns of each half of score buffer i % 2
-              mma_ts(tmem + kColO + h * D, tmem + kColS + (i % kSBufs) * 128 + h * 64 + kk * 8,
-                     desc_at(v_desc, (h * 4 + kk) * 2048), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
-            else
-              mma_ss(tmem + kColO + h * D, desc_at(p_desc, h * kPanelBytes + kk * 32),
-                     desc_at(v_desc, (h * 4 + kk) * 2048), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < 4; ++kk)   // P_i sits in the first 32 columns of each half of score buffer i % 2
+            mma_ts(tmem + kColO + h * kD, tmem + kColS + (i % 2) * 128 + h * 64 + kk * 8,
+                   desc_at(v_desc, (h * 4 + kk) * 2048), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
         }
         mma_commit(&bars->v_empty[s]);
         mma_commit(&bars->o_done[i & 1]);
@@ -261,26 +246,21 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
 
       for (int j = 0; ok && j < n_kv; ++j) {
         const int s = j % kStages;
-        // With P in the only score buffer, P_{j-1} V_{j-1} must be issued before S_j replaces it
-        if (L::kPTmem && kSBufs == 1 && j > 0) ok = issue_pv(j - 1);
-        ok = ok && mbar_wait(&bars->k_full[s], (j / kStages) & 1, abort_flag);
-        const int sb = j % kSBufs;
-        // With P in TMEM, score buffer sb is next overwritten by S_j only after P_{j-2} V_{j-2},
-        // which was issued earlier by this same thread: the tensor pipe keeps them in order.
-        if (!L::kPTmem && ok && j >= kSBufs)
-          ok = mbar_wait(&bars->s_free[sb], (j / kSBufs - 1) & 1, abort_flag);
-        if (!ok) break;
+        // Score buffer sb is overwritten by S_j only after P_{j-2} V_{j-2}, which was issued earlier
+        // by this same thread: the tensor pipe keeps them in order.
+        const int sb = j % 2;
+        if (!(ok = mbar_wait(&bars->k_full[s], (j / kStages) & 1, abort_flag))) break;
         tc_fence_after_sync();
         const SmemDescBase k_desc{k_desc0.lo + s * (kStageBytes >> 4), k_desc0.hi};
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
+        for (int kk = 0; kk < kD / 16; ++kk) {
           const uint32_t off = (kk / 4) * kPanelBytes + (kk % 4) * 32;
           mma_ss(tmem + kColS + sb * 128, desc_at(q_desc, off), desc_at(k_desc, off), idesc_s,
                  kk > 0 ? 1u : 0u);
         }
         mma_commit(&bars->k_empty[s]);
         mma_commit(&bars->s_full[sb]);
-        if (!(L::kPTmem && kSBufs == 1) && j > 0) ok = issue_pv(j - 1);
+        if (j > 0) ok = issue_pv(j - 1);
       }
       if (ok) issue_pv(n_kv - 1);
     }
@@ -291,51 +271,37 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     const int row = quad * 32 + lane;     // row within the tile = TMEM lane
     const int r = q0 + row;               // query index
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-    const uint32_t tO = tlane + kColO + half * D;  // this half's output accumulator
+    const uint32_t tO = tlane + kColO + half * kD;  // this half's output accumulator
     const float scale_log2 = scale * kLog2e;
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
-    uint8_t* p_row0 = smem + L::kP + half * kPanelBytes + row * 128;
     // waits for P_i V_i (tile i) to have completed
     auto wait_pv = [&](int i) { return mbar_wait(&bars->o_done[i & 1], (i >> 1) & 1, abort_flag); };
     float m = -INFINITY, l = 0.f;  // running max (log2 units, scaled) and sum of this half-row
     bool ok = true;
 
     for (int j = 0; j < n_kv; ++j) {
-      const int sb = j % kSBufs;
+      const int sb = j % 2;
       const uint32_t tS = tlane + kColS + sb * 128 + half * 64;
-      if (!(ok = mbar_wait(&bars->s_full[sb], (j / kSBufs) & 1, abort_flag))) break;
+      if (!(ok = mbar_wait(&bars->s_full[sb], (j / 2) & 1, abort_flag))) break;
       tc_fence_after_sync();
       const int c0 = j * kBN + half * 64;  // first key of this thread's 64 columns
       // Only the diagonal tile needs the causal mask: columns beyond `limit` are dropped.
       const bool diagonal = (j == n_kv - 1);
       const int limit = r - c0;
 
-      // The thread's 64 scores are read from TMEM (both 32-column loads in flight together).
-      // At D = 128 (registers to spare) they stay in registers for the max and for the
-      // exponentials and S is handed back to the MMA warp at once; at D = 64 (two CTAs per SM,
-      // 96 registers) they are read a second time after the max instead of being kept.
-      constexpr bool kKeepScores = (D == 128);
+      // The thread's 64 scores, both 32-column loads in flight together; they stay in registers for the
+      // max and for the exponentials.
       uint32_t xa[32], xb[32];
-      auto load_scores = [&]() {
-        tmem_ld32(tS, xa);
-        tmem_ld32(tS + 32, xb);
-        tmem_wait_ld();
-        if (diagonal) {
+      tmem_ld32(tS, xa);
+      tmem_ld32(tS + 32, xb);
+      tmem_wait_ld();
+      if (diagonal) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i > limit) xa[i] = 0xff800000u;  // -inf
-            if (32 + i > limit) xb[i] = 0xff800000u;
-          }
+        for (int i = 0; i < 32; ++i) {
+          if (i > limit) xa[i] = 0xff800000u;  // -inf
+          if (32 + i > limit) xb[i] = 0xff800000u;
         }
-      };
-      auto release_scores = [&]() {  // S is in registers: the next QK^T may overwrite it
-        if (!L::kPTmem) {
-          tc_fence_before_sync();
-          mbar_arrive(&bars->s_free[sb]);
-        }
-      };
-      load_scores();
-      if (kKeepScores) release_scores();
+      }
       // max of the raw scores (scale > 0 commutes with max)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -343,18 +309,16 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         mx4[i & 3] = fmax3(mx4[i & 3], __uint_as_float(xa[i]), __uint_as_float(xb[i]));
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
 
-      bool waited_o = false;
       if (j == 0) {
         m = mx;  // O is first written by an MMA with accumulate = 0: nothing to rescale
       } else if (__any_sync(0xffffffffu, mx > m + kRescaleThreshold)) {
         if (!(ok = wait_pv(j - 1))) break;
-        waited_o = true;
         tc_fence_after_sync();
         const float m_new = fmaxf(m, mx);
         // m = -inf: nothing but zeros has been accumulated so far (every earlier column masked)
         const float corr = (m == -INFINITY) ? 0.f : ex2(m - m_new);
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = 0; c < kD / 32; ++c) {
           uint32_t o[32];
           tmem_ld32(tO + c * 32, o);
           tmem_wait_ld();
@@ -366,18 +330,14 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         l *= corr;
         m = m_new;
       }
-      // P in shared memory: the MMA that read the buffer last (tile j - 1) must have completed
-      if (!L::kPTmem && j > 0 && !waited_o && !(ok = wait_pv(j - 1))) break;
-      uint8_t* p_row = p_row0;
 
       // ---- p = exp2(s * scale * log2e - m), packed two-float FMAs and sums (192 x 8192: 3.43 -> 3.26 ms,
-      // issue slots and power; a share of the exponentials on the FMA pipe: 3.29-3.34); bf16 P goes
-      // to shared memory in the swizzled K-major layout. A half-row with no visible key yet has
+      // issue slots and power; a share of the exponentials on the FMA pipe: 3.29-3.34). A half-row with no visible key yet has
       // m = -inf: its scores are all -inf and must give p = 0, not exp2(nan). ----
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       const float2 sl = make_float2(scale_log2, scale_log2);
       const float neg_m = (m == -INFINITY) ? 0.f : -m;
-      uint32_t pk[L::kPTmem ? 32 : 1];  // packed P of this thread when it goes to TMEM
+      uint32_t pk[32];  // packed P of this thread
       auto process = [&](uint32_t (&x)[32], int ch) {
         float pv[32];
         const float2 nm = make_float2(neg_m, neg_m);
@@ -394,43 +354,22 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
           for (int i = 0; i < 32; ++i)
             pv[i] = (pv[i] != 0.f && philox_keep(rng, idx0 + i, rate)) ? pv[i] * keep_scale : 0.f;
         }
-        if (L::kPTmem) {
-          // bf16 pairs (k, k+1) per 32-bit TMEM column: 16 columns for these 32 probabilities
+        // bf16 pairs (k, k+1) per 32-bit TMEM column: 16 columns for these 32 probabilities
 #pragma unroll
-          for (int i = 0; i < 16; ++i) pk[ch * 16 + i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
-        } else {
-#pragma unroll
-          for (int v4 = 0; v4 < 4; ++v4) {
-            uint4 w;
-            w.x = pack_bf16(pv[v4 * 8 + 0], pv[v4 * 8 + 1]);
-            w.y = pack_bf16(pv[v4 * 8 + 2], pv[v4 * 8 + 3]);
-            w.z = pack_bf16(pv[v4 * 8 + 4], pv[v4 * 8 + 5]);
-            w.w = pack_bf16(pv[v4 * 8 + 6], pv[v4 * 8 + 7]);
-            const int chunk = ch * 4 + v4;  // 16-byte chunk within the 128-byte row
-            *reinterpret_cast<uint4*>(p_row + ((chunk ^ (row & 7)) << 4)) = w;
-          }
-        }
+        for (int i = 0; i < 16; ++i) pk[ch * 16 + i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
       };
-      if (!kKeepScores) {
-        load_scores();
-        release_scores();
-      }
       process(xa, 0);
       process(xb, 1);
       l += (sum2[0].x + sum2[1].x) + (sum2[0].y + sum2[1].y);
-      if (L::kPTmem) {
-        tmem_st32(tS, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-        tmem_wait_st();
-      } else {
-        fence_proxy_async_smem();
-      }
+      tmem_st32(tS, pk);
+      tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(&bars->p_full);
     }
 
     // Epilogue: merge the two halves of each row. out = (O_0 w_0 + O_1 w_1) / (l_0 w_0 + l_1 w_1)
     // with w_h = exp2(m_h - max(m_0, m_1)); lse in natural-log units of the scaled scores.
-    // Each thread of the pair writes half of the row's D outputs.
+    // Each thread of the pair writes half of the row's 128 outputs.
     // The (max, sum) pairs are exchanged through the Q tile's shared memory, which nobody reads
     // any more: every Q K^T has completed before the last s_full was observed.
     float2* stat = reinterpret_cast<float2*>(smem + L::kQ);  // [2][128]
@@ -448,13 +387,13 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       const float w1 = (s1.x == -INFINITY) ? 0.f : ex2(s1.x - m_tot);
       const float l_tot = s0.y * w0 + s1.y * w1;
       const float f0 = w0 / l_tot, f1 = w1 / l_tot;
-      constexpr int kCols = D / 2;  // output columns per thread
-      __nv_bfloat16* dst = out + (static_cast<size_t>(bh) * S + r) * D + half * kCols;
+      constexpr int kCols = kD / 2;  // output columns per thread
+      __nv_bfloat16* dst = out + (static_cast<size_t>(bh) * S + r) * kD + half * kCols;
 #pragma unroll
       for (int c = 0; c < kCols / 32; ++c) {
         uint32_t oa[32], ob[32];
         tmem_ld32(tlane + kColO + half * kCols + c * 32, oa);
-        tmem_ld32(tlane + kColO + D + half * kCols + c * 32, ob);
+        tmem_ld32(tlane + kColO + kD + half * kCols + c * 32, ob);
         tmem_wait_ld();
         if (r < S) {
 #pragma unroll
@@ -484,21 +423,21 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
   if (threadIdx.x == 0 && bars->abort_flag) report_timeout(status, bars->abort_flag);
 }
 
-template <int D, bool DROP>
+template <bool DROP>
 int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k,
                     const uint16_t* v, int BH, int S, float scale, float rate, uint64_t seed,
                     uint64_t offset, int64_t unit0, cudaStream_t st) {
   CUtensorMap mq, mk, mv;
-  if (int rc = make_tensor_map_bf16(&mq, q, BH, S, D, kBM)) return rc;
-  if (int rc = make_tensor_map_bf16(&mk, k, BH, S, D, kBN)) return rc;
-  if (int rc = make_tensor_map_bf16(&mv, v, BH, S, D, kBN)) return rc;
+  if (int rc = make_tensor_map_bf16(&mq, q, BH, S, kD, kBM)) return rc;
+  if (int rc = make_tensor_map_bf16(&mk, k, BH, S, kD, kBN)) return rc;
+  if (int rc = make_tensor_map_bf16(&mv, v, BH, S, kD, kBN)) return rc;
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  auto kern = flash_fwd_bf16_kernel<D, DROP>;
+  auto kern = flash_fwd_bf16_kernel<DROP>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                FwdSmem<D>::kBytes));
+                                FwdSmem::kBytes));
   const LeveledGrid order = leveled_grid(32768, S, BH);   // (16384 and 65536: 0-4 % slower or the same)
-  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kBM - 1) / kBM), dim3(kFwdThreads), FwdSmem<D>::kBytes, st,
+  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kBM - 1) / kBM), dim3(kFwdThreads), FwdSmem::kBytes, st,
                       mq, mk, mv, reinterpret_cast<__nv_bfloat16*>(out), lse, S, scale, rate,
                       make_philox(seed, offset), unit0, order, status));
   return DADATTN_OK;
@@ -531,8 +470,8 @@ extern "C" int dadattn_flash_fwd_bf16(uint16_t* out, float* lse, const uint16_t*
   const bool drop = rate > 0.f;
   if (D == 64)   // head size 64 has a kernel of its own (flash_fwd64_sm100.cu)
     return launch_fwd_bf16_d64(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, nullptr, 0, st);
-  return drop ? launch_fwd_bf16<128, true>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st)
-              : launch_fwd_bf16<128, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
+  return drop ? launch_fwd_bf16<true>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st)
+              : launch_fwd_bf16<false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
 }
 
 extern "C" int dadattn_flash_fwd_bf16_masked(uint16_t* out, float* lse, const uint16_t* q,
