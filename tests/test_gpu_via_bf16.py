@@ -10,6 +10,7 @@ import dadgpt_b200 as dad
 from dadgpt_b200 import _lib
 from dadgpt_b200.attention import device_status, flash_f32_via_bf16_workspace_bytes
 from tests.gpu_util import max_abs, rel_l2
+from tests.test_gpu_f32_tensor_core import _reference
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +44,25 @@ def test_forward_backward_against_oracle(cuda, oracle, S, D):
         else:
             assert rel_l2(got.cpu().numpy(), ref) <= 3e-2, name
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("BH,S", [(60, 700), (300, 100), (170, 257), (40, 1024)])
+def test_several_items_per_cta(cuda, BH, S):
+    """More (key tile, unit) items than SMs: the fp32-result variant of the gradient kernel passes its dQ
+    staging buffer and each item's K / V buffers from item to item. Judged unit by unit against float64."""
+    D, scale = 64, 0.125
+    g = torch.Generator(device=cuda).manual_seed(BH)
+    q, k, v, do = (torch.randn(BH, S, D, device=cuda, generator=g) for _ in range(4))
+    ws = torch.empty(flash_f32_via_bf16_workspace_bytes(BH, S, D), dtype=torch.uint8, device=cuda)
+    out, lse = torch.full_like(q, float("nan")), torch.full((BH, S), float("nan"), device=cuda)
+    grads = [torch.full_like(q, float("nan")) for _ in range(3)]
+    dad.gpu_flash_attention_forward_via_bf16(out, lse, q, k, v, BH, S, D, scale, ws)
+    dad.gpu_flash_attention_backward_via_bf16(*grads, do, out, lse, q, k, v, BH, S, D, scale, ws)
+    assert device_status() == 0
+    want = _reference(*(rounded(t) for t in (q, k, v, do)), scale)
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), (out, lse, *grads), want):
+        err = (a.double() - b).flatten(1).norm(dim=1) / b.flatten(1).norm(dim=1)
+        assert err.max().item() <= 3e-2, name
 
 
 def test_argument_checks_and_precision_switch(cuda):
