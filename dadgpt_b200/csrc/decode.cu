@@ -51,7 +51,7 @@ constexpr int kItemRing = 2;        // items a CTA's producer may be ahead
 constexpr unsigned kTicketGroups = 32;  // first-level counters of the "all lengths read" tickets
 constexpr int kMaxRanked = 256;     // sequences whose lengths a CTA copies and can rank
 constexpr int kMaxCluster = 8;      // CTAs that share a head of one sequence (portable cluster size)
-constexpr long long kBytesPerRank = 262144;   // and the K + V bytes that are worth one of them
+constexpr long long kBytesPerRank = 65536;    // and the K + V bytes that are worth one of them
 
 // A 16-byte piece of a row as float pairs, and the softmax's exponential. Scores are kept in units
 // that exp_of() takes: natural units and expf for fp32 caches, log2 units and ex2 for bf16 ones
@@ -585,10 +585,18 @@ int launch_decode(T* out, const T* q, const T* k_new, const T* v_new, T* k_cache
   DAD_CUDA(cudaGetDevice(&dev));
   DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const long long pairs = static_cast<long long>(B) * H;
-  // CTAs per (sequence, head): as many as the longest sequence there can be has 256 KB of K and V
+  // CTAs per (sequence, head): as many as the longest sequence there can be has 64 KB of K and V
   // for, while all of the call's CTAs still fit on the GPU at once. Beyond that, waiting clusters
   // cost more than the finer cut gives (4 sequences x 24 heads of up to 8000 rows: 131 us with 4 CTAs
-  // each, 145 with 8).
+  // each, 145 with 8). us a call in a CUDA graph, 12 heads x 64, by KB of K and V per CTA:
+  //                                  32      64     128     256
+  //   fp32, 150 rows               3.54    3.88    4.01    4.01
+  //   fp32, 300 rows               4.10    4.31    4.95    6.10
+  //   fp32, 700 rows               4.78    4.78    5.55    7.08
+  //   bf16, 700 rows               4.69    4.91    5.97    6.95
+  //   bf16, 4 x 50-200 rows        4.53    4.27    4.27    4.23
+  //   bf16, 10 x 80-800 rows       8.19    8.36    8.36    8.71
+  // (fp32, 16 heads x 16, 400 rows: 4.22, 3.80 from 64 on.)
   const long long bytes = static_cast<long long>(lengths ? max_len : fixed_len + 1) * 2 * DH * sizeof(T);
   const int resident = kManyPerSm * sms;
   int ranks = 1;

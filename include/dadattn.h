@@ -255,7 +255,7 @@ int dadattn_decode_bf16(uint16_t* out, const uint16_t* q, const uint16_t* k_new,
 /* dadattn_decode_f32 for B sequences at once, on fp32 caches [B,H,max_len,D] with lengths[B] as in
  * dadattn_decode_bf16 (same workspace rules, dadattn_decode_workspace_bytes). Head sizes 16, 32,
  * 64, 128. This is what a batched generation loop over the reference's fp32 model calls once per
- * layer; results equal B separate dadattn_decode_f32 calls. No counterpart in the reference, which
+ * layer; results equal B separate dadattn_decode_f32 calls up to the order of the sums. No counterpart in the reference, which
  * decodes one sequence at a time (src/generate.cpp:94-139). */
 int dadattn_decode_f32_batched(float* out, const float* q, const float* k_new, const float* v_new,
                                float* k_cache, float* v_cache, int32_t* lengths, int B, int H, int D,
