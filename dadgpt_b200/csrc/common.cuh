@@ -199,10 +199,12 @@ int launch_bwd_fused_d64_f32(float* dq32, float* dk32, float* dv32, const float*
 int launch_fwd_f32_tc(float* out, float* lse, const float* q, const float* k, const float* v, int BH, int S, int D,
                       float scale, float rate, uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok,
                       cudaStream_t st);
-// delta = rowsum(dO o O), or nullptr: the kernel then forms it from the rows it loads anyway.
-int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* delta, const float* dout, const float* out,
-                      const float* lse, const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+// delta: scratch of BH * S floats for rowsum(dO o O), which launch_delta_f32_d64 (flash_f32.cu) forms at
+// head size 64.
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, float* delta, const float* dout, const float* out, const float* lse,
+                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st);
+int launch_delta_f32_d64(float* delta, const float* dout, const float* out, int64_t rows, bool vec_ok, cudaStream_t st);
 
 // Launch with programmatic stream serialization: the grid may become resident while its
 // predecessor in the stream drains, runs its set-up (barriers, TMEM, descriptor prefetch), and

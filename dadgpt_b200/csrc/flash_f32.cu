@@ -22,7 +22,6 @@ namespace {
 constexpr int kTile = 64;      // queries per block and keys per shared-memory tile
 constexpr int kThreads = 256;  // 16 x 16 threads
 constexpr int kPStride = kTile + 4;
-constexpr int kDeltaKernelFrom = 512;   // sequence length from which delta gets a kernel of its own
 
 template <int N>   // a multiple of 4
 __device__ __forceinline__ void load_vec(float (&dst)[N], const float* src) {
@@ -238,7 +237,7 @@ flash_fwd_f32_kernel(float* __restrict__ out, float* __restrict__ lse, const flo
 template <int D>
 __global__ void flash_delta_f32_kernel(float* __restrict__ delta, const float* __restrict__ dout,
                                        const float* __restrict__ out, int64_t rows, bool vec_ok) {
-  constexpr int L = D / 4;  // lanes per row: 4, 8, 16, 32
+  constexpr int L = D / 4;  // lanes per row: 16 or 32
   pdl_wait();
   pdl_launch_dependents();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -522,6 +521,11 @@ int check_common(int BH, int S, int d_head, float rate) {
 }
 
 }  // namespace
+
+int launch_delta_f32_d64(float* delta, const float* dout, const float* out, int64_t rows, bool vec_ok, cudaStream_t st) {
+  return launch_delta<64>(delta, dout, out, rows, vec_ok, st);
+}
+
 }  // namespace dadattn
 
 using namespace dadattn;
@@ -567,16 +571,8 @@ extern "C" int dadattn_flash_bwd_f32_dropout(float* dq, float* dk, float* dv, fl
   if (d_head <= 64) {
     const bool vec_ok = aligned(dq, 16) && aligned(dk, 16) && aligned(dv, 16) && aligned(dout, 16) &&
                         aligned(out, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
-    // Short sequences save a launch (the tensor-core kernel forms delta itself); in long ones the
-    // extra rows would make its loaders the bottleneck (8 x 2048 x 64: 88 us, 102 without the delta
-    // kernel; 96 x 200 x 32: 30.4 us without it, 31.9 with it).
-    const bool own_delta = S < kDeltaKernelFrom;
-    if (!own_delta) {
-      auto* delta_of = d_head == 64 ? launch_delta<64> : d_head == 32 ? launch_delta<32> : launch_delta<16>;
-      if (int rc = delta_of(delta, dout, out, static_cast<int64_t>(BH) * S, vec_ok, st)) return rc;
-    }
-    return launch_bwd_f32_tc(dq, dk, dv, own_delta ? nullptr : delta, dout, out, lse, q, k, v, BH, S, d_head, scale,
-                             rate, seed, offset, unit0, vec_ok, st);
+    return launch_bwd_f32_tc(dq, dk, dv, delta, dout, out, lse, q, k, v, BH, S, d_head, scale, rate, seed, offset,
+                             unit0, vec_ok, st);
   }
   return rate > 0.f ? launch_bwd<128, true>(dq, dk, dv, delta, dout, out, lse, q, k, v, BH, S, scale, rate, seed,
                                             offset, unit0, st)

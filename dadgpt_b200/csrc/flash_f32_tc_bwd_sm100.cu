@@ -53,7 +53,8 @@ static_assert(sizeof(BwdBars) <= 256, "barrier block");
 
 struct BwdArgs {
   float *dq, *dk, *dv;
-  const float *dout, *out, *lse, *delta, *q, *k, *v;   // delta: null, or computed by an earlier kernel
+  const float *dout, *out, *lse, *q, *k, *v;
+  float* delta;   // scratch, used only where delta_given
   int BH, S;
   float scale, rate;
   PhiloxRounds rng;
@@ -90,9 +91,20 @@ __device__ __forceinline__ BwdItem bwd_item(int k, int BH, int S) {
   return it;
 }
 
+// Whether delta = rowsum(dO o O) comes from a kernel ahead instead of the rows of O that this one loads
+// beside those of dO. Forming it saves a launch and pays while the loaders have time for the rows: at
+// head sizes below 64, whose rows are short, and while no CTA has a second item. us, formed here / given:
+//   D = 16   32 x 301 15.6 / 17.4   48 x 1024 95.7 / 96.6     8 x 2048 62.4 / 64.4
+//   D = 32   32 x 301 17.0 / 18.7   48 x 1024 107.1 / 106.6   8 x 2048 71.6 / 71.4
+//   D = 64   16 x 200 17.4 / 18.3   8 x 1024 49.3 / 50.2      (64 and 128 items)
+//            32 x 301 23.4 / 23.9   8 x 2048 90.2 / 90.2      (192 and 256 items)
+//            96 x 200 38.3 / 36.6   200 x 256 81.7 / 76.4     48 x 1024 151.1 / 139.7
+constexpr bool delta_given(int D, bool many) { return D == 64 && many; }
+
 template <int D, bool DROP, bool MANY>   // MANY: more items than CTAs
 __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __grid_constant__ BwdArgs args) {
   using L = BwdSmem;
+  constexpr bool kDeltaGiven = delta_given(D, MANY);
   constexpr uint32_t kExtra = 256, kSum1 = 320, kSum2 = 384;   // kSum1: dV; kSum2: dK or dQ
   constexpr int V4 = D / 4;                                    // float4 pieces of a row
   constexpr int NC = D / 4;                                    // columns of a sum per thread
@@ -181,9 +193,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           if (!is_q) {
             const int rv = it.first + i * kStep + t;
             row_lse = t < kStep && rv < S ? __ldg(args.lse + unit + rv) : 0.f;
-            if (args.delta) row_delta = t < kStep && rv < S ? args.delta[unit + rv] : 0.f;
+            if (kDeltaGiven) row_delta = t < kStep && rv < S ? args.delta[unit + rv] : 0.f;
           }
-          if (!is_q && !args.delta) {
+          if (!is_q && !kDeltaGiven) {
             float4 xo[kMine];
             fetch(xo, args.out, it, i);
 #pragma unroll
@@ -200,10 +212,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
           if (!is_q) {
             if (t < kStep) vec[s2 * 128 + t] = row_lse;
-            if (t < kStep && args.delta) vec[s2 * 128 + 64 + t] = row_delta;
+            if (kDeltaGiven && t < kStep) vec[s2 * 128 + 64 + t] = row_delta;
 #pragma unroll
             for (int j = 0; j < kMine; ++j)
-              if (!args.delta && c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
+              if (!kDeltaGiven && c4 == 0 && rt + j * kRowStep < kStep) vec[s2 * 128 + 64 + rt + j * kRowStep] = delta[j];
           }
           fence_proxy_async_smem();
           mbar_arrive(&bars->b2_full[s2]);
@@ -321,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         x1[j] = load4(a1 + j * kRowStep * D, in, args.vec_ok);
         x2[j] = load4(a2 + j * kRowStep * D, in, args.vec_ok);
       }
-      const bool form_delta = it.is_q && !args.delta;
+      const bool form_delta = !kDeltaGiven && it.is_q;
       float4 xo[kMine];
       auto load_out = [&]() {
 #pragma unroll
@@ -388,12 +400,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const bool is_q = it.is_q;
       const int row0 = it.row0, first = it.first, n_it = it.n_it, bh = it.bh;
       if (nxt.valid) prefetch_resident(nxt);
-      if (is_q && !args.delta) compute_sync();   // delta of all rows
+      if (!kDeltaGiven && is_q) compute_sync();   // delta of all rows
       const int r_own = row0 + row;
       const size_t at_own = static_cast<size_t>(bh) * S + r_own;
       const float own_lse = is_q && r_own < S ? __ldg(args.lse + at_own) : 0.f;
       const float own_delta = !is_q ? 0.f
-                              : !args.delta ? reinterpret_cast<const float*>(smem + L::kOwn)[(n & 1) * kRows + row]
+                              : !kDeltaGiven ? reinterpret_cast<const float*>(smem + L::kOwn)[(n & 1) * kRows + row]
                               : r_own < S ? args.delta[at_own] : 0.f;
       const uint64_t unit = static_cast<uint64_t>(args.unit0 + bh) * S;
 
@@ -489,6 +501,8 @@ int launch(const BwdArgs& a, unsigned grid, cudaStream_t st) {
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::kBytes));
   static std::atomic<int> regs{0};
   if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs)) return rc;
+  if (delta_given(D, MANY))
+    if (int rc = launch_delta_f32_d64(a.delta, a.dout, a.out, static_cast<int64_t>(a.BH) * a.S, a.vec_ok, st)) return rc;
   DAD_CUDA(launch_pdl(kern, dim3(grid), dim3(kThreads), BwdSmem::kBytes, st, a));
   return DADATTN_OK;
 }
@@ -506,12 +520,12 @@ int launch(const BwdArgs& a, cudaStream_t st) {
 
 }  // namespace
 
-int launch_bwd_f32_tc(float* dq, float* dk, float* dv, const float* delta, const float* dout, const float* out,
-                      const float* lse, const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
+int launch_bwd_f32_tc(float* dq, float* dk, float* dv, float* delta, const float* dout, const float* out, const float* lse,
+                      const float* q, const float* k, const float* v, int BH, int S, int D, float scale, float rate,
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st) {
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  const BwdArgs a = {dq, dk, dv, dout, out, lse, delta, q, k, v, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
+  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, delta, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
                      status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
