@@ -44,9 +44,12 @@ constexpr int kGStages = 3;                // streamed-tile ring depth
 constexpr int kGThreads = 19 * 32;
 constexpr int kGCompute = 16 * 32;
 // Up to this many CTAs the key tiles go level by level (leveled_grid) and the delta kernel clears the
-// workspace: 24 x 2048 135 -> 112 us, 24 x 300 21.3 -> 19.0, 96 x 2048 445 -> 429, 24 x 8192 1354 -> 1305.
-// With more waves the order gains nothing and the cleared lines, by then out of L2, are better written by
-// a memset ahead of the reads (192 x 8192, 12288 CTAs: 10.35 ms, against 10.45 in the other form).
+// workspace; with more waves the order gains nothing and the cleared lines, by then out of L2, are better
+// written by a memset ahead of the reads. Backward alone, us by CTAs, level by level / unit by unit:
+//     192  24 x 1024   47 / 62      1536  192 x 1024   294-311 / 304-320   3072  192 x 2048  843-882 / 873-884
+//     384  24 x 2048  110 / 133     1800  600 x 300        200 / 206       3072  96 x 4096  1391-1428 / 1430
+//     768  48 x 2048  210 / 229     2048  64 x 4096    876-940 / 948-966   3072  48 x 8192  2540-2580 / 2460-2570
+// (192 x 8192, 12288 CTAs: 10.45 ms / 10.35)
 constexpr int kGLeveledBlocks = 2048;
 constexpr int kPrepareThreads = 256;         // of the delta kernel, whose blocks zero a part of one tile
 constexpr int kGDqTileBytes = kGD * kGSub * 4;   // one dQ^T tile, fp32
