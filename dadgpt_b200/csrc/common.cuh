@@ -117,7 +117,9 @@ __device__ __forceinline__ bool philox_keep(const PhiloxKey& p, uint64_t subsequ
 //  * Of the counter only the low subsequence word changes from draw to draw. The first round's
 //    product with the offset word is one number for the call, the second round's product with what
 //    comes of it one for the thread, and neither reaches the other lane before the third round: 13
-//    widening products, two high and one low are left of 20.
+//    widening products, three high and one low are left of 20. The pipe that multiplies integers sets the
+//    pace: at 192 x 1024 the mask kernel takes 250 us (265 with 19 widening products) and keeps it busy
+//    84 % of the time, at 54 % of the issue slots.
 struct PhiloxRounds {
   uint32_t k0[10], k1[9];   // key words of rounds 0..9 (the last round needs only k0)
   uint32_t c0, c1;          // low counter words: offset / 4
@@ -229,9 +231,9 @@ cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaSt
 // (whose tensors then stay in L2 while they are worked on), inside a group level by level. Blocks are
 // handed out in index order, so the long ones start first and the short ones fill the gaps at the end.
 // With one unit after the other, a launch of a few waves ended on whatever tile came last: the forward
-// at 24 x 2048 x 128 took 43.7 us, now 36.5, 96 x 512 23.0 and 21.3, 24 x 8192 428 and 403. Grid
-// dimensions rather than a division of one block index: those stay in uniform registers (2 % of the
-// forward's time).
+// at 24 x 2048 x 128 took 44.1 us, level by level 37.1, 96 x 512 23.6 and 22.6, 24 x 8192 433 and 417,
+// 192 x 8192 3427 and 3405. Grid dimensions rather than a division of one block index: those stay in
+// uniform registers (2 % of the forward's time).
 struct LeveledGrid {
   int group, units;
 };

@@ -8,8 +8,8 @@
 //     stages (8 KB of K, 8 KB of V) with bulk copies; four consumer warps read them from shared
 //     memory 512 contiguous bytes at a time. What is in flight does not depend on how the arithmetic
 //     is getting on: with loads and arithmetic taking turns in the same warps the kernel reached
-//     5.0 TB/s on 64 sequences x 12 heads of up to 1024 rows and 4.1 on 4 x 24 of up to 8000 at head
-//     size 128, now 5.8 and 5.4 (6.7 on 128 x 24 x 128);
+//     4.75 TB/s on 64 sequences x 12 heads of up to 1024 rows and 4.26 on 4 x 24 of up to 8000 at head
+//     size 128, now 5.56-5.7 and 4.85-5.2 (6.8 on 128 x 24 x 128; the lengths are drawn);
 //   * q.k partial sums are reduced over a row's D*sizeof(T)/16 lanes with warp shuffles; each lane
 //     keeps an online-softmax state (max, sum, D/lanes accumulators) for the rows it has seen. The
 //     row groups of a tile are handled without branches so that their latencies overlap: a CTA's
@@ -18,7 +18,7 @@
 //     a counter, the next item's rows already on their way while one is merged. Few pairs: the CTAs
 //     of a cluster share a pair and merge through distributed shared memory. Neither needs records in
 //     global memory, and a pair's merge costs no trip through L2 (8 sequences x 8 heads of up to 400
-//     rows: 6.9 us a layer with records and tickets, 4.0 now);
+//     rows, early start: 6.9 us a layer with records and tickets, 3.9 now);
 //   * the append is fused: the warp that owns row `len` takes k_new/v_new from the token's vectors,
 //     uses them, and stores them into the cache;
 //   * every CTA draws a ticket once it has copied the lengths; the holder of the last one stores

@@ -331,8 +331,8 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         m = m_new;
       }
 
-      // ---- p = exp2(s * scale * log2e - m), packed two-float FMAs and sums (192 x 8192: 3.43 -> 3.26 ms,
-      // issue slots and power; a share of the exponentials on the FMA pipe: 3.29-3.34). A half-row with no visible key yet has
+      // ---- p = exp2(s * scale * log2e - m), packed two-float FMAs and sums (192 x 8192: 3.41 -> 3.32 ms,
+      // 24 x 8192 419 -> 405 us, 24 x 2048 37.1 -> 36.8; a share of the exponentials on the FMA pipe was no faster). A half-row with no visible key yet has
       // m = -inf: its scores are all -inf and must give p = 0, not exp2(nan). ----
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       const float2 sl = make_float2(scale_log2, scale_log2);

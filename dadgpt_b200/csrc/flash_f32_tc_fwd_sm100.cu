@@ -9,8 +9,9 @@
 //               P V is added to an fp32 register sum, so the output is never rescaled in tensor memory
 //   warps 16-26 fetch fp32 K / V rows, split them in registers, fill the shared-memory rings
 //   warp 27     issues the products: P V of step i, scores of step i + 2, P V of step i + 1, ...
-// A step costs 2304 clocks of tensor pipe at head size 64 (24 + 24 products of 48) and about 1700
-// issue slots per scheduler.
+// A step costs 2304 clocks of tensor pipe at head size 64 (24 + 24 products of 48; the pipe's counter
+// takes 32) and about 2100 issue slots per scheduler, and takes about 3550 clocks (48 x 1024): the planes
+// of a step are stored only after the last step's sums have been taken.
 // CTAs are persistent where there are more items than SMs, as in the backward: the rings run on across
 // items and the next Q is fetched and split while the last sums complete (48 x 1024 x 64: 58 -> 55.6 us,
 // 148 x 512: 57.0 -> 46.6, 72 x 777: 69.9 -> 62.0).
