@@ -39,11 +39,6 @@ constexpr int kWarpLoader0 = 16, kWarpIssuer = 27;
 constexpr int kRegsLaunch = 72, kRegsCompute = 88, kRegsHelper = 48;
 static_assert(kComputeThreads * kRegsCompute + (kThreads - kComputeThreads) * kRegsHelper <= kThreads * kRegsLaunch, "register pool exceeded");
 
-// Waits in these kernels: few plain polls before the suspending form. Sixteen compute warps that poll
-// take issue slots from the loaders, which then set the pace.
-constexpr uint32_t kPolls = 16;
-#define tile_wait(bar, parity, abort_flag) mbar_wait_at<kPolls>(bar, parity, abort_flag, __LINE__)
-
 // Plane pairs of the six products, smallest first.
 __device__ __forceinline__ constexpr int product_a(int i) { return i == 0 ? 2 : i == 1 ? 0 : i == 2 ? 1 : i == 3 ? 1 : 0; }
 __device__ __forceinline__ constexpr int product_b(int i) { return i == 0 ? 0 : i == 1 ? 2 : i == 2 ? 1 : i == 3 ? 0 : i == 4 ? 1 : 0; }

@@ -98,6 +98,8 @@ namespace {
 
 using namespace ptx;
 
+#define hot_wait(bar, parity, abort_flag) mbar_wait_at<24>(bar, parity, abort_flag, __LINE__)
+
 constexpr int kBM = 128;          // query rows per CTA
 constexpr int kBN = 128;          // keys per tile
 constexpr int kStages = 2;        // K/V ring depth
@@ -202,11 +204,11 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         uint8_t* kdst = smem + L::kK + s * kPanels * kPanelBytes;
         uint8_t* vdst = smem + L::kV + s * kPanels * kPanelBytes;
         // K's slot frees when Q K^T of its previous tenant is done, V's when P V is done
-        if (use > 0 && !mbar_wait(&bars->k_empty[s], (use - 1) & 1, abort_flag)) break;
+        if (use > 0 && !hot_wait(&bars->k_empty[s], (use - 1) & 1, abort_flag)) break;
         mbar_arrive_expect_tx(&bars->k_full[s], kPanels * kPanelBytes);
         for (int p = 0; p < kPanels; ++p)
           tma_load_3d(kdst + p * kPanelBytes, &map_k, &bars->k_full[s], p * 64, j * kBN, bh);
-        if (use > 0 && !mbar_wait(&bars->v_empty[s], (use - 1) & 1, abort_flag)) break;
+        if (use > 0 && !hot_wait(&bars->v_empty[s], (use - 1) & 1, abort_flag)) break;
         mbar_arrive_expect_tx(&bars->v_full[s], kPanels * kPanelBytes);
         for (int p = 0; p < kPanels; ++p)
           tma_load_3d(vdst + p * kPanelBytes, &map_v, &bars->v_full[s], p * 64, j * kBN, bh);
@@ -221,13 +223,13 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       const SmemDescBase k_desc0 = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
       const SmemDescBase v_desc0 = make_desc_base_sw128(smem_u32(smem + L::kV), kPanelBytes);
       constexpr uint32_t kStageBytes = kPanels * kPanelBytes;
-      bool ok = mbar_wait(&bars->q_full, 0, abort_flag);
+      bool ok = hot_wait(&bars->q_full, 0, abort_flag);
 
       // O_h[:, 64 pn .. 64 pn + 63] (+)= P_i[:, 64 h .. 64 h + 63] V_i[64 h .. 64 h + 63, :]
       auto issue_pv = [&](int i) -> bool {
         const int s = i % kStages;
-        if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
-        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!hot_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!hot_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         const SmemDescBase v_desc{v_desc0.lo + s * (kStageBytes >> 4), v_desc0.hi};
         // One MMA per 16 keys covers all 128 output columns: the V tile is MN-major, its 64-column
@@ -249,7 +251,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         // Score buffer sb is overwritten by S_j only after P_{j-2} V_{j-2}, which was issued earlier
         // by this same thread: the tensor pipe keeps them in order.
         const int sb = j % 2;
-        if (!(ok = mbar_wait(&bars->k_full[s], (j / kStages) & 1, abort_flag))) break;
+        if (!(ok = hot_wait(&bars->k_full[s], (j / kStages) & 1, abort_flag))) break;
         tc_fence_after_sync();
         const SmemDescBase k_desc{k_desc0.lo + s * (kStageBytes >> 4), k_desc0.hi};
 #pragma unroll
@@ -275,14 +277,14 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     const float scale_log2 = scale * kLog2e;
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
     // waits for P_i V_i (tile i) to have completed
-    auto wait_pv = [&](int i) { return mbar_wait(&bars->o_done[i & 1], (i >> 1) & 1, abort_flag); };
+    auto wait_pv = [&](int i) { return hot_wait(&bars->o_done[i & 1], (i >> 1) & 1, abort_flag); };
     float m = -INFINITY, l = 0.f;  // running max (log2 units, scaled) and sum of this half-row
     bool ok = true;
 
     for (int j = 0; j < n_kv; ++j) {
       const int sb = j % 2;
       const uint32_t tS = tlane + kColS + sb * 128 + half * 64;
-      if (!(ok = mbar_wait(&bars->s_full[sb], (j / 2) & 1, abort_flag))) break;
+      if (!(ok = hot_wait(&bars->s_full[sb], (j / 2) & 1, abort_flag))) break;
       tc_fence_after_sync();
       const int c0 = j * kBN + half * 64;  // first key of this thread's 64 columns
       // Only the diagonal tile needs the causal mask: columns beyond `limit` are dropped.
@@ -376,7 +378,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     if (ok) {
       stat[half * 128 + row] = make_float2(m, l);
       mbar_arrive(&bars->stat_full);
-      ok = mbar_wait(&bars->stat_full, 0, abort_flag) &&
+      ok = hot_wait(&bars->stat_full, 0, abort_flag) &&
            wait_pv(n_kv - 1);
     }
     if (ok) {

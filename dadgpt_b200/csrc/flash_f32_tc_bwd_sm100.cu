@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
           for (int j = 0; j < kMine; ++j) sp[j] = split4(x[j]);
           fetch(x, is_q ? args.k : args.q, it, i);   // on its way while B2 goes to shared memory
-          if (lap2 > 0 && !(ok = tile_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
+          if (lap2 > 0 && !(ok = mbar_wait(&bars->b2_empty[s2], (lap2 - 1) & 1, abort_flag))) break;
           put(smem + L::kB2 + s2 * 3 * kPlaneB, sp);
           if (!is_q) {
             if (t < kStep) vec[s2 * 128 + t] = row_lse;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           const bool more = i + 1 < it.n_it;
           if (more || nxt.valid)
             fetch(x, (more ? is_q : nxt.is_q) ? args.v : args.dout, more ? it : nxt, more ? i + 1 : 0);
-          if (g >= 2 && !(ok = tile_wait(&bars->b1_empty[s], ((g >> 1) - 1) & 1, abort_flag))) break;
+          if (g >= 2 && !(ok = mbar_wait(&bars->b1_empty[s], ((g >> 1) - 1) & 1, abort_flag))) break;
           put(smem + L::kB1 + s * 3 * kPlaneB, sp);
           fence_proxy_async_smem();
           mbar_arrive(&bars->b1_full[s]);
@@ -255,10 +255,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
               mma_ss(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
                      idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
         };
-        if (!tile_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx + 64, a2, b2);
-        if (!tile_wait(&bars->b1_full[s], par, abort_flag)) return false;
+        if (!mbar_wait(&bars->b1_full[s], par, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx, a1, b1);
         mma_commit(&bars->x_full[s]);
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         const int s2 = i % 3;
         const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
         const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
-        if (!tile_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 streamed rows kk lie over the 16 columns their scores came from
         if (!is_q) {
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       for (int n = 0; ok && (MANY || n < 1); ++n) {
         const BwdItem it = MANY ? bwd_item<MANY>(n, args.BH, S) : item0;
         if (!it.valid) break;
-        ok = tile_wait(&bars->a_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        ok = mbar_wait(&bars->a_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_sums(g + i, it.is_q) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 
     float sum1[NC], sum2[NC];
     auto take_sums = [&](int i, bool is_q) -> bool {
-      if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       if (!is_q) tmem_add<NC>(tlane + kSum1 + cg * NC, sum1);
       tmem_add<NC>(tlane + kSum2 + cg * NC, sum2);
@@ -416,9 +416,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       for (int i = 0; i < n_it; ++i, ++step) {
         const int s = step & 1;
         const int col0 = first + i * kStep + cg * 16;        // streamed row of this thread's first column
-        if (!(ok = tile_wait(&bars->x_full[s], (step >> 1) & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->x_full[s], (step >> 1) & 1, abort_flag))) break;
         // (the row scalars came with B2)
-        if (!is_q && !(ok = tile_wait(&bars->b2_full[step % 3], (step / 3) & 1, abort_flag))) break;
+        if (!is_q && !(ok = mbar_wait(&bars->b2_full[step % 3], (step / 3) & 1, abort_flag))) break;
         tc_fence_after_sync();
         const uint32_t tx = tlane + s * 128 + cg * 16;
         float2 p[8], g[8];

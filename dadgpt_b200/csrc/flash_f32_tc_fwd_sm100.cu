@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
           float4 x[kMine];
           Split4 sp[kMine];
           auto put = [&](uint8_t* tile, uint64_t* empty, uint64_t* full) -> bool {
-            if (lap > 0 && !tile_wait(empty, (lap - 1) & 1, abort_flag)) return false;
+            if (lap > 0 && !mbar_wait(empty, (lap - 1) & 1, abort_flag)) return false;
 #pragma unroll
             for (int j = 0; j < kMine; ++j)
               if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         const int s = i % kStages;
         const uint32_t tx = tmem + (i & 1) * 64;
         const SmemDescBase kd{k0.lo + s * (3 * kPlaneB >> 4), k0.hi};
-        if (!tile_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int m = 0; m < 6; ++m)
@@ -198,8 +198,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         const int s = i % kStages;
         const uint32_t tx = tmem + (i & 1) * 64;
         const SmemDescBase vd{v0.lo + s * (3 * kPlaneB >> 4), v0.hi};
-        if (!tile_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
-        if (!tile_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 keys kk lie over the 16 columns their scores came from
 #pragma unroll
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       for (int n = 0; ok && (MANY || n < 1); ++n) {
         const FwdItem it = MANY ? fwd_item<MANY>(n, args.BH, S) : item0;
         if (!it.valid) break;
-        ok = tile_wait(&bars->q_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        ok = mbar_wait(&bars->q_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_pv(g + i) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     const float keep_scale = DROP ? 1.0f / (1.0f - args.rate) : 1.0f;
     float m = -FLT_MAX, l = 0.f, o[NC];
     auto take_sums = [&](int i) -> bool {
-      if (!tile_wait(&bars->acc_done, i & 1, abort_flag)) return false;
+      if (!mbar_wait(&bars->acc_done, i & 1, abort_flag)) return false;
       tc_fence_after_sync();
       tmem_add<NC>(tlane + kSum + cg * NC, o);
       return true;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       for (int c = 0; c < NC; ++c) o[c] = 0.f;
 
       for (int i = 0; i < n_it; ++i, ++step) {
-        if (!(ok = tile_wait(&bars->x_full[step & 1], (step >> 1) & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->x_full[step & 1], (step >> 1) & 1, abort_flag))) break;
         tc_fence_after_sync();
         const uint32_t tx = tlane + (step & 1) * 64 + cg * 16;
         const int c0 = i * kStep + cg * 16;

@@ -54,6 +54,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// (does not suspend)
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -66,29 +67,28 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-constexpr uint32_t kSpinLimit = 1u << 24;  // with the back-off below: a few seconds
-// Non-blocking polls before the suspending wait takes over. More than a few hundred cost time:
-// the polling of waiting warps competes for issue slots with the warps that still work.
-constexpr uint32_t kHotPolls = 128;
+constexpr uint32_t kSpinLimit = 1u << 21;  // a try_wait that fails has been suspended for about 3000 clocks: seconds
 
 // Waits for the phase with the given parity to complete. `abort_flag` (shared memory) is
 // polled too: once any thread of the CTA has given up, everybody leaves quickly. The thread
 // whose own wait runs out leaves `site` (the source line of the wait, through DAD_MBAR_WAIT)
 // in the flag, from where the kernel's exit path copies it next to the device status word.
-template <uint32_t HOT = kHotPolls>
-__device__ __forceinline__ bool mbar_wait_at(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                             int site) {
-  // Most waits in these kernels are short (a few hundred clocks: the next link of a pipeline). A
-  // suspending try_wait that has to be woken costs more than that, so the wait starts as a plain
-  // poll and only then turns into the suspending form with back-off.
-  for (uint32_t i = 0; i < HOT; ++i)
+//
+// The wait is a handful of instructions, and has to be: kernels with six roles hold some thirty of them.
+// As 128 polls, which the compiler unrolled, ahead of a try_wait loop with back-off, they made 280 of the
+// 333 KB of the head-size-64 gradient kernel; the warps stood still for instructions (a wait that was
+// ready took 200-400 clocks), and a step at 192 x 1024 x 64 took 200 us, so written 187. POLLS plain polls
+// come before the wait that suspends: 2 against none are worth 0.3 %, 24 cost the head-size-64 kernels 5 %
+// and gain the head-size-128 forward, whose code is short, 2 % (3.31 -> 3.25 ms at 192 x 8192).
+template <int POLLS = 2>
+__device__ __forceinline__ bool mbar_wait_at(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site) {
+#pragma unroll
+  for (int i = 0; i < POLLS; ++i)
     if (mbar_test_wait(bar, parity)) return true;
+#pragma unroll 1
   for (uint32_t i = 0; i < kSpinLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (i > 32) {
-      if (*abort_flag) return false;
-      __nanosleep(i > 4096 ? 256 : 32);
-    }
+    if (*abort_flag) return false;
   }
   atomicCAS(const_cast<int*>(abort_flag), 0, site);
   return false;
