@@ -13,20 +13,26 @@
 // run; dadattn_set_bwd_deterministic(1) selects the two-kernel path of
 // flash_bwd_bf16_sm100.cu, which has no such sums.
 //
-// Rows of the score tile are queries (one TMEM lane each), so lse and delta are per-thread
-// scalars. P and dS are written once, bf16, row-major [query][key] in the 128-byte swizzled
-// layout: dS is the K-major A operand of dQ = dS K, and the same bytes read as an MN-major A
-// operand are dS^T (resp. P^T) for dK (resp. dV). The Q / dO tiles are K-major A operands of the
-// score GEMMs and MN-major B operands of dK / dV; K is the K-major B operand of S and the
-// MN-major B operand of dQ.
-//   warps 0-15   compute: four warps per TMEM lane quadrant, 32 of the 128 key columns each
+// Rows of the score tile are keys (one TMEM lane each): S^T = K Q^T and dP^T = V dO^T, so that P^T and
+// dS^T, packed to bf16, are the A operands of dV and dK from tensor memory. dS^T is also written to shared
+// memory, [key][query] in the 128-byte swizzled layout, as the MN-major A operand of dQ. That leaves room
+// for a third Q / dO stage and takes 64 KB a tile off shared memory, whose 128 bytes a clock the products,
+// the stores and the TMA share (272 KB a tile). What the time was before, 4140 clocks a tile against 1660
+// of the products: with two stages a tile's loads (2000 clocks beside the reduce-adds) started when dV / dK
+// of the tile two back were through and held up the products of the tile between; dQ had one staging
+// buffer, 3600 clocks from one use to the next. Now 2700-2800 (192 x 1024: 117 -> 84 us), set by the
+// issuing thread (2500 clocks for 32 products, their waits and commits) and the arithmetic (2200) alike.
+// Measured and not kept: two issuing warps, each with its own accumulators (13 % slower), dK's A operand
+// from shared memory (more traffic), the next group's tiles prefetched into L2 (2 % slower).
+//   warps 0-15   compute: four warps per TMEM lane quadrant, 32 of the 128 query columns each
 //   warp 16      TMA producer           warp 17      MMA issuer + TMEM owner
-//   warp 18      dQ reducer: issues the TMA reduce-adds and the dK / dV stores   (warp 19 idle)
+//   warp 18      reducer: issues the TMA reduce-adds of dQ and the dK / dV stores
+//   warp 19      row scalars: -lse log2e and -delta scale of each tile's queries
 //   warps 20-23  accumulator drain: one thread per TMEM lane takes each tile's dQ, and each
-//                item's dK / dV, out of tensor memory into the shared-memory staging buffers,
+//                item's dK / dV, out of tensor memory into the shared-memory staging panels,
 //                while the compute warps are already on the next tile's arithmetic
 // The roles are whole warpgroups so that registers can move between them (setmaxnreg): the
-// compute warps hold two packed tiles' worth of values and get 96 registers, the others 56 / 40.
+// compute warps hold a tile's 32 probabilities and gradients a thread and get 96 registers, the others 48.
 #include <cuda_bf16.h>
 
 #include <cfloat>
@@ -45,46 +51,38 @@ constexpr int kFPanel = 128 * 128;        // [128 rows][64 bf16] swizzled panel
 constexpr int kFThreads = 24 * 32;
 constexpr int kFCompute = 16 * 32;
 constexpr int kFDrain = 4 * 32;           // one thread per TMEM lane
-constexpr int kWarpProducer = 16, kWarpIssuer = 17, kWarpReducer = 18, kWarpDrain0 = 20;
+constexpr int kWarpProducer = 16, kWarpIssuer = 17, kWarpReducer = 18, kWarpScalars = 19, kWarpDrain0 = 20;
 // Registers per thread after the warpgroups have rebalanced. The pool is what the CTA was launched
 // with (kRegsLaunch per thread, the most that 768 threads can have): an increase beyond it would
 // wait for ever.
-constexpr int kRegsLaunch = 80, kRegsCompute = 96, kRegsHelper = 56, kRegsDrain = 40;
+constexpr int kRegsLaunch = 80, kRegsCompute = 96, kRegsHelper = 48, kRegsDrain = 48;
 static_assert(kFCompute * kRegsCompute + 128 * kRegsHelper + kFDrain * kRegsDrain <= kFThreads * kRegsLaunch,
               "the warpgroups ask for more registers than the CTA owns");
 static_assert(kFThreads * kRegsLaunch <= 65536 && (kRegsLaunch + 8) * kFThreads > 65536,
               "kRegsLaunch is not what the compiler gives a CTA of this size");
-constexpr int kFStages = 2;
+constexpr int kFStages = 3;
 constexpr int kFRing = 4;                 // entries of the work-item ring (a power of two)
 constexpr float kFLog2e = 1.4426950408889634f;
-constexpr int kVecBox = 132;   // fp32 words one row-scalar load brings in
 
 struct FusedSmem {
   static constexpr int kK = 0;                          // two buffers: items alternate
   static constexpr int kV = kK + 2 * kFPanel;
   static constexpr int kQ = kV + 2 * kFPanel;
   static constexpr int kDO = kQ + kFStages * kFPanel;
-  static constexpr int kP = kDO + kFStages * kFPanel;   // [128 q][128 keys] bf16, two panels
-  static constexpr int kDS = kP + 2 * kFPanel;
+  static constexpr int kDS = kDO + kFStages * kFPanel;  // dS^T [128 keys][128 q] bf16, two panels
   static constexpr int kDQ = kDS + 2 * kFPanel;         // [128 q][64] fp32, two 128-byte panels
-  static constexpr int kBars = kDQ + 2 * kFPanel;
-  // Per-row scalars of a query tile, one buffer per Q / dO stage: lse and delta of kVecBox rows
-  // each (the tile's 128 and up to three before them: a TMA load starts on a 16-byte boundary),
-  // every vector on its own 128-byte boundary.
-  static constexpr int kBarsBytes = 384;
-  static constexpr int kVec = kBars + kBarsBytes;
-  static constexpr int kVecDelta = 640, kVecStride = 1280;
-  static constexpr int kBytes = kVec + kFStages * kVecStride;
-  static_assert(kVec % 128 == 0 && kVecBox * 4 <= kVecDelta, "row-scalar buffers misplaced");
+  static constexpr int kVec = kDQ + 2 * kFPanel;        // two buffers of [2][128] row scalars
+  static constexpr int kBars = kVec + 2 * 2 * kFT * 4;
+  static constexpr int kBarsBytes = 512;
+  static constexpr int kBytes = kBars + kBarsBytes;
   static_assert(kBytes <= 232448, "shared memory budget of one CTA exceeded");
 };
 
 struct FusedBars {
-  uint64_t kv_full[2], dkv_sent[2], q_full[kFStages], do_full[kFStages], qdo_empty[kFStages];
+  uint64_t kv_full[2], kv_empty[2], qdo_full[kFStages], qdo_empty[kFStages];
   uint64_t item_ready[kFRing], item_free[kFRing];
-  uint64_t x_full, x_free, w_full, acc_done, dq_drained, dq_staged, dq_sent, dkv_staged[2], vec_full[kFStages];
-  uint64_t dkv_drained;
-  int ring[kFRing];
+  uint64_t s_full[2], p_full, dp_full, w_full, acc_done, dq_drained, dkv_drained, staged[2], sent[2];
+  int2 ring[kFRing];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -123,11 +121,9 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
       : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_wait_read1() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
@@ -140,6 +136,23 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+
+// prmt with the sign-replicating selectors (8 + byte number): each selected byte of the result is 0xff or 0.
+template <uint32_t SEL>
+__device__ __forceinline__ uint32_t byte_signs(uint32_t w) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(d) : "r"(w), "n"(SEL));
+  return d;
 }
 
 // One item of work = (key tile kt, batch x head bh): the CTA that takes it streams the n_it query
@@ -162,20 +175,22 @@ __device__ __forceinline__ Item decode_item(int item, int BH, int n_tiles, int g
   return t;
 }
 
-// Items are handed out by a global counter; the producer thread takes them and publishes each
-// through a four-entry ring in shared memory, which the other roles read in the same order.
+// Items are handed out by a global counter; the producer thread takes them and publishes each, decoded
+// (the divisions would sit in every role's chain), through a four-entry ring in shared memory, which the
+// other roles read in the same order. An entry beyond the last item has n_it = 0.
 struct ItemFeed {
   FusedBars* bars;
   volatile int* abort_flag;
-  int n_read;
-  // the next item of this CTA, or n_items when there is none (or the kernel is aborting)
-  __device__ __forceinline__ int fetch(int n_items) {
+  int n_tiles, n_read;
+  // the next item of this CTA; n_it = 0 when there is none (or the kernel is aborting)
+  __device__ __forceinline__ Item fetch() {
     const int slot = n_read & (kFRing - 1);
-    if (!mbar_wait(&bars->item_ready[slot], (n_read / kFRing) & 1, abort_flag)) return n_items;
-    const int v = *reinterpret_cast<volatile int*>(&bars->ring[slot]);
+    if (!mbar_wait(&bars->item_ready[slot], (n_read / kFRing) & 1, abort_flag)) return Item{n_tiles, 0, 0};
+    const volatile int2& e = bars->ring[slot];
+    const int kt = e.x, bh = e.y;
     mbar_arrive(&bars->item_free[slot]);
     ++n_read;
-    return v;
+    return Item{kt, bh, n_tiles - kt};
   }
 };
 
@@ -187,15 +202,16 @@ __global__ void __launch_bounds__(kFThreads, 1)
 flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                        const __grid_constant__ CUtensorMap map_dqw, const __grid_constant__ CUtensorMap map_dk,
-                       const __grid_constant__ CUtensorMap map_dv, const __grid_constant__ CUtensorMap map_lse,
-                       const __grid_constant__ CUtensorMap map_delta, int lse_shift,
-                       int* __restrict__ item_counter, int BH, int S,
+                       const __grid_constant__ CUtensorMap map_dv, const float* __restrict__ lse,
+                       const float* __restrict__ delta, int* __restrict__ item_counter, int BH, int S,
                        int heads, int group_bh, float scale, float rate, PhiloxKey rng, int64_t unit0,
                        const uint32_t* __restrict__ mask_bits, int* __restrict__ status) {
   using L = FusedSmem;
   constexpr int D = kFD;
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 320, kColDQ = 384;
+  // S^T and dP^T (fp32, 128 queries each), dV, dK, dQ (64 each), P^T as packed bf16. dS^T goes back over
+  // dP^T: each thread packs its 32 queries into the first 16 of the 32 columns it has read.
+  constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 320, kColDQ = 384, kColP = 448;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   FusedBars* bars = reinterpret_cast<FusedBars*>(smem + L::kBars);
@@ -212,28 +228,25 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->dkv_sent[s], 1);
+      mbar_init(&bars->kv_empty[s], 1);
+      mbar_init(&bars->s_full[s], 2);       // the product and the tile's row scalars
+      mbar_init(&bars->staged[s], kFDrain);
+      mbar_init(&bars->sent[s], 1);
     }
     for (int s = 0; s < kFStages; ++s) {
-      mbar_init(&bars->q_full[s], 1);
-      mbar_init(&bars->do_full[s], 1);
+      mbar_init(&bars->qdo_full[s], 1);
       mbar_init(&bars->qdo_empty[s], 1);
     }
     for (int s = 0; s < kFRing; ++s) {
       mbar_init(&bars->item_ready[s], 1);
-      mbar_init(&bars->item_free[s], kFCompute + kFDrain + 2);   // compute, drain, MMA issuer, reducer
+      mbar_init(&bars->item_free[s], kFCompute + kFDrain + 32 + 2);   // compute, drain, row scalars, MMA issuer, reducer
     }
-    mbar_init(&bars->x_full, 1);
-    mbar_init(&bars->x_free, kFCompute);
+    mbar_init(&bars->p_full, kFCompute);
+    mbar_init(&bars->dp_full, 1);
     mbar_init(&bars->w_full, kFCompute);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->dq_drained, kFDrain);
-    mbar_init(&bars->dq_staged, kFDrain);
     mbar_init(&bars->dkv_drained, kFDrain);
-    mbar_init(&bars->dq_sent, 1);
-    mbar_init(&bars->dkv_staged[0], kFDrain);
-    mbar_init(&bars->dkv_staged[1], kFDrain);
-    for (int s = 0; s < kFStages; ++s) mbar_init(&bars->vec_full[s], 1);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -259,28 +272,30 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       prefetch_tensormap(&map_k);
       prefetch_tensormap(&map_v);
       prefetch_tensormap(&map_do);
-      prefetch_tensormap(&map_lse);
-      prefetch_tensormap(&map_delta);
       int n_pub = 0;
-      auto publish = [&](int item) -> bool {
+      auto publish = [&](const Item& t) -> bool {
         const int slot = n_pub & (kFRing - 1);
         if (n_pub >= kFRing &&
             !mbar_wait(&bars->item_free[slot], (n_pub / kFRing - 1) & 1, abort_flag))
           return false;
-        *reinterpret_cast<volatile int*>(&bars->ring[slot]) = item;
+        volatile int2& e = bars->ring[slot];
+        e.x = t.kt;
+        e.y = t.bh;
         mbar_arrive(&bars->item_ready[slot]);
         ++n_pub;
         return true;
       };
       // the first item is the CTA's own index; the counter hands out the rest
-      int cur = static_cast<int>(blockIdx.x);
-      bool ok = publish(cur);
+      auto decode = [&](int item) -> Item {
+        return item < n_items ? decode_item(item, BH, n_tiles, group_bh) : Item{n_tiles, 0, 0};
+      };
+      Item t = decode(static_cast<int>(blockIdx.x));
+      bool ok = publish(t);
       int g = 0;
-      for (int j = 0; ok && cur < n_items; ++j) {
-        const Item t = decode_item(cur, BH, n_tiles, group_bh);
-        // K / V go to the buffer of the item before last, once its dK / dV have left that buffer
+      for (int j = 0; ok && t.n_it > 0; ++j) {
+        // K / V go to the buffer of the item before last, once its products are through
         const int kb = j & 1;
-        if (ok && j >= 2) ok = mbar_wait(&bars->dkv_sent[kb], ((j >> 1) - 1) & 1, abort_flag);
+        if (ok && j >= 2) ok = mbar_wait(&bars->kv_empty[kb], ((j >> 1) - 1) & 1, abort_flag);
         if (!ok) break;
         const int ub = t.bh / heads, uh = t.bh - ub * heads;   // (batch, head) of the unit
         mbar_arrive_expect_tx(&bars->kv_full[kb], 2 * kFPanel);
@@ -289,118 +304,113 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // The following item (or the end mark) is claimed only now, and published at once: the
         // other roles look one item ahead. Every item a CTA holds in advance is work that no idle
         // CTA can take near the end of the kernel, so it holds as few as it can.
-        const int nxt = static_cast<int>(gridDim.x) + atomicAdd(item_counter, 1);
+        const Item nxt = decode(static_cast<int>(gridDim.x) + atomicAdd(item_counter, 1));
         ok = publish(nxt);
         for (int i = 0; ok && i < t.n_it; ++i, ++g) {
           const int s = g % kFStages, use = g / kFStages;
           if (use > 0 && !(ok = mbar_wait(&bars->qdo_empty[s], (use - 1) & 1, abort_flag))) break;
           const int q0 = (t.kt + i) * kFT;
-          mbar_arrive_expect_tx(&bars->q_full[s], kFPanel);
-          tma_load_4d(smem + L::kQ + s * kFPanel, &map_q, &bars->q_full[s], 0, q0, uh, ub);
-          mbar_arrive_expect_tx(&bars->do_full[s], kFPanel);
-          tma_load_4d(smem + L::kDO + s * kFPanel, &map_do, &bars->do_full[s], 0, q0, uh, ub);
-          // The tile's row scalars ride the same ring: the stage is free once the GEMMs of the
-          // tile that used it have completed, and those followed the arithmetic that read the
-          // scalars. The load starts at the 16-byte boundary at or below the tile's first row.
-          const int at = t.bh * S + q0;
-          mbar_arrive_expect_tx(&bars->vec_full[s], 2 * kVecBox * 4);
-          tma_load_1d(smem + L::kVec + s * L::kVecStride, &map_lse, &bars->vec_full[s], (at + lse_shift) & ~3);
-          tma_load_1d(smem + L::kVec + s * L::kVecStride + L::kVecDelta, &map_delta, &bars->vec_full[s], at & ~3);
+          mbar_arrive_expect_tx(&bars->qdo_full[s], 2 * kFPanel);
+          tma_load_4d(smem + L::kQ + s * kFPanel, &map_q, &bars->qdo_full[s], 0, q0, uh, ub);
+          tma_load_4d(smem + L::kDO + s * kFPanel, &map_do, &bars->qdo_full[s], 0, q0, uh, ub);
         }
-        cur = nxt;
+        t = nxt;
       }
     }
   } else if (warp == kWarpIssuer) {
     // ------------------------------ MMA issuer ------------------------------
     if (elect_one()) {
-      constexpr uint32_t idesc_x = make_idesc_bf16(128, 128, 0, 0);   // S, dP: both K-major
-      constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, 1, 1);    // dV, dK: A and B MN-major
-      constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, 0, 1);    // dQ: A K-major, B MN-major
+      constexpr uint32_t idesc_x = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both K-major
+      constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, 0, 1);    // dV, dK: A in tensor memory, B MN-major
+      constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, 1, 1);    // dQ: A and B MN-major
       const SmemDescBase k0_desc = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
       const SmemDescBase v0_desc = make_desc_base_sw128(smem_u32(smem + L::kV), 0);
       const SmemDescBase q0_desc = make_desc_base_sw128(smem_u32(smem + L::kQ), 0);
       const SmemDescBase do0_desc = make_desc_base_sw128(smem_u32(smem + L::kDO), 0);
-      // P / dS read as MN-major A: the two 64-key panels are kFPanel apart (leading byte offset)
-      const SmemDescBase p_t = make_desc_base_sw128(smem_u32(smem + L::kP), kFPanel);
+      // dS^T read as MN-major A (M = queries): the two 64-query panels are kFPanel apart
       const SmemDescBase ds_t = make_desc_base_sw128(smem_u32(smem + L::kDS), kFPanel);
-      const SmemDescBase ds_k = make_desc_base_sw128(smem_u32(smem + L::kDS), 0);
 
-      // S = Q K^T and dP = dO V^T of tile g (counted over all items of this CTA), K / V buffer kb
-      auto issue_x = [&](int g, int kb) -> bool {
-        const int s = g % kFStages;
-        const uint32_t par = (g / kFStages) & 1;
+      // S^T = K Q^T of the tile in stage s (the g-th of this CTA), K / V buffer kb
+      auto issue_s = [&](int g, int s, int kb) {
         const SmemDescBase qd{q0_desc.lo + s * (kFPanel >> 4), q0_desc.hi};
-        const SmemDescBase dd{do0_desc.lo + s * (kFPanel >> 4), do0_desc.hi};
         const SmemDescBase kd{k0_desc.lo + kb * (kFPanel >> 4), k0_desc.hi};
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk)
+          mma_ss(tmem + kColS, desc_at(kd, kk * 32), desc_at(qd, kk * 32), idesc_x, kk > 0 ? 1u : 0u);
+        mma_commit(&bars->s_full[g & 1]);
+      };
+      // dP^T = V dO^T
+      auto issue_dp = [&](int s, int kb) {
+        const SmemDescBase dd{do0_desc.lo + s * (kFPanel >> 4), do0_desc.hi};
         const SmemDescBase vd{v0_desc.lo + kb * (kFPanel >> 4), v0_desc.hi};
-        if (!mbar_wait(&bars->q_full[s], par, abort_flag)) return false;
-        tc_fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          mma_ss(tmem + kColS, desc_at(qd, kk * 32), desc_at(kd, kk * 32), idesc_x, kk > 0 ? 1u : 0u);
-        if (!mbar_wait(&bars->do_full[s], par, abort_flag)) return false;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          mma_ss(tmem + kColDP, desc_at(dd, kk * 32), desc_at(vd, kk * 32), idesc_x, kk > 0 ? 1u : 0u);
-        mma_commit(&bars->x_full);
-        return true;
-      };
-      // dV += P^T dO, dK += dS^T Q (fresh accumulators on an item's first tile), dQ_tile = dS K
-      auto issue_acc = [&](int g, int item, bool first_of_item) -> bool {
-        const int kb = item & 1;
-        const int s = g % kFStages;
-        const SmemDescBase qd{q0_desc.lo + s * (kFPanel >> 4), q0_desc.hi};
-        const SmemDescBase dd{do0_desc.lo + s * (kFPanel >> 4), do0_desc.hi};
-        const SmemDescBase kd{k0_desc.lo + kb * (kFPanel >> 4), k0_desc.hi};
-        if (!mbar_wait(&bars->w_full, g & 1, abort_flag)) return false;
-        // a new item's first products overwrite dV / dK: the drain warps must have taken the
-        // previous item's out of tensor memory
-        if (first_of_item && item > 0 && !mbar_wait(&bars->dkv_drained, (item - 1) & 1, abort_flag)) return false;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < kFT / 16; ++kk) {   // K dimension = 128 queries, 16 per MMA
-          const uint32_t acc = (!first_of_item || kk > 0) ? 1u : 0u;
-          // A = P^T / dS^T: 16 query rows (2048 bytes) further down per step; B = dO / Q rows
-          mma_ss(tmem + kColDV, desc_at(p_t, kk * 2048), desc_at(dd, kk * 2048), idesc_t, acc);
-          mma_ss(tmem + kColDK, desc_at(ds_t, kk * 2048), desc_at(qd, kk * 2048), idesc_t, acc);
-        }
-        // Q and dO of this stage are last read by the products above: the stage goes back to the
-        // producer now, not after dQ, which only needs dS and K.
-        mma_commit(&bars->qdo_empty[s]);
-        // the previous tile's dQ must have left tensor memory before this one overwrites it; the
-        // compute warps read it right after they publish P / dS, while dV / dK are running
-        if (g > 0 && !mbar_wait(&bars->dq_drained, (g - 1) & 1, abort_flag)) return false;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < kFT / 16; ++kk) {   // K dimension = 128 keys
-          mma_ss(tmem + kColDQ, desc_at(ds_k, (kk / 4) * kFPanel + (kk % 4) * 32),
-                 desc_at(kd, kk * 2048), idesc_q, kk > 0 ? 1u : 0u);
-        }
-        mma_commit(&bars->acc_done);
-        return true;
+          mma_ss(tmem + kColDP, desc_at(vd, kk * 32), desc_at(dd, kk * 32), idesc_x, kk > 0 ? 1u : 0u);
+        mma_commit(&bars->dp_full);
       };
 
-      ItemFeed feed{bars, abort_flag, 0};
-      int cur = feed.fetch(n_items);
-      int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
-      bool ok = cur < n_items && mbar_wait(&bars->kv_full[0], 0, abort_flag) && issue_x(0, 0);
-      int g = 0;
-      for (int j = 0; ok && cur < n_items; ++j) {
-        const int n_it = decode_item(cur, BH, n_tiles, group_bh).n_it;
+      ItemFeed feed{bars, abort_flag, n_tiles, 0};
+      int n_it = feed.fetch().n_it, n_nxt = 0;
+      bool ok = n_it > 0 && mbar_wait(&bars->kv_full[0], 0, abort_flag) && mbar_wait(&bars->qdo_full[0], 0, abort_flag);
+      if (ok) {
+        tc_fence_after_sync();
+        issue_s(0, 0, 0);
+        issue_dp(0, 0);
+      }
+      int g = 0, s = 0;          // tile and its stage
+      uint32_t par = 0;          // parity of that stage's full barrier
+      for (int j = 0; ok && n_it > 0; ++j) {
+        const int kb = j & 1;
         for (int i = 0; ok && i < n_it; ++i, ++g) {
-          // The next tile's score GEMMs go first, so the arithmetic on them overlaps this tile's
-          // accumulating GEMMs; across an item boundary they use the other K / V buffer.
-          if (i + 1 < n_it) {
-            ok = mbar_wait(&bars->x_free, g & 1, abort_flag) && issue_x(g + 1, j & 1);
-          } else if (nxt < n_items) {
-            const int kbn = (j + 1) & 1;
-            ok = mbar_wait(&bars->x_free, g & 1, abort_flag) &&
-                 mbar_wait(&bars->kv_full[kbn], ((j + 1) >> 1) & 1, abort_flag) && issue_x(g + 1, kbn);
+          const bool last = i + 1 == n_it;
+          if (last) n_nxt = feed.fetch().n_it;   // (published when the producer came to this item)
+          const int sn = s + 1 == kFStages ? 0 : s + 1;
+          const uint32_t parn = sn == 0 ? par ^ 1u : par;
+          const bool more = !last || n_nxt > 0;
+          const int kbn = last ? kb ^ 1 : kb;
+          const SmemDescBase qd{q0_desc.lo + s * (kFPanel >> 4), q0_desc.hi};
+          const SmemDescBase dd{do0_desc.lo + s * (kFPanel >> 4), do0_desc.hi};
+          const SmemDescBase kd{k0_desc.lo + kb * (kFPanel >> 4), k0_desc.hi};
+          // P^T of this tile is there, and its scores have been read: dV += P^T dO, 16 queries per MMA, and
+          // the next tile's scores (across an item boundary from the other K / V buffer), while dS is being
+          // formed. A new item's first products overwrite dV / dK: the drain warps must have taken the
+          // previous item's out of tensor memory.
+          if (!(ok = mbar_wait(&bars->p_full, g & 1, abort_flag))) break;
+          if (more && !(ok = (!last || mbar_wait(&bars->kv_full[kbn], ((j + 1) >> 1) & 1, abort_flag)) &&
+                             mbar_wait(&bars->qdo_full[sn], parn, abort_flag)))
+            break;
+          tc_fence_after_sync();
+          if (more) issue_s(g + 1, sn, kbn);
+          if (i == 0 && j > 0) {
+            if (!(ok = mbar_wait(&bars->dkv_drained, (j - 1) & 1, abort_flag))) break;
+            tc_fence_after_sync();
           }
-          ok = ok && issue_acc(g, j, i == 0);
+#pragma unroll
+          for (int kk = 0; kk < kFT / 16; ++kk)
+            mma_ts(tmem + kColDV, tmem + kColP + kk * 8, desc_at(dd, kk * 2048), idesc_t, (i > 0 || kk > 0) ? 1u : 0u);
+          // dK += dS^T Q
+          if (!(ok = mbar_wait(&bars->w_full, g & 1, abort_flag))) break;
+          tc_fence_after_sync();
+#pragma unroll
+          for (int kk = 0; kk < kFT / 16; ++kk)
+            mma_ts(tmem + kColDK, tmem + kColDP + (kk / 2) * 32 + (kk % 2) * 8, desc_at(qd, kk * 2048), idesc_t,
+                   (i > 0 || kk > 0) ? 1u : 0u);
+          // dS^T has been read out of its columns once dK is through: the next tile's dP^T may follow
+          if (more) issue_dp(sn, kbn);
+          // Q and dO of this stage are last read by the products above
+          mma_commit(&bars->qdo_empty[s]);
+          // dQ = dS K, 16 keys per MMA. The previous tile's dQ must have left tensor memory before.
+          if (g > 0 && !(ok = mbar_wait(&bars->dq_drained, (g - 1) & 1, abort_flag))) break;
+          tc_fence_after_sync();
+#pragma unroll
+          for (int kk = 0; kk < kFT / 16; ++kk)
+            mma_ss(tmem + kColDQ, desc_at(ds_t, kk * 2048), desc_at(kd, kk * 2048), idesc_q, kk > 0 ? 1u : 0u);
+          mma_commit(&bars->acc_done);
+          if (last) mma_commit(&bars->kv_empty[kb]);
+          s = sn;
+          par = parn;
         }
-        cur = nxt;
-        nxt = cur < n_items ? feed.fetch(n_items) : n_items;
+        n_it = n_nxt;
       }
     }
   } else if (warp == kWarpReducer) {
@@ -410,61 +420,88 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const uint64_t keep = l2_policy_evict_last();
       prefetch_tensormap(&map_dk);
       prefetch_tensormap(&map_dv);
-      ItemFeed feed{bars, abort_flag, 0};
-      int cur = feed.fetch(n_items);
-      int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
-      int g = 0;   // uses of the dQ staging buffer: one per tile, and with F32 one per item for its dV
+      ItemFeed feed{bars, abort_flag, n_tiles, 0};
+      uint32_t turn = 0;   // parity of the staging panels' use
+      auto hand_back = [&]() {
+        bulk_wait_read<1>();
+        mbar_arrive(&bars->sent[0]);
+        bulk_wait_read<0>();
+        mbar_arrive(&bars->sent[1]);
+        turn ^= 1u;
+      };
       bool ok = true;
-      for (int j = 0; ok && cur < n_items; ++j) {
-        const Item t = decode_item(cur, BH, n_tiles, group_bh);
-        for (int i = 0; ok && i < t.n_it; ++i, ++g) {
-          if (F32 && i + 1 == t.n_it) {
-            if (!(ok = mbar_wait(&bars->dq_staged, g & 1, abort_flag))) break;
-            tma_store_3d(&map_dv, smem + L::kDQ, 0, t.kt * kFT, t.bh);
-            tma_store_3d(&map_dv, smem + L::kDQ + kFPanel, 32, t.kt * kFT, t.bh);
-            bulk_commit();
-            bulk_wait_read0();
-            mbar_arrive(&bars->dq_sent);
-            ++g;
-          }
-          if (!(ok = mbar_wait(&bars->dq_staged, g & 1, abort_flag))) break;
-          const int q0 = (t.kt + i) * kFT;
-          tma_reduce_add_3d(&map_dqw, smem + L::kDQ, 0, q0, t.bh, keep);
-          tma_reduce_add_3d(&map_dqw, smem + L::kDQ + kFPanel, 32, q0, t.bh, keep);
-          bulk_commit();
-          if (i + 1 < t.n_it) {
-            bulk_wait_read0();
-            mbar_arrive(&bars->dq_sent);
-          } else {
-            // The item's dK / dV were staged (in its K / V buffers) before the dQ of its last
-            // tile. Their stores go behind the reduce, so that the dQ staging buffer is handed
-            // back as soon as the reduce has read it; the K / V buffers follow.
-            // One barrier per K / V buffer, not one for all items: after a single-tile item the
-            // compute warps stage the next item's dK / dV without needing this warp, so a single
-            // barrier could run two phases ahead of a late reducer, whose parity wait would then
-            // never be satisfied (and the compute warps in turn wait for this warp's dq_sent).
-            // The next phase of dkv_staged[j & 1] belongs to item j + 2 and cannot complete
-            // before this warp has handed back the staging buffer of item j's last tile.
-            if (!(ok = mbar_wait(&bars->dkv_staged[j & 1], (j >> 1) & 1, abort_flag))) break;
-            if (F32) {   // dK: columns 0-31 in the K buffer, 32-63 in the V buffer
-              tma_store_3d(&map_dk, smem + L::kK + (j & 1) * kFPanel, 0, t.kt * kFT, t.bh);
-              tma_store_3d(&map_dk, smem + L::kV + (j & 1) * kFPanel, 32, t.kt * kFT, t.bh);
-            } else {
-              const int ub = t.bh / heads, uh = t.bh - ub * heads;
-              tma_store_4d(&map_dk, smem + L::kK + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
-              tma_store_4d(&map_dv, smem + L::kV + (j & 1) * kFPanel, 0, t.kt * kFT, uh, ub);
+      for (Item t = feed.fetch(); ok && t.n_it > 0; t = feed.fetch()) {
+        for (int i = 0; ok && i < t.n_it; ++i) {
+          const int q0 = (t.kt + i) * kFT, k0 = t.kt * kFT;
+          if (i + 1 == t.n_it) {
+            // The item is complete: dV and dK take a turn of the panels ahead of the last tile's dQ (one
+            // each if the panels are fp32)
+            const int ub = t.bh / heads, uh = t.bh - ub * heads;
+            for (int a = 0; ok && a < (F32 ? 2 : 1); ++a) {
+              for (int p = 0; ok && p < 2; ++p) {
+                if (!(ok = mbar_wait(&bars->staged[p], turn, abort_flag))) break;
+                if (F32) tma_store_3d(a ? &map_dk : &map_dv, smem + L::kDQ + p * kFPanel, p * 32, k0, t.bh);
+                else tma_store_4d(p ? &map_dk : &map_dv, smem + L::kDQ + p * kFPanel, 0, k0, uh, ub);
+                bulk_commit();
+              }
+              if (ok) hand_back();
             }
-            bulk_commit();
-            bulk_wait_read1();
-            mbar_arrive(&bars->dq_sent);
-            bulk_wait_read0();
-            mbar_arrive(&bars->dkv_sent[j & 1]);
           }
+          for (int p = 0; ok && p < 2; ++p) {
+            if (!(ok = mbar_wait(&bars->staged[p], turn, abort_flag))) break;
+            tma_reduce_add_3d(&map_dqw, smem + L::kDQ + p * kFPanel, p * 32, q0, t.bh, keep);
+            bulk_commit();
+          }
+          if (ok) hand_back();
         }
-        cur = nxt;
-        nxt = cur < n_items ? feed.fetch(n_items) : n_items;
       }
       bulk_wait0();   // every sum and store has landed before the CTA retires
+    }
+  } else {
+    // ------------------------------ row scalars ------------------------------
+    // -lse log2e and -delta scale of each tile's 128 queries, from memory through registers (a tile
+    // ahead: the SM's path to L2 is busy with the reduce-adds) into one of two buffers. Queries beyond S
+    // contribute nothing: p = exp2(-inf). Buffer g % 2 is free once the products of tile g - 2, which
+    // follow the arithmetic that read it, have given their stage back; that barrier's next phase needs
+    // this warp's scalars of tile g + 1.
+    float* vec = reinterpret_cast<float*>(smem + L::kVec);
+    ItemFeed feed{bars, abort_flag, n_tiles, 0};
+    Item t = feed.fetch();
+    Item nxt = t.n_it > 0 ? feed.fetch() : t;
+    float rl[4], rd[4];
+    auto request = [&](int q_tile, int bh) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int q = q_tile * kFT + c * 32 + lane;
+        const int64_t at = static_cast<int64_t>(bh) * S + q;
+        rl[c] = q < S ? lse[at] : INFINITY;
+        rd[c] = q < S ? delta[at] : 0.f;
+      }
+    };
+    if (t.n_it > 0) request(t.kt, t.bh);
+    bool ok = true;
+    int g = 0, s2 = kFStages - 2;   // the tile; stage of tile g - 2
+    uint32_t par2 = 1;              // and the parity of that use
+    while (ok && t.n_it > 0) {
+      for (int i = 0; i < t.n_it; ++i, ++g) {
+        if (g >= 2 && !(ok = mbar_wait(&bars->qdo_empty[s2], par2, abort_flag))) break;
+        if (++s2 == kFStages) s2 = 0, par2 ^= 1u;
+        float* dst = vec + (g & 1) * (2 * kFT) + lane;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          dst[c * 32] = -rl[c] * kFLog2e;
+          dst[kFT + c * 32] = -rd[c] * scale;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->s_full[g & 1]);
+        if (i + 1 < t.n_it) {
+          request(t.kt + i + 1, t.bh);
+        } else if (nxt.n_it > 0) {
+          request(nxt.kt, nxt.bh);
+        }
+      }
+      t = nxt;
+      if (ok && t.n_it > 0) nxt = feed.fetch();
     }
   }
   } else if (warp >= kWarpDrain0) {
@@ -473,229 +510,222 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int quad = warp % 4;
     const int row = quad * 32 + lane;     // TMEM lane = query row (dQ) or key row (dK / dV)
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-    ItemFeed feed{bars, abort_flag, 0};
-    int cur = feed.fetch(n_items);
-    int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
+    ItemFeed feed{bars, abort_flag, n_tiles, 0};
     bool ok = true;
-    int g = 0, used = 0;   // tiles; uses of the dQ staging buffer
-    // 64 fp32 accumulator columns -> two swizzled panels [128 rows][32 fp32]
-    auto stage_f32 = [&](uint32_t col, uint8_t* panel0, uint8_t* panel1) {
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t o[16];
-        tmem_ld16(tlane + col + c * 16, o);
-        tmem_wait_ld();
-        uint8_t* dst = (c < 2 ? panel0 : panel1) + row * 128;
+    int g = 0;
+    uint32_t back = 1;   // parity of the staging panels' return from their last use (none yet: passes)
+    // 32 fp32 accumulator columns -> a swizzled panel [128 rows][32 fp32]
+    auto stage_f32 = [&](const uint32_t (&o)[32], int p) {
+      uint8_t* dst = smem + L::kDQ + p * kFPanel + row * 128;
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4)
-          *reinterpret_cast<uint4*>(dst + ((((c & 1) * 4 + c4) ^ (row & 7)) << 4)) =
-              make_uint4(o[4 * c4], o[4 * c4 + 1], o[4 * c4 + 2], o[4 * c4 + 3]);
-      }
+      for (int c4 = 0; c4 < 8; ++c4)
+        *reinterpret_cast<uint4*>(dst + ((c4 ^ (row & 7)) << 4)) =
+            make_uint4(o[4 * c4], o[4 * c4 + 1], o[4 * c4 + 2], o[4 * c4 + 3]);
+      fence_proxy_async_smem();
+      mbar_arrive(&bars->staged[p]);
     };
-    for (int j = 0; ok && cur < n_items; ++j) {
-      const int n_it = decode_item(cur, BH, n_tiles, group_bh).n_it;
-      for (int i = 0; i < n_it; ++i, ++g, ++used) {
-        // the staging buffer back from its previous use, then this tile's GEMMs
-        if (used > 0 && !(ok = mbar_wait(&bars->dq_sent, (used - 1) & 1, abort_flag))) break;
+    // 64 accumulator columns through both panels as fp32; `drained` gets an arrival once they are read
+    auto turn_f32 = [&](uint32_t col, uint64_t* drained) -> bool {
+#pragma unroll 1
+      for (int p = 0; p < 2; ++p) {
+        uint32_t o[32];
+        tmem_ld32(tlane + col + p * 32, o);
+        tmem_wait_ld();
+        if (p == 1 && drained) {
+          tc_fence_before_sync();
+          mbar_arrive(drained);
+        }
+        if (!mbar_wait(&bars->sent[p], back, abort_flag)) return false;
+        stage_f32(o, p);
+      }
+      back ^= 1u;
+      return true;
+    };
+    for (Item t = feed.fetch(); ok && t.n_it > 0; t = feed.fetch()) {
+      for (int i = 0; i < t.n_it; ++i, ++g) {
         if (!(ok = mbar_wait(&bars->acc_done, g & 1, abort_flag))) break;
         tc_fence_after_sync();
-        if (F32 && i + 1 == n_it) {
-          // The item is complete: dV through the dQ staging buffer (before this tile's dQ), dK through
-          // the item's own K and V buffers, both as fp32 panels.
-          const int kb = j & 1;
-          stage_f32(kColDV, smem + L::kDQ, smem + L::kDQ + kFPanel);
-          fence_proxy_async_smem();
-          mbar_arrive(&bars->dq_staged);
-          ++used;
-          stage_f32(kColDK, smem + L::kK + kb * kFPanel, smem + L::kV + kb * kFPanel);
-          tc_fence_before_sync();
-          mbar_arrive(&bars->dkv_drained);          // the next item's products may overwrite dV / dK
-          fence_proxy_async_smem();
-          mbar_arrive(&bars->dkv_staged[kb]);
-          if (!(ok = mbar_wait(&bars->dq_sent, (used - 1) & 1, abort_flag))) break;
-        } else if (i + 1 == n_it) {
-          // The item is complete: dK / dV, tensor memory -> bf16 rows in the item's own K / V
-          // buffers (every GEMM that read them has completed), from where the reducer warp
-          // stores them. Sixteen columns at a time; dV is columns [0, 64), dK [64, 128).
-          const int kb = j & 1;
+        if (i + 1 == t.n_it) {
+          // The item is complete: dV and dK leave through the dQ staging panels, ahead of this tile's dQ.
+          // (Staged in the item's own K / V buffers, they held up the K / V loads of the item after next:
+          // short items waited 5000 clocks for theirs.) dkv_drained: the next item's products may overwrite.
+          if (F32) {
+            if (!(ok = turn_f32(kColDV, nullptr) && turn_f32(kColDK, &bars->dkv_drained))) break;
+          } else {
 #pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            uint32_t o[16];
-            tmem_ld16(tlane + kColDV + c * 16, o);   // kColDK = kColDV + 64
-            tmem_wait_ld();
-            uint8_t* dst = smem + (c < 4 ? L::kV : L::kK) + kb * kFPanel + row * 128;
+            for (int c = 0; c < 4; ++c) {   // 32 columns at a time; dV is columns [0, 64), dK [64, 128)
+              uint32_t o[32];
+              tmem_ld32(tlane + kColDV + c * 32, o);   // kColDK = kColDV + 64
+              tmem_wait_ld();
+              if (c == 3) {
+                tc_fence_before_sync();
+                mbar_arrive(&bars->dkv_drained);
+              }
+              const int p = c / 2;
+              if ((c & 1) == 0 && !(ok = mbar_wait(&bars->sent[p], back, abort_flag))) break;
+              uint8_t* dst = smem + L::kDQ + p * kFPanel + row * 128;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int chunk = (c & 3) * 2 + h;
-              *reinterpret_cast<uint4*>(dst + ((chunk ^ (row & 7)) << 4)) = make_uint4(
-                  pack_bf16(__uint_as_float(o[8 * h + 0]), __uint_as_float(o[8 * h + 1])),
-                  pack_bf16(__uint_as_float(o[8 * h + 2]), __uint_as_float(o[8 * h + 3])),
-                  pack_bf16(__uint_as_float(o[8 * h + 4]), __uint_as_float(o[8 * h + 5])),
-                  pack_bf16(__uint_as_float(o[8 * h + 6]), __uint_as_float(o[8 * h + 7])));
+              for (int h = 0; h < 4; ++h)
+                *reinterpret_cast<uint4*>(dst + ((((c & 1) * 4 + h) ^ (row & 7)) << 4)) = make_uint4(
+                    pack_bf16(__uint_as_float(o[8 * h + 0]), __uint_as_float(o[8 * h + 1])),
+                    pack_bf16(__uint_as_float(o[8 * h + 2]), __uint_as_float(o[8 * h + 3])),
+                    pack_bf16(__uint_as_float(o[8 * h + 4]), __uint_as_float(o[8 * h + 5])),
+                    pack_bf16(__uint_as_float(o[8 * h + 6]), __uint_as_float(o[8 * h + 7])));
+              if (c & 1) {
+                fence_proxy_async_smem();
+                mbar_arrive(&bars->staged[p]);
+              }
             }
-          }
-          tc_fence_before_sync();
-          mbar_arrive(&bars->dkv_drained);          // the next item's products may overwrite dV / dK
-          fence_proxy_async_smem();
-          mbar_arrive(&bars->dkv_staged[kb]);
-        }
-        // dQ of the tile: tensor memory -> swizzled fp32 staging ([2 panels][128 rows][32 fp32]),
-        // which the reducer warp sends on
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t o[16];
-          tmem_ld16(tlane + kColDQ + c * 16, o);
-          tmem_wait_ld();
-          if (c == 3) {
-            tc_fence_before_sync();
-            mbar_arrive(&bars->dq_drained);          // the next tile's dQ may overwrite this one
-          }
-          uint8_t* dq_row = smem + L::kDQ + (c / 2) * kFPanel + row * 128;
-#pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            const int chunk = (c & 1) * 4 + c4;
-            *reinterpret_cast<uint4*>(dq_row + ((chunk ^ (row & 7)) << 4)) =
-                make_uint4(o[4 * c4], o[4 * c4 + 1], o[4 * c4 + 2], o[4 * c4 + 3]);
+            if (!ok) break;
+            back ^= 1u;
           }
         }
-        fence_proxy_async_smem();
-        mbar_arrive(&bars->dq_staged);
+        // dQ of the tile: tensor memory -> swizzled fp32 staging, a panel of 32 columns at a time, which
+        // the reducer warp sends on: one panel is staged while the other is being read. dq_drained: the
+        // next tile's dQ may overwrite this one.
+        if (!(ok = turn_f32(kColDQ, &bars->dq_drained))) break;
       }
-      cur = nxt;
-      nxt = (ok && cur < n_items) ? feed.fetch(n_items) : n_items;
     }
   } else {
     // ------------------------------ compute warps ------------------------------
     setmaxnreg_inc<kRegsCompute>();
     const int quad = warp % 4;            // TMEM lane quadrant of this warp
-    const int cg = warp / 4;              // which 32 key columns of the 128
-    const int row = quad * 32 + lane;     // query row within the tile = TMEM lane
+    const int cg = warp / 4;              // which 32 query columns of the 128
+    const int row = quad * 32 + lane;     // key row within the tile = TMEM lane
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     const float scale_log2 = scale * kFLog2e;
-    const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
-    uint8_t* p_row = smem + L::kP + (cg / 2) * kFPanel + row * 128;
+    const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f, grad_scale = scale * keep_scale;
     uint8_t* ds_row = smem + L::kDS + (cg / 2) * kFPanel + row * 128;
+    const float* vec = reinterpret_cast<const float*>(smem + L::kVec) + cg * 32;
     bool ok = true;
 
-    // Per-row scalars (lse and delta of the tile's 128 queries) come from the producer's loads:
-    // global loads of the compute warps would queue behind the dQ reduce traffic on the SM's
-    // path to L2, for thousands of clocks. Queries beyond S contribute nothing (p = exp2(-inf)).
-    // Keep bits of this thread's 32 key columns for one tile: word cg of the row's record,
-    // fetched a tile ahead like the row scalars.
-    auto load_keep = [&](bool valid, int q_tile, int k_tile, int bh) -> uint32_t {
-      if (DROP != 2 || !valid) return 0u;
-      return __ldg(mask_bits + mask_bits_record(bh, q_tile, k_tile, row, n_tiles) * 4 + cg);
+    // Keep bits: bit 8 b + 7 - k of a lane's word is for query 4 k + b of its 32, so that k shifts to the
+    // left bring those of queries 4 k .. 4 k + 3 to the four bytes' signs, from where one prmt makes a mask.
+    // From a drawn mask (DROP 2) this lane fetches the word of one query for the warp's 32 keys; a 32 x 32
+    // bit transposition across the warp turns it round.
+    auto transpose_bits = [&](uint32_t w) -> uint32_t {
+      uint32_t m = 0x0000ffffu;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1, m ^= m << d) {
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, w, d);
+        w = (lane & d) ? ((w & ~m) | ((o >> d) & m)) : ((w & m) | ((o & m) << d));
+      }
+      return w;
     };
 
-    ItemFeed feed{bars, abort_flag, 0};
-    int cur = feed.fetch(n_items);
-    int nxt = cur < n_items ? feed.fetch(n_items) : n_items;
-    uint32_t keep_word = 0u, next_keep = 0u;
-    if (DROP == 2 && cur < n_items) {
-      const Item t0 = decode_item(cur, BH, n_tiles, group_bh);
-      next_keep = load_keep(true, t0.kt, t0.kt, t0.bh);
-    }
-    int g = 0, j = 0;
+    ItemFeed feed{bars, abort_flag, n_tiles, 0};
+    int g = 0;
 
-    for (; ok && cur < n_items; ++j) {
-      const Item t = decode_item(cur, BH, n_tiles, group_bh);
-      const int k0 = t.kt * kFT;
+    for (Item t = feed.fetch(); ok && t.n_it > 0; t = feed.fetch()) {
       for (int i = 0; i < t.n_it; ++i, ++g) {
-        const int q = (t.kt + i) * kFT + row;
         const bool diagonal = (i == 0);
-        const int vs = g % kFStages;
-        const float* vbuf = reinterpret_cast<const float*>(smem + L::kVec + vs * L::kVecStride);
-        if (DROP == 2) {
-          // the next tile's keep bits: requested here, first used in that tile
-          keep_word = next_keep;
-          if (i + 1 < t.n_it) {
-            next_keep = load_keep(true, t.kt + i + 1, t.kt, t.bh);
-          } else {
-            const Item tn = decode_item(nxt < n_items ? nxt : 0, BH, n_tiles, group_bh);
-            next_keep = load_keep(nxt < n_items, tn.kt, tn.kt, tn.bh);
+        uint32_t keep_word = 0u;
+        if (DROP == 2)   // (there by the time the exponentials are done)
+          keep_word = __ldg(mask_bits + mask_bits_record(t.bh, t.kt + i, t.kt, cg * 32 + 4 * (7 - (lane & 7)) + (lane >> 3), n_tiles) * 4 + quad);
+        // the scores and the tile's row scalars
+        if (!(ok = mbar_wait(&bars->s_full[g & 1], (g >> 1) & 1, abort_flag))) break;
+        tc_fence_after_sync();
+        const float* v_lse = vec + (g & 1) * (2 * kFT);
+        const float* v_delta = v_lse + kFT;
+        uint32_t x[32];   // S^T, then p
+        tmem_ld32(tlane + kColS + cg * 32, x);
+        tmem_wait_ld();
+        if (diagonal) {   // the causal compare only exists on an item's first tile
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (row > cg * 32 + c) x[c] = 0xff800000u;   // -inf: p = 0
+        }
+#pragma unroll
+        for (int c = 0; c < 32; c += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(v_lse + c);   // (all lanes want the same four)
+          const float2 e0 = ffma2(make_float2(__uint_as_float(x[c]), __uint_as_float(x[c + 1])),
+                                  make_float2(scale_log2, scale_log2), make_float2(l.x, l.y));
+          const float2 e1 = ffma2(make_float2(__uint_as_float(x[c + 2]), __uint_as_float(x[c + 3])),
+                                  make_float2(scale_log2, scale_log2), make_float2(l.z, l.w));
+          x[c] = __float_as_uint(ex2(e0.x));
+          x[c + 1] = __float_as_uint(ex2(e0.y));
+          x[c + 2] = __float_as_uint(ex2(e1.x));
+          x[c + 3] = __float_as_uint(ex2(e1.y));
+        }
+
+        if (DROP == 1 && (!diagonal || quad <= cg)) {   // (beyond the diagonal there is nothing to drop)
+          const uint64_t q = static_cast<uint64_t>(t.kt + i) * kFT + cg * 32;
+          const uint64_t idx = (static_cast<uint64_t>(unit0 + t.bh) * S + q) * S + t.kt * kFT + row;
+#pragma unroll 4
+          for (int c = 0; c < 32; ++c)
+            keep_word |= (philox_keep(rng, idx + static_cast<uint64_t>(c) * S, rate) ? 1u : 0u) << (8 * (c & 3) + 7 - (c >> 2));
+        }
+        if (DROP == 2) keep_word = transpose_bits(keep_word);
+        // dP^T of this tile follows dV of the tile before, whose P^T has then been read
+        if (!(ok = mbar_wait(&bars->dp_full, g & 1, abort_flag))) break;
+        tc_fence_after_sync();
+        uint32_t w[16];   // 32 queries = 16 packed columns = two K steps of the dV / dK products
+#pragma unroll
+        for (int c = 0; c < 32; c += 4) {
+          float2 p0 = make_float2(__uint_as_float(x[c]), __uint_as_float(x[c + 1]));
+          float2 p1 = make_float2(__uint_as_float(x[c + 2]), __uint_as_float(x[c + 3]));
+          if (DROP) {
+            p0 = fmul2(p0, make_float2(keep_scale, keep_scale));
+            p1 = fmul2(p1, make_float2(keep_scale, keep_scale));
+          }
+          w[c / 2] = pack_bf16(p0.x, p0.y);
+          w[c / 2 + 1] = pack_bf16(p1.x, p1.y);
+          if (DROP) {
+            w[c / 2] &= byte_signs<0x9988>(keep_word << (c / 4));
+            w[c / 2 + 1] &= byte_signs<0xbbaa>(keep_word << (c / 4));
           }
         }
-        // (one barrier per stage: its next completion needs the stage back from the GEMMs of tile
-        // g, hence this thread's own P / dS, so the phase cannot run away from a slow waiter)
-        if (!(ok = mbar_wait(&bars->vec_full[vs], (g / kFStages) & 1, abort_flag))) break;
-        const int at = t.bh * S + (t.kt + i) * kFT;     // the tile's first row in the [BH, S] vectors
-        const bool in = q < S;
-        const float row_lse2 = in ? vbuf[((at + lse_shift) & 3) + row] * kFLog2e : INFINITY;
-        const float row_delta_s = in ? vbuf[L::kVecDelta / 4 + (at & 3) + row] * scale : 0.f;
-        if (!(ok = mbar_wait(&bars->x_full, g & 1, abort_flag))) break;
-        tc_fence_after_sync();
-        // Sixteen columns at a time: the packed results have to wait in registers for the P / dS
-        // buffers, and nothing here may spill (local memory shares the path the reduce-adds load).
-        uint32_t pw[16], dw[16];
+        tmem_st16(tlane + kColP + cg * 16, w);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(&bars->p_full);   // (the scores are in registers, too: the next tile's may overwrite them)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          uint32_t x1[16], x2[16];
-          tmem_ld16(tlane + kColS + cg * 32 + h * 16, x1);
+          uint32_t x2[16];
           tmem_ld16(tlane + kColDP + cg * 32 + h * 16, x2);
           tmem_wait_ld();
-          if (h == 1) {
-            tc_fence_before_sync();
-            mbar_arrive(&bars->x_free);  // scores are in registers: the next tile's GEMMs may overwrite
-          }
-          // ds = p (dP - delta) scale as p * fma(dP, scale, -delta scale), two columns at a time
-          // with packed two-float instructions; the causal compare only exists on an item's first
-          // (diagonal) tile
-          auto pair = [&](int cc, bool masked, uint32_t& pw_, uint32_t& dw_) {
-            const int key = k0 + cg * 32 + h * 16 + cc;
-            const float2 e = ffma2(make_float2(__uint_as_float(x1[cc]), __uint_as_float(x1[cc + 1])),
-                                   make_float2(scale_log2, scale_log2), make_float2(-row_lse2, -row_lse2));
-            float2 p = make_float2(ex2(e.x), ex2(e.y));
-            if (masked) {
-              if (key > q) p.x = 0.f;
-              if (key + 1 > q) p.y = 0.f;
-            }
-            float2 gr = make_float2(__uint_as_float(x2[cc]), __uint_as_float(x2[cc + 1]));
-            float2 pd = p;
-            if (DROP == 1) {
-              const uint64_t idx = (static_cast<uint64_t>(unit0 + t.bh) * S + q) * S + key;
-              const float m0 = (p.x != 0.f && philox_keep(rng, idx, rate)) ? keep_scale : 0.f;
-              const float m1 = (p.y != 0.f && philox_keep(rng, idx + 1, rate)) ? keep_scale : 0.f;
-              pd = fmul2(p, make_float2(m0, m1));
-              gr = fmul2(gr, make_float2(m0, m1));
-            } else if (DROP == 2) {
-              const float m0 = ((keep_word >> (h * 16 + cc)) & 1u) ? keep_scale : 0.f;
-              const float m1 = ((keep_word >> (h * 16 + cc + 1)) & 1u) ? keep_scale : 0.f;
-              pd = fmul2(p, make_float2(m0, m1));
-              gr = fmul2(gr, make_float2(m0, m1));
-            }
-            const float2 ds = fmul2(p, ffma2(gr, make_float2(scale, scale), make_float2(-row_delta_s, -row_delta_s)));
-            pw_ = pack_bf16(pd.x, pd.y);
-            dw_ = pack_bf16(ds.x, ds.y);
-          };
-          if (diagonal) {
+          // ds = p (dP - delta) scale as p * fma(dP, scale, -delta scale)
 #pragma unroll
-            for (int cc = 0; cc < 16; cc += 2) pair(cc, true, pw[h * 8 + cc / 2], dw[h * 8 + cc / 2]);
-          } else {
-#pragma unroll
-            for (int cc = 0; cc < 16; cc += 2) pair(cc, false, pw[h * 8 + cc / 2], dw[h * 8 + cc / 2]);
+          for (int c = 0; c < 16; c += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(v_delta + h * 16 + c);
+            uint32_t* gr = x2 + c;
+            if (DROP) {
+              const uint32_t k4 = keep_word << (h * 4 + c / 4);
+              gr[0] &= byte_signs<0x8888>(k4);
+              gr[1] &= byte_signs<0x9999>(k4);
+              gr[2] &= byte_signs<0xaaaa>(k4);
+              gr[3] &= byte_signs<0xbbbb>(k4);
+            }
+            const int at = h * 16 + c;
+            const float2 ds0 = fmul2(make_float2(__uint_as_float(x[at]), __uint_as_float(x[at + 1])),
+                                     ffma2(make_float2(__uint_as_float(gr[0]), __uint_as_float(gr[1])),
+                                           make_float2(grad_scale, grad_scale), make_float2(d4.x, d4.y)));
+            const float2 ds1 = fmul2(make_float2(__uint_as_float(x[at + 2]), __uint_as_float(x[at + 3])),
+                                     ffma2(make_float2(__uint_as_float(gr[2]), __uint_as_float(gr[3])),
+                                           make_float2(grad_scale, grad_scale), make_float2(d4.z, d4.w)));
+            w[at / 2] = pack_bf16(ds0.x, ds0.y);
+            w[at / 2 + 1] = pack_bf16(ds1.x, ds1.y);
           }
         }
-        // P / dS of tile g-1 consumed and its dQ complete in tensor memory
+        // dS^T of tile g-1 consumed
         if (g > 0) {
           if (!(ok = mbar_wait(&bars->acc_done, (g - 1) & 1, abort_flag))) break;
           tc_fence_after_sync();
         }
+        tmem_st16(tlane + kColDP + cg * 32, w);
 #pragma unroll
         for (int v4 = 0; v4 < 4; ++v4) {
           const int chunk = (cg & 1) * 4 + v4;  // 16-byte chunk within the 128-byte row of the panel
-          const int off = (chunk ^ (row & 7)) << 4;
-          *reinterpret_cast<uint4*>(p_row + off) =
-              make_uint4(pw[4 * v4], pw[4 * v4 + 1], pw[4 * v4 + 2], pw[4 * v4 + 3]);
-          *reinterpret_cast<uint4*>(ds_row + off) =
-              make_uint4(dw[4 * v4], dw[4 * v4 + 1], dw[4 * v4 + 2], dw[4 * v4 + 3]);
+          *reinterpret_cast<uint4*>(ds_row + ((chunk ^ (row & 7)) << 4)) =
+              make_uint4(w[4 * v4], w[4 * v4 + 1], w[4 * v4 + 2], w[4 * v4 + 3]);
         }
+        tmem_wait_st();
+        tc_fence_before_sync();
         fence_proxy_async_smem();
         mbar_arrive(&bars->w_full);
       }
-      cur = nxt;
-      nxt = (ok && cur < n_items) ? feed.fetch(n_items) : n_items;
+      if (!ok) break;
     }
-
   }
 
   tc_fence_before_sync();
@@ -800,33 +830,6 @@ int make_dq_workspace_map(CUtensorMap* map, float* ws, int BH, int S) {
   return DADATTN_OK;
 }
 
-// A [n] fp32 vector of per-row scalars as a 1-D map with boxes of kVecBox words. `base` need not
-// be 16-byte aligned: the map starts at the boundary below it and *shift is the number of words
-// in between, which the kernel adds to its row index.
-int make_row_scalar_map(CUtensorMap* map, const float* base, int64_t n, int* shift) {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  if (!fn) return fail(DADATTN_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  const uintptr_t addr = reinterpret_cast<uintptr_t>(base);
-  if (addr % 4) return fail(DADATTN_E_ARG, "a float vector is not 4-byte aligned");
-  *shift = static_cast<int>((addr % 16) / 4);
-  const cuuint64_t dims[1] = {static_cast<cuuint64_t>(n + *shift)};
-  const cuuint64_t strides[1] = {0};   // unused with one dimension
-  const cuuint32_t box[1] = {kVecBox};
-  const cuuint32_t estr[1] = {1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 1, reinterpret_cast<void*>(addr - addr % 16), dims,
-                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(DADATTN_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return DADATTN_OK;
-}
-
 }  // namespace
 }  // namespace dadattn
 namespace dadattn {
@@ -846,8 +849,7 @@ static int launch_fused_kernel(float* dq_ws, uint16_t* dk, uint16_t* dv, float* 
                                const uint16_t* k, const uint16_t* v, int BH, int S, const UnitLayout& lay, float scale,
                                float rate, const PhiloxKey& rng, int64_t unit0, const uint32_t* mask_bits,
                                cudaStream_t st) {
-  CUtensorMap mq, mk, mv, mdo, mws, mdk, mdv, mlse, mdelta;
-  int lse_shift = 0, delta_shift = 0;   // the workspace is 256-byte aligned: delta needs none
+  CUtensorMap mq, mk, mv, mdo, mws, mdk, mdv;
   if (int rc = make_tensor_map_bf16_units(&mq, q, BH, S, kFD, kFT, lay)) return rc;
   if (int rc = make_tensor_map_bf16_units(&mk, k, BH, S, kFD, kFT, lay)) return rc;
   if (int rc = make_tensor_map_bf16_units(&mv, v, BH, S, kFD, kFT, lay)) return rc;
@@ -860,13 +862,9 @@ static int launch_fused_kernel(float* dq_ws, uint16_t* dk, uint16_t* dv, float* 
     if (int rc = make_tensor_map_bf16_units(&mdv, dv, BH, S, kFD, kFT, lay)) return rc;
   }
   if (int rc = make_dq_workspace_map(&mws, dq_ws, BH, S)) return rc;
-  // (the kernel indexes the [BH, S] vectors with 32-bit TMA coordinates)
   if (static_cast<int64_t>(BH) * S > INT32_MAX - 1024)
     return fail(DADATTN_E_UNSUPPORTED, "BH * S = %lld rows exceed what the fused backward addresses",
                 static_cast<long long>(BH) * S);
-  if (int rc = make_row_scalar_map(&mlse, lse, static_cast<int64_t>(BH) * S, &lse_shift)) return rc;
-  if (int rc = make_row_scalar_map(&mdelta, delta, static_cast<int64_t>(BH) * S, &delta_shift)) return rc;
-  if (delta_shift != 0) return fail(DADATTN_E_ARG, "the backward workspace is not 16-byte aligned");
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
   // One persistent CTA per SM; the CTAs draw (key tile, batch x head) items from a counter.
@@ -887,7 +885,7 @@ static int launch_fused_kernel(float* dq_ws, uint16_t* dk, uint16_t* dv, float* 
   static std::atomic<int> regs_seen[4];
   if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kRegsLaunch, regs_seen[variant])) return rc;
   DAD_CUDA(launch_pdl(kern, grid, dim3(kFThreads), FusedSmem::kBytes, st, mq, mk, mv, mdo, mws, mdk, mdv,
-                      mlse, mdelta, lse_shift, item_counter, BH, S, lay.heads, group_bh, scale, rate,
+                      lse, delta, item_counter, BH, S, lay.heads, group_bh, scale, rate,
                       rng, unit0, mask_bits, status));
   return DADATTN_OK;
 }

@@ -80,7 +80,7 @@ constexpr uint32_t kSpinLimit = 1u << 21;  // a try_wait that fails has been sus
 // ready took 200-400 clocks), and a step at 192 x 1024 x 64 took 200 us, so written 187. POLLS plain polls
 // come before the wait that suspends: 2 against none are worth 0.3 %, 24 cost the head-size-64 kernels 5 %
 // and gain the head-size-128 forward, whose code is short, 2 % (3.31 -> 3.25 ms at 192 x 8192).
-template <int POLLS = 2>
+template <int POLLS = 0>
 __device__ __forceinline__ bool mbar_wait_at(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site) {
 #pragma unroll
   for (int i = 0; i < POLLS; ++i)
