@@ -62,6 +62,10 @@ static_assert(kFThreads * kRegsLaunch <= 65536 && (kRegsLaunch + 8) * kFThreads 
               "kRegsLaunch is not what the compiler gives a CTA of this size");
 constexpr int kFStages = 3;
 constexpr int kFRing = 4;                 // entries of the work-item ring (a power of two)
+// Rows of all units up to which they are one group. Backward alone, us, one group / groups of up to 65536
+// rows: 48 x 2048 90.9 / 95.9, 24 x 4096 152 / 159; above, as groups of 98304 rows / of 65536: 192 x 1024
+// 114.5 / 113.0, 144 x 700 67 / 62. Groups as even as they come: 72 x 777 as 64 + 8 units 47.5, as one 42.
+constexpr int kFAllInL2 = 98304;
 constexpr float kFLog2e = 1.4426950408889634f;
 
 struct FusedSmem {
@@ -868,16 +872,15 @@ static int launch_fused_kernel(float* dq_ws, uint16_t* dk, uint16_t* dv, float* 
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
   // One persistent CTA per SM; the CTAs draw (key tile, batch x head) items from a counter.
-  // Batch x head units are worked on in groups whose Q, dO and dQ rows (1 KiB per query) stay
-  // well inside L2.
+  // Batch x head units are worked on in even groups whose Q, dO and dQ rows (1 KiB per query) stay
+  // well inside L2; in one where all of them fit, since every group but the last ends on its short items.
   const int64_t n_items = static_cast<int64_t>((S + kFT - 1) / kFT) * BH;
   if (n_items > INT32_MAX / 2) return fail(DADATTN_E_UNSUPPORTED, "too many (key tile, batch x head) items");
   int dev = 0, sms = 0;
   DAD_CUDA(cudaGetDevice(&dev));
   DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
-  int group_bh = 65536 / S;
-  group_bh = group_bh < 1 ? 1 : (group_bh > 64 ? 64 : group_bh);
+  const int group_bh = static_cast<int64_t>(BH) * S <= kFAllInL2 ? BH : leveled_grid(65536, S, BH).group;
   const int variant = f32_dk ? 3 : rate > 0.f ? (mask_bits ? 2 : 1) : 0;
   auto kern = variant == 3 ? flash_bwd_fused_kernel<0, true> : variant == 2 ? flash_bwd_fused_kernel<2, false>
               : variant == 1 ? flash_bwd_fused_kernel<1, false> : flash_bwd_fused_kernel<0, false>;
