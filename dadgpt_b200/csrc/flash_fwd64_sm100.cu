@@ -24,8 +24,9 @@
 //     as packed bf16 over the first half of the same columns, from where the P V product takes
 //     it as its A operand;
 //   * scale-and-subtract and the row sums run as packed two-float instructions (fma.rn.f32x2,
-//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in four as a
-//     cubic on the FMA pipe (a bf16x2 exp2 on the special-function unit was tried: no faster, and
+//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in eight as a
+//     cubic on the FMA pipe (48 x 4096 forward under the power cap: 146.8 us; one in four 149, none
+//     148.5; a bf16x2 exp2 on the special-function unit was tried: no faster, and
 //     it cost a digit of lse): the softmax is bound by instruction issue, not by any one unit;
 //   * CTAs are persistent: barriers, tensor memory and descriptors are set up once, items are
 //     dealt out heaviest first in a fixed serpentine order (no global counter to reset), the
@@ -436,6 +437,16 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               if (i > limit) xa[i] = 0xff800000u;  // -inf
           }
         };
+        if (diagonal && c * 64 + half * 32 > quad * 32 + 31) {   // the warp's block lies beyond the diagonal
+          uint32_t zero[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) zero[i] = 0u;
+          tmem_st16(tS, zero);
+          tmem_wait_st();
+          tc_fence_before_sync();
+          mbar_arrive(&bars->p_full[X][c]);
+          continue;   // (an item's first block: m stays -inf)
+        }
         load_scores();
         float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -482,7 +493,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int i = 0; i < 32; i += 2) {
           const float2 e = ffma2(make_float2(__uint_as_float(xa[i]), __uint_as_float(xa[i + 1])), sl, nm);
           float2 p;
-          if ((i & 7) == 6) {   // one pair in four on the FMA pipe
+          if ((i & 15) == 14) {   // one pair in eight on the FMA pipe
             p = ex2_poly2(e);
           } else {
             p.x = ex2(e.x);

@@ -77,9 +77,10 @@ constexpr uint32_t kSpinLimit = 1u << 21;  // a try_wait that fails has been sus
 // The wait is a handful of instructions, and has to be: kernels with six roles hold some thirty of them.
 // As 128 polls, which the compiler unrolled, ahead of a try_wait loop with back-off, they made 280 of the
 // 333 KB of the head-size-64 gradient kernel; the warps stood still for instructions (a wait that was
-// ready took 200-400 clocks), and a step at 192 x 1024 x 64 took 200 us, so written 187. POLLS plain polls
-// come before the wait that suspends: 2 against none are worth 0.3 %, 24 cost the head-size-64 kernels 5 %
-// and gain the head-size-128 forward, whose code is short, 2 % (3.31 -> 3.25 ms at 192 x 8192).
+// ready took 200-400 clocks), and a step at 192 x 1024 x 64 took 200 us, so written 187. A hand-over
+// from one warp to another takes 125 clocks when the waiter is suspended in try_wait and 210-290 when it
+// polls with test_wait; POLLS plain polls ahead are for the head-size-128 forward, whose code is short: 24
+// are worth 2 % there (3.31 -> 3.25 ms at 192 x 8192) and cost the head-size-64 kernels 5 %.
 template <int POLLS = 0>
 __device__ __forceinline__ bool mbar_wait_at(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site) {
 #pragma unroll
