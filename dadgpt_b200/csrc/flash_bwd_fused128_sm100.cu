@@ -11,18 +11,22 @@
 // P^T and dS^T go back into tensor memory as packed bf16 and are the A operands of dV / dK from
 // there (tcgen05.mma with A in TMEM): an MMA with both operands in shared memory reads them at
 // 128 B/clk, and with the TMA loads, the stores and the dQ staging the shared-memory traffic of
-// a step (336 KB when P^T / dS^T lived there), not the tensor core, set the step time. dS^T is
+// a step (336 KB when P^T / dS^T lived there, now 224) weighs as much as the products. dS^T is
 // also written, bf16, [key][query] in the 128-byte swizzled layout, as the MN-major B operand
 // of dQ^T, whose A operand is the resident K tile read MN-major. Computing dQ transposed keeps
 // all 128 TMEM lanes busy (M = 128 head dims) although a step has only 64 queries.
-// Each step's dQ^T tile (32 KB fp32) goes TMEM -> staging in shared memory -> bulk reduce-add
-// into an fp32 workspace laid out tile by tile ([BH][64-query block][128 dims][64 queries], rows
-// swizzled as staged), which a last pass transposes and rounds to bf16. The sums into the
-// workspace happen in whatever order the CTAs reach them, so dQ may differ in its last bits from
-// run to run; dadattn_set_bwd_deterministic(1) selects the two-kernel path.
-//   warp 0      TMA producer          warp 1      MMA issuer + TMEM owner
-//   warps 2-17  compute: four warps per TMEM lane quadrant, each taking 16 of the 64 query columns
-//   warp 18     dQ reducer
+// Each step's dQ^T tile (32 KB fp32) goes from tensor memory through registers of four drain warps into an
+// fp32 workspace by red.global.add.v4, laid out so that a warp's lanes, one head dim each, add 512
+// consecutive bytes ([BH][64-query block][16 groups of 4 queries][128 dims][4 queries]): 1290 clocks a tile
+// and SM, as fast as bulk reduce-adds from shared memory (1390; rows of 256 bytes apart, a lane on each,
+// take 2400), without the 64 KB a step that staging costs where shared memory sets the pace. A last pass
+// rounds the workspace to bf16. The sums happen in whatever order the CTAs reach them, so dQ may differ in
+// its last bits from run to run; dadattn_set_bwd_deterministic(1) selects the two-kernel path.
+//   warps 0-15   compute: four warps per TMEM lane quadrant, each taking 16 of the 64 query columns
+//   warp 16      TMA producer          warp 17      MMA issuer + TMEM owner
+//   warp 18      row scalars: -lse log2e and -delta scale of each step's queries      (warp 19 idle)
+//   warps 20-23  drain: dQ^T out of tensor memory, one thread per lane, while the compute warps are
+//                already on the next step's arithmetic
 #include <cuda_bf16.h>
 
 #include <cfloat>
@@ -35,14 +39,28 @@ namespace {
 
 using namespace ptx;
 
+// Two plain polls ahead of the suspending wait: 192 x 8192 10.30 ms, none 10.39, 8 10.39, 24 10.37 (each before
+// the products were issued by a whole warp).
+#define polled_wait(bar, parity, abort_flag) mbar_wait_at<2>(bar, parity, abort_flag, __LINE__)
+#define polled_warp_wait(bar, parity, abort_flag) __all_sync(0xffffffffu, polled_wait(bar, parity, abort_flag))
+
 constexpr int kGD = 128;                   // head size
 constexpr int kGKeys = 128;                // keys owned by a CTA
 constexpr int kGSub = 64;                  // queries per step
 constexpr int kGPanel = 128 * 128;         // [128 rows][64 bf16] swizzled panel
 constexpr int kGSubPanel = 64 * 128;       // [64 rows][64 bf16] swizzled panel
-constexpr int kGStages = 3;                // streamed-tile ring depth
-constexpr int kGThreads = 19 * 32;
+constexpr int kGStages = 4;                // streamed-tile ring depth
+constexpr int kGThreads = 24 * 32;
 constexpr int kGCompute = 16 * 32;
+constexpr int kGDrain = 4 * 32;
+constexpr int kGWarpProducer = 16, kGWarpIssuer = 17, kGWarpScalars = 18, kGWarpDrain0 = 20;
+// Registers per thread once the warpgroups have rebalanced; the pool is what the CTA starts with. (The
+// drain threads hold a row of 64 sums.)
+constexpr int kGRegsLaunch = 80, kGRegsCompute = 88, kGRegsHelper = 48, kGRegsDrain = 80;
+static_assert(kGCompute * kGRegsCompute + 128 * kGRegsHelper + kGDrain * kGRegsDrain <= kGThreads * kGRegsLaunch,
+              "the warpgroups ask for more registers than the CTA owns");
+static_assert(kGThreads * kGRegsLaunch <= 65536 && (kGRegsLaunch + 8) * kGThreads > 65536,
+              "kGRegsLaunch is not what the compiler gives a CTA of this size");
 // Up to this many CTAs the key tiles go level by level (leveled_grid) and the delta kernel clears the
 // workspace; with more waves the order gains nothing and the cleared lines, by then out of L2, are better
 // written by a memset ahead of the reads. Backward alone, us by CTAs, level by level / unit by unit:
@@ -63,29 +81,24 @@ struct G128Smem {
   static constexpr int kQ = kV + kTile;
   static constexpr int kDO = kQ + kGStages * kSubTile;
   static constexpr int kDS = kDO + kGStages * kSubTile;  // [128 keys][64 q] bf16, one panel
-  static constexpr int kDQ = kDS + kGPanel;              // [128 dims][64 q] fp32 staging
-  static constexpr int kVec = kDQ + kGDqTileBytes;       // lse*log2e, delta: 2 x [2][64] fp32
+  static constexpr int kVec = kDS + kGPanel;             // two buffers of [2][64] row scalars
   static constexpr int kBars = kVec + 2 * 2 * 64 * 4;
   static constexpr int kBytes = kBars + 256;
   static_assert(kBytes <= 232448, "shared memory budget of one CTA exceeded");
 };
 
 struct G128Bars {
-  uint64_t kv_full, q_full[kGStages], do_full[kGStages], qdo_empty[kGStages];
-  uint64_t x_full, x_free, w_full, acc_done, vec_full, dq_drained, dq_staged, dq_sent;
+  uint64_t kv_full, qdo_full[kGStages], qdo_empty[kGStages];
+  uint64_t x_full[2], x_free, w_full, acc_done, dq_drained;
   uint32_t tmem_base;
   int abort_flag;
 };
 
-__device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, const void* smem_src, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-               ::"l"(gdst), "r"(smem_u32(smem_src)), "r"(bytes) : "memory");
+__device__ __forceinline__ void red_add4(float* to, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(__uint_as_float(a)),
+               "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
+               : "memory");
 }
-__device__ __forceinline__ void bulk_commit_g() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0_g() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_wait0_g() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
@@ -104,10 +117,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
-// 16-byte chunk `c` (0..15) of staging / workspace row `row` (256 bytes = 64 fp32) sits at chunk
-// c ^ (row & 15): a warp writing one chunk of 32 consecutive rows then spreads over all banks.
-__host__ __device__ __forceinline__ int dq_chunk(int c, int row) { return c ^ (row & 15); }
-
 template <bool DROP, bool LEVELED>
 __global__ void __launch_bounds__(kGThreads, 1)
 flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -115,7 +124,8 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
                           __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
                           float* __restrict__ dq_ws, const float* __restrict__ lse,
                           const float* __restrict__ delta, int S, float scale, float rate,
-                          PhiloxKey rng, int64_t unit0, LeveledGrid order, int* __restrict__ status) {
+                          const __grid_constant__ PhiloxRounds rng, int64_t unit0, LeveledGrid order,
+                          int* __restrict__ status) {
   using L = G128Smem;
   constexpr int D = kGD;
   constexpr uint32_t kTmemCols = 512;
@@ -127,7 +137,6 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   extern __shared__ __align__(1024) uint8_t smem[];
   G128Bars* bars = reinterpret_cast<G128Bars*>(smem + L::kBars);
   volatile int* abort_flag = &bars->abort_flag;
-  float* vec = reinterpret_cast<float*>(smem + L::kVec);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n_sub = (S + kGSub - 1) / kGSub;
@@ -145,22 +154,19 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
     for (int s = 0; s < kGStages; ++s) {
-      mbar_init(&bars->q_full[s], 1);
-      mbar_init(&bars->do_full[s], 1);
+      mbar_init(&bars->qdo_full[s], 1);
       mbar_init(&bars->qdo_empty[s], 1);
     }
-    mbar_init(&bars->x_full, 1);
+    mbar_init(&bars->x_full[0], 2);      // the products and the step's row scalars
+    mbar_init(&bars->x_full[1], 2);
     mbar_init(&bars->x_free, kGCompute);
     mbar_init(&bars->w_full, kGCompute);
     mbar_init(&bars->acc_done, 1);
-    mbar_init(&bars->vec_full, kGCompute);
-    mbar_init(&bars->dq_drained, kGCompute);
-    mbar_init(&bars->dq_staged, kGCompute);
-    mbar_init(&bars->dq_sent, 1);
+    mbar_init(&bars->dq_drained, kGDrain);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 1) {
+  if (warp == kGWarpIssuer) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
     tmem_relinquish();
   }
@@ -171,7 +177,9 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   pdl_wait();
   pdl_launch_dependents();
 
-  if (warp == 0) {
+  if (warp >= kGWarpProducer && warp < kGWarpDrain0) {
+  setmaxnreg_dec<kGRegsHelper>();
+  if (warp == kGWarpProducer) {
     // ------------------------------ TMA producer ------------------------------
     if (elect_one()) {
       prefetch_tensormap(&map_k);
@@ -185,21 +193,19 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       }
       for (int i = 0; i < n_it; ++i) {
         const int s = i % kGStages, use = i / kGStages;
-        if (use > 0 && !mbar_wait(&bars->qdo_empty[s], (use - 1) & 1, abort_flag)) break;
+        if (use > 0 && !polled_wait(&bars->qdo_empty[s], (use - 1) & 1, abort_flag)) break;
         const int q0 = (first + i) * kGSub;
-        mbar_arrive_expect_tx(&bars->q_full[s], L::kSubTile);
-        for (int p = 0; p < 2; ++p)
-          tma_load_3d(smem + L::kQ + s * L::kSubTile + p * kGSubPanel, &map_q, &bars->q_full[s],
-                      p * 64, q0, bh);
-        mbar_arrive_expect_tx(&bars->do_full[s], L::kSubTile);
-        for (int p = 0; p < 2; ++p)
-          tma_load_3d(smem + L::kDO + s * L::kSubTile + p * kGSubPanel, &map_do, &bars->do_full[s],
-                      p * 64, q0, bh);
+        mbar_arrive_expect_tx(&bars->qdo_full[s], 2 * L::kSubTile);
+        for (int p = 0; p < 2; ++p) {
+          tma_load_3d(smem + L::kQ + s * L::kSubTile + p * kGSubPanel, &map_q, &bars->qdo_full[s], p * 64, q0, bh);
+          tma_load_3d(smem + L::kDO + s * L::kSubTile + p * kGSubPanel, &map_do, &bars->qdo_full[s], p * 64, q0, bh);
+        }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == kGWarpIssuer) {
     // ------------------------------ MMA issuer ------------------------------
-    if (elect_one()) {
+    {   // (the whole warp: mma_ss_warp)
+      const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       constexpr uint32_t idesc_x = make_idesc_bf16(128, 64, 0, 0);    // S^T, dP^T: both K-major
       constexpr uint32_t idesc_a = make_idesc_bf16(128, D, 0, 1);     // dV, dK: B MN-major
       constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, 1, 1);    // dQ^T: A and B MN-major
@@ -211,49 +217,47 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       // streamed tiles: K-major B of the score GEMMs, MN-major B (panels kGSubPanel apart) of dV / dK
       const SmemDescBase q_desc0 = make_desc_base_sw128(smem_u32(smem + L::kQ), kGSubPanel);
       const SmemDescBase do_desc0 = make_desc_base_sw128(smem_u32(smem + L::kDO), kGSubPanel);
-      bool ok = mbar_wait(&bars->kv_full, 0, abort_flag);
+      bool ok = polled_warp_wait(&bars->kv_full, 0, abort_flag);
 
       auto issue_x = [&](int i) -> bool {
         const int s = i % kGStages;
         const uint32_t par = (i / kGStages) & 1;
         const SmemDescBase qd{q_desc0.lo + s * (L::kSubTile >> 4), q_desc0.hi};
         const SmemDescBase dd{do_desc0.lo + s * (L::kSubTile >> 4), do_desc0.hi};
-        if (!mbar_wait(&bars->q_full[s], par, abort_flag)) return false;
+        if (!polled_warp_wait(&bars->qdo_full[s], par, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          mma_ss(tmem + kColS, desc_at(k_kmaj, (kk / 4) * kGPanel + (kk % 4) * 32),
-                 desc_at(qd, (kk / 4) * kGSubPanel + (kk % 4) * 32), idesc_x, kk > 0 ? 1u : 0u);
-        if (!mbar_wait(&bars->do_full[s], par, abort_flag)) return false;
+          mma_ss_warp(tm + kColS, desc_at(k_kmaj, (kk / 4) * kGPanel + (kk % 4) * 32),
+                 desc_at(qd, (kk / 4) * kGSubPanel + (kk % 4) * 32), idesc_x, kk > 0 ? 1u : 0u, lead);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          mma_ss(tmem + kColDP, desc_at(v_kmaj, (kk / 4) * kGPanel + (kk % 4) * 32),
-                 desc_at(dd, (kk / 4) * kGSubPanel + (kk % 4) * 32), idesc_x, kk > 0 ? 1u : 0u);
-        mma_commit(&bars->x_full);
+          mma_ss_warp(tm + kColDP, desc_at(v_kmaj, (kk / 4) * kGPanel + (kk % 4) * 32),
+                 desc_at(dd, (kk / 4) * kGSubPanel + (kk % 4) * 32), idesc_x, kk > 0 ? 1u : 0u, lead);
+        mma_commit_warp(&bars->x_full[i & 1], lead);
         return true;
       };
       auto issue_acc = [&](int i) -> bool {
         const int s = i % kGStages;
         const SmemDescBase qd{q_desc0.lo + s * (L::kSubTile >> 4), q_desc0.hi};
         const SmemDescBase dd{do_desc0.lo + s * (L::kSubTile >> 4), do_desc0.hi};
-        if (!mbar_wait(&bars->w_full, i & 1, abort_flag)) return false;
+        if (!polled_warp_wait(&bars->w_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < kGSub / 16; ++kk) {   // K dimension = 64 queries, 16 per MMA
           const uint32_t acc = (i > 0 || kk > 0) ? 1u : 0u;
-          mma_ts(tmem + kColDV, tmem + kColP + kk * 8, desc_at(dd, kk * 2048), idesc_a, acc);
-          mma_ts(tmem + kColDK, tmem + kColDSt + kk * 8, desc_at(qd, kk * 2048), idesc_a, acc);
+          mma_ts_warp(tm + kColDV, tm + kColP + kk * 8, desc_at(dd, kk * 2048), idesc_a, acc, lead);
+          mma_ts_warp(tm + kColDK, tm + kColDSt + kk * 8, desc_at(qd, kk * 2048), idesc_a, acc, lead);
         }
-        // the previous step's dQ^T must have left tensor memory before this one overwrites it;
-        // the compute warps read it right after they publish P^T / dS^T, while dV / dK are running
-        if (i > 0 && !mbar_wait(&bars->dq_drained, (i - 1) & 1, abort_flag)) return false;
+        mma_commit_warp(&bars->qdo_empty[s], lead);   // Q and dO of this stage are last read by the products above
+        // the previous step's dQ^T must have left tensor memory before this one overwrites it
+        if (i > 0 && !polled_warp_wait(&bars->dq_drained, (i - 1) & 1, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < kGKeys / 16; ++kk)    // K dimension = 128 keys
-          mma_ss(tmem + kColDQ, desc_at(k_mn, kk * 2048), desc_at(ds_desc, kk * 2048), idesc_q,
-                 kk > 0 ? 1u : 0u);
-        mma_commit(&bars->qdo_empty[s]);
-        mma_commit(&bars->acc_done);
+          mma_ss_warp(tm + kColDQ, desc_at(k_mn, kk * 2048), desc_at(ds_desc, kk * 2048), idesc_q,
+                 kk > 0 ? 1u : 0u, lead);
+        mma_commit_warp(&bars->acc_done, lead);
         return true;
       };
 
@@ -261,121 +265,127 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       for (int i = 0; ok && i < n_it; ++i) {
         // the next step's score GEMMs go first: the arithmetic on them overlaps this step's
         // accumulating GEMMs
-        if (i + 1 < n_it) ok = mbar_wait(&bars->x_free, i & 1, abort_flag) && issue_x(i + 1);
+        if (i + 1 < n_it) ok = polled_warp_wait(&bars->x_free, i & 1, abort_flag) && issue_x(i + 1);
         ok = ok && issue_acc(i);
       }
     }
-  } else if (warp == 18) {
-    // ------------------------------ dQ reducer ------------------------------
-    if (elect_one()) {
-      for (int i = 0; i < n_it; ++i) {
-        if (!mbar_wait(&bars->dq_staged, i & 1, abort_flag)) break;
-        float* dst = dq_ws + (static_cast<size_t>(bh) * n_sub + first + i) * (kGD * kGSub);
-        bulk_reduce_add_f32(dst, smem + L::kDQ, kGDqTileBytes);
-        bulk_commit_g();
-        bulk_wait_read0_g();
-        mbar_arrive(&bars->dq_sent);
+  } else if (warp == kGWarpScalars) {
+    // ------------------------------ row scalars ------------------------------
+    // -lse log2e and -delta scale of each step's 64 queries, requested a step ahead, into one of two buffers.
+    // Queries beyond S contribute nothing: p = exp2(-inf). Buffer i % 2 is free once the products of step
+    // i - 2, which follow the arithmetic that read it, have given their stage back; that barrier's next phase
+    // is a later step's, which needs these scalars first.
+    const size_t vec_base = static_cast<size_t>(bh) * S;
+    float rl[2], rd[2];
+    auto request = [&](int i) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int q = (first + i) * kGSub + c * 32 + lane;
+        rl[c] = q < S ? lse[vec_base + q] : INFINITY;
+        rd[c] = q < S ? delta[vec_base + q] : 0.f;
       }
-      bulk_wait0_g();   // every sum has landed before the CTA retires
+    };
+    request(0);
+    for (int i = 0; i < n_it; ++i) {
+      if (i >= 2 && !polled_wait(&bars->qdo_empty[(i - 2) % kGStages], ((i - 2) / kGStages) & 1, abort_flag)) break;
+      float* dst = reinterpret_cast<float*>(smem + L::kVec) + (i & 1) * 128 + lane;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        dst[c * 32] = -rl[c] * kGLog2e;
+        dst[64 + c * 32] = -rd[c] * scale;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->x_full[i & 1]);
+      if (i + 1 < n_it) request(i + 1);
+    }
+  }
+  } else if (warp >= kGWarpDrain0) {
+    // ------------------------------ dQ drain ------------------------------
+    setmaxnreg_dec<kGRegsDrain>();
+    const int quad = warp % 4;
+    const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    float* dst = dq_ws + (static_cast<size_t>(bh) * n_sub + first) * (kGD * kGSub) + (quad * 32 + lane) * 4;
+    for (int i = 0; i < n_it; ++i, dst += kGD * kGSub) {
+      if (!polled_wait(&bars->acc_done, i & 1, abort_flag)) break;
+      tc_fence_after_sync();
+      uint32_t o0[32], o1[32];
+      tmem_ld32(tlane + kColDQ, o0);
+      tmem_ld32(tlane + kColDQ + 32, o1);
+      tmem_wait_ld();
+      tc_fence_before_sync();
+      mbar_arrive(&bars->dq_drained);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) red_add4(dst + c * (kGD * 4), o0[4 * c], o0[4 * c + 1], o0[4 * c + 2], o0[4 * c + 3]);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) red_add4(dst + (8 + c) * (kGD * 4), o1[4 * c], o1[4 * c + 1], o1[4 * c + 2], o1[4 * c + 3]);
     }
   } else {
     // ------------------------------ compute warps ------------------------------
-    const int cw = warp - 2;              // 0..15
+    setmaxnreg_inc<kGRegsCompute>();
     const int quad = warp % 4;            // TMEM lane quadrant of this warp
-    const int cg = cw / 4;                // which 16 query columns of the 64
-    const int ct = cw * 32 + lane;        // 0..511 among the compute threads
-    const int row = quad * 32 + lane;     // key within the tile (and head dim of dQ^T) = TMEM lane
+    const int cg = warp / 4;              // which 16 query columns of the 64
+    const int row = quad * 32 + lane;     // key within the tile = TMEM lane
     const int key = k0 + row;
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
     const float scale_log2 = scale * kGLog2e;
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
-    const size_t vec_base = static_cast<size_t>(bh) * S;
+    const float* vec = reinterpret_cast<const float*>(smem + L::kVec) + cg * 16;
     uint8_t* ds_row = smem + L::kDS + row * 128;
-    uint8_t* dq_row = smem + L::kDQ + row * 256;
     bool ok = true;
-    // Per-column vectors (lse log2e and delta of the step's 64 queries): threads 0-127 fetch
-    // them one step ahead into a register and publish them through one of two shared-memory
-    // buffers, so that neither the global load nor a buffer hand-over sits in the step's chain.
-    auto fetch_vec = [&](int i) -> float {
-      const int qv = (first + i) * kGSub + (ct & 63);
-      if (ct >= 128 || i >= n_it || qv >= S) return ct < 64 ? INFINITY : 0.f;
-      return ct < 64 ? lse[vec_base + qv] * kGLog2e : delta[vec_base + qv];
-    };
-    float next_vec = fetch_vec(0);
-
-    // dQ^T of step t: TMEM [128 dims][64 q] -> staging (rows swizzled), which the reducer sends
-    // on. The caller has seen acc_done of step t.
-    auto drain_dq = [&](int t) -> bool {
-      uint32_t o[16];
-      tmem_ld16(tlane + kColDQ + cg * 16, o);
-      tmem_wait_ld();
-      tc_fence_before_sync();
-      mbar_arrive(&bars->dq_drained);
-      // the reduce of the previous step must have finished reading the staging buffer
-      if (t > 0 && !mbar_wait(&bars->dq_sent, (t - 1) & 1, abort_flag)) return false;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(dq_row + (dq_chunk(cg * 4 + c, row) << 4)) =
-            make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-      fence_proxy_async_smem();
-      mbar_arrive(&bars->dq_staged);
-      return true;
-    };
 
     for (int i = 0; i < n_it; ++i) {
-      const int q0 = (first + i) * kGSub;
-      const bool diagonal = i < 2;   // sub-tiles that straddle the diagonal need the comparison
-      // Buffer i % 2 was last read in step i-2, and every thread finished that step before it
-      // arrived at vec_full(i-1), which this thread has already seen complete.
-      float* v_lse = vec + (i & 1) * 128;
-      float* v_delta = v_lse + 64;
-      if (ct < 128) v_lse[ct] = next_vec;   // threads 64-127 land in v_delta
-      next_vec = fetch_vec(i + 1);
-      mbar_arrive(&bars->vec_full);
-      if (!(ok = mbar_wait(&bars->vec_full, i & 1, abort_flag))) break;
-      if (!(ok = mbar_wait(&bars->x_full, i & 1, abort_flag))) break;
+      const int q0 = (first + i) * kGSub + cg * 16;   // this thread's first query
+      const float* v_lse = vec + (i & 1) * 128;
+      const float* v_delta = v_lse + 64;
+      if (!(ok = polled_wait(&bars->x_full[i & 1], (i >> 1) & 1, abort_flag))) break;
       tc_fence_after_sync();
-
-      const int cbase = cg * 16;
       uint32_t x1[16], x2[16];
-      tmem_ld16(tlane + kColS + cbase, x1);
-      tmem_ld16(tlane + kColDP + cbase, x2);
+      tmem_ld16(tlane + kColS + cg * 16, x1);
+      tmem_ld16(tlane + kColDP + cg * 16, x2);
       tmem_wait_ld();
       tc_fence_before_sync();
-      mbar_arrive(&bars->x_free);  // scores are in registers: the next step's GEMMs may overwrite
+      mbar_arrive(&bars->x_free);  // scores are in registers: the next step's products may overwrite them
 
+      if (i < 2) {   // sub-tiles that straddle the diagonal
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          if (key > q0 + c) x1[c] = 0xff800000u;   // -inf: p = 0
+      }
+      uint32_t keep = 0xffffu;
+      if (DROP) {   // (draws only for pairs that count: key <= query < S)
+        const int lo = max(key - q0, 0), hi = min(S - q0, 16);
+        keep = lo < hi ? philox_keep_bits<2>(rng, (static_cast<uint64_t>(unit0 + bh) * S + q0 + lo) * S + key,
+                                             static_cast<uint32_t>(S), hi - lo) << lo
+                       : 0u;
+      }
       uint32_t pw[8], dw[8];
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
         // 128-bit broadcast reads: all lanes of a warp want the same four columns
-        const float4 a = *reinterpret_cast<const float4*>(v_lse + cbase + c);
-        const float4 b = *reinterpret_cast<const float4*>(v_delta + cbase + c);
-        const float l2[4] = {a.x, a.y, a.z, a.w}, dl[4] = {b.x, b.y, b.z, b.w};
-        float pv[4], dv4[4];
+        const float4 a = *reinterpret_cast<const float4*>(v_lse + c);
+        const float4 b = *reinterpret_cast<const float4*>(v_delta + c);
+        const float2 l2[2] = {make_float2(a.x, a.y), make_float2(a.z, a.w)}, dl[2] = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int query = q0 + cbase + c + e;
-          float p = ex2(fmaf(__uint_as_float(x1[c + e]), scale_log2, -l2[e]));
-          if (diagonal && key > query) p = 0.f;
-          float g = __uint_as_float(x2[c + e]);
-          float pd = p;
+        for (int h = 0; h < 2; ++h) {
+          const int e = c + 2 * h;
+          const float2 t = ffma2(make_float2(__uint_as_float(x1[e]), __uint_as_float(x1[e + 1])),
+                                 make_float2(scale_log2, scale_log2), l2[h]);
+          const float2 p = make_float2(ex2(t.x), ex2(t.y));
+          float2 pd = p, g = make_float2(__uint_as_float(x2[e]), __uint_as_float(x2[e + 1]));
           if (DROP) {
-            const uint64_t idx = (static_cast<uint64_t>(unit0 + bh) * S + query) * S + key;
-            const float mk = (p != 0.f && philox_keep(rng, idx, rate)) ? keep_scale : 0.f;
-            pd = p * mk;
-            g *= mk;
+            const float2 mk = make_float2((keep >> e) & 1u ? keep_scale : 0.f, (keep >> (e + 1)) & 1u ? keep_scale : 0.f);
+            pd = fmul2(p, mk);
+            g = fmul2(g, mk);
           }
-          pv[e] = pd;
-          dv4[e] = p * (g - dl[e]) * scale;
+          // ds = p (dP - delta) scale as p * fma(dP, scale, -delta scale)
+          const float2 ds = fmul2(p, ffma2(g, make_float2(scale, scale), dl[h]));
+          pw[e / 2] = pack_bf16(pd.x, pd.y);
+          dw[e / 2] = pack_bf16(ds.x, ds.y);
         }
-        pw[c / 2] = pack_bf16(pv[0], pv[1]);
-        pw[c / 2 + 1] = pack_bf16(pv[2], pv[3]);
-        dw[c / 2] = pack_bf16(dv4[0], dv4[1]);
-        dw[c / 2 + 1] = pack_bf16(dv4[2], dv4[3]);
       }
-      // P^T / dS^T of step i-1 consumed and its dQ^T complete in tensor memory
+      // P^T / dS^T of step i-1 consumed
       if (i > 0) {
-        if (!(ok = mbar_wait(&bars->acc_done, (i - 1) & 1, abort_flag))) break;
+        if (!(ok = polled_wait(&bars->acc_done, (i - 1) & 1, abort_flag))) break;
         tc_fence_after_sync();
       }
       // sixteen queries = eight packed columns = one K step of the dV / dK MMAs
@@ -392,16 +402,12 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       tc_fence_before_sync();
       fence_proxy_async_smem();
       mbar_arrive(&bars->w_full);
-      if (i > 0 && !(ok = drain_dq(i - 1))) break;
     }
 
-    // the last step's dQ^T, then dV (column groups 0, 1) and dK (2, 3), 64 head dims each
-    if (ok && (ok = mbar_wait(&bars->acc_done, (n_it - 1) & 1, abort_flag))) {
+    // dV (column groups 0, 1) and dK (2, 3), 64 head dims each
+    if (ok && polled_wait(&bars->acc_done, (n_it - 1) & 1, abort_flag)) {
       tc_fence_after_sync();
-      ok = drain_dq(n_it - 1);
-    }
-    if (ok) {
-      __nv_bfloat16* dst = (cg < 2 ? dv : dk) + (vec_base + key) * D + (cg & 1) * 64;
+      __nv_bfloat16* dst = (cg < 2 ? dv : dk) + (static_cast<size_t>(bh) * S + key) * D + (cg & 1) * 64;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t o[32];
@@ -422,7 +428,7 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == kGWarpIssuer) {
     __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem, kTmemCols);
@@ -463,27 +469,30 @@ __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __rest
   if (r < rows && c == 0) delta[r] = sum;
 }
 
-// Workspace tile [128 dims][64 queries] fp32 (rows swizzled as staged) -> dq[q][128] bf16.
-// One CTA of 256 threads per tile: thread t takes query t % 64 and 32 head dims.
-__global__ void fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict__ dq_ws,
-                                        int S, int n_sub) {
+// Workspace tile [16 groups of 4 queries][128 dims][4 queries] fp32 -> dq[q][128] bf16. One CTA of 256 threads
+// per tile: thread t takes head dims 2 (t % 64) and the next, so that a warp reads 1 KB and writes 128 bytes of
+// a row in one piece.
+__global__ void __launch_bounds__(256)
+fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict__ dq_ws, int S, int n_sub) {
   pdl_wait();
   const int bh = blockIdx.y, blk = blockIdx.x;
-  const float* tile = dq_ws + (static_cast<size_t>(bh) * n_sub + blk) * (kGD * kGSub);
-  const int qi = threadIdx.x % 64, dg = threadIdx.x / 64;
-  const int q = blk * kGSub + qi;
-  uint32_t w[16];
+  const float4* tile = reinterpret_cast<const float4*>(dq_ws + (static_cast<size_t>(bh) * n_sub + blk) * (kGD * kGSub));
+  const int d = (threadIdx.x % 64) * 2, g0 = threadIdx.x / 64;
+  float4 a[4], b[4];
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {
-    const int d0 = dg * 32 + j, d1 = d0 + 1;
-    const float a = tile[d0 * 64 + (dq_chunk(qi / 4, d0) << 2) + (qi & 3)];
-    const float b = tile[d1 * 64 + (dq_chunk(qi / 4, d1) << 2) + (qi & 3)];
-    w[j / 2] = pack_bf16(a, b);
+  for (int j = 0; j < 4; ++j) {
+    a[j] = tile[(g0 + 4 * j) * kGD + d];
+    b[j] = tile[(g0 + 4 * j) * kGD + d + 1];
   }
-  if (q < S) {
-    uint4* dst = reinterpret_cast<uint4*>(dq + (static_cast<size_t>(bh) * S + q) * kGD + dg * 32);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  for (int j = 0; j < 4; ++j) {
+    const int q = blk * kGSub + (g0 + 4 * j) * 4;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(dq + (static_cast<size_t>(bh) * S + q) * kGD + d);
+    const uint32_t w[4] = {pack_bf16(a[j].x, b[j].x), pack_bf16(a[j].y, b[j].y), pack_bf16(a[j].z, b[j].z),
+                           pack_bf16(a[j].w, b[j].w)};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (q + e < S) dst[e * (kGD / 2)] = w[e];
   }
   pdl_launch_dependents();
 }
@@ -491,7 +500,7 @@ __global__ void fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, const fl
 }  // namespace
 
 // Workspace: delta [BH,S] fp32 (padded to 256 bytes), then the dQ^T accumulator
-// [BH][ceil(S/64)][128][64] fp32.
+// [BH][ceil(S/64)][16][128][4] fp32.
 size_t fused128_bwd_workspace_bytes(int BH, int S) {
   const size_t delta_bytes = (static_cast<size_t>(BH) * S * sizeof(float) + 255) / 256 * 256;
   const size_t n_sub = (static_cast<size_t>(S) + kGSub - 1) / kGSub;
@@ -525,12 +534,14 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
                       dim3(static_cast<unsigned>(blocks)), dim3(kPrepareThreads), 0, st, delta, dq_ws,
                       reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out), rows));
   stage_event(1, st);
-  const PhiloxKey rng = make_philox(seed, offset);
+  const PhiloxRounds rng = make_philox_rounds(seed, offset, rate);
   const LeveledGrid order = leveled_grid(32768, S, BH);
   const bool drop = rate > 0.f;
   auto kern = leveled ? (drop ? flash_bwd_fused128_kernel<true, true> : flash_bwd_fused128_kernel<false, true>)
                       : (drop ? flash_bwd_fused128_kernel<true, false> : flash_bwd_fused128_kernel<false, false>);
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G128Smem::kBytes));
+  static std::atomic<int> regs_seen[4];
+  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kGRegsLaunch, regs_seen[2 * leveled + drop])) return rc;
   DAD_CUDA(launch_pdl(kern, leveled ? leveled_blocks(order, by_unit.x) : by_unit, dim3(kGThreads),
                       G128Smem::kBytes, st, mk, mv, mq, mdo, reinterpret_cast<BF*>(dk),
                       reinterpret_cast<BF*>(dv), dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
