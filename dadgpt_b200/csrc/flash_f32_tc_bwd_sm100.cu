@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         }
         it = nxt;
       }
-    } else if (elect_one()) {
+    } else {
+      const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // A, B K-major
       constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // A from tensor memory, B MN-major
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const SmemDescBase b2_0 = make_desc_base_sw128(smem_u32(smem + L::kB2), 0);
       auto issue_x = [&](int i) -> bool {
         const int s = i & 1;
-        const uint32_t par = (i >> 1) & 1, tx = tmem + s * 128;
+        const uint32_t par = (i >> 1) & 1, tx = tm + s * 128;
         const int s2 = i % 3;
         const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
         const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
@@ -252,25 +253,25 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           for (int m = 0; m < 6; ++m)
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk)
-              mma_ss(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
-                     idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
+              mma_ss_warp(td, desc_at(a, product_a(m) * kPlaneA + kk * 32), desc_at(b, product_b(m) * kPlaneB + kk * 32),
+                     idesc_x, (m > 0 || kk > 0) ? 1u : 0u, lead);
         };
-        if (!mbar_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->b2_full[s2], (i / 3) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx + 64, a2, b2);
-        if (!mbar_wait(&bars->b1_full[s], par, abort_flag)) return false;
+        if (!warp_wait(&bars->b1_full[s], par, abort_flag)) return false;
         tc_fence_after_sync();
         product(tx, a1, b1);
-        mma_commit(&bars->x_full[s]);
+        mma_commit_warp(&bars->x_full[s], lead);
         return true;
       };
       auto issue_sums = [&](int i, bool is_q) -> bool {
         const int s = i & 1;
-        const uint32_t tx = tmem + s * 128;
+        const uint32_t tx = tm + s * 128;
         const int s2 = i % 3;
         const SmemDescBase b1{b1_0.lo + s * (3 * kPlaneB >> 4), b1_0.hi};
         const SmemDescBase b2{b2_0.lo + s2 * (3 * kPlaneB >> 4), b2_0.hi};
-        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 streamed rows kk lie over the 16 columns their scores came from
         if (!is_q) {
@@ -279,21 +280,21 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
             for (int kk = 0; kk < kStep / 16; ++kk) {
               const uint32_t at = (product_a(m) == 0 ? 0u : product_a(m) == 1 ? 8u : 64u) + kk * 16;
-              mma_ts(tmem + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 2048), idesc_s,
-                     (m > 0 || kk > 0) ? 1u : 0u);
+              mma_ts_warp(tm + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                     (m > 0 || kk > 0) ? 1u : 0u, lead);
             }
         }
-        mma_commit(&bars->b2_empty[s2]);
+        mma_commit_warp(&bars->b2_empty[s2], lead);
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
-            const uint32_t at = product_a(m) == 0 ? tx + 64 + 8 + kk * 16 : tmem + kExtra + (product_a(m) - 1) * 8 + kk * 16;
-            mma_ts(tmem + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 2048), idesc_s,
-                   (m > 0 || kk > 0) ? 1u : 0u);
+            const uint32_t at = product_a(m) == 0 ? tx + 64 + 8 + kk * 16 : tm + kExtra + (product_a(m) - 1) * 8 + kk * 16;
+            mma_ts_warp(tm + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                   (m > 0 || kk > 0) ? 1u : 0u, lead);
           }
-        mma_commit(&bars->b1_empty[s]);
-        mma_commit(&bars->acc_done);
+        mma_commit_warp(&bars->b1_empty[s], lead);
+        mma_commit_warp(&bars->acc_done, lead);
         return true;
       };
       bool ok = true;
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       for (int n = 0; ok && (MANY || n < 1); ++n) {
         const BwdItem it = MANY ? bwd_item<MANY>(n, args.BH, S) : item0;
         if (!it.valid) break;
-        ok = mbar_wait(&bars->a_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        ok = warp_wait(&bars->a_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_sums(g + i, it.is_q) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }

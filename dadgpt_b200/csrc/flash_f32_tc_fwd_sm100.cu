@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
           if (++s == kStages) s = 0, ++lap;
         }
       }
-    } else if (elect_one()) {
+    } else {
+      const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // Q, K: K-major
       constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // P from tensor memory, V MN-major
@@ -180,38 +181,38 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       const SmemDescBase v0 = make_desc_base_sw128(smem_u32(smem + L::kV), 0);
       auto issue_x = [&](int i) -> bool {
         const int s = i % kStages;
-        const uint32_t tx = tmem + (i & 1) * 64;
+        const uint32_t tx = tm + (i & 1) * 64;
         const SmemDescBase kd{k0.lo + s * (3 * kPlaneB >> 4), k0.hi};
-        if (!mbar_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->k_full[s], (i / kStages) & 1, abort_flag)) return false;
         tc_fence_after_sync();
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
-            mma_ss(tx, desc_at(qd, product_a(m) * kPlaneA + kk * 32), desc_at(kd, product_b(m) * kPlaneB + kk * 32),
-                   idesc_x, (m > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(&bars->x_full[i & 1]);
-        mma_commit(&bars->k_empty[s]);
+            mma_ss_warp(tx, desc_at(qd, product_a(m) * kPlaneA + kk * 32), desc_at(kd, product_b(m) * kPlaneB + kk * 32),
+                   idesc_x, (m > 0 || kk > 0) ? 1u : 0u, lead);
+        mma_commit_warp(&bars->x_full[i & 1], lead);
+        mma_commit_warp(&bars->k_empty[s], lead);
         return true;
       };
       auto issue_pv = [&](int i) -> bool {
         const int s = i % kStages;
-        const uint32_t tx = tmem + (i & 1) * 64;
+        const uint32_t tx = tm + (i & 1) * 64;
         const SmemDescBase vd{v0.lo + s * (3 * kPlaneB >> 4), v0.hi};
-        if (!mbar_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
-        if (!mbar_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->p_full, i & 1, abort_flag)) return false;
         tc_fence_after_sync();
         // the planes of 16 keys kk lie over the 16 columns their scores came from
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
-            const uint32_t at = product_a(m) == 2 ? tmem + kExtra + kk * 8 : tx + kk * 16 + product_a(m) * 8;
-            mma_ts(tmem + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 2048), idesc_s,
-                   (m > 0 || kk > 0) ? 1u : 0u);
+            const uint32_t at = product_a(m) == 2 ? tm + kExtra + kk * 8 : tx + kk * 16 + product_a(m) * 8;
+            mma_ts_warp(tm + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+                   (m > 0 || kk > 0) ? 1u : 0u, lead);
           }
-        mma_commit(&bars->v_empty[s]);
-        mma_commit(&bars->acc_done);
+        mma_commit_warp(&bars->v_empty[s], lead);
+        mma_commit_warp(&bars->acc_done, lead);
         return true;
       };
       bool ok = true;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       for (int n = 0; ok && (MANY || n < 1); ++n) {
         const FwdItem it = MANY ? fwd_item<MANY>(n, args.BH, S) : item0;
         if (!it.valid) break;
-        ok = mbar_wait(&bars->q_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
+        ok = warp_wait(&bars->q_full, n & 1, abort_flag) && issue_x(g) && (it.n_it < 2 || issue_x(g + 1));
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_pv(g + i) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }

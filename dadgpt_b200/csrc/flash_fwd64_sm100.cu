@@ -268,14 +268,15 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     // S_X = Q_X K(g+1, c)^T, the scores two sub-steps ahead, into the buffer that P_X(g, c) has
     // just left (also across an item boundary). A ring stage and a Q buffer are released by both
     // issuers: each commits (or, where its group has nothing to do with the tile, arrives) once.
-    if (elect_one()) {
-      const int X = (warp == 1) ? 0 : 1;
+    {   // (whole warps: mma_ss_warp)
+      const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
+      const int X = __reduce_max_sync(0xffffffffu, warp == 1 ? 0u : 1u);
       constexpr uint32_t idesc_s = make_idesc_bf16(kT, 64, 0, 0);    // Q, K: K-major; 64 keys
       constexpr uint32_t idesc_o = make_idesc_bf16(kT, kHD, 0, 1);   // P from TMEM, V MN-major
       const SmemDescBase q_desc0 = make_desc_base_sw128(smem_u32(smem + L::kQ), 0);
       const SmemDescBase k_desc0 = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
       const SmemDescBase v_desc0 = make_desc_base_sw128(smem_u32(smem + L::kV), 0);
-      const uint32_t tSx = tmem + kColS + X * 128, tOx = tmem + kColO + X * 2 * kHD;
+      const uint32_t tSx = tm + kColS + X * 128, tOx = tm + kColO + X * 2 * kHD;
       int n_pv = 0;      // sub-steps of this group whose P V products have been issued
       int n_done = 0;    // items finished so far in which the group took part
       bool ok = true;
@@ -287,27 +288,27 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const SmemDescBase kd{k_desc0.lo + (g % kKvStages) * (kPanel >> 4), k_desc0.hi};
 #pragma unroll
         for (int kk = 0; kk < kHD / 16; ++kk)
-          mma_ss(tSx + c * 64, desc_at(qd, kk * 32), desc_at(kd, c * 8192 + kk * 32), idesc_s, kk > 0 ? 1u : 0u);
-        mma_commit(&bars->s_full[X][c]);
+          mma_ss_warp(tSx + c * 64, desc_at(qd, kk * 32), desc_at(kd, c * 8192 + kk * 32), idesc_s, kk > 0 ? 1u : 0u, lead);
+        mma_commit_warp(&bars->s_full[X][c], lead);
       };
       // O_(X,h) (+)= P_(X,h) V[keys 64 c + 32 h .. + 31] of ring tile g, both halves. P of half h
       // sits in the first 16 columns of its 32 columns of buffer c, 16 keys (8 columns of packed
       // bf16 pairs) per MMA; V is MN-major, 16 keys = 2048 bytes further down.
       auto issue_pv = [&](int g, int c, bool first_of_item) -> bool {
         // the epilogue of the group's previous item must have read O_X before it is overwritten
-        if (first_of_item && n_done > 0 && !mbar_wait(&bars->o_free[X], (n_done - 1) & 1, abort_flag))
+        if (first_of_item && n_done > 0 && !warp_wait(&bars->o_free[X], (n_done - 1) & 1, abort_flag))
           return false;
-        if (!mbar_wait(&bars->p_full[X][c], (n_pv >> 1) & 1, abort_flag)) return false;
+        if (!warp_wait(&bars->p_full[X][c], (n_pv >> 1) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         const SmemDescBase vd{v_desc0.lo + (g % kKvStages) * (kPanel >> 4), v_desc0.hi};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk)
-            mma_ts(tOx + h * kHD, tSx + c * 64 + h * 32 + kk * 8, desc_at(vd, (c * 4 + h * 2 + kk) * 2048),
-                   idesc_o, (!first_of_item || kk > 0) ? 1u : 0u);
+            mma_ts_warp(tOx + h * kHD, tSx + c * 64 + h * 32 + kk * 8, desc_at(vd, (c * 4 + h * 2 + kk) * 2048),
+                   idesc_o, (!first_of_item || kk > 0) ? 1u : 0u, lead);
         }
-        mma_commit(&bars->o_done[X][n_pv & 1]);
+        mma_commit_warp(&bars->o_done[X][n_pv & 1], lead);
         ++n_pv;
         return true;
       };
@@ -320,15 +321,15 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       F64Item nxt = f64_item<ONE>(deal, 1, BH, n_tiles, n_items);
       int g = 0;
       if (cur.valid) {
-        ok = mbar_wait(&bars->q_full[0], 0, abort_flag) && mbar_wait(&bars->k_full[0], 0, abort_flag);
+        ok = warp_wait(&bars->q_full[0], 0, abort_flag) && warp_wait(&bars->k_full[0], 0, abort_flag);
         if (ok) {
           tc_fence_after_sync();
           if (n_of(cur) > 0 && begin_of(cur) == 0) {
             issue_s(0, 0, 0);
             issue_s(0, 0, 1);
-            if (end_of(cur) == 1) mma_commit(&bars->q_empty[0]);   // the item's only score products of this group
+            if (end_of(cur) == 1) mma_commit_warp(&bars->q_empty[0], lead);   // the item's only score products of this group
           }
-          if (n_of(cur) == 0) mbar_arrive(&bars->q_empty[0]);
+          if (n_of(cur) == 0 && lead) mbar_arrive(&bars->q_empty[0]);
         }
       }
       for (int k = 0; ok && cur.valid; ++k) {
@@ -345,7 +346,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           // also where this group has nothing to do with the tile: an idle issuer must not run
           // ahead and arrive twice within one phase of a release barrier.
           bool issued = false;
-          ok = mbar_wait(&bars->v_full[s], (g / kKvStages) & 1, abort_flag);
+          ok = warp_wait(&bars->v_full[s], (g / kKvStages) & 1, abort_flag);
           // the group has scores to form in the next tile
           const bool s_next = have_next && n_of(ni) > 0 && nj >= begin_of(ni) && nj < end_of(ni);
           bool next_ready = false;
@@ -357,8 +358,8 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             if (ok && s_next) {
               if (!next_ready) {
-                if (nj == begin_of(ni)) ok = mbar_wait(&bars->q_full[nqb], ((last ? k + 1 : k) >> 1) & 1, abort_flag);
-                ok = ok && mbar_wait(&bars->k_full[(g + 1) % kKvStages], ((g + 1) / kKvStages) & 1, abort_flag);
+                if (nj == begin_of(ni)) ok = warp_wait(&bars->q_full[nqb], ((last ? k + 1 : k) >> 1) & 1, abort_flag);
+                ok = ok && warp_wait(&bars->k_full[(g + 1) % kKvStages], ((g + 1) / kKvStages) & 1, abort_flag);
                 if (ok) tc_fence_after_sync();
                 next_ready = true;
               }
@@ -366,18 +367,18 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 issue_s(nqb, g + 1, c);
                 issued = true;
                 // the item's last scores of this group
-                if (c == 1 && nj + 1 == end_of(ni)) mma_commit(&bars->q_empty[nqb]);
+                if (c == 1 && nj + 1 == end_of(ni)) mma_commit_warp(&bars->q_empty[nqb], lead);
               }
             }
           }
           if (ok && have_next && n_of(ni) == 0 && nj == 0) {
             // the next item has no tile for this group: hand its Q buffer back (once it is loaded)
-            if (last) ok = mbar_wait(&bars->q_full[nqb], ((k + 1) >> 1) & 1, abort_flag);
-            if (ok) mbar_arrive(&bars->q_empty[nqb]);
+            if (last) ok = warp_wait(&bars->q_full[nqb], ((k + 1) >> 1) & 1, abort_flag);
+            if (ok && lead) mbar_arrive(&bars->q_empty[nqb]);
           }
           // this issuer's share of the stage's release: after every product of its that reads it
           if (ok) {
-            if (issued) mma_commit(&bars->kv_empty[s]); else mbar_arrive(&bars->kv_empty[s]);
+            if (issued) mma_commit_warp(&bars->kv_empty[s], lead); else if (lead) mbar_arrive(&bars->kv_empty[s]);
           }
         }
         if (n_x > 0) ++n_done;
