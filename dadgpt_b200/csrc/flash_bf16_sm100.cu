@@ -127,7 +127,11 @@ struct FwdSmem {
 
 struct FwdBars {
   uint64_t q_full, k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
-  uint64_t s_full[2], p_full, o_done[2], stat_full;  // P_j V_j commits to o_done[j & 1]
+  // p_full: one per score buffer. S_{j+1} is formed before P_j is complete, so that a warp can store P_{j+1}
+  // while another still works on tile j: with one barrier for both its second arrival stood in for the other's
+  // first, and P_j V_j read scores for probabilities (rows of infinities in one call of five at 8 x 3080 with
+  // dropout, whose draws set the warps apart). P_{j+2} needs S_{j+2}, which is issued after p_full of tile j.
+  uint64_t s_full[2], p_full[2], o_done[2], stat_full;  // P_j V_j commits to o_done[j & 1]
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -170,7 +174,8 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_init(&bars->v_empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) mbar_init(&bars->s_full[b], 1);
-    mbar_init(&bars->p_full, kSoftmaxThreads);
+    mbar_init(&bars->p_full[0], kSoftmaxThreads);
+    mbar_init(&bars->p_full[1], kSoftmaxThreads);
     mbar_init(&bars->o_done[0], 1);
     mbar_init(&bars->o_done[1], 1);
     mbar_init(&bars->stat_full, kSoftmaxThreads);
@@ -229,7 +234,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       auto issue_pv = [&](int i) -> bool {
         const int s = i % kStages;
         if (!hot_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
-        if (!hot_wait(&bars->p_full, i & 1, abort_flag)) return false;
+        if (!hot_wait(&bars->p_full[i & 1], (i >> 1) & 1, abort_flag)) return false;
         tc_fence_after_sync();
         const SmemDescBase v_desc{v_desc0.lo + s * (kStageBytes >> 4), v_desc0.hi};
         // One MMA per 16 keys covers all 128 output columns: the V tile is MN-major, its 64-column
@@ -366,7 +371,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       tmem_st32(tS, pk);
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&bars->p_full);
+      mbar_arrive(&bars->p_full[sb]);
     }
 
     // Epilogue: merge the two halves of each row. out = (O_0 w_0 + O_1 w_1) / (l_0 w_0 + l_1 w_1)
