@@ -352,11 +352,12 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
           if (key > q0 + c) x1[c] = 0xff800000u;   // -inf: p = 0
       }
       uint32_t keep = 0xffffu;
-      if (DROP) {   // (draws only for pairs that count: key <= query < S)
-        const int lo = max(key - q0, 0), hi = min(S - q0, 16);
-        keep = lo < hi ? philox_keep_bits<2>(rng, (static_cast<uint64_t>(unit0 + bh) * S + q0 + lo) * S + key,
-                                             static_cast<uint32_t>(S), hi - lo) << lo
-                       : 0u;
+      if (DROP) {
+        // where the warp's 32 x 16 block has visible pairs (the same number of draws in every lane: a warp's loop
+        // runs as long as its longest lane's)
+        if (q0 + 15 >= k0 + quad * 32)
+          keep = philox_keep_bits<2>(rng, (static_cast<uint64_t>(unit0 + bh) * S + q0) * S + key, static_cast<uint32_t>(S), 16);
+        __syncwarp();
       }
       uint32_t pw[8], dw[8];
 #pragma unroll

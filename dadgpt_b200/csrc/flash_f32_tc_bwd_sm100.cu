@@ -456,14 +456,13 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         // ds = p (dP - delta) scale, with dropout on P and dP alike
         uint32_t keep = 0xffffu;
         if (DROP) {
-          // (draws only for pairs that count: key <= query < S)
-          if (is_q) {
-            keep = philox_keep_bits<2>(args.rng, (unit + r_own) * S + col0, 1u, r_own < S ? min(r_own - col0 + 1, 16) : 0);
-          } else {
-            const int lo = max(r_own - col0, 0), hi = min(S - col0, 16);
-            keep = lo < hi ? philox_keep_bits<2>(args.rng, (unit + col0 + lo) * S + r_own, static_cast<uint32_t>(S), hi - lo) << lo
-                           : 0u;
-          }
+          // where the warp's 32 x 16 block has visible pairs. The same number of draws in every lane: a warp's
+          // loop runs as long as its longest lane's, and a constant count needs no bounds (32 x 301 x 32 with
+          // dropout: 53.7 -> 52.8 us a step).
+          if (is_q ? col0 <= row0 + quad * 32 + 31 : col0 + 15 >= row0 + quad * 32)
+            keep = is_q ? philox_keep_bits<2>(args.rng, (unit + r_own) * S + col0, 1u, 16)
+                        : philox_keep_bits<2>(args.rng, (unit + col0) * S + r_own, static_cast<uint32_t>(S), 16);
+          __syncwarp();
         }
 #pragma unroll
         for (int c = 0; c < 8; ++c) {

@@ -342,8 +342,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         }
         if (DROP) {
           const uint64_t at = (static_cast<uint64_t>(args.unit0 + bh) * S + r) * S + c0;
-          // (no draws for keys beyond the row's own nor for rows beyond the sequence)
-          const uint32_t keep = philox_keep_bits<4>(args.rng, at, 1u, r < S ? min(r - c0 + 1, 16) : 0);
+          // (where the warp's block has visible pairs; the same number of draws in every lane)
+          const uint32_t keep = c0 <= row0 + quad * 32 + 31 ? philox_keep_bits<4>(args.rng, at, 1u, 16) : 0u;
+          __syncwarp();
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             p[c] = fmul2(p[c], make_float2((keep >> (2 * c)) & 1u ? keep_scale : 0.f, (keep >> (2 * c + 1)) & 1u ? keep_scale : 0.f));
