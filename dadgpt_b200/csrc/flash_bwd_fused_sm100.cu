@@ -22,8 +22,8 @@
 // of the tile two back were through and held up the products of the tile between; dQ had one staging
 // buffer, 3600 clocks from one use to the next. Now 2700-2800 (192 x 1024: 117 -> 84 us), set by the
 // issuing thread (2500 clocks for 32 products, their waits and commits) and the arithmetic (2200) alike.
-// Measured and not kept: two issuing warps, each with its own accumulators (13 % slower), dK's A operand
-// from shared memory (more traffic), the next group's tiles prefetched into L2 (2 % slower).
+// Measured and not kept: two issuing warps, each with its own accumulators (backward 113 -> 126 us), the whole
+// warp issuing (the same), the next group's tiles prefetched into L2 (117 -> 120).
 //   warps 0-15   compute: four warps per TMEM lane quadrant, 32 of the 128 query columns each
 //   warp 16      TMA producer           warp 17      MMA issuer + TMEM owner
 //   warp 18      reducer: issues the TMA reduce-adds of dQ and the dK / dV stores
