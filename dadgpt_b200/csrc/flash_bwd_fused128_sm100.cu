@@ -346,10 +346,25 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       tc_fence_before_sync();
       mbar_arrive(&bars->x_free);  // scores are in registers: the next step's products may overwrite them
 
-      if (i < 2) {   // sub-tiles that straddle the diagonal
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {
+        // 128-bit broadcast reads, here and below: all lanes of a warp want the same four columns
+        const float4 l4 = *reinterpret_cast<const float4*>(v_lse + c);
+        const float2 e0 = ffma2(make_float2(__uint_as_float(x1[c]), __uint_as_float(x1[c + 1])),
+                                make_float2(scale_log2, scale_log2), make_float2(l4.x, l4.y));
+        const float2 e1 = ffma2(make_float2(__uint_as_float(x1[c + 2]), __uint_as_float(x1[c + 3])),
+                                make_float2(scale_log2, scale_log2), make_float2(l4.z, l4.w));
+        x1[c] = __float_as_uint(ex2(e0.x));
+        x1[c + 1] = __float_as_uint(ex2(e0.y));
+        x1[c + 2] = __float_as_uint(ex2(e1.x));
+        x1[c + 3] = __float_as_uint(ex2(e1.y));
+      }
+      // Sub-tiles that straddle the diagonal. (Behind the exponentials: a score of -inf would be p = NaN where the
+      // query's lse is, and with it dV of keys that the query does not see.)
+      if (i < 2) {
 #pragma unroll
         for (int c = 0; c < 16; ++c)
-          if (key > q0 + c) x1[c] = 0xff800000u;   // -inf: p = 0
+          if (key > q0 + c) x1[c] = 0u;
       }
       uint32_t keep = 0xffffu;
       if (DROP) {
@@ -362,16 +377,12 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       uint32_t pw[8], dw[8];
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
-        // 128-bit broadcast reads: all lanes of a warp want the same four columns
-        const float4 a = *reinterpret_cast<const float4*>(v_lse + c);
         const float4 b = *reinterpret_cast<const float4*>(v_delta + c);
-        const float2 l2[2] = {make_float2(a.x, a.y), make_float2(a.z, a.w)}, dl[2] = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
+        const float2 dl[2] = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int e = c + 2 * h;
-          const float2 t = ffma2(make_float2(__uint_as_float(x1[e]), __uint_as_float(x1[e + 1])),
-                                 make_float2(scale_log2, scale_log2), l2[h]);
-          const float2 p = make_float2(ex2(t.x), ex2(t.y));
+          const float2 p = make_float2(__uint_as_float(x1[e]), __uint_as_float(x1[e + 1]));
           float2 pd = p, g = make_float2(__uint_as_float(x2[e]), __uint_as_float(x2[e + 1]));
           if (DROP) {
             const float2 mk = make_float2((keep >> e) & 1u ? keep_scale : 0.f, (keep >> (e + 1)) & 1u ? keep_scale : 0.f);

@@ -634,11 +634,6 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         uint32_t x[32];   // S^T, then p
         tmem_ld32(tlane + kColS + cg * 32, x);
         tmem_wait_ld();
-        if (diagonal) {   // the causal compare only exists on an item's first tile
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (row > cg * 32 + c) x[c] = 0xff800000u;   // -inf: p = 0
-        }
 #pragma unroll
         for (int c = 0; c < 32; c += 4) {
           const float4 l = *reinterpret_cast<const float4*>(v_lse + c);   // (all lanes want the same four)
@@ -650,6 +645,13 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           x[c + 1] = __float_as_uint(ex2(e0.y));
           x[c + 2] = __float_as_uint(ex2(e1.x));
           x[c + 3] = __float_as_uint(ex2(e1.y));
+        }
+        // The causal compare only exists on an item's first tile. (Behind the exponentials: a score of -inf would
+        // be p = NaN where the query's lse is, and with it dV of keys that the query does not see.)
+        if (diagonal) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (row > cg * 32 + c) x[c] = 0u;
         }
 
         if (DROP == 1 && (!diagonal || quad <= cg)) {   // (beyond the diagonal there is nothing to drop)
