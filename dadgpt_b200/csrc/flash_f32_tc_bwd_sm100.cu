@@ -377,11 +377,15 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     };
     BwdItem it{}, nxt = MANY ? bwd_item<MANY>(0, args.BH, S) : item0;
     int step = 0;   // over all items
+    int left = 0;   // where a wait runs out: the first item whose barrier has not been joined
 #pragma unroll(MANY ? 1 : 2)
     for (int n = 0; MANY || n < 2; ++n) {
       if (nxt.valid) load_resident(nxt, n);
       if (n > 0) {   // the results of the item before
-        if (!(ok = take_sums(step - 1, it.is_q))) break;
+        if (!(ok = take_sums(step - 1, it.is_q))) {
+          left = n;
+          break;
+        }
         const int rows = min(kRows, S - it.row0);
         const size_t at = (static_cast<size_t>(it.bh) * S + it.row0) * D;
         if constexpr (MANY) {
@@ -482,7 +486,22 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         tc_fence_before_sync();
         mbar_arrive(&bars->p_full);
       }
-      if (!ok) break;
+      if (!ok) {
+        left = n + 1;
+        break;
+      }
+    }
+    // A warp that has given up joins the named barriers that are left: nothing bounds the wait of the others there.
+    if (!ok) {
+      if constexpr (!MANY) {
+        compute_sync();   // (ahead of the results; that of a dQ item's delta comes before its first wait)
+      } else if constexpr (!kDeltaGiven) {
+        for (;; ++left) {
+          const BwdItem e = bwd_item<MANY>(left, args.BH, S);
+          if (!e.valid) break;
+          if (e.is_q) compute_sync();
+        }
+      }
     }
     tc_fence_before_sync();
   }

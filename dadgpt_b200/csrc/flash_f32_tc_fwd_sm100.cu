@@ -267,11 +267,15 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     };
     FwdItem it{}, nxt = MANY ? fwd_item<MANY>(0, args.BH, S) : item0;
     int step = 0;   // over all items
+    int synced = 0; // where a wait runs out: the barriers of the row's warps joined until then
 #pragma unroll(MANY ? 1 : 2)
     for (int n = 0; MANY || n < 2; ++n) {
       if (nxt.valid) load_resident(nxt);
       if (n > 0) {   // the results of the item before
-        if (!(ok = take_sums(step - 1))) break;
+        if (!(ok = take_sums(step - 1))) {
+          synced = step + n - 1;
+          break;
+        }
         float* own = part + ((step + n - 1) & 1) * 512;   // (the buffers of `part` alternate over steps and results)
         own[cg * 128 + row] = l;
         rows_sync();
@@ -301,7 +305,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       for (int c = 0; c < NC; ++c) o[c] = 0.f;
 
       for (int i = 0; i < n_it; ++i, ++step) {
-        if (!(ok = mbar_wait(&bars->x_full[step & 1], (step >> 1) & 1, abort_flag))) break;
+        if (!(ok = mbar_wait(&bars->x_full[step & 1], (step >> 1) & 1, abort_flag))) {
+          synced = step + n;
+          break;
+        }
         tc_fence_after_sync();
         const uint32_t tx = tlane + (step & 1) * 64 + cg * 16;
         const int c0 = i * kStep + cg * 16;
@@ -351,7 +358,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         }
         l = fmaf(l, corr, sum.x + sum.y);
         if (i > 0) {   // and with it the planes of step i - 1 are free
-          if (!(ok = take_sums(step - 1))) break;
+          if (!(ok = take_sums(step - 1))) {
+            synced = step + n + 1;
+            break;
+          }
 #pragma unroll
           for (int c = 0; c < NC; ++c) o[c] *= corr;
         }
@@ -361,6 +371,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         mbar_arrive(&bars->p_full);
       }
       if (!ok) break;
+    }
+    // A warp that has given up joins the named barriers that are left: nothing bounds the wait of the others there.
+    if (!ok) {
+      for (int n = 0; MANY || n < 1; ++n) {
+        const FwdItem e = MANY ? fwd_item<MANY>(n, args.BH, S) : item0;
+        if (!e.valid) break;
+        for (int i = 0; i <= e.n_it; ++i)
+          if (--synced < 0) rows_sync();
+      }
+      if (!MANY) compute_sync();
     }
     tc_fence_before_sync();
   }
