@@ -153,6 +153,17 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(kDecodeWarps * 32) : "memory");
 }
+// The same, and whether any consumer thread brought a true one.
+__device__ __forceinline__ bool consumers_any(bool mine) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, 2, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(static_cast<uint32_t>(mine)), "n"(kDecodeWarps * 32)
+      : "memory");
+  return any != 0;
+}
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kDecodeThreads, kManyPerSm)
@@ -520,7 +531,9 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
       }
       if (ranks == 1) {
         if (s.row1 == 0 && s.h == 0 && threadIdx.x == 0) atomicExch(status, DADATTN_E_ARG);
-        consumers_sync();   // sh.acc / sh.m are read: the next item may write them
+        // sh.acc / sh.m are read: the next item may write them. The warps go on together or not at all: one whose
+        // wait ran out would be missing at the named barriers of the next item.
+        if (consumers_any(!ok)) have = false;
       }
     }
   }

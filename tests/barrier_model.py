@@ -12,6 +12,7 @@ what they execute, in the order of the CUDA source:
     ("bulk", reads)             a store or reduce-add out of shared memory: reads after any delay
     ("bulk_wait", n)            until all but the n youngest of those have read
     ("sync", name, n)           a named barrier of n roles
+    ("any", name, n, flag)      the same with a reduction: yields whether any of the n flags was set
 
 A role that is several warps is several agents, each with its own part of the data and its own arrivals
 (`need`: arrivals per phase): one agent for all of them would hide that they can be a tile apart.
@@ -44,7 +45,7 @@ class Model:
         self.cells = {}
         self.tma, self.bulk = [], []
         self.queues = {}
-        self.syncs = {}                   # name -> [completed generations, arrivals]
+        self.syncs = {}                   # name -> [completed generations, arrivals, flags so far, last result]
         self.aborted = False
         self.abort_after = rng.randrange(1, 1200) if abort else None
 
@@ -73,20 +74,21 @@ class Model:
             return (c - op[2]) % 2 == 1   # the parity that the hardware looks at
         if op[0] == "bulk_wait":
             return all(b is None for b in self.bulk[:max(0, len(self.bulk) - op[1])])
-        return self.syncs[op[1]][0] > op[2]   # sync: op[2] is the generation it joined
+        return self.syncs[op[1]][0] > op[2]   # sync, any: op[2] is the generation it joined
 
     def issue(self, who, op):
         """Executes an operation; returns it if the agent has to wait for it."""
         kind = op[0]
         if kind in ("wait", "bulk_wait"):
             return op
-        if kind == "sync":
-            state = self.syncs.setdefault(op[1], [0, 0])
+        if kind in ("sync", "any"):
+            state = self.syncs.setdefault(op[1], [0, 0, False, False])
             joined = state[0]
             state[1] += 1
+            state[2] |= kind == "any" and op[3]
             if state[1] == op[2]:
-                state[0], state[1] = joined + 1, 0
-            return ("sync", op[1], joined)
+                state[:] = joined + 1, 0, False, state[2]
+            return (kind, op[1], joined)
         if kind == "arrive":
             self.arrive(op[1])
         elif kind == "tma":
@@ -157,10 +159,15 @@ class Model:
             if who not in agents:
                 self.run_async(who.removeprefix("queue "))
                 continue
-            failed = who in failing
+            failed, before = who in failing, pending[who]
             pending[who] = None
             try:
-                op = agents[who].throw(Aborted()) if failed else next(agents[who])
+                if failed:
+                    op = agents[who].throw(Aborted())
+                elif before is not None and before[0] == "any":
+                    op = agents[who].send(self.syncs[before[1]][3])
+                else:
+                    op = next(agents[who])
             except (StopIteration, Aborted):
                 alive.discard(who)
                 self.finished(who, alive)
