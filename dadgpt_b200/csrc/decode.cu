@@ -344,6 +344,7 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
       // After a wait that ran out the claims are made all the same: the workspace stays usable.
       while (next < n_items) next = claim();
       settle_ticket();
+      settle_ring(sh.full, stages, lap * stages + st);
     }
   } else {
     // ------------------------------ consumers ------------------------------

@@ -131,7 +131,7 @@ struct FwdBars {
   // while another still works on tile j: with one barrier for both its second arrival stood in for the other's
   // first, and P_j V_j read scores for probabilities (rows of infinities in one call of five at 8 x 3080 with
   // dropout, whose draws set the warps apart). P_{j+2} needs S_{j+2}, which is issued after p_full of tile j.
-  uint64_t s_full[2], p_full[2], o_done[2], stat_full;  // P_j V_j commits to o_done[j & 1]
+  uint64_t s_full[2], p_full[2], o_done[2], stat_full, settled;  // P_j V_j commits to o_done[j & 1]
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -179,6 +179,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars->o_done[0], 1);
     mbar_init(&bars->o_done[1], 1);
     mbar_init(&bars->stat_full, kSoftmaxThreads);
+    mbar_init(&bars->settled, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -204,6 +205,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_arrive_expect_tx(&bars->q_full, kPanels * kPanelBytes);
       for (int p = 0; p < kPanels; ++p)
         tma_load_3d(smem + L::kQ + p * kPanelBytes, &map_q, &bars->q_full, p * 64, q0, bh);
+      int n_k = 0, n_v = 0;   // tiles loaded
       for (int j = 0; j < n_kv; ++j) {
         const int s = j % kStages, use = j / kStages;
         uint8_t* kdst = smem + L::kK + s * kPanels * kPanelBytes;
@@ -213,11 +215,16 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         mbar_arrive_expect_tx(&bars->k_full[s], kPanels * kPanelBytes);
         for (int p = 0; p < kPanels; ++p)
           tma_load_3d(kdst + p * kPanelBytes, &map_k, &bars->k_full[s], p * 64, j * kBN, bh);
+        ++n_k;
         if (use > 0 && !hot_wait(&bars->v_empty[s], (use - 1) & 1, abort_flag)) break;
         mbar_arrive_expect_tx(&bars->v_full[s], kPanels * kPanelBytes);
         for (int p = 0; p < kPanels; ++p)
           tma_load_3d(vdst + p * kPanelBytes, &map_v, &bars->v_full[s], p * 64, j * kBN, bh);
+        ++n_v;
       }
+      settle(&bars->q_full, 0);
+      settle_ring(bars->k_full, kStages, n_k);
+      settle_ring(bars->v_full, kStages, n_v);
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -270,6 +277,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         if (j > 0) ok = issue_pv(j - 1);
       }
       if (ok) issue_pv(n_kv - 1);
+      settle_products(&bars->settled);
     }
   } else {
     // ------------------------------ softmax ------------------------------

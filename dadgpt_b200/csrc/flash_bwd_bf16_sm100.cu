@@ -68,7 +68,7 @@ struct BwdSmem {
 
 struct BwdBars {
   uint64_t r_full, c1_full[3], c2_full[3], c_empty[3];
-  uint64_t x_full[2], x_free[2], w_full, acc_done, vec_full;
+  uint64_t x_full[2], x_free[2], w_full, acc_done, vec_full, settled;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -127,6 +127,7 @@ flash_bwd_bf16_kernel(const __grid_constant__ CUtensorMap map_r1,
     mbar_init(&bars->w_full, kComputeThreads);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->vec_full, kComputeThreads);
+    mbar_init(&bars->settled, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -155,7 +156,8 @@ flash_bwd_bf16_kernel(const __grid_constant__ CUtensorMap map_r1,
         tma_load_3d(smem + L::kR1 + p * kPanelBytes, &map_r1, &bars->r_full, p * 64, row0, bh);
         tma_load_3d(smem + L::kR2 + p * kPanelBytes, &map_r2, &bars->r_full, p * 64, row0, bh);
       }
-      for (int i = 0; i < n_it; ++i) {
+      int i = 0;
+      for (; i < n_it; ++i) {
         const int s = i % kStages, use = i / kStages;
         if (use > 0 && !mbar_wait(&bars->c_empty[s], (use - 1) & 1, abort_flag)) break;
         const int c_row0 = (first + i) * kSubRows;
@@ -168,6 +170,9 @@ flash_bwd_bf16_kernel(const __grid_constant__ CUtensorMap map_r1,
           tma_load_3d(smem + L::kC2 + s * L::kSub + p * kSubPanelBytes, &map_c2,
                       &bars->c2_full[s], p * 64, c_row0, bh);
       }
+      settle(&bars->r_full, 0);
+      settle_ring(bars->c1_full, kStages, i);
+      settle_ring(bars->c2_full, kStages, i);
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -237,6 +242,7 @@ flash_bwd_bf16_kernel(const __grid_constant__ CUtensorMap map_r1,
                issue_x(i + kXBufs);
         ok = ok && issue_acc(i);
       }
+      settle_products(&bars->settled);
     }
   } else {
     // ------------------------------ compute warps ------------------------------

@@ -89,7 +89,7 @@ struct G128Smem {
 
 struct G128Bars {
   uint64_t kv_full, qdo_full[kGStages], qdo_empty[kGStages];
-  uint64_t x_full[2], x_free, w_full, acc_done, dq_drained;
+  uint64_t x_full[2], x_free, w_full, acc_done, dq_drained, settled;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -163,6 +163,7 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
     mbar_init(&bars->w_full, kGCompute);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->dq_drained, kGDrain);
+    mbar_init(&bars->settled, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -191,7 +192,8 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
         tma_load_3d(smem + L::kK + p * kGPanel, &map_k, &bars->kv_full, p * 64, k0, bh);
         tma_load_3d(smem + L::kV + p * kGPanel, &map_v, &bars->kv_full, p * 64, k0, bh);
       }
-      for (int i = 0; i < n_it; ++i) {
+      int i = 0;
+      for (; i < n_it; ++i) {
         const int s = i % kGStages, use = i / kGStages;
         if (use > 0 && !polled_wait(&bars->qdo_empty[s], (use - 1) & 1, abort_flag)) break;
         const int q0 = (first + i) * kGSub;
@@ -201,6 +203,8 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
           tma_load_3d(smem + L::kDO + s * L::kSubTile + p * kGSubPanel, &map_do, &bars->qdo_full[s], p * 64, q0, bh);
         }
       }
+      settle(&bars->kv_full, 0);
+      settle_ring(bars->qdo_full, kGStages, i);
     }
   } else if (warp == kGWarpIssuer) {
     // ------------------------------ MMA issuer ------------------------------
@@ -268,6 +272,7 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
         if (i + 1 < n_it) ok = polled_warp_wait(&bars->x_free, i & 1, abort_flag) && issue_x(i + 1);
         ok = ok && issue_acc(i);
       }
+      settle_products_warp(&bars->settled, lead);
     }
   } else if (warp == kGWarpScalars) {
     // ------------------------------ row scalars ------------------------------

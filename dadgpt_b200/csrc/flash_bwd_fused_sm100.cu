@@ -85,7 +85,7 @@ struct FusedSmem {
 struct FusedBars {
   uint64_t kv_full[2], kv_empty[2], qdo_full[kFStages], qdo_empty[kFStages];
   uint64_t item_ready[kFRing], item_free[kFRing];
-  uint64_t s_full[2], p_full, dp_full, w_full, acc_done, dq_drained, dkv_drained, staged[2], sent[2];
+  uint64_t s_full[2], p_full, dp_full, w_full, acc_done, dq_drained, dkv_drained, staged[2], sent[2], settled;
   int2 ring[kFRing];
   uint32_t tmem_base;
   int abort_flag;
@@ -251,6 +251,7 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->dq_drained, kFDrain);
     mbar_init(&bars->dkv_drained, kFDrain);
+    mbar_init(&bars->settled, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
   }
@@ -295,8 +296,8 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       };
       Item t = decode(static_cast<int>(blockIdx.x));
       bool ok = publish(t);
-      int g = 0;
-      for (int j = 0; ok && t.n_it > 0; ++j) {
+      int g = 0, j = 0;
+      for (; ok && t.n_it > 0; ++j) {
         // K / V go to the buffer of the item before last, once its products are through
         const int kb = j & 1;
         if (ok && j >= 2) ok = mbar_wait(&bars->kv_empty[kb], ((j >> 1) - 1) & 1, abort_flag);
@@ -320,6 +321,8 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         t = nxt;
       }
+      settle_ring(bars->kv_full, 2, j);
+      settle_ring(bars->qdo_full, kFStages, g);
     }
   } else if (warp == kWarpIssuer) {
     // ------------------------------ MMA issuer ------------------------------
@@ -416,6 +419,7 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         n_it = n_nxt;
       }
+      settle_products(&bars->settled);
     }
   } else if (warp == kWarpReducer) {
     // ------------------------------ dQ reducer / dK, dV writer ------------------------------

@@ -45,7 +45,7 @@ struct BwdSmem {
   static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
 };
 struct BwdBars {
-  uint64_t a_full, p_full, acc_done;
+  uint64_t a_full, p_full, acc_done, settled;
   uint64_t b1_full[2], b1_empty[2], b2_full[3], b2_empty[3], x_full[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     mbar_init(&bars->a_full, kComputeThreads);
     mbar_init(&bars->p_full, kComputeThreads);
     mbar_init(&bars->acc_done, 1);
+    mbar_init(&bars->settled, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->b1_full[s], kLoaderThreads);
       mbar_init(&bars->b1_empty[s], 1);
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_sums(g + i, it.is_q) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }
+      settle_products_warp(&bars->settled, lead);
     }
   } else {
     setmaxnreg_inc<kRegsCompute>();

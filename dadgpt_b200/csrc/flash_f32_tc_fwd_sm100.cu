@@ -36,7 +36,7 @@ struct FwdSmem {
   static_assert(kBytes <= 232448, "shared memory of a CTA exceeded");
 };
 struct FwdBars {
-  uint64_t q_full, p_full, acc_done, x_full[2];
+  uint64_t q_full, p_full, acc_done, x_full[2], settled;
   uint64_t k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
   uint32_t tmem_base;
   int abort_flag;
@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     mbar_init(&bars->q_full, kComputeThreads);
     mbar_init(&bars->p_full, kComputeThreads);
     mbar_init(&bars->acc_done, 1);
+    mbar_init(&bars->settled, 1);
     for (int s = 0; s < 2; ++s) mbar_init(&bars->x_full[s], 1);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&bars->k_full[s], kLoaderThreads);
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
         for (int i = 0; ok && i < it.n_it; ++i) ok = issue_pv(g + i) && (i + 2 >= it.n_it || issue_x(g + i + 2));
         g += it.n_it;
       }
+      settle_products_warp(&bars->settled, lead);
     }
   } else {
     setmaxnreg_inc<kRegsCompute>();

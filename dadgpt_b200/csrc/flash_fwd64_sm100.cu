@@ -81,7 +81,7 @@ struct F64Smem {
 struct F64Bars {
   uint64_t q_full[2], q_empty[2];
   uint64_t k_full[kKvStages], v_full[kKvStages], kv_empty[kKvStages];
-  uint64_t s_full[2][2], p_full[2][2], o_done[2][2], o_free[2], stat_full[2];   // [group][buffer]
+  uint64_t s_full[2][2], p_full[2][2], o_done[2][2], o_free[2], stat_full[2], settled[2];   // [group][buffer]
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -207,6 +207,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       mbar_init(&bars->o_done[b][1], 1);
       mbar_init(&bars->o_free[b], 2 * kHalfThreads);
       mbar_init(&bars->stat_full[b], 2 * kHalfThreads);
+      mbar_init(&bars->settled[b], 1);
     }
     for (int s = 0; s < kKvStages; ++s) {
       mbar_init(&bars->k_full[s], 1);
@@ -235,9 +236,9 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       prefetch_tensormap(&map_q);
       prefetch_tensormap(&map_k);
       prefetch_tensormap(&map_v);
-      int g = 0;  // K/V tiles loaded so far, over all items
+      int g = 0, k = 0;  // K/V tiles and Q pairs loaded so far, over all items
       bool ok = true;
-      for (int k = 0; ok; ++k) {
+      for (; ok; ++k) {
         const F64Item it = f64_item<ONE>(deal, k, BH, n_tiles, n_items);
         if (!it.valid) break;
         const int qb = k & 1;
@@ -260,6 +261,9 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           tma_load_4d(smem + L::kV + s * kPanel, &map_v, &bars->v_full[s], 0, row0, uh, ub);
         }
       }
+      settle_ring(bars->q_full, 2, k);
+      settle_ring(bars->k_full, kKvStages, g);
+      settle_ring(bars->v_full, kKvStages, g);
     }
   } else if (warp == 1 || warp == 18) {
     // ------------------------------ MMA issuers ------------------------------
@@ -385,6 +389,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         cur = nxt;
         nxt = f64_item<ONE>(deal, k + 2, BH, n_tiles, n_items);
       }
+      settle_products_warp(&bars->settled[X], lead);
     }
   } else {
     // ------------------------------ softmax groups ------------------------------

@@ -237,6 +237,31 @@ __device__ __forceinline__ void mma_commit_warp(uint64_t* bar, uint32_t lead) {
       : "memory");
 }
 
+// ---- leaving ------------------------------------------------------------------------------------
+// A CTA must not retire with loads on their way into its shared memory or products at work on it and on its
+// tensor memory, also where a bounded wait ran out and nobody took up what it had issued. So the issuing
+// threads wait for their last copies and products before they join the exit, in every run: they have
+// nothing else to do by then. Bounded like every wait (some 10 ms; the abort flag is not looked at).
+constexpr uint32_t kSettleLimit = 1u << 12;
+__device__ __forceinline__ void settle(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < kSettleLimit; ++i)
+    if (mbar_try_wait(bar, parity)) return;
+}
+// `issued` loads so far, dealt to the ring's stages in turn
+__device__ __forceinline__ void settle_ring(uint64_t* full, int stages, int issued) {
+#pragma unroll 1
+  for (int s = 0; s < stages && s < issued; ++s) settle(&full[s], ((issued - 1 - s) / stages) & 1);
+}
+__device__ __forceinline__ void settle_products(uint64_t* unused_bar) {
+  mma_commit(unused_bar);
+  settle(unused_bar, 0);
+}
+__device__ __forceinline__ void settle_products_warp(uint64_t* unused_bar, uint32_t lead) {
+  mma_commit_warp(unused_bar, lead);
+  settle(unused_bar, 0);
+}
+
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulation.
 // a_mn_major / b_mn_major: 0 = K-major (K contiguous in shared memory), 1 = MN-major.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int a_mn_major,

@@ -13,6 +13,7 @@ what they execute, in the order of the CUDA source:
     ("bulk_wait", n)            until all but the n youngest of those have read
     ("sync", name, n)           a named barrier of n roles
     ("any", name, n, flag)      the same with a reduction: yields whether any of the n flags was set
+    ("settle", barrier, k)      a wait that does not look at the abort flag (for copies and products on their way)
 
 A role that is several warps is several agents, each with its own part of the data and its own arrivals
 (`need`: arrivals per phase): one agent for all of them would hide that they can be a tile apart.
@@ -21,6 +22,8 @@ Two things are checked. A parity wait is only right while its barrier has seen k
 ahead it blocks for ever (on the GPU until the bounded wait expires), behind it passes too early. And every cell
 (a tile in shared memory, columns of tensor memory) carries a tag for its contents: whoever reads names the tag
 that must be there. A product or store reads when it runs, which may be long after it was issued.
+
+When the last agent has come to its end the CTA retires: no load may be on its way and no product at work.
 
 With `abort` one wait of the run gives up as if its bound had been reached. From there on every wait that is not
 ready fails, as it does once the CTA's abort flag is up (the agent sees `Aborted`), contents are no longer
@@ -43,7 +46,7 @@ class Model:
         self.rng = rng
         self.done, self.count = {}, {}    # completed phases, arrivals in the current one
         self.cells = {}
-        self.tma, self.bulk = [], []
+        self.tma, self.bulk, self.loads = [], [], {}   # loads: how many each barrier has been given
         self.queues = {}
         self.syncs = {}                   # name -> [completed generations, arrivals, flags so far, last result]
         self.aborted = False
@@ -51,6 +54,25 @@ class Model:
 
     def agents(self):
         raise NotImplementedError
+
+    # ---- how issuing threads leave ----
+    def producing(self, body):
+        """A producer's loads are waited for at its end, whether or not one of its waits gave up."""
+        try:
+            yield from body
+        except Aborted:
+            pass
+        for bar, n in sorted(self.loads.items()):
+            yield ("settle", bar, n - 1)
+
+    def issuing(self, body, bar="settled"):
+        """And an issuer's products, by a barrier that nothing else uses."""
+        try:
+            yield from body
+        except Aborted:
+            pass
+        yield ("commit", bar)
+        yield ("settle", bar, 0)
 
     # ---- primitives ----
     def arrive(self, name):
@@ -67,7 +89,7 @@ class Model:
                 raise Violation(f"{cell} holds {self.cells.get(cell)}, {tag} expected")
 
     def ready(self, op):
-        if op[0] == "wait":
+        if op[0] in ("wait", "settle"):
             c = self.done.get(op[1], 0)
             if c - op[2] not in (0, 1) and not self.aborted:
                 raise Violation(f"{op[1]}: waiter wants completion {op[2]}, barrier has completed {c}")
@@ -79,7 +101,7 @@ class Model:
     def issue(self, who, op):
         """Executes an operation; returns it if the agent has to wait for it."""
         kind = op[0]
-        if kind in ("wait", "bulk_wait"):
+        if kind in ("wait", "bulk_wait", "settle"):
             return op
         if kind in ("sync", "any"):
             state = self.syncs.setdefault(op[1], [0, 0, False, False])
@@ -93,6 +115,7 @@ class Model:
             self.arrive(op[1])
         elif kind == "tma":
             self.tma.append((op[1], op[2] if len(op) > 2 else []))
+            self.loads[op[1]] = self.loads.get(op[1], 0) + 1
         elif kind in ("mma", "commit"):
             self.queues.setdefault(who, []).append(op)
         elif kind == "read":
@@ -149,7 +172,6 @@ class Model:
             if not movable:
                 if alive:
                     raise Violation(f"stuck: { {n: pending[n][1:] for n in sorted(alive)} }")
-                self.at_exit()
                 return
             who = self.rng.choice(movable)
             if who == slow and self.rng.random() < 0.9 and len(movable) > 1:
@@ -170,16 +192,11 @@ class Model:
                     op = next(agents[who])
             except (StopIteration, Aborted):
                 alive.discard(who)
-                self.finished(who, alive)
+                if not alive and (self.tma or any(op[0] == "mma" for q in self.queues.values() for op in q)):
+                    raise Violation("loads or products at work at the exit") from None
                 continue
             pending[who] = self.issue(who, op)
         raise Violation("did not finish")
-
-    def finished(self, who, alive):
-        """An agent has come to its end."""
-
-    def at_exit(self):
-        """Everything has come to its end."""
 
 
 def survives(make, seeds):

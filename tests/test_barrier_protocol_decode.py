@@ -65,7 +65,7 @@ class Decode(Model):
             n += 1
 
     def agents(self):
-        return {"producer": self.producer(), **{f"consumer{w}": self.consumer(w) for w in WARPS}}
+        return {"producer": self.producing(self.producer()), **{f"consumer{w}": self.consumer(w) for w in WARPS}}
 
 
 ITEMS = [[9, 3, 0, 1], [0, 0, 0, 0], [1, 1, 1, 1, 1], [5], [2, 7, 2]]
@@ -80,3 +80,12 @@ def test_every_schedule_ends(abort):
 def test_consumers_have_to_agree_on_whether_they_go_on():
     found = survives(lambda s: Decode([2, 2, 2, 2], random.Random(s), agreed=False, abort=True), range(500))
     assert found is not None and "stuck" in found[1]
+
+
+def test_the_model_catches_rows_on_their_way_when_the_block_retires():
+    class Leaves(Decode):
+        def producing(self, body):
+            return body
+
+    found = survives(lambda s: Leaves([4, 4, 4], random.Random(s), abort=True), range(500))
+    assert found is not None and "at work" in found[1]

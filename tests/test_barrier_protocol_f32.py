@@ -108,7 +108,7 @@ class Forward(Model):
                 yield ("sync", "compute", 2)
 
     def agents(self):
-        return {"issuer": self.issuer(), **{f"loader{t}": self.loader(t) for t in PARTS},
+        return {"issuer": self.issuing(self.issuer()), **{f"loader{t}": self.loader(t) for t in PARTS},
                 **{f"compute{a}": self.compute(a) for a in PARTS}}
 
 
@@ -225,7 +225,7 @@ class Backward(Model):
                 turn += 1
 
     def agents(self):
-        return {"issuer": self.issuer(), **{f"loader{t}": self.loader(t) for t in PARTS},
+        return {"issuer": self.issuing(self.issuer()), **{f"loader{t}": self.loader(t) for t in PARTS},
                 **{f"compute{a}": self.compute(a) for a in PARTS}}
 
 
@@ -288,3 +288,12 @@ def test_the_model_catches_two_stages_released_as_three():
     with pytest.raises(Violation):
         for seed in range(200):
             Short([(False, 9)], random.Random(seed)).run()
+
+
+def test_the_model_catches_products_at_work_when_the_block_retires():
+    class Leaves(Forward):
+        def issuing(self, body, bar="settled"):
+            return body
+
+    found = survives(lambda s: Leaves([3, 3], random.Random(s), abort=True), range(500))
+    assert found is not None and "at work" in found[1]
