@@ -73,9 +73,10 @@ struct F64Smem {
   static constexpr int kQ = 0;                                // [2 items][A, B] panels
   static constexpr int kK = kQ + 4 * kPanel;
   static constexpr int kV = kK + kKvStages * kPanel;
-  static constexpr int kStat = kV + kKvStages * kPanel;      // float2 [group][half][128]: (max, sum)
-  static constexpr int kBars = kStat + 2 * 2 * 128 * 8;
+  static constexpr int kStat = kV + kKvStages * kPanel;      // float2 [2 items][group][half][128]: (max, sum)
+  static constexpr int kBars = kStat + 2 * 2 * 2 * 128 * 8;
   static constexpr int kBytes = kBars + 512;
+  static_assert(kBytes <= 232448, "shared memory budget of one CTA exceeded");
 };
 
 struct F64Bars {
@@ -528,7 +529,10 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       // ---- epilogue: merge the two halves of each row. out = (O_0 w_0 + O_1 w_1) / (l_0 w_0 +
       // l_1 w_1) with w_h = exp2(m_h - max(m_0, m_1)); lse in natural-log units of the scaled
       // scores. Each thread of the pair writes 32 of the row's 64 outputs. ----
-      float2* stat = reinterpret_cast<float2*>(smem + L::kStat) + X * 256;   // [half][128]
+      // (Two buffers: the scores of an item of one tile do not wait for the epilogue of the item before, so that a
+      // half may be here again while a warp of the other has not read its row's pairs. A third time needs scores that
+      // come behind products, and those the probabilities that both halves store after the first.)
+      float2* stat = reinterpret_cast<float2*>(smem + L::kStat) + ((n_item & 1) * 2 + X) * 256;   // [half][128]
       const int r = qt * kT + row;          // query index
       stat[half * 128 + row] = make_float2(m, l2.x + l2.y);
       mbar_arrive(&bars->stat_full[X]);
