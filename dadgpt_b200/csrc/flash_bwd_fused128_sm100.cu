@@ -61,14 +61,6 @@ static_assert(kGCompute * kGRegsCompute + 128 * kGRegsHelper + kGDrain * kGRegsD
               "the warpgroups ask for more registers than the CTA owns");
 static_assert(kGThreads * kGRegsLaunch <= 65536 && (kGRegsLaunch + 8) * kGThreads > 65536,
               "kGRegsLaunch is not what the compiler gives a CTA of this size");
-// Up to this many CTAs the key tiles go level by level (leveled_grid) and the delta kernel clears the
-// workspace; with more waves the order gains nothing and the cleared lines, by then out of L2, are better
-// written by a memset ahead of the reads. Backward alone, us by CTAs, level by level / unit by unit:
-//     192  24 x 1024   47 / 62      1536  192 x 1024   294-311 / 304-320   3072  192 x 2048  843-882 / 873-884
-//     384  24 x 2048  110 / 133     1800  600 x 300        200 / 206       3072  96 x 4096  1391-1428 / 1430
-//     768  48 x 2048  210 / 229     2048  64 x 4096    876-940 / 948-966   3072  48 x 8192  2540-2580 / 2460-2570
-// (192 x 8192, 12288 CTAs: 10.45 ms / 10.35)
-constexpr int kGLeveledBlocks = 2048;
 constexpr int kPrepareThreads = 256;         // of the delta kernel, whose blocks zero a part of one tile
 constexpr int kGDqTileBytes = kGD * kGSub * 4;   // one dQ^T tile, fp32
 constexpr float kGLog2e = 1.4426950408889634f;
@@ -117,7 +109,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
-template <bool DROP, bool LEVELED>
+template <bool DROP>
 __global__ void __launch_bounds__(kGThreads, 1)
 flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
@@ -141,8 +133,8 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n_sub = (S + kGSub - 1) / kGSub;
   // key tile `own` streams the query sub-tiles 2*own .. n_sub-1 (low `own` = most work = first)
-  int own = static_cast<int>(blockIdx.x), bh = blockIdx.y;
-  if (LEVELED && !leveled_block(order, own, bh)) return;
+  int own, bh;
+  if (!leveled_block(order, own, bh)) return;
   const int first = 2 * own;
   const int n_it = n_sub - first;
   const int k0 = own * kGKeys;
@@ -454,9 +446,8 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
 }
 
 // delta[r] = sum_d dO[r,d] O[r,d] (reference flash_delta_kernel, cuda/attention.cu:76-85): 16
-// lanes per row of 128. With ZERO also zeros into the workspace, 32 bytes per thread (a memset of its
-// own between two kernels costs short calls about 3 us).
-template <bool ZERO>
+// lanes per row of 128. Also zeros into the workspace, 32 bytes per thread (a memset of its own between two
+// kernels costs short calls about 3 us).
 __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __restrict__ dq_ws,
                                         const __nv_bfloat16* __restrict__ dout,
                                         const __nv_bfloat16* __restrict__ out, int64_t rows) {
@@ -466,10 +457,8 @@ __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __rest
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = t / Lr;
   const int c = static_cast<int>(t % Lr) * 8;
-  if (ZERO) {
-    float4* zero = reinterpret_cast<float4*>(dq_ws) + static_cast<int64_t>(blockIdx.x) * (2 * kPrepareThreads);
-    zero[threadIdx.x] = zero[threadIdx.x + kPrepareThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  float4* zero = reinterpret_cast<float4*>(dq_ws) + static_cast<int64_t>(blockIdx.x) * (2 * kPrepareThreads);
+  zero[threadIdx.x] = zero[threadIdx.x + kPrepareThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
   float sum = 0.f;
   if (r < rows) {
     const uint4 a = *reinterpret_cast<const uint4*>(dout + r * D + c);
@@ -543,23 +532,26 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
 
   stage_event(0, st);
   const int64_t rows = static_cast<int64_t>(BH) * S;
-  const dim3 by_unit((S + kGKeys - 1) / kGKeys, BH);
-  const bool leveled = static_cast<int64_t>(by_unit.x) * BH <= kGLeveledBlocks;
-  if (!leveled) DAD_CUDA(cudaMemsetAsync(dq_ws, 0, static_cast<size_t>(BH) * n_sub * kGDqTileBytes, st));
   const int64_t blocks = static_cast<int64_t>(BH) * n_sub * (kGDqTileBytes / (32 * kPrepareThreads));
-  DAD_CUDA(launch_pdl(leveled ? fused128_prepare_kernel<true> : fused128_prepare_kernel<false>,
-                      dim3(static_cast<unsigned>(blocks)), dim3(kPrepareThreads), 0, st, delta, dq_ws,
-                      reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out), rows));
+  DAD_CUDA(launch_pdl(fused128_prepare_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kPrepareThreads), 0, st, delta,
+                      dq_ws, reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out), rows));
   stage_event(1, st);
   const PhiloxRounds rng = make_philox_rounds(seed, offset, rate);
+  // Key tiles level by level over groups of units, whatever the number of CTAs. Backward alone, us (medians), level
+  // by level / unit by unit with a memset ahead:
+  //     192 CTAs  24 x 1024     42 / 59      1800  600 x 300   190 / 199       3072  96 x 4096   1311-1329 / 1379-1389
+  //     384       24 x 2048    105 / 127     2048  64 x 4096   885 / 920       3072  48 x 8192   2338-2357 / 2382-2415
+  //     768       48 x 2048    205 / 220     3000  3000 x 128  320 / 328       3840  30 x 16384  5466-5522 / 5536-5553
+  //    1536      192 x 1024    278 / 290     3072  192 x 2048  808 / 827      12288  192 x 8192  9441-9477 / 9500-9624
+  // (6 x 65536, units one by one: 16.7-17.0 ms / 16.7.) Before the products were issued by a whole warp and dQ
+  // left its staging buffer, unit by unit had been the better one beyond 2048 CTAs.
   const LeveledGrid order = leveled_grid(32768, S, BH);
   const bool drop = rate > 0.f;
-  auto kern = leveled ? (drop ? flash_bwd_fused128_kernel<true, true> : flash_bwd_fused128_kernel<false, true>)
-                      : (drop ? flash_bwd_fused128_kernel<true, false> : flash_bwd_fused128_kernel<false, false>);
+  auto kern = drop ? flash_bwd_fused128_kernel<true> : flash_bwd_fused128_kernel<false>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G128Smem::kBytes));
-  static std::atomic<int> regs_seen[4];
-  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kGRegsLaunch, regs_seen[2 * leveled + drop])) return rc;
-  DAD_CUDA(launch_pdl(kern, leveled ? leveled_blocks(order, by_unit.x) : by_unit, dim3(kGThreads),
+  static std::atomic<int> regs_seen[2];
+  if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kGRegsLaunch, regs_seen[drop])) return rc;
+  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kGKeys - 1) / kGKeys), dim3(kGThreads),
                       G128Smem::kBytes, st, mk, mv, mq, mdo, reinterpret_cast<BF*>(dk),
                       reinterpret_cast<BF*>(dv), dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
   stage_event(2, st);

@@ -1,5 +1,5 @@
 """GPU: bf16 attention at head size 128 where the CTAs go level by level over groups of units: last groups that are
-padded, groups of one unit, and the backward on both sides of the number of CTAs at which it changes its order."""
+padded, groups of one unit, groups of thousands."""
 import pytest
 import torch
 
