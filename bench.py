@@ -15,8 +15,9 @@ checked on rank 0. After its timed regions (never inside them) the run checks wh
 against the CPU oracle and reports that as `verify`.
 
 --impl reference times the reference's own CPU implementation of the path (its host ops driven
-in the reference's call order, oracle/_ref; the C restatement if that library is absent) on the
-host cores, same metric and workload, each step a bounded sample of (batch x head) units.
+in the reference's call order, oracle/_ref) on the host cores, same metric and workload, each step a
+bounded sample of (batch x head) units. Without that library, which is built from the reference's sources,
+it says so in an "unavailable" line: this repository's own restatement of the ops is not the reference.
 """
 from __future__ import annotations
 
@@ -125,12 +126,17 @@ def run_reference_arm(args):
     if rank != 0:
         return
     from dadgpt_b200 import workloads as W
+    from oracle.oracle import RefHost
+    if not RefHost.available():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's sources are absent, its host ops (oracle/_ref) are not built"}), flush=True)
+        return
     shape = W.gpt2(1024)
     cores = os.cpu_count() or 1
     units = min(shape.BH, cores)  # one unit per core per step keeps a step near one second
     for _ in range(min(args.warmup, 1)):
         cpu_pass(units, cores)
-    total, kind = 0.0, "port"
+    total, kind = 0.0, ""
     for _ in range(args.steps):
         dt, kind = cpu_pass(units, cores)
         total += dt
