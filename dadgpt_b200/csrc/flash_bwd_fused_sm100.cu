@@ -51,7 +51,7 @@ constexpr int kFPanel = 128 * 128;        // [128 rows][64 bf16] swizzled panel
 constexpr int kFThreads = 24 * 32;
 constexpr int kFCompute = 16 * 32;
 constexpr int kFDrain = 4 * 32;           // one thread per TMEM lane
-constexpr int kWarpProducer = 16, kWarpIssuer = 17, kWarpReducer = 18, kWarpScalars = 19, kWarpDrain0 = 20;
+constexpr int kWarpProducer = 16, kWarpIssuer = 17, kWarpReducer = 18, kWarpDrain0 = 20;   // (19: row scalars)
 // Registers per thread after the warpgroups have rebalanced. The pool is what the CTA was launched
 // with (kRegsLaunch per thread, the most that 768 threads can have): an increase beyond it would
 // wait for ever.

@@ -94,12 +94,13 @@ __device__ __forceinline__ BwdItem bwd_item(int k, int BH, int S) {
 
 // Whether delta = rowsum(dO o O) comes from a kernel ahead instead of the rows of O that this one loads
 // beside those of dO. Forming it saves a launch and pays while the loaders have time for the rows: at
-// head sizes below 64, whose rows are short, and while no CTA has a second item. us, formed here / given:
+// head sizes below 64, whose rows are short, and while no CTA has a second item. Backward alone, us, formed here /
+// given (D = 16 and 32 before whole warps issued the products):
 //   D = 16   32 x 301 15.6 / 17.4   48 x 1024 95.7 / 96.6     8 x 2048 62.4 / 64.4
 //   D = 32   32 x 301 17.0 / 18.7   48 x 1024 107.1 / 106.6   8 x 2048 71.6 / 71.4
-//   D = 64   16 x 200 17.4 / 18.3   8 x 1024 49.3 / 50.2      (64 and 128 items)
-//            32 x 301 23.4 / 23.9   8 x 2048 90.2 / 90.2      (192 and 256 items)
-//            96 x 200 38.3 / 36.6   200 x 256 81.7 / 76.4     48 x 1024 151.1 / 139.7
+//   D = 64   16 x 200 16.4 / 17.3   8 x 1024 45.5 / 45.7      (64 and 128 items)
+//            32 x 301 21.1 / 21.3   8 x 2048 83-93 / 87-94    (192 and 256 items)
+//            96 x 200 36.6 / 35.2   200 x 256 75.0 / 72.2     48 x 1024 143.0 / 137.2
 constexpr bool delta_given(int D, bool many) { return D == 64 && many; }
 
 template <int D, bool DROP, bool MANY>   // MANY: more items than CTAs
