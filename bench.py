@@ -40,7 +40,7 @@ UNIT = "TFLOP/s"
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the ncu
 # capture summarised in profiles/flash_bf16_fwd_bwd_gpt2_T1024_D64.md.
-NCU_TRAFFIC_BYTES = {"flash_bwd_fused_kernel": 206.1e6}
+NCU_TRAFFIC_BYTES = {"flash_bwd_fused_kernel": 202.6e6}
 
 
 def load_peaks():

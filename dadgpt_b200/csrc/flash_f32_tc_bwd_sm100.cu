@@ -17,7 +17,7 @@
 //               i + 2 (B2's stage is released before B1's, so its refill hides behind the sums'
 //               last products), sums of step i + 1, ...
 // A step costs 2304 (X) + 2304 (dK/dV) or 1152 (dQ) clocks of tensor pipe at head size 64 (48 for a
-// 128 x 64 x 16 product; the pipe's counter takes 32) and, the mean of both kinds, about 3000 issue slots
+// 128 x 64 x 16 product; the pipe's counter takes 32) and, the mean of both kinds, about 2700 issue slots
 // per scheduler, and takes about 4600 clocks (48 x 1024; 4900 before the whole warp issued the products).
 // CTAs are persistent where there are more items than SMs: the streamed rings run on across items, and
 // the next item's resident tiles are fetched and split, and its first products formed, while this one's

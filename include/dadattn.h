@@ -11,9 +11,9 @@
  *  - a 64 KiB array in the library image for dadattn_decode_bf16_noalloc (no allocation call).
  * There is no CPU fallback: without a CUDA device every compute call fails.
  *
- * Device-side waits are bounded. If one runs out, the kernel records DADATTN_E_TIMEOUT and
- * exits; copies and tensor-core operations it had in flight may still land afterwards, so every
- * result enqueued on that device up to the next dadattn_device_status() call is void.
+ * Device-side waits are bounded. If one runs out, the kernel records DADATTN_E_TIMEOUT, waits for its
+ * own copies and products in flight and exits. Its results are incomplete, and later calls may have read
+ * them: every result enqueued on that device up to the next dadattn_device_status() call is void.
  *
  * Tensor layouts follow DadGPT: heads already split, [BH, S, D] contiguous, row-major;
  * lse / delta are [BH, S] fp32. "bf16" pointers are raw 16-bit bfloat16 (uint16_t here so the
