@@ -124,12 +124,17 @@ struct PhiloxRounds {
   uint32_t k0[10], k1[9];   // key words of rounds 0..9 (the last round needs only k0)
   uint32_t c0, c1;          // low counter words: offset / 4
   uint32_t m_lo, m_hi;      // round 0: 0xD2511F53 * c0
-  uint32_t word;            // offset % 4: which word of the block is the draw
+  uint32_t word;            // offset % 4: which word of the block is the draw; 4 more where strides do not fit
   uint32_t drop_below;      // draws below this are dropped (uniform < rate)
 };
-PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate);
+// Whether 31 strides stay within 32 bits, as the shared form of philox_keep_bits takes for granted.
+constexpr bool philox_strides_fit(uint32_t stride) { return 31ull * stride <= 0xffffffffu; }
+static_assert(philox_strides_fit(1) && philox_strides_fit(138547332) && !philox_strides_fit(138547333) &&
+              !philox_strides_fit(0x7fffffff), "the line lies at 2^32 / 31");
+PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate, uint32_t stride = 1);
 
-// Bit i (i < n <= 32): whether the probability of flat index at + i * stride is kept.
+// Bit i (i < n <= 32): whether the probability of flat index at + i * stride is kept. `stride` is at most the one
+// that `p` was made for.
 template <int UNROLL>
 __device__ __forceinline__ uint32_t philox_keep_bits(const PhiloxRounds& p, uint64_t at, uint32_t stride, int n) {
   const uint32_t lo = static_cast<uint32_t>(at), hi = static_cast<uint32_t>(at >> 32);
@@ -157,7 +162,7 @@ __device__ __forceinline__ uint32_t philox_keep_bits(const PhiloxRounds& p, uint
     }
     return bits;
   }
-  const PhiloxKey key = {p.k0[0], p.k1[0], p.c0, p.c1, p.word};
+  const PhiloxKey key = {p.k0[0], p.k1[0], p.c0, p.c1, p.word & 3u};
 #pragma unroll 1
   for (int i = 0; i < n; ++i)
     bits |= (philox_draw(key, at + static_cast<uint64_t>(i) * stride) >= p.drop_below ? 1u : 0u) << i;

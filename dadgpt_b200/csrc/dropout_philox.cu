@@ -93,7 +93,7 @@ uint32_t drop_threshold(float rate) {
 
 }  // namespace
 
-PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate) {
+PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate, uint32_t stride) {
   const PhiloxKey rng = make_philox(seed, offset);
   PhiloxRounds p;
   for (int r = 0; r < 10; ++r) {
@@ -105,7 +105,7 @@ PhiloxRounds make_philox_rounds(uint64_t seed, uint64_t offset, float rate) {
   const uint64_t m = static_cast<uint64_t>(0xD2511F53u) * rng.c0;
   p.m_lo = static_cast<uint32_t>(m);
   p.m_hi = static_cast<uint32_t>(m >> 32);
-  p.word = rng.word;
+  p.word = rng.word | (philox_strides_fit(stride) ? 0u : 4u);
   p.drop_below = drop_threshold(rate);
   return p;
 }

@@ -536,7 +536,7 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
   DAD_CUDA(launch_pdl(fused128_prepare_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kPrepareThreads), 0, st, delta,
                       dq_ws, reinterpret_cast<const BF*>(dout), reinterpret_cast<const BF*>(out), rows));
   stage_event(1, st);
-  const PhiloxRounds rng = make_philox_rounds(seed, offset, rate);
+  const PhiloxRounds rng = make_philox_rounds(seed, offset, rate, static_cast<uint32_t>(S));
   // Key tiles level by level over groups of units, whatever the number of CTAs. Backward alone, us (medians), level
   // by level / unit by unit with a memset ahead:
   //     192 CTAs  24 x 1024     42 / 59      1800  600 x 300   190 / 199       3072  96 x 4096   1311-1329 / 1379-1389

@@ -548,8 +548,8 @@ int launch_bwd_f32_tc(float* dq, float* dk, float* dv, float* delta, const float
                       uint64_t seed, uint64_t offset, int64_t unit0, bool vec_ok, cudaStream_t st) {
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, delta, BH, S, scale, rate, make_philox_rounds(seed, offset, rate), unit0, vec_ok,
-                     status};
+  const BwdArgs a = {dq, dk, dv, dout, out, lse, q, k, v, delta, BH, S, scale, rate, make_philox_rounds(seed, offset, rate, static_cast<uint32_t>(S)),
+                     unit0, vec_ok, status};
   const bool drop = rate > 0.f;
   if (D == 64) return drop ? launch<64, true>(a, st) : launch<64, false>(a, st);
   if (D == 32) return drop ? launch<32, true>(a, st) : launch<32, false>(a, st);
