@@ -74,24 +74,33 @@ int make_tensor_map_bf16(CUtensorMap* map, const void* base, int BH, int S, int 
   return DADATTN_OK;
 }
 
-int make_tensor_map_bf16_units(CUtensorMap* map, const void* base, int units, int S, int D, int box_rows,
-                               const UnitLayout& lay) {
+static int encode_units(CUtensorMap* map, const void* base, bool f32, int units, int S, int D, int box_columns, int box_rows,
+                        CUtensorMapSwizzle swizzle, const UnitLayout& lay) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(DADATTN_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int heads = lay.heads, batch = units / lay.heads;
+  const cuuint64_t size = f32 ? 4 : 2;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S),
                               static_cast<cuuint64_t>(heads), static_cast<cuuint64_t>(batch)};
   // a dimension of extent 1 still needs a legal stride (a multiple of 16 bytes)
-  const cuuint64_t head_stride = heads > 1 ? static_cast<cuuint64_t>(lay.head) * 2 : static_cast<cuuint64_t>(D) * 2;
-  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(lay.row) * 2, head_stride,
-                                 static_cast<cuuint64_t>(lay.batch) * 2};
-  const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};
+  const cuuint64_t head_stride = static_cast<cuuint64_t>(heads > 1 ? lay.head : D) * size;
+  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(lay.row) * size, head_stride,
+                                 static_cast<cuuint64_t>(lay.batch) * size};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_columns), static_cast<cuuint32_t>(box_rows), 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(DADATTN_E_CUDA, "cuTensorMapEncodeTiled (4-D) failed (%d)", (int)r);
   return DADATTN_OK;
+}
+int make_tensor_map_bf16_units(CUtensorMap* map, const void* base, int units, int S, int D, int box_rows,
+                               const UnitLayout& lay) {
+  return encode_units(map, base, false, units, S, D, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, lay);
+}
+int make_tensor_map_rows64(CUtensorMap* map, const void* base, bool f32, int units, int S, int D, int box_rows,
+                           const UnitLayout& lay) {
+  return encode_units(map, base, f32, units, S, D, f32 ? 16 : 32, box_rows, CU_TENSOR_MAP_SWIZZLE_64B, lay);
 }
 
 namespace {

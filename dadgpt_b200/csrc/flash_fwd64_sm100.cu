@@ -98,6 +98,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// TMA store of 32 rows of 64 bytes (a warp's share of the output) to (x, row, head, batch)
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int x, int y, int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+      ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
@@ -174,7 +184,7 @@ __device__ __forceinline__ F64Item f64_item(const F64DealOf<ONE>& deal, int k, i
 template <int DROP, bool F32, bool ONE>
 __global__ void __launch_bounds__(kFwd64Threads, 1)
 flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                   const __grid_constant__ CUtensorMap map_v, void* __restrict__ out,
+                   const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
                    float* __restrict__ lse, int BH, int S, UnitLayout lay, float scale, float rate,
                    PhiloxKey rng, int64_t unit0, const uint4* __restrict__ mask_bits,
                    int* __restrict__ status, const __grid_constant__ F64DealOf<ONE> deal) {
@@ -199,7 +209,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars->q_full[b], 1);
-      mbar_init(&bars->q_empty[b], 2);              // one arrival per issuer
+      mbar_init(&bars->q_empty[b], 16);             // one arrival per softmax warp
       for (int i = 0; i < 2; ++i) {
         mbar_init(&bars->s_full[b][i], 1);
         mbar_init(&bars->p_full[b][i], 2 * kHalfThreads);
@@ -226,10 +236,9 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
-  // Set-up is done; from here on global memory is read, which the previous grid in the stream
-  // may have produced. Once every CTA of this grid is here the next grid may start its set-up.
-  pdl_wait();
-  pdl_launch_dependents();
+  // Set-up is done. Global memory, which the previous grid in the stream may still read or write, is
+  // touched only behind pdl_wait, by the roles that touch it; the products have nothing to wait for but
+  // the producer's loads.
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -237,13 +246,15 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       prefetch_tensormap(&map_q);
       prefetch_tensormap(&map_k);
       prefetch_tensormap(&map_v);
+      prefetch_tensormap(&map_out);
       int g = 0, k = 0;  // K/V tiles and Q pairs loaded so far, over all items
       bool ok = true;
-      for (; ok; ++k) {
-        const F64Item it = f64_item<ONE>(deal, k, BH, n_tiles, n_items);
-        if (!it.valid) break;
+      F64Item it = f64_item<ONE>(deal, 0, BH, n_tiles, n_items);
+      pdl_wait();
+      pdl_launch_dependents();   // once every CTA of this grid is here the next grid may start its set-up
+      for (; ok && it.valid; it = f64_item<ONE>(deal, ++k, BH, n_tiles, n_items)) {
         const int qb = k & 1;
-        // the Q buffer frees when the last score product of the item before last has completed
+        // the Q buffer frees when the results of the item before last, which are staged in it, have left
         if (k >= 2 && !mbar_wait(&bars->q_empty[qb], ((k >> 1) - 1) & 1, abort_flag)) break;
         int ub = it.bh / lay.heads, uh = it.bh - ub * lay.heads;   // (batch, head) of the unit
         const int ub_b = ONE ? it.bh_b / lay.heads : ub, uh_b = ONE ? it.bh_b - ub_b * lay.heads : uh;
@@ -271,8 +282,8 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     // One issuing thread per group. Issuer X walks the K/V ring tiles of all items in order, each
     // tile as two sub-steps of 64 keys. For sub-step (g, c) it issues O_X += P_X V(g, c) and then
     // S_X = Q_X K(g+1, c)^T, the scores two sub-steps ahead, into the buffer that P_X(g, c) has
-    // just left (also across an item boundary). A ring stage and a Q buffer are released by both
-    // issuers: each commits (or, where its group has nothing to do with the tile, arrives) once.
+    // just left (also across an item boundary). A ring stage is released by both issuers: each commits
+    // (or, where its group has nothing to do with the tile, arrives) once.
     {   // (whole warps: mma_ss_warp)
       const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       const int X = __reduce_max_sync(0xffffffffu, warp == 1 ? 0u : 1u);
@@ -332,9 +343,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (n_of(cur) > 0 && begin_of(cur) == 0) {
             issue_s(0, 0, 0);
             issue_s(0, 0, 1);
-            if (end_of(cur) == 1) mma_commit_warp(&bars->q_empty[0], lead);   // the item's only score products of this group
           }
-          if (n_of(cur) == 0 && lead) mbar_arrive(&bars->q_empty[0]);
         }
       }
       for (int k = 0; ok && cur.valid; ++k) {
@@ -371,15 +380,8 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               if (ok) {
                 issue_s(nqb, g + 1, c);
                 issued = true;
-                // the item's last scores of this group
-                if (c == 1 && nj + 1 == end_of(ni)) mma_commit_warp(&bars->q_empty[nqb], lead);
               }
             }
-          }
-          if (ok && have_next && n_of(ni) == 0 && nj == 0) {
-            // the next item has no tile for this group: hand its Q buffer back (once it is loaded)
-            if (last) ok = warp_wait(&bars->q_full[nqb], ((k + 1) >> 1) & 1, abort_flag);
-            if (ok && lead) mbar_arrive(&bars->q_empty[nqb]);
           }
           // this issuer's share of the stage's release: after every product of its that reads it
           if (ok) {
@@ -404,13 +406,27 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
     int t = 0;        // 64-key sub-steps this group has processed so far, over all items
     int n_item = 0;   // items this group has taken part in
+    int owed = -1;    // Q buffer that this warp has staged results in and not yet given back
     bool ok = true;
+    // gives it back, once the store has read it (lane 0 issued that)
+    auto give_back = [&]() {
+      if (owed >= 0 && lane == 0) {
+        bulk_wait_read0();
+        mbar_arrive(&bars->q_empty[owed]);
+      }
+      owed = -1;
+    };
+    if (DROP == 2) pdl_wait();   // (the mask)
 
     for (int k = 0; ok; ++k) {
       const F64Item it = f64_item<ONE>(deal, k, BH, n_tiles, n_items);
       if (!it.valid) break;
       const int n_x = X ? it.n_b : it.n_a;
-      if (n_x == 0) continue;               // nothing for this group
+      if (n_x == 0) {                       // nothing for this group: its share of the Q buffer, once that is loaded
+        give_back();
+        if ((ok = mbar_wait(&bars->q_full[k & 1], (k >> 1) & 1, abort_flag)) && lane == 0) mbar_arrive(&bars->q_empty[k & 1]);
+        continue;
+      }
       const int qt = ONE ? 0 : it.qa + X, bh = ONE && X ? it.bh_b : it.bh;
       float m = -INFINITY;                  // running max of the scaled scores, log2 units
       float2 l2 = make_float2(0.f, 0.f);    // running sum, two interleaved partial sums
@@ -426,6 +442,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             keep_next = __ldg(bits1 + mask_bits_record(bh, qt, (v + 1) >> 1, row, n_tiles) * 4 +
                               ((v + 1) & 1) * 2 + half);
         }
+        if (v == 1) give_back();   // (every item has two sub-steps; the store is long through)
         if (!(ok = mbar_wait(&bars->s_full[X][c], (t >> 1) & 1, abort_flag))) break;
         tc_fence_after_sync();
         const uint32_t tS = tS0 + c * 64;
@@ -546,8 +563,25 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const float w1 = (s1.x == -INFINITY) ? 0.f : ex2(s1.x - m_tot);
       const float l_tot = s0.y * w0 + s1.y * w1;
       const float f0 = w0 / l_tot, f1 = w1 / l_tot;
-      const int ub = bh / lay.heads, uh = bh - ub * lay.heads;
-      const int64_t at = ub * lay.batch + uh * lay.head + r * lay.row + half * 32;
+      // Through shared memory and TMA: as 16-byte stores of one row per lane, 32 lines an instruction, they took
+      // 1800-2400 clocks an item and held up the loads of the next one (192 x 1024: 48.3 us, now 44.3; 48 x 4096
+      // 133 and 125; 192 x 128 6.1 and 5.7, part of it the first item and the descriptors read ahead of pdl_wait).
+      // A warp's 32 rows x 32 columns are its own 2 KB of the group's Q tile, whose last product is behind the last
+      // scores. (fp32 rows of 32 columns would need 4 KB: 16 columns, then the others.)
+      uint8_t* stage = smem + L::kQ + ((k & 1) * 2 + X) * kPanel + (half * 4 + quad) * 2048;
+      auto put = [&](int chunk, uint4 w) {   // 64-byte rows, swizzled
+        *reinterpret_cast<uint4*>(stage + lane * 64 + ((chunk ^ ((lane >> 1) & 3)) << 4)) = w;
+      };
+      auto send = [&](int column) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int ub = bh / lay.heads, uh = bh - ub * lay.heads, row0 = qt * kT + quad * 32;
+        if (lane == 0 && row0 < S) {   // (rows beyond S are not written)
+          tma_store_4d(&map_out, stage, half * 32 + column, row0, uh, ub);
+          bulk_commit();
+        }
+      };
+      if (n_item == 0) pdl_wait();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {   // 16 output columns at a time
         uint32_t oa[16], ob[16];
@@ -558,33 +592,31 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           tc_fence_before_sync();
           mbar_arrive(&bars->o_free[X]);   // O and the statistics have been read: the next item may start
         }
-        if (r < S) {
+        uint32_t w[8];
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            float y[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              y[e] = __uint_as_float(oa[8 * i + e]) * f0 + __uint_as_float(ob[8 * i + e]) * f1;
-            if (F32) {
-              float4* dst = reinterpret_cast<float4*>(static_cast<float*>(out) + at + c * 16 + i * 8);
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {   // rounded to bf16 like every operand, widened again
-                const uint32_t lo = pack_bf16(y[4 * e], y[4 * e + 1]), hi = pack_bf16(y[4 * e + 2], y[4 * e + 3]);
-                dst[e] = make_float4(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u),
-                                     __uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
-              }
-            } else {
-              *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(out) + at + c * 16 + i * 8) = make_uint4(
-                  pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
-            }
+        for (int e = 0; e < 16; e += 2)
+          w[e / 2] = pack_bf16(__uint_as_float(oa[e]) * f0 + __uint_as_float(ob[e]) * f1,
+                               __uint_as_float(oa[e + 1]) * f0 + __uint_as_float(ob[e + 1]) * f1);
+        if (F32) {   // rounded to bf16 like every operand, widened again
+          if (c == 1) {
+            if (lane == 0) bulk_wait_read0();
+            __syncwarp();
           }
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            put(e, make_uint4(w[2 * e] << 16, w[2 * e] & 0xffff0000u, w[2 * e + 1] << 16, w[2 * e + 1] & 0xffff0000u));
+          send(c * 16);
+        } else {
+          put(2 * c, make_uint4(w[0], w[1], w[2], w[3]));
+          put(2 * c + 1, make_uint4(w[4], w[5], w[6], w[7]));
+          if (c == 1) send(0);
         }
       }
+      owed = k & 1;
       ++n_item;
-      if (r < S) {
-        if (half == 0) lse[static_cast<size_t>(bh) * S + r] = (m_tot + log2f(l_tot)) * kLn2;
-      }
+      if (half == 0 && r < S) lse[static_cast<size_t>(bh) * S + r] = (m_tot + log2f(l_tot)) * kLn2;
     }
+    if (lane == 0) bulk_wait0();   // the results have landed before the CTA retires
   }
 
   // ------------------------------ common exit ------------------------------
@@ -639,10 +671,11 @@ template <int DROP, bool F32 = false>
 int launch_fwd64(void* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v,
                  int BH, int S, const UnitLayout& lay, float scale, float rate, uint64_t seed,
                  uint64_t offset, int64_t unit0, const uint32_t* mask_bits, cudaStream_t st) {
-  CUtensorMap mq, mk, mv;
+  CUtensorMap mq, mk, mv, mo;
   if (int rc = make_tensor_map_bf16_units(&mq, q, BH, S, kHD, kT, lay)) return rc;
   if (int rc = make_tensor_map_bf16_units(&mk, k, BH, S, kHD, kT, lay)) return rc;
   if (int rc = make_tensor_map_bf16_units(&mv, v, BH, S, kHD, kT, lay)) return rc;
+  if (int rc = make_tensor_map_rows64(&mo, out, F32, BH, S, kHD, 32, lay)) return rc;
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
   int dev = 0, sms = 0;
@@ -654,7 +687,7 @@ int launch_fwd64(void* out, float* lse, const uint16_t* q, const uint16_t* k, co
   const dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));
   auto launch = [&](auto kern, const auto& deal) -> int {
     DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Smem::kBytes));
-    DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv, out, lse, BH, S, lay, scale,
+    DAD_CUDA(launch_pdl(kern, grid, dim3(kFwd64Threads), F64Smem::kBytes, st, mq, mk, mv, mo, lse, BH, S, lay, scale,
                         rate, make_philox(seed, offset), unit0, reinterpret_cast<const uint4*>(mask_bits), status, deal));
     return DADATTN_OK;
   };

@@ -434,5 +434,8 @@ inline UnitLayout unit_layout(int B, int H, int S, int D, bool interleaved) {
 // pass units = B*H: the map is then (D, S, 1, B*H).
 int make_tensor_map_bf16_units(CUtensorMap* map, const void* base, int units, int S, int D, int box_rows,
                                const UnitLayout& lay);
+// The same over a bf16 or fp32 tensor with boxes of 64-byte rows (32 or 16 columns) and 64-byte swizzle.
+int make_tensor_map_rows64(CUtensorMap* map, const void* base, bool f32, int units, int S, int D, int box_rows,
+                           const UnitLayout& lay);
 
 }  // namespace dadattn
