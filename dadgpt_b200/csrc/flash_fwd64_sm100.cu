@@ -24,10 +24,12 @@
 //     as packed bf16 over the first half of the same columns, from where the P V product takes
 //     it as its A operand;
 //   * scale-and-subtract and the row sums run as packed two-float instructions (fma.rn.f32x2,
-//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in eight as a
-//     cubic on the FMA pipe (48 x 4096 forward under the power cap: 146.8 us; one in four 149, none
-//     148.5; a bf16x2 exp2 on the special-function unit was tried: no faster, and
-//     it cost a digit of lse): the softmax is bound by instruction issue, not by any one unit;
+//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in four as a
+//     cubic on the FMA pipe (us at 192 x 1024 / 48 x 4096: none 44.4 / 129, one in eight 42.8 / 124, one
+//     in four 41.7 / 121, three in eight 42.4 / 122, half 43.7 / 127; a bf16x2 exp2 on the
+//     special-function unit was tried: no faster, and it cost a digit of lse); only the 32 x 32 block
+//     on the diagonal pays for the causal compare: the softmax is bound by instruction issue and the
+//     exp2 unit alike;
 //   * CTAs are persistent: barriers, tensor memory and descriptors are set up once, items are
 //     dealt out heaviest first in a fixed serpentine order (no global counter to reset), the
 //     next item's Q tiles and first K/V tiles are in flight while the current one finishes, and
@@ -447,7 +449,6 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tc_fence_after_sync();
         const uint32_t tS = tS0 + c * 64;
         const bool diagonal = (j == n_x - 1);
-        const int limit = row - c * 64 - half * 32;   // diagonal tile: column i visible iff i <= limit
 
         // ---- the thread's 32 scores: read once, kept in registers for the max and the
         // exponentials ----
@@ -455,10 +456,10 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         auto load_scores = [&]() {
           tmem_ld32(tS, xa);
           tmem_wait_ld();
-          if (diagonal) {
+          if (diagonal && c * 2 + half == quad) {   // the block on the diagonal; those below it see all keys
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (i > limit) xa[i] = 0xff800000u;  // -inf
+              if (i > lane) xa[i] = 0xff800000u;  // -inf
           }
         };
         if (diagonal && c * 64 + half * 32 > quad * 32 + 31) {   // the warp's block lies beyond the diagonal
@@ -517,7 +518,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int i = 0; i < 32; i += 2) {
           const float2 e = ffma2(make_float2(__uint_as_float(xa[i]), __uint_as_float(xa[i + 1])), sl, nm);
           float2 p;
-          if ((i & 15) == 14) {   // one pair in eight on the FMA pipe
+          if ((i & 7) == 2) {   // one pair in four on the FMA pipe
             p = ex2_poly2(e);
           } else {
             p.x = ex2(e.x);
