@@ -477,12 +477,13 @@ __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __rest
 
 // Workspace tile [16 groups of 4 queries][128 dims][4 queries] fp32 -> dq[q][128] bf16. One CTA of 256 threads
 // per tile: thread t takes head dims 2 (t % 64) and the next, so that a warp reads 1 KB and writes 128 bytes of
-// a row in one piece.
+// a row in one piece. The sums are read for the last time: their lines need not go out to memory.
 __global__ void __launch_bounds__(256)
-fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict__ dq_ws, int S, int n_sub) {
+fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, float* __restrict__ dq_ws, int S, int n_sub) {
   pdl_wait();
   const int bh = blockIdx.y, blk = blockIdx.x;
-  const float4* tile = reinterpret_cast<const float4*>(dq_ws + (static_cast<size_t>(bh) * n_sub + blk) * (kGD * kGSub));
+  float* sums = dq_ws + (static_cast<size_t>(bh) * n_sub + blk) * (kGD * kGSub);
+  const float4* tile = reinterpret_cast<const float4*>(sums);
   const int d = (threadIdx.x % 64) * 2, g0 = threadIdx.x / 64;
   float4 a[4], b[4];
 #pragma unroll
@@ -500,6 +501,9 @@ fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict_
     for (int e = 0; e < 4; ++e)
       if (q + e < S) dst[e * (kGD / 2)] = w[e];
   }
+  __syncthreads();
+  static_assert(kGDqTileBytes == 256 * 128, "a line of the tile per thread");
+  discard_line(sums + threadIdx.x * 32);
   pdl_launch_dependents();
 }
 
@@ -556,7 +560,7 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
                       reinterpret_cast<BF*>(dv), dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
   stage_event(2, st);
   DAD_CUDA(launch_pdl(fused128_convert_kernel, dim3(n_sub, BH), dim3(256), 0, st,
-                      reinterpret_cast<BF*>(dq), static_cast<const float*>(dq_ws), S, n_sub));
+                      reinterpret_cast<BF*>(dq), dq_ws, S, n_sub));
   stage_event(3, st);
   return DADATTN_OK;
 }

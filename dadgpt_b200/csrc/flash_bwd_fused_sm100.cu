@@ -767,9 +767,7 @@ __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restric
   if (t == 0) *item_counter = 0;
   float sum = 0.f;
   if (r < rows) {
-    float4* z = reinterpret_cast<float4*>(dq_ws + r * D + c);
-    z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-    z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    zero_32_bytes(dq_ws + r * D + c);   // (whole sectors)
     // where row r = (unit, s) lies in dO and O: heads-split rows are simply consecutive
     int64_t at = r * D + c;
     if (INTERLEAVED) {
@@ -792,15 +790,18 @@ __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restric
   if (r < rows && c == 0) delta[r] = sum;
 }
 
-// dQ workspace (fp32) -> dq (bf16).
+// dQ workspace (fp32) -> dq (bf16). The sums are read for the last time: their lines, which would go out to memory
+// in the middle of later kernels (50 MB at 192 x 1024, of the step's 490 MB of memory traffic), are dropped. Step at
+// 192 x 1024 154.5 -> 152.1 us, 24 x 512 29.9 -> 28.9.
 template <bool INTERLEAVED>
-__global__ void fused_convert_kernel(__nv_bfloat16* __restrict__ dq, const float* __restrict__ dq_ws,
+__global__ void fused_convert_kernel(__nv_bfloat16* __restrict__ dq, float* __restrict__ dq_ws,
                                      int64_t n8, int S, UnitLayout lay) {
   pdl_wait();
   pdl_launch_dependents();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= n8) return;
-  const float4 a = *reinterpret_cast<const float4*>(dq_ws + t * 8), b = *reinterpret_cast<const float4*>(dq_ws + t * 8 + 4);
+  float4 a, b;
+  load_32_bytes(dq_ws + t * 8, a, b);
   // workspace row r = (unit, s), 8 elements at column c; heads-split dq has the same order
   int64_t at = t * 8;
   if (INTERLEAVED) {
@@ -812,6 +813,8 @@ __global__ void fused_convert_kernel(__nv_bfloat16* __restrict__ dq, const float
   }
   *reinterpret_cast<uint4*>(dq + at) =
       make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+  __syncwarp();   // (the line's four readers have their values; they are there together, a row being eight lanes)
+  if (t % 4 == 0) discard_line(dq_ws + t * 8);
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -937,7 +940,7 @@ int launch_bwd_fused_d64(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* workspa
   const int64_t n8 = rows * kFD / 8;
   DAD_CUDA(launch_pdl(heads > 0 ? fused_convert_kernel<true> : fused_convert_kernel<false>,
                       dim3(static_cast<unsigned>((n8 + 255) / 256)), dim3(256), 0,
-                      st, reinterpret_cast<BF*>(dq), static_cast<const float*>(dq_ws), n8, S, lay));
+                      st, reinterpret_cast<BF*>(dq), dq_ws, n8, S, lay));
   stage_event(3, st);
   return DADATTN_OK;
 }

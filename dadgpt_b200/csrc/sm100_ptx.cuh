@@ -344,6 +344,22 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// ---- 32-byte accesses to global memory (sm_100): the address a multiple of 32 ------------------
+__device__ __forceinline__ void load_32_bytes(const float* from, float4& a, float4& b) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(from)
+               : "memory");
+}
+__device__ __forceinline__ void zero_32_bytes(float* to) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"l"(to), "f"(0.f) : "memory");
+}
+// What the 128 bytes at `line` (a multiple of 128) hold is not needed any more, and need not be written to memory
+// when the line leaves L2. For scratch that its next use writes before it reads.
+__device__ __forceinline__ void discard_line(void* line) {
+  asm volatile("discard.global.L2 [%0], 128;" ::"l"(line) : "memory");
+}
+
 // ---- packed two-float arithmetic and three-input max (sm_100) --------------------------------
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   float2 d;
