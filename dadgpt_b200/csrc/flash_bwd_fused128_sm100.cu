@@ -447,17 +447,18 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
 
 // delta[r] = sum_d dO[r,d] O[r,d] (reference flash_delta_kernel, cuda/attention.cu:76-85): 16
 // lanes per row of 128. Also zeros into the workspace, 32 bytes per thread (a memset of its own between two
-// kernels costs short calls about 3 us).
+// kernels costs short calls about 3 us). From the last row on, as the pass that rounds: the gradient kernel starts with
+// the first, whose lines L2 then still holds (64 x 2048 backward 269-274 -> 261-268 us, 192 x 1024 260-264 -> 258-259).
 __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __restrict__ dq_ws,
                                         const __nv_bfloat16* __restrict__ dout,
                                         const __nv_bfloat16* __restrict__ out, int64_t rows) {
   constexpr int D = kGD, Lr = D / 8;
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t block = gridDim.x - 1 - blockIdx.x, t = block * blockDim.x + threadIdx.x;
   const int64_t r = t / Lr;
   const int c = static_cast<int>(t % Lr) * 8;
-  float4* zero = reinterpret_cast<float4*>(dq_ws) + static_cast<int64_t>(blockIdx.x) * (2 * kPrepareThreads);
+  float4* zero = reinterpret_cast<float4*>(dq_ws) + block * (2 * kPrepareThreads);
   zero[threadIdx.x] = zero[threadIdx.x + kPrepareThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
   float sum = 0.f;
   if (r < rows) {
@@ -481,7 +482,7 @@ __global__ void fused128_prepare_kernel(float* __restrict__ delta, float* __rest
 __global__ void __launch_bounds__(256)
 fused128_convert_kernel(__nv_bfloat16* __restrict__ dq, float* __restrict__ dq_ws, int S, int n_sub) {
   pdl_wait();
-  const int bh = blockIdx.y, blk = blockIdx.x;
+  const int bh = gridDim.y - 1 - blockIdx.y, blk = blockIdx.x;
   float* sums = dq_ws + (static_cast<size_t>(bh) * n_sub + blk) * (kGD * kGSub);
   const float4* tile = reinterpret_cast<const float4*>(sums);
   const int d = (threadIdx.x % 64) * 2, g0 = threadIdx.x / 64;

@@ -752,6 +752,9 @@ flash_bwd_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 // zero fill of the fp32 dQ workspace, in one pass over the rows. The fill waits for the kernel ahead
 // like every other access: the workspace may lie where that kernel still reads or writes (an arena
 // hands its bytes on from call to call), and kernels release their dependents before they are done.
+// Blocks take the rows from the end, here and in the pass that rounds: the gradient kernel starts with the first units,
+// whose lines are then the last to have come into L2, and leaves those of the last ones there (192 x 1024 step 168.9
+// -> 167.7 us, behind fp32 tensors 74.1 -> 73.7).
 template <bool INTERLEAVED>
 __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restrict__ dq_ws,
                                      int* __restrict__ item_counter,
@@ -759,7 +762,7 @@ __global__ void fused_prepare_kernel(float* __restrict__ delta, float* __restric
                                      const __nv_bfloat16* __restrict__ out, int64_t rows, int S,
                                      UnitLayout lay) {
   constexpr int D = kFD, Lr = D / 8;  // 8 lanes per row
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = static_cast<int64_t>(gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = t / Lr;   // row of the [BH, S] index space: delta and the workspace are heads-split
   const int c = static_cast<int>(t % Lr) * 8;
   pdl_wait();
@@ -798,7 +801,7 @@ __global__ void fused_convert_kernel(__nv_bfloat16* __restrict__ dq, float* __re
                                      int64_t n8, int S, UnitLayout lay) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = static_cast<int64_t>(gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= n8) return;
   float4 a, b;
   load_32_bytes(dq_ws + t * 8, a, b);

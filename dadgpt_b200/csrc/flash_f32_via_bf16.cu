@@ -83,12 +83,13 @@ __global__ void __launch_bounds__(256) via_forward_inputs_kernel(CastList list, 
 
 // Everything the gradient kernel needs, in one pass over the rows (head size 64, eight lanes per row):
 // q, k, v, dout -> bf16, delta = rowsum(bf16(dout) o out) in fp32, zeros into dq and the item counter.
+// From the last row on: the gradient kernel starts with the first, whose lines L2 then still holds.
 __global__ void __launch_bounds__(256)
 via_backward_inputs_kernel(CastList list, const float* __restrict__ out, float* __restrict__ dq,
                            float* __restrict__ delta, int* __restrict__ item_counter, int64_t n8) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = static_cast<int64_t>(gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   if (t == 0) *item_counter = 0;
   const bool in = t < n8;
   float4 x[4][2], o[2];
