@@ -16,7 +16,8 @@
 //     rate is the length of that chain (branching on each row: 12-24 % slower);
 //   * many (sequence, head) pairs: persistent CTAs, the longest sequences first, items handed out by
 //     a counter, the next item's rows already on their way while one is merged. Few pairs: the CTAs
-//     of a cluster share a pair and merge through distributed shared memory. Neither needs records in
+//     of a cluster share one, or the same head of a long and a short sequence, and merge through distributed
+//     shared memory. Neither needs records in
 //     global memory, and a pair's merge costs no trip through L2 (8 sequences x 8 heads of up to 400
 //     rows, early start: 6.9 us a layer with records and tickets, 3.9 now);
 //   * the append is fused: the warp that owns row `len` takes k_new/v_new from the token's vectors,
@@ -50,7 +51,8 @@ constexpr int kMaxStages = 4;
 constexpr int kItemRing = 2;        // items a CTA's producer may be ahead
 constexpr unsigned kTicketGroups = 32;  // first-level counters of the "all lengths read" tickets
 constexpr int kMaxRanked = 256;     // sequences whose lengths a CTA copies and can rank
-constexpr int kMaxCluster = 8;      // CTAs that share a head of one sequence (portable cluster size)
+constexpr int kMaxCluster = 8;      // CTAs that share a head of one sequence or two (portable cluster size)
+constexpr int kMaxPaired = 64;      // sequences of a call up to which clusters share two
 constexpr long long kBytesPerRank = 65536;    // and the K + V bytes that are worth one of them
 
 // A 16-byte piece of a row as float pairs, and the softmax's exponential. Scores are kept in units
@@ -104,11 +106,20 @@ inline size_t workspace_bytes(int B, int H, int D, int max_len) {
 }
 
 // ---- the kernel --------------------------------------------------------------------------------
-// ranks == 1: persistent CTAs take whole (sequence, head) items, the items of longer sequences first
+// How a call's (sequence, head) pairs are dealt out. Each way is an instance of its own: in one kernel that branched on
+// it, every one carried the others' registers and branches (bf16, us a layer, one kernel -> instances: 64 sequences x 12
+// heads x 64 17.4 -> 17.2, all of 512 rows 18.4 -> 17.7, 1 x 24 heads x 128 of 7900 rows 21.2 -> 20.5, 2 x 12 19.2 -> 18.0).
+enum class Deal { kPersistent, kCluster, kPairCluster };
+// kPersistent: persistent CTAs take whole (sequence, head) items, the items of longer sequences first
 // (`reorder`): CTA c item c, then whatever a global counter hands out. The producer is already loading
 // the next item's rows while the consumers finish the current one.
-// ranks > 1: the `ranks` CTAs of a thread-block cluster share the rows of one item and merge
+// kCluster: the `ranks` CTAs of a thread-block cluster share the rows of one item and merge
 // through distributed shared memory: no records in global memory, no tickets, no second kernel.
+// kPairCluster: a cluster shares the same head of two sequences, the longest of the call with the shortest and so on,
+// and each gets of its CTAs what its length, read here, asks for. With a cluster for each, the longest ones' read alone at
+// the end (bf16, 24 heads x 128, us a layer, before -> now: rows 1000 / 3000 / 5000 / 7000 38.6 -> 35.5, 7900 and three
+// of 1000 40.1 -> 29.0, 4 x 4000 35.5 -> 35.2, 7000 / 3000 / 5000 37.7 -> 36.8; 16 x 12 heads, up to 1900 rows 22.7 ->
+// 21.2). Parts that ran on from one sequence into the other, all exactly even, were slower: 38.2, 28.8, 38.0 and 23.5.
 template <typename T, int D>
 struct DecodeTile {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
@@ -124,12 +135,13 @@ struct DecodeShared {
   float m[kDecodeWarps], l[kDecodeWarps];
   float acc[kDecodeWarps][128];          // [warp][d]
   __align__(16) int lens[kMaxRanked];    // the sequence lengths (calls of up to kMaxRanked sequences)
+  int2 member[2];                        // kPairCluster: (sequence or -1, length)
   union {
     struct {
       int place[kMaxRanked];             // reorder: rank of each sequence
       int order[kMaxRanked];             // reorder: sequence of each rank
     };
-    float record[kMaxCluster][130];      // ranks > 1: every CTA's partial result, in CTA 0
+    float record[kMaxCluster][130];      // clusters: every CTA's partial result, in the CTA that merges it
   };
 };
 
@@ -141,10 +153,10 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-// stores to the same shared-memory variable of the cluster's CTA 0
-__device__ __forceinline__ uint32_t cluster_rank0_address(const void* own) {
+// stores to the same shared-memory variable of another CTA of the cluster
+__device__ __forceinline__ uint32_t cluster_address(const void* own, int cta) {
   uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(ptx::smem_u32(own)));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(ptx::smem_u32(own)), "r"(cta));
   return a;
 }
 __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
@@ -165,14 +177,16 @@ __device__ __forceinline__ bool consumers_any(bool mine) {
   return any != 0;
 }
 
-template <typename T, int D>
+template <typename T, int D, Deal DEAL>
 __global__ void __launch_bounds__(kDecodeThreads, kManyPerSm)
 decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned* __restrict__ seq_tickets, const T* __restrict__ q,
               const T* __restrict__ k_new, const T* __restrict__ v_new, T* __restrict__ k_cache,
               T* __restrict__ v_cache, int32_t* __restrict__ lengths, int fixed_len, int B, int H, int max_len,
-              int ranks, int stages, int reorder, int early, float scale, int* __restrict__ status) {
+              int cluster_ctas, int stages, int reorder, int early, float scale, int* __restrict__ status) {
   using namespace ptx;
   using Tile = DecodeTile<T, D>;
+  constexpr bool kPersistent = DEAL == Deal::kPersistent, kPairs = DEAL == Deal::kPairCluster;
+  const int ranks = kPersistent ? 1 : cluster_ctas;
   constexpr int EPL = Elem<T>::kPerLane;  // elements per lane (16 bytes)
   constexpr int LPK = D / EPL;            // lanes per cache row
   constexpr int KPI = 32 / LPK;           // cache rows per warp instruction
@@ -215,10 +229,11 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
   if (snapshot)
     for (int i = threadIdx.x; i < kMaxRanked; i += kDecodeThreads) {
       sh.lens[i] = i < B ? (lengths ? lengths[i] : fixed_len) : INT_MIN;
-      if (reorder) sh.place[i] = 0;
+      if (kPersistent && reorder) sh.place[i] = 0;
     }
+  if (kPairs && threadIdx.x < 2) sh.member[threadIdx.x] = make_int2(-1, -1);
   __syncthreads();
-  if (reorder) {
+  if (kPersistent && reorder) {
     // rank(s) = number of sequences that come before s (longer, or as long with a smaller index);
     // with the count padded to a power of two n_pad (32..256; padding is INT_MIN and comes last),
     // 128 threads share out the n_pad^2 comparisons.
@@ -252,24 +267,57 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
   struct Item {
     int b, h, len, row0, row1;
   };
-  const int n_items = B * H, n_lanes = static_cast<int>(gridDim.x) / ranks;   // items taken up by CTAs at the start
-  auto item = [&](int e) -> Item {
-    Item s;
-    const int p = e / H;
-    s.h = e - p * H;
-    s.b = reorder ? sh.order[p] : p;
-    s.len = snapshot ? sh.lens[s.b] : lengths[s.b];
-    const int rows = s.len >= 0 && s.len < max_len ? s.len + 1 : 0;
-    const int share = (rows + ranks - 1) / ranks;
-    s.row0 = min(rank * share, rows);
-    s.row1 = min(s.row0 + share, rows);
-    return s;
+  const int n_items = B * H, n_lanes = static_cast<int>(gridDim.x);   // kPersistent: items taken up by CTAs at the start
+  auto rows_of = [&](int len) { return len >= 0 && len < max_len ? len + 1 : 0; };
+  int merges = -1;            // which sequence of its cluster a CTA merges, if any, and which CTAs have parts of it
+  int part0 = 0, part1 = ranks;
+  bool second = false;        // whether the CTA's own part is of its cluster's second sequence
+  // CTA `part` of the `parts` that share sequence b's head h
+  auto share_of = [&](int b, int h, int len, int part, int parts) -> Item {
+    const int rows = rows_of(len), share = (static_cast<unsigned>(rows) + parts - 1) / static_cast<unsigned>(max(parts, 1)), row0 = min(part * share, rows);
+    return Item{b, h, len, row0, min(row0 + share, rows)};
   };
-
-  const Item first = item(static_cast<int>(blockIdx.x) / ranks);
+  auto item = [&](int e) -> Item {
+    const int p = e / H, b = kPersistent && reorder ? sh.order[p] : p;
+    return share_of(b, e - p * H, snapshot ? sh.lens[b] : lengths[b], rank, ranks);
+  };
+  Item first;
+  if (!kPairs) {
+    first = item(static_cast<int>(blockIdx.x) / ranks);
+    if (rank == 0) merges = 0;
+  } else {
+    // Cluster c takes head c % H of the c / H-th longest and c / H-th shortest sequence (one, in the middle of an odd
+    // number). Its CTAs are divided so that the largest part is as small as it can be.
+    const int e = static_cast<int>(blockIdx.x) / ranks, g = e / H, t = threadIdx.x;
+    if (t < B) {
+      const int mine = sh.lens[t];
+      int place = 0;
+#pragma unroll 4
+      for (int j = 0; j < B; ++j)
+        place += static_cast<int>(sh.lens[j] > mine) | (static_cast<int>(sh.lens[j] == mine) & static_cast<int>(j < t));
+      if (place == g) sh.member[0] = make_int2(t, mine);
+      else if (place == B - 1 - g) sh.member[1] = make_int2(t, mine);
+    }
+    __syncthreads();
+    const int2 a = sh.member[0], b = sh.member[1];
+    const int rows_a = rows_of(a.y), rows_b = b.x < 0 ? 0 : rows_of(b.y);
+    int cut = rows_b == 0 ? ranks : 0;   // CTAs for the first
+    if (rows_a > 0 && rows_b > 0) {
+      // the whole number below or above what is in proportion, whichever has the smaller largest part
+      const float fa = static_cast<float>(rows_a), fb = static_cast<float>(rows_b);
+      const int below = min(max(static_cast<int>(__fdividef(fa * ranks, fa + fb)), 1), ranks - 1);
+      const int above = min(below + 1, ranks - 1);
+      cut = fa * (ranks - above) <= fb * below ? below : above;
+    }
+    second = rank >= cut;
+    first = second ? share_of(b.x, e - g * H, b.y, rank - cut, ranks - cut) : share_of(a.x, e - g * H, a.y, rank, cut);
+    if (rank < 2 && (rank == 0 ? a.x : b.x) >= 0) merges = rank;
+    part0 = rank == 0 ? 0 : cut;
+    part1 = rank == 0 ? cut : ranks;
+  }
   // "this CTA has started and looked its item up" (record shares memory with the ranking): waited
   // for before the first remote store
-  if (ranks > 1) cluster_arrive();
+  if (!kPersistent) cluster_arrive();
 
   // Every CTA of the call draws a ticket once it has read the lengths; whoever holds the last one
   // knows that nobody will read them again and advances them. Two levels keep the atomics off one
@@ -308,7 +356,7 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
       // One claim per item beyond the CTAs' first ones and one per CTA that finds nothing left: n_items
       // in all, of which the last returns the counter to zero.
       auto claim = [&]() -> int {
-        if (n_lanes >= n_items) return n_items;
+        if (!kPersistent || n_lanes >= n_items) return n_items;
         const unsigned c = atomicAdd(item_counter, 1u);
         if (c == static_cast<unsigned>(n_items - 1)) *item_counter = 0;
         return min(static_cast<int>(c) + n_lanes, n_items);
@@ -464,7 +512,7 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
 
       // the next item; its token vectors arrive while this one is merged
       have = false;
-      if (ranks == 1) {
+      if (kPersistent) {
         const int slot_i = n % kItemRing;
         if (ok && (ok = mbar_wait(&sh.item_ready[slot_i], (n / kItemRing) & 1, abort_flag))) {
           const int e = *reinterpret_cast<volatile int*>(&sh.item[slot_i]);
@@ -517,12 +565,12 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
           ll += sh.l[w] * c;
           aa += sh.acc[w][d] * c;
         }
-        if (ranks == 1) {
+        if (kPersistent) {
           if (s.row1 > 0) out[bh * D + d] = Elem<T>::from_float(aa / ll);
         } else {
-          // hand the share to CTA 0, which is known to run once the cluster's first barrier is through
+          // hand the share to the CTA that merges it, which is known to run once the cluster's first barrier is through
           cluster_wait();
-          const uint32_t rec = cluster_rank0_address(&sh.record[rank][0]);
+          const uint32_t rec = cluster_address(&sh.record[rank][0], second ? 1 : 0);
           st_cluster(rec + d * 4, aa);
           if (d == 0) {
             st_cluster(rec + D * 4, mm);
@@ -530,7 +578,7 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
           }
         }
       }
-      if (ranks == 1) {
+      if (kPersistent) {
         if (s.row1 == 0 && s.h == 0 && threadIdx.x == 0) atomicExch(status, DADATTN_E_ARG);
         // sh.acc / sh.m are read: the next item may write them. The warps go on together or not at all: one whose
         // wait ran out would be missing at the named barriers of the next item.
@@ -539,27 +587,27 @@ decode_kernel(T* __restrict__ out, unsigned* __restrict__ item_counter, unsigned
     }
   }
 
-  if (ranks > 1) {
-    // Threads without a share to hand over join the first barrier here; after the second, CTA 0 merges.
+  if (!kPersistent) {
+    // Threads without a share to hand over join the first barrier here; after the second the shares are merged.
     const int d = threadIdx.x;
     if (d >= D) cluster_wait();
     cluster_arrive();
     cluster_wait();
-    if (rank == 0) {
-      const Item& s = first;
-      if (s.len >= 0 && s.len < max_len) {
+    if (merges >= 0) {
+      const int b = kPairs ? sh.member[merges].x : first.b, len = kPairs ? sh.member[merges].y : first.len;
+      if (len >= 0 && len < max_len) {
         if (d < D) {
           float mm = -FLT_MAX;
-          for (int j = 0; j < ranks; ++j) mm = fmaxf(mm, sh.record[j][D]);
+          for (int j = part0; j < part1; ++j) mm = fmaxf(mm, sh.record[j][D]);
           float ll = 0.f, aa = 0.f;
-          for (int j = 0; j < ranks; ++j) {
+          for (int j = part0; j < part1; ++j) {
             const float c = Elem<T>::exp_of(sh.record[j][D] - mm);   // a share without rows has m = -FLT_MAX: 0
             ll += sh.record[j][D + 1] * c;
             aa += sh.record[j][d] * c;
           }
-          out[(static_cast<size_t>(s.b) * H + s.h) * D + d] = Elem<T>::from_float(aa / ll);
+          out[(static_cast<size_t>(b) * H + first.h) * D + d] = Elem<T>::from_float(aa / ll);
         }
-      } else if (s.h == 0 && d == 0) {
+      } else if (first.h == 0 && d == 0) {
         atomicExch(status, DADATTN_E_ARG);
       }
     }
@@ -592,9 +640,6 @@ int launch_decode(T* out, const T* q, const T* k_new, const T* v_new, T* k_cache
   // of the lengths
   unsigned* item_counter = tickets;
   unsigned* seq_tickets = tickets ? tickets + static_cast<size_t>(B) * H : nullptr;
-  auto kern = decode_kernel<T, DH>;
-  // (a cheap host call, 0.06 us)
-  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(decode_smem(kMaxStages))));
   int dev = 0, sms = 0;
   DAD_CUDA(cudaGetDevice(&dev));
   DAD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -615,11 +660,23 @@ int launch_decode(T* out, const T* q, const T* k_new, const T* v_new, T* k_cache
   const int resident = kManyPerSm * sms;
   int ranks = 1;
   while (ranks < kMaxCluster && ranks * kBytesPerRank < bytes && pairs * ranks * 2 <= resident) ranks *= 2;
+  // Two or four CTAs for each: a cluster of four or eight for two sequences, where the lengths are on the device (the
+  // ranking reads them all: up to kMaxPaired) and the spare CTAs of an odd one fit, too.
+  Deal deal = ranks > 1 ? Deal::kCluster : Deal::kPersistent;
   // (without a workspace there is no counter to deal items from: one CTA each)
-  const long long grid = ranks > 1 || !item_counter ? pairs * ranks : min(pairs, static_cast<long long>(resident));
-  const int stages = grid <= static_cast<long long>(kFewPerSm) * sms ? kFewStages : kManyStages;
+  long long grid = ranks > 1 || !item_counter ? pairs * ranks : min(pairs, static_cast<long long>(resident));
+  const long long paired = static_cast<long long>((B + 1) / 2) * H * ranks * 2;
+  if (lengths && ranks > 1 && ranks < kMaxCluster && B >= 2 && B <= kMaxPaired && paired * 100 <= resident * 95LL)
+    deal = Deal::kPairCluster, ranks *= 2, grid = paired;
+  // (clusters of eight with the deeper ring fit 48 times, which leaves the next call's no room to set themselves up in)
+  const long long few = deal == Deal::kPairCluster && ranks == kMaxCluster ? 2 * sms : kFewPerSm * sms;
+  const int stages = grid <= few ? kFewStages : kManyStages;
   // Longest first pays once a CTA takes more than one item; the in-kernel ranking handles 32..256 sequences.
   const int reorder = B >= 32 && B <= kMaxRanked && pairs > grid;
+  auto kern = deal == Deal::kPersistent ? decode_kernel<T, DH, Deal::kPersistent>
+              : deal == Deal::kCluster ? decode_kernel<T, DH, Deal::kCluster> : decode_kernel<T, DH, Deal::kPairCluster>;
+  // (a cheap host call, 0.06 us)
+  DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(decode_smem(kMaxStages))));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kDecodeThreads);
