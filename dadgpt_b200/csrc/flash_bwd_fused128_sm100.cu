@@ -113,7 +113,7 @@ template <bool DROP>
 __global__ void __launch_bounds__(kGThreads, 1)
 flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
-                          __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
+                          const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv,
                           float* __restrict__ dq_ws, const float* __restrict__ lse,
                           const float* __restrict__ delta, int S, float scale, float rate,
                           const __grid_constant__ PhiloxRounds rng, int64_t unit0, LeveledGrid order,
@@ -413,24 +413,31 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       mbar_arrive(&bars->w_full);
     }
 
-    // dV (column groups 0, 1) and dK (2, 3), 64 head dims each
+    // dV (column groups 0, 1) and dK (2, 3), 64 head dims each, through shared memory and TMA: a warp's 32 keys x 64 dims
+    // are 4 KB of the Q ring, whose tiles the last products have read. As 16-byte stores of one row per lane, 32 rows
+    // an instruction, they took 6800 clocks a CTA (backward, us: 192 x 1024 267 -> 247, 72 x 777 80 -> 73, 192 x 128 30.5 ->
+    // 26.8, 24 x 2048 103 -> 95.6, 192 x 8192 9590 -> 9390).
     if (ok && polled_wait(&bars->acc_done, (n_it - 1) & 1, abort_flag)) {
       tc_fence_after_sync();
-      __nv_bfloat16* dst = (cg < 2 ? dv : dk) + (static_cast<size_t>(bh) * S + key) * D + (cg & 1) * 64;
+      uint8_t* stage = smem + L::kQ + cg * kGPanel + quad * 32 * 128;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t o[32];
         tmem_ld32(tlane + (cg < 2 ? kColDV : kColDK) + (cg & 1) * 64 + c * 32, o);
         tmem_wait_ld();
-        if (key < S) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(dst + c * 32 + i * 8) = make_uint4(
-                pack_bf16(__uint_as_float(o[8 * i + 0]), __uint_as_float(o[8 * i + 1])),
-                pack_bf16(__uint_as_float(o[8 * i + 2]), __uint_as_float(o[8 * i + 3])),
-                pack_bf16(__uint_as_float(o[8 * i + 4]), __uint_as_float(o[8 * i + 5])),
-                pack_bf16(__uint_as_float(o[8 * i + 6]), __uint_as_float(o[8 * i + 7])));
-        }
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(
+              pack_bf16(__uint_as_float(o[8 * i + 0]), __uint_as_float(o[8 * i + 1])),
+              pack_bf16(__uint_as_float(o[8 * i + 2]), __uint_as_float(o[8 * i + 3])),
+              pack_bf16(__uint_as_float(o[8 * i + 4]), __uint_as_float(o[8 * i + 5])),
+              pack_bf16(__uint_as_float(o[8 * i + 6]), __uint_as_float(o[8 * i + 7])));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0 && k0 + quad * 32 < S) {   // (rows beyond S are not written)
+        bulk_store_3d(cg < 2 ? &map_dv : &map_dk, stage, (cg & 1) * 64, k0 + quad * 32, bh);
+        bulk_store_read();
       }
     }
   }
@@ -527,11 +534,13 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
   const int n_sub = (S + kGSub - 1) / kGSub;
   float* delta = static_cast<float*>(workspace);
   float* dq_ws = reinterpret_cast<float*>(static_cast<char*>(workspace) + delta_bytes);
-  CUtensorMap mk, mv, mq, mdo;
+  CUtensorMap mk, mv, mq, mdo, mdk, mdv;
   if (int rc = make_tensor_map_bf16(&mk, k, BH, S, kGD, kGKeys)) return rc;
   if (int rc = make_tensor_map_bf16(&mv, v, BH, S, kGD, kGKeys)) return rc;
   if (int rc = make_tensor_map_bf16(&mq, q, BH, S, kGD, kGSub)) return rc;
   if (int rc = make_tensor_map_bf16(&mdo, dout, BH, S, kGD, kGSub)) return rc;
+  if (int rc = make_tensor_map_bf16(&mdk, dk, BH, S, kGD, 32)) return rc;
+  if (int rc = make_tensor_map_bf16(&mdv, dv, BH, S, kGD, 32)) return rc;
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
 
@@ -557,8 +566,7 @@ int launch_bwd_fused_d128(uint16_t* dq, uint16_t* dk, uint16_t* dv, void* worksp
   static std::atomic<int> regs_seen[2];
   if (int rc = check_launch_registers(reinterpret_cast<const void*>(kern), kGRegsLaunch, regs_seen[drop])) return rc;
   DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kGKeys - 1) / kGKeys), dim3(kGThreads),
-                      G128Smem::kBytes, st, mk, mv, mq, mdo, reinterpret_cast<BF*>(dk),
-                      reinterpret_cast<BF*>(dv), dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
+                      G128Smem::kBytes, st, mk, mv, mq, mdo, mdk, mdv, dq_ws, lse, static_cast<const float*>(delta), S, scale, rate, rng, unit0, order, status));
   stage_event(2, st);
   DAD_CUDA(launch_pdl(fused128_convert_kernel, dim3(n_sub, BH), dim3(256), 0, st,
                       reinterpret_cast<BF*>(dq), dq_ws, S, n_sub));

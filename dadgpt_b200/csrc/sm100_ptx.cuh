@@ -144,6 +144,17 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// TMA store out of shared memory to (x, y, z), as a group of its own; the memory may be written again, and the CTA
+// leave, behind bulk_store_read().
+__device__ __forceinline__ void bulk_store_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];\n\t"
+      "cp.async.bulk.commit_group;"
+      ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_store_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
 // 1-D form, for vectors of per-row scalars. x times the element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_1d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x) {
   asm volatile(
