@@ -174,7 +174,22 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     return;
   }
 
+  // The tiles of the ring's stage s, by the producing thread
+  auto load_k = [&](int s, int j) {
+    mbar_arrive_expect_tx(&bars->k_full[s], kPanels * kPanelBytes);
+    for (int p = 0; p < kPanels; ++p)
+      tma_load_3d(smem + L::kK + (s * kPanels + p) * kPanelBytes, &map_k, &bars->k_full[s], p * 64, j * kBN, bh);
+  };
+  auto load_v = [&](int s, int j) {
+    mbar_arrive_expect_tx(&bars->v_full[s], kPanels * kPanelBytes);
+    for (int p = 0; p < kPanels; ++p)
+      tma_load_3d(smem + L::kV + (s * kPanels + p) * kPanelBytes, &map_v, &bars->v_full[s], p * 64, j * kBN, bh);
+  };
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_q);
+    prefetch_tensormap(&map_k);
+    prefetch_tensormap(&map_v);
+    prefetch_tensormap(&map_out);
     mbar_init(&bars->q_full, 1);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&bars->k_full[s], 1);
@@ -191,7 +206,16 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars->settled, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
+    // The first tiles are requested here: they need this thread's barriers, and nothing of what the others set up (192 x
+    // 1024 93.4 -> 91.9 us, 192 x 128 11.8 -> 11.3)
+    pdl_wait();
+    mbar_arrive_expect_tx(&bars->q_full, kPanels * kPanelBytes);
+    for (int p = 0; p < kPanels; ++p)
+      tma_load_3d(smem + L::kQ + p * kPanelBytes, &map_q, &bars->q_full, p * 64, q0, bh);
+    load_k(0, 0);
+    load_v(0, 0);
   }
+  __syncwarp();
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
     tmem_relinquish();
@@ -207,28 +231,16 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (elect_one()) {
-      prefetch_tensormap(&map_q);
-      prefetch_tensormap(&map_k);
-      prefetch_tensormap(&map_v);
-      mbar_arrive_expect_tx(&bars->q_full, kPanels * kPanelBytes);
-      for (int p = 0; p < kPanels; ++p)
-        tma_load_3d(smem + L::kQ + p * kPanelBytes, &map_q, &bars->q_full, p * 64, q0, bh);
-      int n_k = 0, n_v = 0;   // tiles loaded
-      for (int j = 0; j < n_kv; ++j) {
+    if (lane == 0) {
+      int n_k = 1, n_v = 1;   // tiles loaded
+      for (int j = 1; j < n_kv; ++j) {
         const int s = j % kStages, use = j / kStages;
-        uint8_t* kdst = smem + L::kK + s * kPanels * kPanelBytes;
-        uint8_t* vdst = smem + L::kV + s * kPanels * kPanelBytes;
         // K's slot frees when Q K^T of its previous tenant is done, V's when P V is done
         if (use > 0 && !hot_wait(&bars->k_empty[s], (use - 1) & 1, abort_flag)) break;
-        mbar_arrive_expect_tx(&bars->k_full[s], kPanels * kPanelBytes);
-        for (int p = 0; p < kPanels; ++p)
-          tma_load_3d(kdst + p * kPanelBytes, &map_k, &bars->k_full[s], p * 64, j * kBN, bh);
+        load_k(s, j);
         ++n_k;
         if (use > 0 && !hot_wait(&bars->v_empty[s], (use - 1) & 1, abort_flag)) break;
-        mbar_arrive_expect_tx(&bars->v_full[s], kPanels * kPanelBytes);
-        for (int p = 0; p < kPanels; ++p)
-          tma_load_3d(vdst + p * kPanelBytes, &map_v, &bars->v_full[s], p * 64, j * kBN, bh);
+        load_v(s, j);
         ++n_v;
       }
       settle(&bars->q_full, 0);
