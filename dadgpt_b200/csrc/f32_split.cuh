@@ -70,9 +70,17 @@ __device__ __forceinline__ Split4 split4(float4 x) {
   }
   return s;
 }
-// Columns 4 c4 .. 4 c4 + 3 of a row into the three planes of a tile (128-byte swizzle).
+// Rows of a streamed tile are as wide as the head, so that the sums' products, which read them MN-major, are too: at
+// 64 columns for every head size those of 32 and 16 took 33 clocks a product instead of 17 and 10 (backward, us:
+// 48 x 1024 x 16 87 -> 73, x 32 99 -> 94; forward and backward 64 x 300 x 16 39.4 -> 33, 32 x 301 x 32 24.5 -> 23.2, 16 x
+// 64 x 16 9.9 -> 9.3).
+template <int D>
+constexpr int kStreamRow = 2 * D;
+// Columns 4 c4 .. 4 c4 + 3 of a row into the three planes of a tile with rows of ROW_BYTES and the swizzle of that width.
+template <int ROW_BYTES = 128>
 __device__ __forceinline__ void store_split(uint8_t* tile, int plane_bytes, int row, int c4, const Split4& s) {
-  uint8_t* at = tile + row * 128 + ((((c4 >> 1) ^ (row & 7)) << 4) | ((c4 & 1) << 3));
+  const int swizzle = ROW_BYTES == 128 ? row & 7 : ROW_BYTES == 64 ? (row >> 1) & 3 : (row >> 2) & 1;
+  uint8_t* at = tile + row * ROW_BYTES + ((((c4 >> 1) ^ swizzle) << 4) | ((c4 & 1) << 3));
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * plane_bytes) = s.p[i];
 }

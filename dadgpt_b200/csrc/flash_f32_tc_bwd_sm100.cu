@@ -144,11 +144,6 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
-  // Columns D..63 of the streamed tiles are read by the sums' products (64 columns wide): zeros.
-  if (D < 64)
-    for (int i = threadIdx.x; i < 5 * 3 * kPlaneB / 16; i += kThreads)
-      reinterpret_cast<uint4*>(smem + L::kB1)[i] = make_uint4(0, 0, 0, 0);
-  if (D < 64) fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -189,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
           auto put = [&](uint8_t* to, const Split4 (&v)[kMine]) {
 #pragma unroll
             for (int j = 0; j < kMine; ++j)
-              if (rt + j * kRowStep < kStep) store_split(to, kPlaneB, rt + j * kRowStep, c4, v[j]);
+              if (rt + j * kRowStep < kStep) store_split<kStreamRow<D>>(to, kPlaneB, rt + j * kRowStep, c4, v[j]);
           };
           float delta[kMine];
           Split4 sp[kMine];
@@ -239,11 +234,11 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
       const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // A, B K-major
-      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // A from tensor memory, B MN-major
+      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, D, 0, 1);       // A from tensor memory, B MN-major
       const SmemDescBase a1 = make_desc_base_sw128(smem_u32(smem + L::kA1), 0);
       const SmemDescBase a2 = make_desc_base_sw128(smem_u32(smem + L::kA2), 0);
-      const SmemDescBase b1_0 = make_desc_base_sw128(smem_u32(smem + L::kB1), 0);
-      const SmemDescBase b2_0 = make_desc_base_sw128(smem_u32(smem + L::kB2), 0);
+      const SmemDescBase b1_0 = make_desc_base_rows<kStreamRow<D>>(smem_u32(smem + L::kB1));
+      const SmemDescBase b2_0 = make_desc_base_rows<kStreamRow<D>>(smem_u32(smem + L::kB2));
       auto issue_x = [&](int i) -> bool {
         const int s = i & 1;
         const uint32_t par = (i >> 1) & 1, tx = tm + s * 128;
@@ -282,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
             for (int kk = 0; kk < kStep / 16; ++kk) {
               const uint32_t at = (product_a(m) == 0 ? 0u : product_a(m) == 1 ? 8u : 64u) + kk * 16;
-              mma_ts_warp(tm + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+              mma_ts_warp(tm + kSum1, tx + at, desc_at(b2, product_b(m) * kPlaneB + kk * 16 * kStreamRow<D>), idesc_s,
                      (m > 0 || kk > 0) ? 1u : 0u, lead);
             }
         }
@@ -292,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_f32_tc_kernel(const __g
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
             const uint32_t at = product_a(m) == 0 ? tx + 64 + 8 + kk * 16 : tm + kExtra + (product_a(m) - 1) * 8 + kk * 16;
-            mma_ts_warp(tm + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+            mma_ts_warp(tm + kSum2, at, desc_at(b1, product_b(m) * kPlaneB + kk * 16 * kStreamRow<D>), idesc_s,
                    (m > 0 || kk > 0) ? 1u : 0u, lead);
           }
         mma_commit_warp(&bars->b1_empty[s], lead);

@@ -113,12 +113,6 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
     tmem_alloc(&bars->tmem_base, 256);
     tmem_relinquish();
   }
-  // Columns D..63 of the V tiles are read by the P V products (64 columns wide): zeros.
-  if (D < 64) {
-    for (int i = threadIdx.x; i < kStages * 3 * kPlaneB / 16; i += kThreads)
-      reinterpret_cast<uint4*>(smem + L::kV)[i] = make_uint4(0, 0, 0, 0);
-    fence_proxy_async_smem();
-  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -156,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
             if (lap > 0 && !mbar_wait(empty, (lap - 1) & 1, abort_flag)) return false;
 #pragma unroll
             for (int j = 0; j < kMine; ++j)
-              if (rt + j * kRowStep < kStep) store_split(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
+              if (rt + j * kRowStep < kStep) store_split<kStreamRow<D>>(tile, kPlaneB, rt + j * kRowStep, c4, sp[j]);
             fence_proxy_async_smem();
             mbar_arrive(full);
             return true;
@@ -176,10 +170,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
       const uint32_t lead = elect_one(), tm = __reduce_max_sync(0xffffffffu, tmem);   // (known to be uniform, so)
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t idesc_x = make_idesc_bf16(kRows, kStep, 0, 0);   // Q, K: K-major
-      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, 64, 0, 1);      // P from tensor memory, V MN-major
+      constexpr uint32_t idesc_s = make_idesc_bf16(kRows, D, 0, 1);       // P from tensor memory, V MN-major
       const SmemDescBase qd = make_desc_base_sw128(smem_u32(smem + L::kQ), 0);
-      const SmemDescBase k0 = make_desc_base_sw128(smem_u32(smem + L::kK), 0);
-      const SmemDescBase v0 = make_desc_base_sw128(smem_u32(smem + L::kV), 0);
+      const SmemDescBase k0 = make_desc_base_rows<kStreamRow<D>>(smem_u32(smem + L::kK));
+      const SmemDescBase v0 = make_desc_base_rows<kStreamRow<D>>(smem_u32(smem + L::kV));
       auto issue_x = [&](int i) -> bool {
         const int s = i % kStages;
         const uint32_t tx = tm + (i & 1) * 64;
@@ -209,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_f32_tc_kernel(const __g
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
             const uint32_t at = product_a(m) == 2 ? tm + kExtra + kk * 8 : tx + kk * 16 + product_a(m) * 8;
-            mma_ts_warp(tm + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 2048), idesc_s,
+            mma_ts_warp(tm + kSum, at, desc_at(vd, product_b(m) * kPlaneB + kk * 16 * kStreamRow<D>), idesc_s,
                    (m > 0 || kk > 0) ? 1u : 0u, lead);
           }
         mma_commit_warp(&bars->v_empty[s], lead);

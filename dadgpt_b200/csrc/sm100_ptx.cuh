@@ -310,6 +310,15 @@ __device__ __forceinline__ SmemDescBase make_desc_base_sw128(uint32_t smem_addr,
   const uint64_t d = make_smem_desc_sw128(smem_addr, lbo_bytes);
   return SmemDescBase{static_cast<uint32_t>(d), static_cast<uint32_t>(d >> 32)};
 }
+// For tiles whose rows are 64 or 32 bytes (32 or 16 bf16), with the swizzle of that width (Swizzle<2, 4, 3> and
+// <1, 4, 3> on the address), 8-row groups one after the other. As above for both majors; an MN-major operand is one
+// such row wide.
+template <int ROW_BYTES>
+__device__ __forceinline__ SmemDescBase make_desc_base_rows(uint32_t smem_addr) {
+  static_assert(ROW_BYTES == 128 || ROW_BYTES == 64 || ROW_BYTES == 32, "a swizzle's width");
+  constexpr uint32_t layout = ROW_BYTES == 128 ? 2 : ROW_BYTES == 64 ? 4 : 6;   // SWIZZLE_128B, _64B, _32B
+  return SmemDescBase{(smem_addr & 0x3FFFF) >> 4, static_cast<uint32_t>(8 * ROW_BYTES >> 4) | 1u << 14 | layout << 29};
+}
 // Descriptor of the same tile advanced by `byte_offset` (a multiple of 16 that stays inside the
 // tile, so the 14-bit address field cannot carry into its neighbours).
 __device__ __forceinline__ uint64_t desc_at(SmemDescBase b, uint32_t byte_offset) {
