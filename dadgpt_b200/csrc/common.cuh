@@ -184,6 +184,10 @@ inline size_t dropout_mask_bits_bytes(int BH, int S) {
   return static_cast<size_t>(BH) * (n_tiles * (n_tiles + 1) / 2) * kMaskTile * 16;
 }
 
+// Forward at head size 128 without dropout, two query tiles per CTA (flash_fwd128_sm100.cu), and where that is the better.
+bool fwd128_pairs_pay(int BH, int S);
+int launch_fwd_bf16_d128_pairs(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v, int BH,
+                               int S, float scale, cudaStream_t st);
 // Forward at head size 64 (flash_fwd64_sm100.cu). mask_bits != nullptr with rate > 0: keep bits
 // from dadattn_dropout_mask_bits; mask_bits == nullptr with rate > 0: the Philox mask is drawn
 // inside the kernel. heads > 0: tensors are the interleaved [B*S, heads*64] activations.
@@ -254,10 +258,14 @@ inline dim3 leveled_blocks(const LeveledGrid& g, int n_levels) {
   return g.group == 1 ? dim3(n_levels, 1, groups) : dim3(g.group, n_levels, groups);
 }
 // False for the blocks that pad the last group.
-__device__ __forceinline__ bool leveled_block(const LeveledGrid& g, int& level, int& bh) {
-  level = g.group == 1 ? blockIdx.x : blockIdx.y;
-  bh = blockIdx.z * g.group + (g.group == 1 ? 0 : blockIdx.x);
+template <typename Index>
+__device__ __forceinline__ bool leveled_item(const LeveledGrid& g, const Index& block, int& level, int& bh) {
+  level = g.group == 1 ? block.x : block.y;
+  bh = block.z * g.group + (g.group == 1 ? 0 : block.x);
   return bh < g.units;
+}
+__device__ __forceinline__ bool leveled_block(const LeveledGrid& g, int& level, int& bh) {
+  return leveled_item(g, blockIdx, level, bh);
 }
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

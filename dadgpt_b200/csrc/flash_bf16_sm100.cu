@@ -20,8 +20,8 @@
 // S_{j+1} is issued before P_j V_j, so the tensor core works on the next tile while the
 // exponentials of the current one are computed; the scores are double-buffered in TMEM.
 //
-// Head size 128; size 64 has the persistent two-tile kernel of flash_fwd64_sm100.cu. The entry points
-// of both are here.
+// Head size 128, launches that do not fill the GPU and dropout; the others have the persistent two-tile kernel of
+// flash_fwd128_sm100.cu, head size 64 that of flash_fwd64_sm100.cu. The entry points of all are here.
 //
 // Every mbarrier wait is bounded (sm100_ptx.cuh). If one runs out, the CTA raises its abort
 // flag, everybody falls through to the common exit, TMEM is freed, and DADATTN_E_TIMEOUT is
@@ -525,6 +525,9 @@ extern "C" int dadattn_flash_fwd_bf16(uint16_t* out, float* lse, const uint16_t*
   const bool drop = rate > 0.f;
   if (D == 64)   // head size 64 has a kernel of its own (flash_fwd64_sm100.cu)
     return launch_fwd_bf16_d64(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, nullptr, 0, st);
+  // (a draw costs more than the rest of the arithmetic: with dropout the larger number of smaller items is the better
+  // one, 192 x 512 119 us against 142)
+  if (!drop && fwd128_pairs_pay(BH, S)) return launch_fwd_bf16_d128_pairs(out, lse, q, k, v, BH, S, scale, st);
   return drop ? launch_fwd_bf16<true>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st)
               : launch_fwd_bf16<false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
 }
