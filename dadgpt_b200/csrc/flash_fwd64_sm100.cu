@@ -24,12 +24,14 @@
 //     as packed bf16 over the first half of the same columns, from where the P V product takes
 //     it as its A operand;
 //   * scale-and-subtract and the row sums run as packed two-float instructions (fma.rn.f32x2,
-//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in four as a
+//     add.rn.f32x2), the row max as three-input max, and one pair of exponentials in eight as a
 //     cubic on the FMA pipe (us at 192 x 1024 / 48 x 4096: none 44.4 / 129, one in eight 42.8 / 124, one
-//     in four 41.7 / 121, three in eight 42.4 / 122, half 43.7 / 127; a bf16x2 exp2 on the
-//     special-function unit was tried: no faster, and it cost a digit of lse); only the 32 x 32 block
-//     on the diagonal pays for the causal compare: the softmax is bound by instruction issue and the
-//     exp2 unit alike;
+//     in four 41.7 / 121, half 43.7 / 127). It is the last pair of sixteen columns: the first fourteen rows
+//     of a sequence, whose probabilities are the largest, see exact ones only (with columns 2 and 3 of
+//     eight and a cubic of 1.0e-4 their lse was off by 4e-5 instead of 3e-7, and results there by a unit
+//     of bf16). A bf16x2 exp2 on the special-function unit was tried: no faster, and it cost a digit of
+//     lse. Only the 32 x 32 block on the diagonal pays for the causal compare: the softmax is bound by
+//     instruction issue and the exp2 unit alike;
 //   * CTAs are persistent: barriers, tensor memory and descriptors are set up once, items are
 //     dealt out heaviest first in a fixed serpentine order (no global counter to reset), the
 //     next item's Q tiles and first K/V tiles are in flight while the current one finishes, and
@@ -518,7 +520,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int i = 0; i < 32; i += 2) {
           const float2 e = ffma2(make_float2(__uint_as_float(xa[i]), __uint_as_float(xa[i + 1])), sl, nm);
           float2 p;
-          if ((i & 7) == 2) {   // one pair in four on the FMA pipe
+          if ((i & 15) == 14) {   // one pair in eight on the FMA pipe
             p = ex2_poly2(e);
           } else {
             p.x = ex2(e.x);
