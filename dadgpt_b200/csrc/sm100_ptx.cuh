@@ -420,9 +420,10 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 // 2^x for two values on the FMA pipe, x at most a few tens: integer part through the float-rounding trick, fraction
 // in [-0.5, 0.5] through its Taylor cubic (largest relative error 7.9e-4, below bf16's half ulp of 2e-3, but not below
 // what lse has: for few of a row's exponentials). Arguments below -127 (masked scores are -inf) come as -127, whose
-// integer part takes the exponent of 1.0 to zero: exactly 0.
+// power of two is put together as 0: exactly 0. NaN stays NaN: it passes the maximum and the product of the two parts
+// (an integer add into the exponent would make it FLT_MAX).
 __device__ __forceinline__ float2 ex2_poly2(float2 x0) {
-  float2 x;   // (NaN stays NaN, and ends as a number that bf16 rounds to infinity)
+  float2 x;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(x.x) : "f"(x0.x), "f"(-127.f));
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(x.y) : "f"(x0.y), "f"(-127.f));
   const float2 big = make_float2(12582912.f, 12582912.f);  // 1.5 * 2^23
@@ -431,10 +432,9 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x0) {
   float2 p = ffma2(f, make_float2(0.0555041087f, 0.0555041087f), make_float2(0.2402265070f, 0.2402265070f));
   p = ffma2(p, f, make_float2(0.6931471806f, 0.6931471806f));
   p = ffma2(p, f, make_float2(1.0f, 1.0f));
-  float2 r;
-  r.x = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
-  r.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
-  return r;
+  const float2 two_n = make_float2(__int_as_float((__float_as_int(t.x) << 23) + 0x3f800000),
+                                   __int_as_float((__float_as_int(t.y) << 23) + 0x3f800000));
+  return fmul2(p, two_n);
 }
 
 
