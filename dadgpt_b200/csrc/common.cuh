@@ -184,7 +184,10 @@ inline size_t dropout_mask_bits_bytes(int BH, int S) {
   return static_cast<size_t>(BH) * (n_tiles * (n_tiles + 1) / 2) * kMaskTile * 16;
 }
 
-// Forward at head size 128 without dropout, two query tiles per CTA (flash_fwd128_sm100.cu), and where that is the better.
+// Forward at head size 128 without dropout. Up to kFwd128OneSumRows rows: one maximum, sum and accumulator per row, two query
+// tiles per CTA (flash_fwd128_sm100.cu) where that is the better, else one (flash_bf16_sm100.cu), with the same results.
+// Beyond: flash_bf16_sm100.cu with those of each half of a row.
+constexpr int kFwd128OneSumRows = 2048;
 bool fwd128_pairs_pay(int BH, int S);
 int launch_fwd_bf16_d128_pairs(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v, int BH,
                                int S, float scale, cudaStream_t st);

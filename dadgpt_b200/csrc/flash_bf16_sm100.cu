@@ -11,7 +11,8 @@
 //               tile, warps 6-9 columns 64-127 (a warp may only touch the TMEM lane quadrant
 //               warp_id % 4). Each half keeps its OWN running max / sum and its OWN output
 //               accumulator in TMEM, so the two threads of a row never synchronise inside the
-//               loop; the halves are merged once, in the epilogue (split-K inside the CTA).
+//               loop; the halves are merged once, in the epilogue (split-K inside the CTA). Up to
+//               2048 rows without dropout they agree on one of each (ONE_SUM).
 //               Eight softmax warps give every scheduler two warps to hide the FFMA -> MUFU ->
 //               FADD latencies behind each other.
 //               A thread reads its 64 scores with tcgen05.ld, writes P as packed bf16 over them,
@@ -131,7 +132,8 @@ struct FwdSmem {
   static constexpr int kK = kQ + kPanels * kPanelBytes;
   static constexpr int kV = kK + kStages * kPanels * kPanelBytes;
   static constexpr int kBars = kV + kStages * kPanels * kPanelBytes;
-  static constexpr int kBytes = kBars + 256;
+  static constexpr int kMax = kBars + 512;               // ONE_SUM: a tile's maxima, [2][half][row]
+  static constexpr int kBytes = kMax + 2 * 2 * kBM * 4;
 };
 
 struct FwdBars {
@@ -141,11 +143,21 @@ struct FwdBars {
   // first, and P_j V_j read scores for probabilities (rows of infinities in one call of five at 8 x 3080 with
   // dropout, whose draws set the warps apart). P_{j+2} needs S_{j+2}, which is issued after p_full of tile j.
   uint64_t s_full[2], p_full[2], o_done[2], stat_full, settled;  // P_j V_j commits to o_done[j & 1]
+  uint64_t max_full[2][2][4];   // ONE_SUM: a warp's 32 maxima of tile j are there, [j & 1][half][quadrant]
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(FwdBars) <= 512, "barrier block");
 
-template <bool DROP>
+// ONE_SUM: a row's two halves agree on its maximum, tile by tile, and add into one accumulator, as the rows of
+// flash_fwd128_sm100.cu do, in the same order: launches of up to kFwd128OneSumRows rows take that kernel or this one by
+// the number of their units, and a unit's result is the same bit for bit. (The maxima go through shared memory and are
+// looked at behind half of the exponentials: 24 x 2048 36.0 -> 36.6 us, 4 x 2048 17.8 -> 18.1; looked at ahead of them, by
+// a barrier of the two warps, 37.7 and 19.7. Against float64 at 192 x 1024: out 2.04e-3 of its norm either way of dealing,
+// lse 2.9e-7 rms; with two sums 2.02e-3, because the largest probability of each half is then an exact 1, and 2.9e-7.)
+// Else each half has a maximum, a sum and an accumulator of its own, merged
+// at the end.
+template <bool DROP, bool ONE_SUM>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k,
@@ -204,6 +216,8 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars->o_done[1], 1);
     mbar_init(&bars->stat_full, kSoftmaxThreads);
     mbar_init(&bars->settled, 1);
+    if (ONE_SUM)
+      for (int i = 0; i < 16; ++i) mbar_init(&bars->max_full[0][0][0] + i, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
     // The first tiles are requested here: they need this thread's barriers, and nothing of what the others set up (192 x
@@ -258,7 +272,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       constexpr uint32_t kStageBytes = kPanels * kPanelBytes;
       bool ok = hot_wait(&bars->q_full, 0, abort_flag);
 
-      // O_h[:, 64 pn .. 64 pn + 63] (+)= P_i[:, 64 h .. 64 h + 63] V_i[64 h .. 64 h + 63, :]
+      // O_h[:, 64 pn .. 64 pn + 63] (+)= P_i[:, 64 h .. 64 h + 63] V_i[64 h .. 64 h + 63, :]; ONE_SUM: one O for both
       auto issue_pv = [&](int i) -> bool {
         const int s = i % kStages;
         if (!hot_wait(&bars->v_full[s], (i / kStages) & 1, abort_flag)) return false;
@@ -271,8 +285,8 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)   // P_i sits in the first 32 columns of each half of score buffer i % 2
-            mma_ts(tmem + kColO + h * kD, tmem + kColS + (i % 2) * 128 + h * 64 + kk * 8,
-                   desc_at(v_desc, (h * 4 + kk) * 2048), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+            mma_ts(tmem + kColO + (ONE_SUM ? 0 : h * kD), tmem + kColS + (i % 2) * 128 + h * 64 + kk * 8,
+                   desc_at(v_desc, (h * 4 + kk) * 2048), idesc_o, (i > 0 || kk > 0 || (ONE_SUM && h > 0)) ? 1u : 0u);
         }
         mma_commit(&bars->v_empty[s]);
         mma_commit(&bars->o_done[i & 1]);
@@ -307,7 +321,9 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     const int row = quad * 32 + lane;     // row within the tile = TMEM lane
     const int r = q0 + row;               // query index
     const uint32_t tlane = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-    const uint32_t tO = tlane + kColO + half * kD;  // this half's output accumulator
+    // what this thread rescales: its half's accumulator, or half the columns of the only one
+    const uint32_t tO = tlane + kColO + half * (ONE_SUM ? kD / 2 : kD);
+    float* maxima = reinterpret_cast<float*>(smem + L::kMax) + row;
     const float scale_log2 = scale * kLog2e;
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
     // waits for P_i V_i (tile i) to have completed
@@ -356,18 +372,24 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
 #pragma unroll
       for (int i = 0; i < 32; ++i)
         mx4[i & 3] = fmax3(mx4[i & 3], __uint_as_float(xa[i]), __uint_as_float(xb[i]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+      float mx = __fmul_rn(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])), scale_log2);
 
-      if (j == 0) {
-        m = mx;  // O is first written by an MMA with accumulate = 0: nothing to rescale
-      } else if (__any_sync(0xffffffffu, mx > m + kRescaleThreshold)) {
-        if (!(ok = wait_pv(j - 1))) break;
+      // ONE_SUM: the other half's maximum of the row. (A buffer is written again two tiles on, behind the wait for the
+      // other half's next maxima, which come after it has read these.)
+      auto agree = [&]() -> bool {
+        if (!hot_wait(&bars->max_full[sb][1 - half][quad], (j >> 1) & 1, abort_flag)) return false;
+        mx = fmaxf(mx, maxima[(sb * 2 + 1 - half) * kBM]);
+        return true;
+      };
+      // the accumulators and the sum get the scale of the larger maximum
+      auto rescale = [&]() -> bool {
+        if (!wait_pv(j - 1)) return false;
         tc_fence_after_sync();
         const float m_new = fmaxf(m, mx);
         // m = -inf: nothing but zeros has been accumulated so far (every earlier column masked)
         const float corr = (m == -INFINITY) ? 0.f : ex2(m - m_new);
 #pragma unroll 1
-        for (int c = 0; c < kD / 32; ++c) {
+        for (int c = 0; c < (ONE_SUM ? kD / 2 : kD) / 32; ++c) {
           uint32_t o[32];
           tmem_ld32(tO + c * 32, o);
           tmem_wait_ld();
@@ -376,19 +398,30 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
           tmem_st32(tO + c * 32, o);
         }
         tmem_wait_st();
-        l *= corr;
+        l = __fmul_rn(l, corr);
         m = m_new;
+        return true;
+      };
+      if (ONE_SUM) {
+        maxima[(sb * 2 + half) * kBM] = mx;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->max_full[sb][half][quad]);
+        if (j == 0 && !(ok = agree())) break;
       }
+      if (j == 0)
+        m = mx;  // O is first written by an MMA with accumulate = 0: nothing to rescale
+      else if (!ONE_SUM && __any_sync(0xffffffffu, mx > m + kRescaleThreshold) && !(ok = rescale()))
+        break;
 
       // ---- p = exp2(s * scale * log2e - m), packed two-float FMAs and sums (192 x 8192: 3.41 -> 3.32 ms,
       // 24 x 8192 419 -> 405 us, 24 x 2048 37.1 -> 36.8; a share of the exponentials on the FMA pipe was no faster). A half-row with no visible key yet has
       // m = -inf: its scores are all -inf and must give p = 0, not exp2(nan). ----
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       const float2 sl = make_float2(scale_log2, scale_log2);
-      const float neg_m = (m == -INFINITY) ? 0.f : -m;
       uint32_t pk[32];  // packed P of this thread
       auto process = [&](uint32_t (&x)[32], int ch) {
         float pv[32];
+        const float neg_m = (m == -INFINITY) ? 0.f : -m;
         const float2 nm = make_float2(neg_m, neg_m);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
@@ -406,6 +439,16 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
         for (int i = 0; i < 16; ++i) pk[ch * 16 + i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
       };
       process(xa, 0);
+      if (ONE_SUM && j > 0) {
+        // The other half's maximum is looked at only now. The exponentials above were computed with the one before, which
+        // stands for nearly every tile; where it does not they are computed again.
+        if (!(ok = agree())) break;
+        if (__any_sync(0xffffffffu, mx > m + kRescaleThreshold)) {
+          if (!(ok = rescale())) break;
+          sum2[0] = sum2[1] = make_float2(0.f, 0.f);
+          process(xa, 0);
+        }
+      }
       process(xb, 1);
       l += (sum2[0].x + sum2[1].x) + (sum2[0].y + sum2[1].y);
       tmem_st32(tS, pk);
@@ -443,14 +486,15 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       for (int c = 0; c < kCols / 32; ++c) {
         uint32_t oa[32], ob[32];
         tmem_ld32(tlane + kColO + half * kCols + c * 32, oa);
-        tmem_ld32(tlane + kColO + kD + half * kCols + c * 32, ob);
+        if (!ONE_SUM) tmem_ld32(tlane + kColO + kD + half * kCols + c * 32, ob);
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float y[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            y[e] = __uint_as_float(oa[8 * i + e]) * f0 + __uint_as_float(ob[8 * i + e]) * f1;
+            y[e] = ONE_SUM ? __uint_as_float(oa[8 * i + e]) * f0
+                           : __uint_as_float(oa[8 * i + e]) * f0 + __uint_as_float(ob[8 * i + e]) * f1;
           *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + i) ^ (lane & 7)) << 4)) =
               make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]),
                          pack_bf16(y[6], y[7]));
@@ -477,7 +521,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
   if (threadIdx.x == 0 && bars->abort_flag) report_timeout(status, bars->abort_flag);
 }
 
-template <bool DROP>
+template <bool DROP, bool ONE_SUM>
 int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k,
                     const uint16_t* v, int BH, int S, float scale, float rate, uint64_t seed,
                     uint64_t offset, int64_t unit0, cudaStream_t st) {
@@ -488,7 +532,7 @@ int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t
   if (int rc = make_tensor_map_bf16(&mo, out, BH, S, kD, 32)) return rc;
   int* status = device_status_word();
   if (!status) return DADATTN_E_CUDA;
-  auto kern = flash_fwd_bf16_kernel<DROP>;
+  auto kern = flash_fwd_bf16_kernel<DROP, ONE_SUM>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 FwdSmem::kBytes));
   const LeveledGrid order = leveled_grid(32768, S, BH);   // (16384 and 65536: 0-4 % slower or the same)
@@ -527,9 +571,11 @@ extern "C" int dadattn_flash_fwd_bf16(uint16_t* out, float* lse, const uint16_t*
     return launch_fwd_bf16_d64(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, nullptr, 0, st);
   // (a draw costs more than the rest of the arithmetic: with dropout the larger number of smaller items is the better
   // one, 192 x 512 119 us against 142)
-  if (!drop && fwd128_pairs_pay(BH, S)) return launch_fwd_bf16_d128_pairs(out, lse, q, k, v, BH, S, scale, st);
-  return drop ? launch_fwd_bf16<true>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st)
-              : launch_fwd_bf16<false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
+  if (drop) return launch_fwd_bf16<true, false>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st);
+  // The arithmetic goes by S alone, so that a unit's result does not depend on the units it is computed with.
+  if (S > kFwd128OneSumRows) return launch_fwd_bf16<false, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
+  if (fwd128_pairs_pay(BH, S)) return launch_fwd_bf16_d128_pairs(out, lse, q, k, v, BH, S, scale, st);
+  return launch_fwd_bf16<false, true>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
 }
 
 extern "C" int dadattn_flash_fwd_bf16_masked(uint16_t* out, float* lse, const uint16_t* q,

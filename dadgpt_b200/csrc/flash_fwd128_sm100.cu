@@ -11,7 +11,8 @@
 //     softmax warpgroup, scores and accumulator in tensor memory and issuing thread: while A's threads compute
 //     exponentials the tensor pipe runs B's products and vice versa. Sequences of one tile: that tile of two units;
 //   * one thread per row: no statistics to exchange, one accumulator per tile (a second one for each half of a
-//     row would not fit beside two tiles' scores). Its 128 scores are read once and stay in registers. (Two threads
+//     row would not fit beside two tiles' scores). Its 128 scores are read once and stay in registers. Launches
+//     that do not fill the GPU take the one-tile kernel of flash_bf16_sm100.cu, in a form that gives the same bits. (Two threads
 //     per row, sixteen softmax warps, with the maximum agreed by a barrier of two warps: 192 x 1024 72.4 us instead
 //     of 70, 192 x 128 10.2 instead of 9.0);
 //   * the probabilities go back over the scores as packed bf16, and the P V product of the first 64 keys is issued
@@ -396,7 +397,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (F128Item it = feed.fetch(x); ok && it.n_kv > 0; it = feed.fetch(x)) {
       const int n = it.n, bh = it.unit, q0 = it.q0, r = q0 + row;
       if (n == 0) continue;
-      float m = -INFINITY, l = 0.f;       // running max (log2 units, scaled) and sum of the row
+      float m = -INFINITY, l[2] = {0.f, 0.f};   // running max (log2 units, scaled) of the row, and its sum by halves of the tiles
       for (int j = 0; j < n; ++j, ++g) {
         const bool diagonal = j == n - 1;
         if (!(ok = mbar_wait(&bars->s_full[x], g & 1, abort_flag))) break;
@@ -419,7 +420,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             mx4[i & 3] = fmax3(mx4[i & 3], __uint_as_float(s[c][i]), __uint_as_float(s[c + 1][i]));
-        const float mx = fmaxf(fmax3(mx4[0], mx4[1], mx4[2]), mx4[3]) * scale_log2;
+        const float mx = __fmul_rn(fmaxf(fmax3(mx4[0], mx4[1], mx4[2]), mx4[3]), scale_log2);
         if (j == 0) {
           m = mx;  // O is first written by a product that does not accumulate: nothing to rescale
         } else if (__any_sync(0xffffffffu, mx > m + kRescaleAt)) {
@@ -437,17 +438,23 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tmem_st32(tO + c * 32, o);
           }
           tmem_wait_st();
-          l *= corr;
+          l[0] = __fmul_rn(l[0], corr);
+          l[1] = __fmul_rn(l[1], corr);
           m = m_new;
         }
         // p = exp2(s scale log2e - m). A row whose scores are all -inf so far must give p = 0, not exp2(NaN).
-        float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        float2 sum2[2];
         const float2 sl = make_float2(scale_log2, scale_log2);
         const float neg_m = (m == -INFINITY) ? 0.f : -m;
         const float2 nm = make_float2(neg_m, neg_m);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];   // bf16 pairs (k, k + 1) per column
+          // The keys' halves have sums of their own, as the one-tile kernel's two threads per row do. The second's begin
+          // with a zero made of the first's: where they are independent the compiler interleaves the halves, and the
+          // first probabilities are late (48 x 1024 24.5 -> 26.5 us, 96 x 512 17.7 -> 18.2).
+          if (c == 0) sum2[0] = sum2[1] = make_float2(0.f, 0.f);
+          if (c == 2) sum2[0] = fmul2(sum2[0], make_float2(0.f, 0.f)), sum2[1] = fmul2(sum2[1], make_float2(0.f, 0.f));
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float2 e = ffma2(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sl, nm);
@@ -460,9 +467,9 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tmem_wait_st();
             tc_fence_before_sync();
             mbar_arrive(&bars->p_full[x][c / 2]);
+            l[c / 2] += (sum2[0].x + sum2[1].x) + (sum2[0].y + sum2[1].y);
           }
         }
-        l += (sum2[0].x + sum2[1].x) + (sum2[0].y + sum2[1].y);
       }
       if (!ok) break;
 
@@ -470,7 +477,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       // which nobody reads any more: every Q K^T has completed before the last s_full was observed.
       if (!(ok = mbar_wait(&bars->o_done[x], u & 1, abort_flag))) break;
       tc_fence_after_sync();
-      const float l_tot = l * ex2(m - m);   // (NaN where the max is not finite)
+      const float l_tot = (l[0] + l[1]) * ex2(m - m);   // (NaN where the max is not finite)
       const float f = 1.0f / l_tot;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -539,20 +546,22 @@ int launch(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, cons
 
 }  // namespace
 
-// Whether items of two query tiles are the better ones. A short launch is over sooner with a tile per CTA: half the
-// work in its longest item. So: sequences of up to three tiles, once the tiles do not fit the GPU at once; others,
-// where the CTAs' mean number of K / V steps is 0.8 of the longest item's. us, one tile / two, by that quotient:
-//     24 x 128   5.6 / 7.0 (24 tiles)   80 x 256   10.6 / 9.4 (160)   60 x 384  13.1 / 11.3 (180)   192 x 128  11.0 / 8.9 (192)
-//     32 x 777  17.1 / 20.7  0.6        40 x 777   19.1 / 20.7  0.7   48 x 1024 27.2 / 24.4  0.8    48 x 777   23.3 / 21.6 0.9
-//     24 x 2048 36.1 / 44    0.7        48 x 2048  66.4 / 59.9  1.5   96 x 512  22.0 / 17.5  1.9   192 x 1024  91.8 / 69.4 3.2
-// Not beyond 2048 rows: a long launch runs at the power cap, and there the one-tile kernel does its work for less
-// (192 x 8192 forward and backward in a loop 13010 us, 13476 with this one; alone and short, 48 x 4096 222 / 208 us).
+// Whether items of two query tiles are the better ones, for up to kFwd128OneSumRows rows. A short launch is over sooner
+// with a tile per CTA: half the work in its longest item. So: sequences of up to three tiles, once the tiles do not fit
+// the GPU at once; others, where the CTAs' mean number of K / V steps is 0.8 of the longest item's. us, one tile / two,
+// by that quotient:
+//     24 x 128   5.6 / 6.9 (24 tiles)   80 x 256   11.7 / 10.5 (160)  60 x 384  12.5 / 11.3 (180)  192 x 128  12.1 / 9.6 (192)
+//     32 x 777  15.6 / 18.9  0.6        40 x 777   17.6 / 19.1  0.7   48 x 1024 27.5 / 24.5  0.8   48 x 777   23.2 / 21.8 0.9
+//     24 x 2048 36.6 / 40.1  0.7        48 x 2048  67.3 / 59.4  1.5   96 x 512  21.9 / 17.6  1.9   192 x 1024 92.4 / 68.7 3.2
+// Longer sequences keep a maximum, a sum and an accumulator for each half of a row, whatever their number: the line is in
+// rows because a unit's result may not go by the units beside it. Two tiles are slower there where they leave CTAs idle
+// or the launch runs at the power cap (16 x 3000 53 / 64, 24 x 8192 380 / 418, 192 x 8192 forward and backward in a loop
+// 12650 / 13080) and faster between (48 x 4096 213 / 198, 192 x 4096 826-905 / 812-840).
 bool fwd128_pairs_pay(int BH, int S) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
   const long long n = (static_cast<long long>(S) + kT - 1) / kT, pairs = n / 2;
-  if (n > 16) return false;
   if (n <= 3) return n * BH > sms;
   return 10 * (pairs * (pairs + 1) + (n % 2 ? n : 0)) * BH >= 8 * n * sms;   // (steps of a unit's items)
 }
