@@ -660,16 +660,32 @@ int launch_decode(T* out, const T* q, const T* k_new, const T* v_new, T* k_cache
   const int resident = kManyPerSm * sms;
   int ranks = 1;
   while (ranks < kMaxCluster && ranks * kBytesPerRank < bytes && pairs * ranks * 2 <= resident) ranks *= 2;
-  // Two or four CTAs for each: a cluster of four or eight for two sequences, where the lengths are on the device (the
-  // ranking reads them all: up to kMaxPaired) and the spare CTAs of an odd one fit, too.
+  // Two or four CTAs for each: a cluster of four or eight for two sequences, where the lengths are on the device. It is
+  // for lengths that differ; equal ones are 0-7 % slower with it. Not where clusters are the last to fit: they wait for
+  // each other, and the next call's have no room to set themselves up in. Clusters of eight take up to 84 % of the GPU's
+  // places for CTAs, of four up to 92 %. Nor beyond kMaxPaired sequences, all of whose lengths every CTA ranks. us a call
+  // in a CUDA graph, bf16, head size 128, a cluster for each / for two, by the longest of evenly spread lengths and (")
+  // of one long sequence, the others an eighth of it:
+  //   clusters of eight         1000           2000           6000           2000 "         6000 "
+  //   4 x 20 heads, 320 CTAs                   12.8 / 12.2    27.2 / 25.1    12.4 / 10.5    26.9 / 20.7
+  //   4 x 31, 496            11.9 / 11.9       15.9 / 16.3    36.2 / 34.6    16.1 / 13.2    36.8 / 26.7
+  //   8 x 16, 512            11.4 / 12.4       16.5 / 16.7    37.8 / 36.5    13.8 / 12.1    32.4 / 25.1
+  //   4 x 33, 528            11.2 / 12.6       16.1 / 18.4    35.2 / 37.8    16.4 / 13.7    37.6 / 27.6
+  //   of four: 8 x 34, 544   18.2 / 17.4       28.5 / 27.3    68.4 / 65.8    26.3 / 21.4    66.5 / 52.6
+  //   4 x 70, 560            16.2 / 18.1       27.8 / 30.1    74.4 / 76.8    28.1 / 22.6    71.0 / 55.1
+  //   64 x 4, 512            18.0 / 18.6       28.1 / 27.1    69.2 / 65.6    20.6 / 17.5    50.7 / 40.3
+  //   96 x 2, 384            14.6 / 15.4       128 x 2, 512   17.1 / 19.0    96 x 1, clusters of eight  9.3 / 10.9
   Deal deal = ranks > 1 ? Deal::kCluster : Deal::kPersistent;
   // (without a workspace there is no counter to deal items from: one CTA each)
   long long grid = ranks > 1 || !item_counter ? pairs * ranks : min(pairs, static_cast<long long>(resident));
   const long long paired = static_cast<long long>((B + 1) / 2) * H * ranks * 2;
-  if (lengths && ranks > 1 && ranks < kMaxCluster && B >= 2 && B <= kMaxPaired && paired * 100 <= resident * 95LL)
+  if (lengths && ranks > 1 && ranks < kMaxCluster && B >= 2 && B <= kMaxPaired &&
+      paired * 100 <= resident * (ranks * 2 == kMaxCluster ? 84LL : 92LL))
     deal = Deal::kPairCluster, ranks *= 2, grid = paired;
-  // (clusters of eight with the deeper ring fit 48 times, which leaves the next call's no room to set themselves up in)
-  const long long few = deal == Deal::kPairCluster && ranks == kMaxCluster ? 2 * sms : kFewPerSm * sms;
+  // The deeper ring for clusters of eight as long as some more would fit (48 do on 148 SMs; 4, 8 or 2 sequences, spread
+  // up to 2000 rows, deeper / not: 320 CTAs 12.2 / 12.4, 368 13.4 / 13.9, 384 13.9 / 14.0 and, one long, 9.8 / 9.3, 400
+  // 18.0 / 14.1).
+  const long long few = deal == Deal::kPairCluster && ranks == kMaxCluster ? sms * 5LL / 2 : kFewPerSm * sms;
   const int stages = grid <= few ? kFewStages : kManyStages;
   // Longest first pays once a CTA takes more than one item; the in-kernel ranking handles 32..256 sequences.
   const int reorder = B >= 32 && B <= kMaxRanked && pairs > grid;
