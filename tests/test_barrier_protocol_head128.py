@@ -62,9 +62,6 @@ class Forward(Model):
                 yield ("write", ("out", h), j - 1)
             yield ("write", ("scores", j & 1, h), ("p", j))
             yield ("arrive", self.wait_p(j)[0])
-        yield from self.results(h)
-
-    def results(self, h):
         yield ("write", "q", "stat")
         yield ("write", ("stat", h), True)
         yield ("arrive", "stat_full")
@@ -218,46 +215,11 @@ class TwoKernel(Model):
                 **{f"compute{a}": self.compute(a) for a in PARTS}}
 
 
-class ForwardOneSum(Forward):
-    """The form with one maximum and one accumulator per row: a row's halves tell each other their maxima of every tile,
-    and look at the other's behind some of their own exponentials."""
-    def __init__(self, n, rng, abort=False, max_buffers=2, max_full=2):
-        super().__init__(n, rng, abort)
-        self.max_buffers, self.max_full = max_buffers, max_full
-        self.grows = [j > 0 and rng.random() < 0.3 for j in range(n)]   # (both see the same two maxima)
-
-    def issuer(self):
-        for op in super().issuer():
-            if op[0] == "mma" and any(c[0] == "out" for c, _ in op[2]):   # both halves' products write all of O
-                i = op[2][0][1]
-                first = op[2][0][0][1] == 0
-                before = [(("out", h), i - 1 if first else ("half", i)) for h in PARTS] if i or not first else []
-                op = ("mma", [r for r in op[1] if r[0][0] != "out"] + before, [(("out", h), ("half", i) if first else i) for h in PARTS])
-            yield op
-
-    def softmax(self, h):
-        for j in range(self.n):
-            b, f = j % self.max_buffers, j % self.max_full
-            yield ("wait", f"s_full[{j & 1}]", j >> 1)
-            yield ("read", ("scores", j & 1, h), ("s", j))
-            yield ("write", ("max", b, h), j)
-            yield ("arrive", f"max_full[{f}, {h}]")
-            yield ("wait", f"max_full[{f}, {1 - h}]", j // self.max_full)
-            yield ("read", ("max", b, 1 - h), j)
-            if self.grows[j]:
-                yield ("wait", f"o_done[{(j - 1) & 1}]", (j - 1) >> 1)
-                yield ("read", ("out", h), j - 1)
-                yield ("write", ("out", h), j - 1)
-            yield ("write", ("scores", j & 1, h), ("p", j))
-            yield ("arrive", self.wait_p(j)[0])
-        yield from self.results(h)
-
-
 LENGTHS = (1, 2, 3, 5, 17)
 
 
 @pytest.mark.parametrize("abort", [False, True], ids=["runs", "gives_up"])
-@pytest.mark.parametrize("make", [Forward, ForwardOneSum, Backward, *(lambda n, rng, abort, b=b, kv=kv: TwoKernel(n, rng, b, kv, abort)
+@pytest.mark.parametrize("make", [Forward, Backward, *(lambda n, rng, abort, b=b, kv=kv: TwoKernel(n, rng, b, kv, abort)
                                                        for b in (1, 2) for kv in (False, True))])
 def test_every_schedule(make, abort):
     for n in LENGTHS:
@@ -268,11 +230,6 @@ def test_the_forward_needs_a_probability_barrier_per_score_buffer():
     """With one for both, a warp a tile ahead stood in for another's arrival, and products ran on scores."""
     found = survives(lambda s: Forward(8, random.Random(s), p_full=1), range(300))
     assert found is not None and ("scores" in found[1] or "p_full" in found[1])
-
-
-@pytest.mark.parametrize("missing", [{"max_buffers": 1}, {"max_full": 1}])
-def test_the_agreed_maximum_needs_two_buffers_with_a_barrier_each(missing):
-    assert survives(lambda s: ForwardOneSum(9, random.Random(s), **missing), range(300)) is not None
 
 
 def _without(base, role, gone):
@@ -288,8 +245,7 @@ def _without(base, role, gone):
 
 
 @pytest.mark.parametrize("base,role,gone", [(Forward, "producer", "k_empty"), (Forward, "producer", "v_empty"), (Forward, "softmax", "o_done"),
-                                            (Forward, "softmax", "stat_full"), (ForwardOneSum, "softmax", "o_done"), (ForwardOneSum, "softmax", "max_full"),
-                                            (ForwardOneSum, "producer", "v_empty"), (Backward, "issuer", "x_free"), (Backward, "issuer", "dq_drained"),
+                                            (Forward, "softmax", "stat_full"), (Backward, "issuer", "x_free"), (Backward, "issuer", "dq_drained"),
                                             (Backward, "compute", "acc_done"), (Backward, "scalars", "qdo_empty"), (Backward, "producer", "qdo_empty")])
 def test_the_models_miss_no_wait_that_is_left_out(base, role, gone):
     assert survives(lambda s: _without(base, role, gone)(9, random.Random(s)), range(300)) is not None
