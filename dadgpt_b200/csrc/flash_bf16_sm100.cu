@@ -503,8 +503,9 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0 && q0 + quad * 32 < S) {   // (rows beyond S are not written)
-        bulk_store_3d(&map_out, stage, half * kCols, q0 + quad * 32, bh);
-        bulk_store_read();
+        tma_store_3d(&map_out, stage, half * kCols, q0 + quad * 32, bh);
+        bulk_commit();
+        bulk_wait_read<0>();
       }
       if (half == 0 && r < S) lse[static_cast<size_t>(bh) * S + r] = (m_tot + log2f(l_tot)) * kLn2;
     }
@@ -546,7 +547,6 @@ int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t
 }  // namespace dadattn
 
 using namespace dadattn;
-
 
 extern "C" int dadattn_flash_bf16_supported(int d_head) { return d_head == 64 || d_head == 128; }
 

@@ -98,16 +98,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  "r"(taddr)
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 
 template <bool DROP>
 __global__ void __launch_bounds__(kGThreads, 1)
@@ -446,8 +436,9 @@ flash_bwd_fused128_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0 && k0 + quad * 32 < S) {   // (rows beyond S are not written)
-        bulk_store_3d(cg < 2 ? &map_dv : &map_dk, stage, (cg & 1) * 64, k0 + quad * 32, bh);
-        bulk_store_read();
+        tma_store_3d(cg < 2 ? &map_dv : &map_dk, stage, (cg & 1) * 64, k0 + quad * 32, bh);
+        bulk_commit();
+        bulk_wait_read<0>();
       }
     }
   }

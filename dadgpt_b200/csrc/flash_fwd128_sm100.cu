@@ -79,23 +79,6 @@ struct F128Bars {
 };
 static_assert(sizeof(F128Bars) <= 512, "barrier block");
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
-      : "memory");
-}
-// TMA store of a [32 rows][64 bf16] swizzled block (a warp's half of its results) to (x, row, unit)
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // ---- the grid's queue -------------------------------------------------------------------------------
 // Asks for a block of this grid that has not started yet, in its place; the answer (16 bytes) completes on `bar`.
 // Not asked again once the answer was that there is none.
@@ -501,7 +484,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (q0 + quad * 32 < S)
           for (int p = 0; p < 2; ++p) tma_store_3d(&map_out, stage + p * kPanel, p * 64, q0 + quad * 32, bh);
         bulk_commit();
-        bulk_wait_read0();
+        bulk_wait_read<0>();
         mbar_arrive(&bars->q_empty[x]);
       }
       __syncwarp();

@@ -92,36 +92,6 @@ struct F64Bars {
 };
 static_assert(sizeof(F64Bars) <= 512, "barrier block");
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-// TMA store of 32 rows of 64 bytes (a warp's share of the output) to (x, row, head, batch)
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int x, int y, int z, int w) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-      ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-      "r"(r[15]), "r"(taddr)
-      : "memory");
-}
-
 // ---- work items --------------------------------------------------------------------------------
 // Item e (0 = heaviest): query-tile pair p = n_pairs - 1 - e / BH of (batch, head) e % BH.
 // Which items a CTA takes, in order, is fixed before the launch; every role computes the same
@@ -415,7 +385,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     // gives it back, once the store has read it (lane 0 issued that)
     auto give_back = [&]() {
       if (owed >= 0 && lane == 0) {
-        bulk_wait_read0();
+        bulk_wait_read<0>();
         mbar_arrive(&bars->q_empty[owed]);
       }
       owed = -1;
@@ -602,7 +572,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                                __uint_as_float(oa[e + 1]) * f0 + __uint_as_float(ob[e + 1]) * f1);
         if (F32) {   // rounded to bf16 like every operand, widened again
           if (c == 1) {
-            if (lane == 0) bulk_wait_read0();
+            if (lane == 0) bulk_wait_read<0>();
             __syncwarp();
           }
 #pragma unroll
