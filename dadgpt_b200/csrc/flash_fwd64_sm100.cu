@@ -346,6 +346,11 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             if (ok && s_next) {
               if (!next_ready) {
+                // An issuer does not wait for K and Q of tiles and items that its group has nothing to do with, and yet
+                // cannot take an old phase for the present one: tile g is there only once the other issuer has given
+                // back tile g - kKvStages, behind its own wait for K of the tile after that and for Q of the item two before
+                // `ni` (an item that leaves a group idle has three tiles or more, the one between one or more).
+                static_assert(kKvStages <= 4, "an idle issuer could take an old phase of q_full for the present one");
                 if (nj == begin_of(ni)) ok = warp_wait(&bars->q_full[nqb], ((last ? k + 1 : k) >> 1) & 1, abort_flag);
                 ok = ok && warp_wait(&bars->k_full[(g + 1) % kKvStages], ((g + 1) / kKvStages) & 1, abort_flag);
                 if (ok) tc_fence_after_sync();
