@@ -120,6 +120,8 @@ enum class Deal { kPersistent, kCluster, kPairCluster };
 // the end (bf16, 24 heads x 128, us a layer, before -> now: rows 1000 / 3000 / 5000 / 7000 38.6 -> 35.5, 7900 and three
 // of 1000 40.1 -> 29.0, 4 x 4000 35.5 -> 35.2, 7000 / 3000 / 5000 37.7 -> 36.8; 16 x 12 heads, up to 1900 rows 22.7 ->
 // 21.2). Parts that ran on from one sequence into the other, all exactly even, were slower: 38.2, 28.8, 38.0 and 23.5.
+// A sequence's sums, and with them the last bits of its result, are divided by its partner's length then; in every deal they
+// go by the number of (sequence, head) pairs.
 template <typename T, int D>
 struct DecodeTile {
   static constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
