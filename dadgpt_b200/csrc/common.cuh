@@ -186,11 +186,13 @@ inline size_t dropout_mask_bits_bytes(int BH, int S) {
 
 // Forward at head size 128 without dropout. Up to kFwd128OneSumRows rows: one maximum, sum and accumulator per row, two query
 // tiles per CTA (flash_fwd128_sm100.cu) where that is the better, else one (flash_bf16_sm100.cu), with the same results.
-// Beyond: flash_bf16_sm100.cu with those of each half of a row.
+// Beyond: flash_bf16_sm100.cu with those of each half of a row, which launch_fwd_bf16_d128_two_sums takes at every S.
 constexpr int kFwd128OneSumRows = 2048;
 bool fwd128_pairs_pay(int BH, int S);
 int launch_fwd_bf16_d128_pairs(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v, int BH,
                                int S, float scale, cudaStream_t st);
+int launch_fwd_bf16_d128_two_sums(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v,
+                                  int BH, int S, float scale, cudaStream_t st);
 // Forward at head size 64 (flash_fwd64_sm100.cu). mask_bits != nullptr with rate > 0: keep bits
 // from dadattn_dropout_mask_bits; mask_bits == nullptr with rate > 0: the Philox mask is drawn
 // inside the kernel. heads > 0: tensors are the interleaved [B*S, heads*64] activations.

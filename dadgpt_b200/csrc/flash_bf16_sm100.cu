@@ -544,6 +544,12 @@ int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t
 }
 
 }  // namespace
+
+int launch_fwd_bf16_d128_two_sums(uint16_t* out, float* lse, const uint16_t* q, const uint16_t* k, const uint16_t* v,
+                                  int BH, int S, float scale, cudaStream_t st) {
+  return launch_fwd_bf16<false, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
+}
+
 }  // namespace dadattn
 
 using namespace dadattn;
@@ -573,7 +579,7 @@ extern "C" int dadattn_flash_fwd_bf16(uint16_t* out, float* lse, const uint16_t*
   // one, 192 x 512 119 us against 142)
   if (drop) return launch_fwd_bf16<true, false>(out, lse, q, k, v, BH, S, scale, rate, seed, offset, unit0, st);
   // The arithmetic goes by S alone, so that a unit's result does not depend on the units it is computed with.
-  if (S > kFwd128OneSumRows) return launch_fwd_bf16<false, false>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
+  if (S > kFwd128OneSumRows) return launch_fwd_bf16_d128_two_sums(out, lse, q, k, v, BH, S, scale, st);
   if (fwd128_pairs_pay(BH, S)) return launch_fwd_bf16_d128_pairs(out, lse, q, k, v, BH, S, scale, st);
   return launch_fwd_bf16<false, true>(out, lse, q, k, v, BH, S, scale, 0.f, 0, 0, 0, st);
 }

@@ -190,7 +190,10 @@ extern "C" int dadattn_flash_fwd_f32_via_bf16(float* out, float* lse, const floa
     return launch_fwd_bf16_d64_f32(out, lse, bq, bk, bv, BH, S, scale, st);
   }
   if (int rc = launch_cast(true, in, 3, elems, st)) return rc;
-  if (int rc = dadattn_flash_fwd_bf16(bo, lse, bq, bk, bv, BH, S, D, scale, 0.f, 0, 0, 0, stream)) return rc;
+  if (!aligned(lse, 4)) return fail(DADATTN_E_ARG, "via bf16: lse must be 4-byte aligned");
+  // Sums by halves of a row at every S: the results are fp32 tensors, which callers compare as such, and their bits are
+  // those that this entry point has always given.
+  if (int rc = launch_fwd_bf16_d128_two_sums(bo, lse, bq, bk, bv, BH, S, scale, st)) return rc;
   CastList back = {{bo}, {out}};
   return launch_cast(false, back, 1, elems, st);
 }
