@@ -127,13 +127,17 @@ constexpr int kPanels = kD / 64;  // 128-byte wide panels of a row
 // the scores they were computed from and read by the MMA as its A operand: an MMA with both operands
 // in shared memory reads 8 KB per 64 clocks, all of an SM's shared-memory bandwidth, so every byte of
 // P kept out of shared memory counts.
+template <bool ONE_SUM>
 struct FwdSmem {
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kPanels * kPanelBytes;
   static constexpr int kV = kK + kStages * kPanels * kPanelBytes;
   static constexpr int kBars = kV + kStages * kPanels * kPanelBytes;
-  static constexpr int kMax = kBars + 512;               // ONE_SUM: a tile's maxima, [2][half][row]
-  static constexpr int kBytes = kMax + 2 * 2 * kBM * 4;
+  static constexpr int kMaxFull = kBars + 256;           // ONE_SUM: barriers [2][half][quadrant] of
+  static constexpr int kMax = kMaxFull + 128;            // a tile's maxima [2][half][row]
+  // An SM that is set up for 164 KB has room beside this for blocks of the next kernel (1 KB each); with the maxima's 2 KB
+  // it has none: 128 x 33 behind fp32 tensors 10.8 -> 12.9 us.
+  static constexpr int kBytes = ONE_SUM ? kMax + 2 * 2 * kBM * 4 : kBars + 256;
 };
 
 struct FwdBars {
@@ -143,11 +147,10 @@ struct FwdBars {
   // first, and P_j V_j read scores for probabilities (rows of infinities in one call of five at 8 x 3080 with
   // dropout, whose draws set the warps apart). P_{j+2} needs S_{j+2}, which is issued after p_full of tile j.
   uint64_t s_full[2], p_full[2], o_done[2], stat_full, settled;  // P_j V_j commits to o_done[j & 1]
-  uint64_t max_full[2][2][4];   // ONE_SUM: a warp's 32 maxima of tile j are there, [j & 1][half][quadrant]
   uint32_t tmem_base;
   int abort_flag;
 };
-static_assert(sizeof(FwdBars) <= 512, "barrier block");
+static_assert(sizeof(FwdBars) <= 256, "barrier block");
 
 // ONE_SUM: a row's two halves agree on its maximum, tile by tile, and add into one accumulator, as the rows of
 // flash_fwd128_sm100.cu do, in the same order: launches of up to kFwd128OneSumRows rows take that kernel or this one by
@@ -164,7 +167,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
                       float* __restrict__ lse, int S, float scale, float rate, const __grid_constant__ PhiloxRounds rng,
                       int64_t unit0, LeveledGrid order, int* __restrict__ status) {
-  using L = FwdSmem;
+  using L = FwdSmem<ONE_SUM>;
   // TMEM columns: two S buffers [0,256) so that Q K^T of the next tile runs while this tile's softmax
   // still reads its scores, O_0 [256,384), O_1 [384,512).
   constexpr uint32_t kTmemCols = 512;
@@ -217,7 +220,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars->stat_full, kSoftmaxThreads);
     mbar_init(&bars->settled, 1);
     if (ONE_SUM)
-      for (int i = 0; i < 16; ++i) mbar_init(&bars->max_full[0][0][0] + i, 1);
+      for (int i = 0; i < 16; ++i) mbar_init(reinterpret_cast<uint64_t*>(smem + L::kMaxFull) + i, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
     // The first tiles are requested here: they need this thread's barriers, and nothing of what the others set up (192 x
@@ -324,6 +327,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
     // what this thread rescales: its half's accumulator, or half the columns of the only one
     const uint32_t tO = tlane + kColO + half * (ONE_SUM ? kD / 2 : kD);
     float* maxima = reinterpret_cast<float*>(smem + L::kMax) + row;
+    uint64_t* max_full = reinterpret_cast<uint64_t*>(smem + L::kMaxFull) + quad;   // a warp's 32 maxima are there
     const float scale_log2 = scale * kLog2e;
     const float keep_scale = DROP ? 1.0f / (1.0f - rate) : 1.0f;
     // waits for P_i V_i (tile i) to have completed
@@ -377,7 +381,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       // ONE_SUM: the other half's maximum of the row. (A buffer is written again two tiles on, behind the wait for the
       // other half's next maxima, which come after it has read these.)
       auto agree = [&]() -> bool {
-        if (!hot_wait(&bars->max_full[sb][1 - half][quad], (j >> 1) & 1, abort_flag)) return false;
+        if (!hot_wait(&max_full[(sb * 2 + 1 - half) * 4], (j >> 1) & 1, abort_flag)) return false;
         mx = fmaxf(mx, maxima[(sb * 2 + 1 - half) * kBM]);
         return true;
       };
@@ -405,7 +409,7 @@ flash_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q,
       if (ONE_SUM) {
         maxima[(sb * 2 + half) * kBM] = mx;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->max_full[sb][half][quad]);
+        if (lane == 0) mbar_arrive(&max_full[(sb * 2 + half) * 4]);
         if (j == 0 && !(ok = agree())) break;
       }
       if (j == 0)
@@ -535,9 +539,9 @@ int launch_fwd_bf16(uint16_t* out, float* lse, const uint16_t* q, const uint16_t
   if (!status) return DADATTN_E_CUDA;
   auto kern = flash_fwd_bf16_kernel<DROP, ONE_SUM>;
   DAD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                FwdSmem::kBytes));
+                                FwdSmem<ONE_SUM>::kBytes));
   const LeveledGrid order = leveled_grid(32768, S, BH);   // (16384 and 65536: 0-4 % slower or the same)
-  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kBM - 1) / kBM), dim3(kFwdThreads), FwdSmem::kBytes, st,
+  DAD_CUDA(launch_pdl(kern, leveled_blocks(order, (S + kBM - 1) / kBM), dim3(kFwdThreads), FwdSmem<ONE_SUM>::kBytes, st,
                       mq, mk, mv, mo, lse, S, scale, rate,
                       make_philox_rounds(seed, offset, rate), unit0, order, status));
   return DADATTN_OK;
