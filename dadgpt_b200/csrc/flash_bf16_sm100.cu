@@ -12,7 +12,7 @@
 //               warp_id % 4). Each half keeps its OWN running max / sum and its OWN output
 //               accumulator in TMEM, so the two threads of a row never synchronise inside the
 //               loop; the halves are merged once, in the epilogue (split-K inside the CTA). Up to
-//               2048 rows without dropout they agree on one of each (ONE_SUM).
+//               2048 rows of bf16 tensors without dropout they agree on one of each (ONE_SUM).
 //               Eight softmax warps give every scheduler two warps to hide the FFMA -> MUFU ->
 //               FADD latencies behind each other.
 //               A thread reads its 64 scores with tcgen05.ld, writes P as packed bf16 over them,
